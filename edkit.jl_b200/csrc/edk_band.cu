@@ -393,7 +393,12 @@ edk_status band_lowest_device(int p, int nev, const std::vector<int>& m,
   // each operator's own last step), as the host form does
   std::vector<std::vector<double>> prev(nops), cand(nops);
   std::vector<int> finished(nops, 0), hstop(nops, 0);
-  std::vector<double> ha((size_t)nops * d.vcols), hb((size_t)nops * d.vcols);
+  // the lowest nk eigenvalues of each Lanczos matrix, on the device
+  // (edk_tridiag.cu): nev + 4 candidates and four more for values that merge
+  int nk = nev + 8;
+  DevBuf evd;
+  EDK_RETURN_IF(evd.alloc_async((size_t)nops * nk * sizeof(double), st));
+  std::vector<double> hev((size_t)nops * nk);
   const unsigned rows = (unsigned)((d.nmax + 255) / 256);
   int left = nops;
   for (int k = 0; k < kmax && left > 0; ++k) {
@@ -418,23 +423,42 @@ edk_status band_lowest_device(int p, int nev, const std::vector<int>& m,
     for (int q = 0; q < nops && !look; ++q)
       look = !finished[q] && k + 1 == std::min(hn[q], kBandSteps);
     if (!look) continue;
-    EDK_TRY_CUDA(cudaMemcpyAsync(ha.data(), alpha.p, ha.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
-    EDK_TRY_CUDA(cudaMemcpyAsync(hb.data(), beta.p, hb.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
-    EDK_TRY_CUDA(cudaMemcpyAsync(hstop.data(), stop.p, nops * sizeof(int), cudaMemcpyDeviceToHost, st));
-    EDK_TRY_CUDA(cudaStreamSynchronize(st));
+    // (repeated with twice as many values while one matrix has too few
+    // distinct ones among them)
+    std::vector<std::vector<double>> dist(nops);
+    for (bool again = true; again;) {
+      again = false;
+      EDK_RETURN_IF(tridiag_lowest_device(nops, alpha.as<double>(), beta.as<double>(), d.vcols,
+                                          nullptr, stop.as<int>(), k + 1, nk, evd.as<double>(), st));
+      EDK_TRY_CUDA(cudaMemcpyAsync(hev.data(), evd.p, hev.size() * sizeof(double),
+                                   cudaMemcpyDeviceToHost, st));
+      EDK_TRY_CUDA(cudaMemcpyAsync(hstop.data(), stop.p, nops * sizeof(int),
+                                   cudaMemcpyDeviceToHost, st));
+      EDK_TRY_CUDA(cudaStreamSynchronize(st));
+      for (int q = 0; q < nops; ++q) {
+        if (finished[q]) continue;
+        const int mm = hstop[q] > 0 ? hstop[q] : k + 1;
+        std::vector<double>& dd = dist[q];  // distinct values: closer than 1e-12 relative merge
+        dd.clear();
+        for (int t = 0; t < std::min(nk, mm); ++t) {
+          const double x = hev[(size_t)q * nk + t];
+          if (dd.empty() || x - dd.back() > 1e-12 * std::max(1.0, std::fabs(x))) dd.push_back(x);
+        }
+        again = again || ((int)dd.size() < nev + 4 && nk < mm);
+      }
+      if (again) {
+        nk = std::min(2 * nk, k + 1);
+        EDK_RETURN_IF(evd.alloc_async((size_t)nops * nk * sizeof(double), st));
+        hev.resize((size_t)nops * nk);
+      }
+    }
     bool changed = false;
     for (int q = 0; q < nops; ++q) {
       if (finished[q]) continue;
       const int own = std::min(hn[q], kBandSteps);
-      const int mm = hstop[q] > 0 ? hstop[q] : k + 1;
       const bool last = hstop[q] > 0 || k + 1 >= own;
       if (!last && (k + 1) % 10 != 0) continue;
-      std::vector<double> ev(mm);
-      tridiag_eigvals(mm, ha.data() + (size_t)q * d.vcols, hb.data() + (size_t)q * d.vcols,
-                      ev.data());
-      std::vector<double> dd;  // distinct values: closer than 1e-12 relative merge
-      for (double x : ev)
-        if (dd.empty() || x - dd.back() > 1e-12 * std::max(1.0, std::fabs(x))) dd.push_back(x);
+      const std::vector<double>& dd = dist[q];
       bool conv = last;
       if (!conv && (int)dd.size() >= nev + 4 && (int)prev[q].size() >= nev + 4) {
         conv = true;

@@ -9,8 +9,9 @@
 // its slice of the concatenated buffers.  The step index j, the recurrence
 // coefficients alpha/beta, 1/beta and the per-operator stop flags live on the
 // device, so a step has no host round trip: it is captured once into a CUDA
-// graph and replayed.  The host looks at alpha/beta only every check_every
-// steps (tridiagonal eigenvalues, convergence).  One step per operator q:
+// graph and replayed.  Every check_every steps the device solves the
+// tridiagonal problems and tests convergence (edk_tridiag.cu); the host reads
+// only how many operators are left.  One step per operator q:
 //   wt_q = H_q v_j                       (row-gather matvec)
 //   s = V_q^H wt_q ; alpha_j = Re s_j     (CGS sweep 1, FP64 block partials)
 //   w_q = wt_q - V_q s ; u = V_q^H w_q    (one pass: k_rupdate_dots)
@@ -803,8 +804,11 @@ struct BatchEngine {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t gexec = nullptr;
   bool graph_ok = false;
+  cudaStream_t side = nullptr;     // the first operator's copy stream
+  cudaEvent_t checked = nullptr;   // the last convergence check has run
 
   ~BatchEngine() {
+    if (checked) cudaEventDestroy(checked);
     if (gexec) cudaGraphExecDestroy(gexec);
     if (graph) cudaGraphDestroy(graph);
   }
@@ -864,6 +868,10 @@ struct BatchEngine {
       Ds.push_back(o.D);
     }
     totalD = woff;
+    if (!ops[0]->cstream)
+      EDK_TRY_CUDA(cudaStreamCreateWithFlags(&ops[0]->cstream, cudaStreamNonBlocking));
+    side = ops[0]->cstream;
+    EDK_TRY_CUDA(cudaEventCreateWithFlags(&checked, cudaEventDisableTiming));
     EDK_RETURN_IF(split_rows());
     EDK_RETURN_IF(dops.alloc_async(hops.size() * sizeof(BOp), st));
     EDK_TRY_CUDA(cudaMemcpyAsync(dops.p, hops.data(), hops.size() * sizeof(BOp),
@@ -1177,51 +1185,53 @@ struct BatchEngine {
   }
 };
 
-// Run the batch until every operator is done or max steps.
+// Run the batch until every operator is done or max steps.  Convergence checks
+// (every `check_every` steps) run on the device between two steps and set the
+// stop flags there; the host reads only how many operators are left, on the
+// copy stream while the next step already runs, so a check leaves the GPU no
+// gap (the step that runs past the last check finds every operator stopped).
 edk_status run_batch(BatchEngine& E, int max_steps, int nev, double tol, int check_every,
                      std::vector<OpResult>& res, int* nchecks = nullptr) {
   const int nops = E.nops;
   res.assign(nops, OpResult{});
-  std::vector<double> ha((size_t)nops * E.m), hb((size_t)nops * E.m);
-  std::vector<int> hdone(nops), hsteps(nops);
-  std::vector<std::vector<double>> prev(nops);
   EDK_RETURN_IF(E.capture());
-  int every = check_every > 0 ? check_every : 10;
+  DevBuf ev, seen, left;
+  EDK_RETURN_IF(ev.alloc_async((size_t)nops * nev * sizeof(double), E.st));
+  EDK_RETURN_IF(seen.alloc_async((size_t)nops * sizeof(int), E.st));
+  EDK_RETURN_IF(left.alloc_async(sizeof(int), E.st));
+  EDK_TRY_CUDA(cudaMemsetAsync(seen.p, 0, (size_t)nops * sizeof(int), E.st));
+  const int every = check_every > 0 ? check_every : 10;
+  bool pending = false;
   for (int j = 0; j < max_steps; ++j) {
     EDK_RETURN_IF(E.run_step());
-    bool last = (j + 1 == max_steps);
+    if (pending) {
+      int h = 0;
+      EDK_TRY_CUDA(cudaStreamWaitEvent(E.side, E.checked, 0));
+      EDK_TRY_CUDA(cudaMemcpyAsync(&h, left.p, sizeof(int), cudaMemcpyDeviceToHost, E.side));
+      EDK_TRY_CUDA(cudaStreamSynchronize(E.side));
+      pending = false;
+      if (h == 0) break;
+    }
+    const bool last = (j + 1 == max_steps);
     if (!last && !((j + 1) % every == 0 && tol > 0)) continue;
     if (nchecks) ++*nchecks;
-    EDK_TRY_CUDA(cudaMemcpyAsync(hdone.data(), E.done.p, nops * sizeof(int), cudaMemcpyDeviceToHost, E.st));
-    EDK_TRY_CUDA(cudaMemcpyAsync(hsteps.data(), E.nsteps.p, nops * sizeof(int), cudaMemcpyDeviceToHost, E.st));
-    EDK_TRY_CUDA(cudaMemcpyAsync(ha.data(), E.alpha.p, ha.size() * 8, cudaMemcpyDeviceToHost, E.st));
-    EDK_TRY_CUDA(cudaMemcpyAsync(hb.data(), E.beta.p, hb.size() * 8, cudaMemcpyDeviceToHost, E.st));
-    EDK_TRY_CUDA(cudaStreamSynchronize(E.st));
-    bool all_done = true;
-    bool changed = false;
-    for (int q = 0; q < nops; ++q) {
-      if (hdone[q]) continue;
-      int mq = hsteps[q];
-      if (tol > 0 && mq >= nev) {
-        std::vector<double> w(mq);
-        if (tridiag_eigvals(mq, ha.data() + (size_t)q * E.m, hb.data() + (size_t)q * E.m, w.data()) == 0) {
-          bool conv = !prev[q].empty();
-          for (int k = 0; k < nev && k < mq && conv; ++k)
-            conv = std::fabs(w[k] - prev[q][k]) <= tol * std::max(1.0, std::fabs(w[k]));
-          prev[q].assign(w.begin(), w.begin() + std::min(nev, mq));
-          if (conv) { hdone[q] = 1; changed = true; continue; }
-        }
-      }
-      all_done = false;
+    if (tol > 0) {
+      EDK_RETURN_IF(tridiag_check_device(nops, E.alpha.as<double>(), E.beta.as<double>(), E.m,
+                                         E.nsteps.as<int>(), nev, ev.as<double>(), tol,
+                                         seen.as<int>(), E.done.as<int>(), left.as<int>(), E.st));
+      EDK_TRY_CUDA(cudaEventRecord(E.checked, E.st));
+      pending = true;
     }
-    if (changed)
-      EDK_TRY_CUDA(cudaMemcpyAsync(E.done.p, hdone.data(), nops * sizeof(int), cudaMemcpyHostToDevice, E.st));
-    if (all_done) break;
   }
+  EDK_RETURN_IF(tridiag_lowest_device(nops, E.alpha.as<double>(), E.beta.as<double>(), E.m,
+                                      E.nsteps.as<int>(), nullptr, 0, nev, ev.as<double>(), E.st));
+  std::vector<double> ha((size_t)nops * E.m), hb((size_t)nops * E.m), he((size_t)nops * nev);
+  std::vector<int> hdone(nops), hsteps(nops);
   EDK_TRY_CUDA(cudaMemcpyAsync(hdone.data(), E.done.p, nops * sizeof(int), cudaMemcpyDeviceToHost, E.st));
   EDK_TRY_CUDA(cudaMemcpyAsync(hsteps.data(), E.nsteps.p, nops * sizeof(int), cudaMemcpyDeviceToHost, E.st));
   EDK_TRY_CUDA(cudaMemcpyAsync(ha.data(), E.alpha.p, ha.size() * 8, cudaMemcpyDeviceToHost, E.st));
   EDK_TRY_CUDA(cudaMemcpyAsync(hb.data(), E.beta.p, hb.size() * 8, cudaMemcpyDeviceToHost, E.st));
+  EDK_TRY_CUDA(cudaMemcpyAsync(he.data(), ev.p, he.size() * 8, cudaMemcpyDeviceToHost, E.st));
   EDK_TRY_CUDA(cudaStreamSynchronize(E.st));
   for (int q = 0; q < nops; ++q) {
     OpResult& r = res[q];
@@ -1229,34 +1239,44 @@ edk_status run_batch(BatchEngine& E, int max_steps, int nev, double tol, int che
     r.steps = hsteps[q];
     r.a.assign(ha.begin() + (size_t)q * E.m, ha.begin() + (size_t)q * E.m + r.steps);
     r.b.assign(hb.begin() + (size_t)q * E.m, hb.begin() + (size_t)q * E.m + r.steps);
-    if (r.steps > 0) {
-      std::vector<double> w(r.steps);
-      tridiag_eigvals(r.steps, r.a.data(), r.b.data(), w.data());
-      r.ev.assign(w.begin(), w.begin() + std::min(nev, r.steps));
-    }
+    const double* w = he.data() + (size_t)q * nev;
+    r.ev.assign(w, w + std::min(nev, r.steps));
   }
   return EDK_OK;
 }
 
 // FP64 start vectors for the refinement of each operator into out (wdt
 // layout): the sum of its `nev` lowest Ritz vectors, so the refined Krylov
-// space holds every wanted eigenvector.
-edk_status ritz_vectors(BatchEngine& E, const std::vector<OpResult>& res, void* out, int nev) {
+// space holds every wanted eigenvector.  With `user` the vectors go to the
+// caller and keep the sign of the QL eigensolver's (tridiag_eigen).
+edk_status ritz_vectors(BatchEngine& E, const std::vector<OpResult>& res, void* out, int nev,
+                        bool user) {
   std::vector<double2> c((size_t)E.nops * E.ncap, make_double2(0.0, 0.0));
   std::vector<int> nc(E.nops, 0);
   for (int q = 0; q < E.nops; ++q) {
     int mq = res[q].steps;
     if (mq <= 0) continue;
-    std::vector<double> w(mq), Q((size_t)mq * mq);
-    if (tridiag_eigen(mq, res[q].a.data(), res[q].b.data(), w.data(), Q.data()) != 0) {
-      set_error("tridiagonal eigensolver did not converge");
-      return EDK_NOT_CONVERGED;
+    const int nk = std::min({nev, mq, (int)res[q].ev.size()});
+    std::vector<double> Q((size_t)mq * nk);
+    for (int e = 0; e < nk; ++e)
+      if (!std::isfinite(res[q].ev[e])) {
+        set_error("tridiagonal eigensolver did not converge");
+        return EDK_NOT_CONVERGED;
+      }
+    tridiag_vectors(mq, res[q].a.data(), res[q].b.data(), nk, res[q].ev.data(), Q.data());
+    double sign = 1.0;
+    if (user) {
+      std::vector<double> w(mq), z(mq);
+      if (tridiag_first_row(mq, res[q].a.data(), res[q].b.data(), w.data(), z.data()) != 0) {
+        set_error("tridiagonal eigensolver did not converge");
+        return EDK_NOT_CONVERGED;
+      }
+      sign = z[0] < 0 ? -1.0 : 1.0;
     }
-    const int nk = std::min(nev, mq);
     for (int k = 0; k < mq; ++k) {
       double v = 0.0;
       for (int e = 0; e < nk; ++e) v += Q[k + (size_t)e * mq];
-      c[(size_t)q * E.ncap + k] = make_double2(v, 0.0);
+      c[(size_t)q * E.ncap + k] = make_double2(sign * v, 0.0);
     }
     nc[q] = mq;
   }
@@ -1383,7 +1403,7 @@ edk_status batch_lanczos(const std::vector<edk_operator*>& ops, const edk_lanczo
   // global element offset of each operator in the concatenated layout
   std::vector<int64_t> goff(nops);
   for (int q = 0; q < nops; ++q) goff[q] = E.hops[q].woff;
-  if (!mixed && ritz_out) EDK_RETURN_IF(ritz_vectors(E, res, ritz_out, 1));
+  if (!mixed && ritz_out) EDK_RETURN_IF(ritz_vectors(E, res, ritz_out, 1, true));
   if (mixed) {
     // FP64 refinement restarted from the sum of the nev lowest Ritz vectors,
     // in one round that may run to max_steps (each operator stops when it
@@ -1394,7 +1414,7 @@ edk_status batch_lanczos(const std::vector<edk_operator*>& ops, const edk_lanczo
     std::vector<int> active(nops);
     for (int q = 0; q < nops; ++q) active[q] = q;
     DevBuf cur;  // start vectors of `active`, compact in that order
-    EDK_RETURN_IF(ritz_vectors(E, res, start.p, o.nev));
+    EDK_RETURN_IF(ritz_vectors(E, res, start.p, o.nev, ritz_out != nullptr));
     void* cur_p = start.p;
     for (int round = 0; round < 4 && !active.empty(); ++round) {
       std::vector<edk_operator*> sub;
@@ -1425,7 +1445,7 @@ edk_status batch_lanczos(const std::vector<edk_operator*>& ops, const edk_lanczo
         // lowest Ritz vectors of the operators this round finalises
         DevBuf gs;
         EDK_RETURN_IF(gs.alloc_async((size_t)F.totalD * esz(wdt), st));
-        EDK_RETURN_IF(ritz_vectors(F, r2, gs.p, 1));
+        EDK_RETURN_IF(ritz_vectors(F, r2, gs.p, 1, true));
         size_t k = 0;
         const bool last_round = round == 3;  // restarts end here: every vector is final
         for (size_t i = 0; i < active.size(); ++i) {
@@ -1441,7 +1461,7 @@ edk_status batch_lanczos(const std::vector<edk_operator*>& ops, const edk_lanczo
       // Ritz vectors of this round (F's layout), then the restarted subset
       DevBuf full;
       EDK_RETURN_IF(full.alloc_async((size_t)F.totalD * esz(wdt), st));
-      EDK_RETURN_IF(ritz_vectors(F, r2, full.p, o.nev));
+      EDK_RETURN_IF(ritz_vectors(F, r2, full.p, o.nev, ritz_out != nullptr));
       int64_t tot = 0;
       for (int i : keep) tot += F.Ds[i];
       DevBuf nb;
@@ -1476,9 +1496,10 @@ edk_status batch_lanczos(const std::vector<edk_operator*>& ops, const edk_lanczo
     for (auto& r : res) {
       int mm = r.steps;
       if (mm <= 0) continue;
-      std::vector<double> w(mm), Q((size_t)mm * mm);
-      if (tridiag_eigen(mm, r.a.data(), r.b.data(), w.data(), Q.data()) == 0)
-        resid = std::max(resid, std::fabs(r.b[mm - 1] * Q[(size_t)mm - 1]));
+      std::vector<double> y(mm);
+      if (r.ev.empty() || !std::isfinite(r.ev[0])) continue;
+      tridiag_vectors(mm, r.a.data(), r.b.data(), 1, r.ev.data(), y.data());
+      resid = std::max(resid, std::fabs(r.b[mm - 1] * y[mm - 1]));
     }
     diag->residual = resid;
     diag->seconds_setup = ts1 - ts0;

@@ -398,5 +398,16 @@ edk_status band_lowest_device(int p, int nev, const std::vector<int>& m,
                               const std::vector<std::vector<const double*>>& B,
                               cudaStream_t st, std::vector<std::vector<double>>& out);
 int tridiag_eigen(int m, const double* a, const double* b, double* w, double* Q);
+int tridiag_first_row(int m, const double* a, const double* b, double* w, double* z);
+// implemented in edk_tridiag.cu: the lowest nk eigenvalues of nops tridiagonal
+// matrices on the device (ev: nops x nk), and the convergence check of a
+// batch on them; inverse iteration on the host
+edk_status tridiag_check_device(int nops, const double* alpha, const double* beta, int64_t ld,
+                                const int* nsteps, int nk, double* ev, double tol, int* seen,
+                                int* done, int* left, cudaStream_t st);
+edk_status tridiag_lowest_device(int nops, const double* alpha, const double* beta, int64_t ld,
+                                 const int* nsteps, const int* nfix, int nall, int nk, double* ev,
+                                 cudaStream_t st);
+void tridiag_vectors(int m, const double* a, const double* b, int nk, const double* w, double* Q);
 double elapsed_ms(cudaEvent_t a, cudaEvent_t b);
 }  // namespace edk

@@ -28,14 +28,17 @@ double elapsed_ms(cudaEvent_t a, cudaEvent_t b) {
 // matrix (diagonal a[0..m-1], off-diagonal b[0..m-2]).  Eigenvalues are
 // returned ascending in w; when Q is non-null it receives the orthonormal
 // eigenvectors as columns (column-major m x m, Q[r + c*m]), ordered like w.
+// With first_row, Q holds only the vectors' first components (m values).
 // Returns 0 on success, -1 if an eigenvalue did not converge in 60 sweeps.
-static int tql(int m, const double* a, const double* b, double* w, double* Q) {
+static int tql(int m, const double* a, const double* b, double* w, double* Q,
+               bool first_row = false) {
   if (m <= 0) return 0;
   std::vector<double> d(a, a + m), e(m, 0.0);
   for (int i = 0; i + 1 < m; ++i) e[i] = b[i];
+  const int rows = first_row ? 1 : m;
   if (Q) {
-    std::fill(Q, Q + (size_t)m * m, 0.0);
-    for (int i = 0; i < m; ++i) Q[i + (size_t)i * m] = 1.0;
+    std::fill(Q, Q + (size_t)rows * m, 0.0);
+    for (int i = 0; i < rows; ++i) Q[i + (size_t)i * rows] = 1.0;
   }
   const double eps = std::numeric_limits<double>::epsilon();
   for (int l = 0; l < m; ++l) {
@@ -74,9 +77,9 @@ static int tql(int m, const double* a, const double* b, double* w, double* Q) {
         d[i + 1] = g + p;
         g = c * r - h;
         if (Q) {
-          for (int q = 0; q < m; ++q) {
-            double* col1 = Q + (size_t)(i + 1) * m;
-            double* col0 = Q + (size_t)i * m;
+          for (int q = 0; q < rows; ++q) {
+            double* col1 = Q + (size_t)(i + 1) * rows;
+            double* col0 = Q + (size_t)i * rows;
             double t = col1[q];
             col1[q] = s * col0[q] + c * t;
             col0[q] = c * col0[q] - s * t;
@@ -95,9 +98,9 @@ static int tql(int m, const double* a, const double* b, double* w, double* Q) {
   std::sort(idx.begin(), idx.end(), [&](int x, int y) { return d[x] < d[y]; });
   for (int i = 0; i < m; ++i) w[i] = d[idx[i]];
   if (Q) {
-    std::vector<double> T((size_t)m * m);
+    std::vector<double> T((size_t)rows * m);
     for (int c = 0; c < m; ++c)
-      for (int r = 0; r < m; ++r) T[r + (size_t)c * m] = Q[r + (size_t)idx[c] * m];
+      for (int r = 0; r < rows; ++r) T[r + (size_t)c * rows] = Q[r + (size_t)idx[c] * rows];
     std::copy(T.begin(), T.end(), Q);
   }
   return 0;
@@ -108,6 +111,11 @@ int tridiag_eigvals(int m, const double* a, const double* b, double* w) {
 }
 int tridiag_eigen(int m, const double* a, const double* b, double* w, double* Q) {
   return tql(m, a, b, w, Q);
+}
+// eigenvalues and the eigenvectors' first components z[m] (signs included),
+// as tridiag_eigen's Q has them in its first row, in O(m^2)
+int tridiag_first_row(int m, const double* a, const double* b, double* w, double* z) {
+  return tql(m, a, b, w, z, true);
 }
 
 }  // namespace edk
