@@ -30,22 +30,42 @@
 
 namespace edk {
 
-// y(:, k) (+)= H x(:, k); blockIdx.y = k.
-template <int BK, class S, class VT, bool GATHER>
+// y(:, k) (+)= H x(:, k); blockIdx.y = k.  TPR lanes share a row.
+template <int BK, class S, class VT, bool GATHER, int TPR>
 __global__ void __launch_bounds__(256) k_apply(BasisDev b, OpDev op, const VT* __restrict__ x,
                                                VT* __restrict__ y, int64_t ldx, int64_t ldy,
                                                int accumulate) {
-  __shared__ uint32_t s_binom[32 * 33];
+  __shared__ uint32_t s_binom[(BK == BK_PROJ_RANK) ? 32 * 33 : 1];
   if constexpr (BK == BK_PROJ_RANK) {
     fill_binom32(s_binom);
     __syncthreads();
   }
   const VT* xk = x + (int64_t)blockIdx.y * ldx;
   VT* yk = y + (int64_t)blockIdx.y * ldy;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < b.D;
-       i += (int64_t)gridDim.x * blockDim.x)
-    gen_row<BK, S, VT, GATHER>(b, op, i, xk, yk, accumulate, s_binom);
+  constexpr int RPB = 256 / TPR;
+  for (int64_t i0 = (int64_t)blockIdx.x * RPB; i0 < b.D; i0 += (int64_t)gridDim.x * RPB) {
+    const int64_t i = i0 + threadIdx.x / TPR;
+    if constexpr (TPR == 1) {
+      if (i < b.D) gen_row<BK, S, VT, GATHER>(b, op, i, xk, yk, accumulate, s_binom);
+    } else {
+      gen_row<BK, S, VT, GATHER, TPR>(b, op, i < b.D ? i : b.D - 1, xk, yk, accumulate, s_binom,
+                                      threadIdx.x % TPR, i < b.D);
+    }
+  }
 }
+
+// Lanes per row of the general gather kernel.  A row is a serial chain of
+// lookups, so a small sector with one lane per row leaves most of the GPU
+// idle: lanes share a row while the rows times the lanes still fit two rounds
+// of the resident threads (148 x 2,048).  Symmetry groups, whose lookup is the
+// longest, take sixteen or four lanes, the others eight.
+// (k, p, z) group sector of L = 22, some 8,360 rows, real vector: 621 us with
+// one lane per row and every group element stepped through the generators, 45
+// us with eight lanes and rotations read off a doubled word, 22 us with sixteen
+// lanes and rotations compared at the zero-run tops (runs_arg32).
+template <int BK> constexpr int many_lanes() { return BK == BK_ABELIAN ? 16 : 8; }
+template <int BK> constexpr int few_lanes() { return BK == BK_ABELIAN ? 4 : 1; }
+bool lanes_fit(int64_t rows, int lanes) { return rows * lanes <= (int64_t)2 * 148 * 2048; }
 
 // Resident blocks per SM asked of the compiler: the rank-search kernels are
 // latency bound and fit 32 registers (8 blocks of 256 threads fill every warp
@@ -131,15 +151,21 @@ edk_status launch_apply(const BasisDev& b, const OpDev& op, const void* x, void*
   bool wide = b.L > 32;
   for (int64_t k0 = 0; k0 < nvec; k0 += 65535) {
     int64_t nk = std::min<int64_t>(nvec - k0, 65535);
-    dim3 grid(apply_grid(b.D), (unsigned)nk);
     const VT* Xk = X + k0 * ldx;
     VT* Yk = Y + k0 * ldy;
-#define EDK_APPLY(BK)                                                                       \
-  case BK:                                                                                  \
-    if (wide) k_apply<BK, uint64_t, VT, GATHER><<<grid, 256, 0, st>>>(b, op, Xk, Yk, ldx, ldy, \
-                                                                       accumulate);         \
-    else k_apply<BK, uint32_t, VT, GATHER><<<grid, 256, 0, st>>>(b, op, Xk, Yk, ldx, ldy,   \
-                                                                  accumulate);              \
+    const int64_t rows = b.D * nk;
+#define EDK_APPLY_T(BK, S, T)                                                                  \
+  k_apply<BK, S, VT, GATHER, GATHER ? (T) : 1>                                                 \
+      <<<dim3(apply_grid(b.D * (GATHER ? (T) : 1)), (unsigned)nk), 256, 0, st>>>(              \
+          b, op, Xk, Yk, ldx, ldy, accumulate);
+#define EDK_APPLY_S(BK, S)                                                                     \
+  if (GATHER && lanes_fit(rows, many_lanes<BK>())) { EDK_APPLY_T(BK, S, many_lanes<BK>()) }    \
+  else if (GATHER && lanes_fit(rows, few_lanes<BK>())) { EDK_APPLY_T(BK, S, few_lanes<BK>()) } \
+  else { EDK_APPLY_T(BK, S, 1) }
+#define EDK_APPLY(BK)                       \
+  case BK:                                  \
+    if (wide) { EDK_APPLY_S(BK, uint64_t) } \
+    else { EDK_APPLY_S(BK, uint32_t) }      \
     break;
     switch (b.bk) {
       EDK_APPLY(BK_TENSOR)
@@ -154,6 +180,8 @@ edk_status launch_apply(const BasisDev& b, const OpDev& op, const void* x, void*
         return EDK_INVALID_ARG;
     }
 #undef EDK_APPLY
+#undef EDK_APPLY_S
+#undef EDK_APPLY_T
     EDK_TRY_CUDA(cudaGetLastError());
   }
   return EDK_OK;

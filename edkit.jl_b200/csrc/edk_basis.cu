@@ -312,13 +312,7 @@ __global__ void k_index(BasisDev b, int64_t n, const uint64_t* states, int64_t* 
                         double2* coeff) {
   __shared__ uint32_t s_binom[32 * 33];
   if (BK == BK_PROJ_RANK) {
-    for (int q = threadIdx.x; q < 32 * 33; q += blockDim.x) {
-      int pp = q / 33, kk = q % 33;
-      uint64_t c = 1;
-      if (kk > pp) c = 0;
-      else for (int r = 1; r <= kk; ++r) c = c * (uint64_t)(pp - kk + r) / (uint64_t)r;
-      s_binom[q] = (uint32_t)c;
-    }
+    fill_binom32(s_binom);
     __syncthreads();
   }
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;

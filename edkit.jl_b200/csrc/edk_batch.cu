@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(256, plan_min_blocks<BK, VT>()) k_bapply_plan(
       int4* dst = reinterpret_cast<int4*>(&s_op);
       for (int e = threadIdx.x; e < (int)(sizeof(BOp) / sizeof(int4)); e += blockDim.x) dst[e] = src[e];
       __syncthreads();
-      ff_tab_fill<BK>(sm, s_op.b, s_op.op.plan.binom);
+      ff_tab_fill<BK>(sm, s_op.b);
       __syncthreads();
       cur = q;
     }

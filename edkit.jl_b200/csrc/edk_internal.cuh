@@ -267,7 +267,6 @@ struct RowPlanDev {
   //       bond of a nearest-neighbour family), or ~0u
   const uint4* slot;
   const double* dg;       // diagonal of the row (operators with diagonal-only generic terms), or null
-  const uint32_t* binom;  // binom[p * 33 + k] = C(p, k), p < 32
   int64_t nslots;         // windows * 256
 };
 constexpr uint32_t kPlanRowMask = (1u << 27) - 1u;
@@ -328,7 +327,7 @@ struct edk_operator {
   int tps = 1;            // threads per state of the fast path (1, 2 or 4; autotuned)
   // row plan of the fast path on rank-searched sectors (edk_plan.cu): built on
   // first use; plan_state 0 not built, 1 built, -1 not available
-  edk::DevBuf p_slot, p_dg, p_binom, p_bad;
+  edk::DevBuf p_slot, p_dg, p_bad;
   int plan_state = 0;
   bool use_plan = true;   // tps == 1 on a rank-searched sector runs the plan kernel
   int use_block = -1;     // several right-hand sides through one SpMM: 1 yes, 0 no, -1 auto

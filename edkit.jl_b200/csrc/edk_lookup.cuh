@@ -163,6 +163,23 @@ __device__ __forceinline__ int64_t colex_rank(uint64_t s, const uint32_t* binom)
   return colex_rank((uint32_t)s, binom);  // rank mode is only enabled for L <= 32
 }
 
+// C(p, k) for p < 32, k <= 32, computed by the compiler; kernels that update or
+// compute ranks copy it to shared memory.
+struct BinomTab { uint32_t v[32 * 33]; };
+constexpr BinomTab make_binom_tab() {
+  BinomTab t{};
+  for (int p = 0; p < 32; ++p) {
+    t.v[p * 33] = 1;
+    for (int k = 1; k <= p; ++k)
+      t.v[p * 33 + k] = t.v[(p - 1) * 33 + k - 1] + t.v[(p - 1) * 33 + k];
+  }
+  return t;
+}
+static __device__ const BinomTab d_binom_tab = make_binom_tab();
+__device__ __forceinline__ void fill_binom32(uint32_t* s_binom) {
+  for (int q = threadIdx.x; q < 32 * 33; q += blockDim.x) s_binom[q] = d_binom_tab.v[q];
+}
+
 // One odometer step over the generators — AbelianBasis.jl:292-299 / 405-414.
 template <class S>
 __device__ __forceinline__ S apply_gen(const GenDev& g, S s, int L, S mask) {
@@ -235,9 +252,42 @@ __device__ __forceinline__ uint32_t canon_runs32(uint32_t s, int L, uint32_t mas
   return m >> (32 - L);
 }
 
+// First minimum over the one-site rotations of the doubled word d of s, at the
+// zero-run tops only (as canon_runs32: about L / 4 candidates of a half-filled
+// state), and its shift: M = i for the rotation right by i, or with LEFT the
+// rotation left by M = L - i; ties keep the smallest M, the identity's 0 first.
+template <bool LEFT>
+__device__ __forceinline__ uint32_t runs_arg32(uint32_t s, int L, uint32_t mask, int& M) {
+  const Dbl32 d = dbl32_top(s, L);
+  uint32_t z = ~s & (((s >> 1) | (s << (L - 1))) & mask);
+  if (L <= 27) {  // M rides in the spare low bits
+    const uint32_t hi_mask = ~((1u << (32 - L)) - 1u);
+    uint32_t m = d.lo & hi_mask;
+    while (z) {
+      const int i = __ffs(z);
+      z &= z - 1;
+      m = min(m, (__funnelshift_r(d.lo, d.hi, i) & hi_mask) | (uint32_t)(LEFT ? L - i : i));
+    }
+    M = (int)(m & ~hi_mask);
+    return m >> (32 - L);
+  }
+  uint32_t m = s;
+  M = 0;
+  while (z) {
+    const int i = __ffs(z);
+    z &= z - 1;
+    const uint32_t r = __funnelshift_r(d.lo, d.hi, i) >> (32 - L);
+    const int q = LEFT ? L - i : i;
+    const bool lt = r < m || (r == m && q < M);
+    m = lt ? r : m;
+    M = lt ? q : M;
+  }
+  return m;
+}
 // first minimum and its translation count M
 __device__ __forceinline__ uint32_t canon_arg32(uint32_t s, int L, int A, int len, uint32_t mask,
                                                 int& M) {
+  if (A == 1) return runs_arg32<false>(s, L, mask, M);
   if (L <= 27) {
     // the spare low bits carry q, so min() keeps the smallest q on ties
     const Dbl32 d = dbl32_top(s, L);
@@ -271,6 +321,11 @@ __device__ __forceinline__ uint32_t canon_arg32(uint32_t s, int L, int A, int le
 __device__ __forceinline__ void canon_par32(uint32_t s, int L, int A, int len, uint32_t mask,
                                             uint32_t& Iam, int& Rr, uint32_t& Ibm, int& M) {
   const uint32_t rs = __brev(s) >> (32 - L);
+  if (A == 1) {
+    Iam = runs_arg32<false>(s, L, mask, Rr);
+    Ibm = runs_arg32<true>(rs, L, mask, M);
+    return;
+  }
   if (L <= 27) {
     const Dbl32 d = dbl32_top(s, L), dr = dbl32_top(rs, L);
     const uint32_t hi_mask = ~((1u << (32 - L)) - 1u);
@@ -303,6 +358,55 @@ __device__ __forceinline__ void canon_par32(uint32_t s, int L, int A, int len, u
     M = lb ? q : M;
     i += A;
   }
+}
+
+// First minimum of the orbit over the commuting generators, in the order of
+// shift_canonical_int (AbelianBasis.jl:428-445: the first generator turns
+// fastest, strict <): q0 turns of the first generator and the o-th setting of
+// the others reach it.  Bound by integer issue, one chain per element: when the
+// first generator is the rotation by one site (every basis with a momentum and
+// unit cell 1, up to 32 sites) its turns are compared at the zero-run tops only;
+// the other generators step once per turn of the first.
+template <class S>
+__device__ __forceinline__ S canon_group(const BasisDev& b, S s, S mask, int& q0, unsigned& o_best) {
+  const GenDev& G0 = b.gens[0];
+  const int n0 = G0.order, L = b.L, shift = G0.shift;
+  unsigned nout = 1;
+  for (int g = 1; g < b.ngen; ++g) nout *= (unsigned)b.gens[g].order;
+  const bool rot = sizeof(S) == 4 && G0.kind == GEN_ROTL && G0.inv_mask == 0 && n0 == L;
+  const bool left = rot && shift == 1, right = rot && shift == L - 1;
+  S bst = s, base = s;
+  q0 = 0;
+  o_best = 0;
+  for (unsigned o = 0; o < nout; ++o) {
+    if (o > 0) {  // odometer step of the generators past the first
+      unsigned turn = 1;
+      for (int g = 1; g < b.ngen; ++g) {
+        base = apply_gen(b.gens[g], base, L, mask);
+        turn *= (unsigned)b.gens[g].order;
+        if (o % turn != 0) break;
+      }
+    }
+    S m = base;
+    int q = 0;
+    if (left) {
+      m = (S)runs_arg32<true>((uint32_t)base, L, (uint32_t)mask, q);
+    } else if (right) {
+      m = (S)runs_arg32<false>((uint32_t)base, L, (uint32_t)mask, q);
+    } else {
+      S cur = base;
+      for (int c = 1; c < n0; ++c) {
+        cur = apply_gen(G0, cur, L, mask);
+        if (cur < m) { m = cur; q = c; }
+      }
+    }
+    if (m < bst) {
+      bst = m;
+      q0 = q;
+      o_best = o;
+    }
+  }
+  return bst;
 }
 
 // Result of index(b, state) on the device.
@@ -394,29 +498,22 @@ __device__ __forceinline__ bool lookup(const BasisDev& b, S s, const uint32_t* b
     decode_val(b, v, h.pos, h.rpos);
     h.pre = n;
     return true;
-  } else {  // BK_ABELIAN: shift_canonical_int, AbelianBasis.jl:428-445
-    int cnt[kMaxGen], best[kMaxGen];
-#pragma unroll
-    for (int g = 0; g < kMaxGen; ++g) { cnt[g] = 0; best[g] = 0; }
-    int64_t order = 1;
-    for (int g = 0; g < b.ngen; ++g) order *= b.gens[g].order;
-    S cur = s, bst = s;
-    for (int64_t t = 0; t < order; ++t) {
-      for (int g = 0; g < b.ngen; ++g) {
-        cur = apply_gen(b.gens[g], cur, b.L, mask);
-        if (++cnt[g] >= b.gens[g].order) cnt[g] = 0; else break;
-      }
-      if (cur < bst) {
-        bst = cur;
-        for (int g = 0; g < b.ngen; ++g) best[g] = cnt[g];
-      }
-    }
+  } else {  // BK_ABELIAN
+    int q0;
+    unsigned o;
+    const S bst = canon_group<S>(b, s, mask, q0, o);
     uint32_t v;
     if (!hash_find(b, bst, v)) return false;
     decode_val(b, v, h.pos, h.rpos);
     double pr = 1.0, pi = 0.0;
     for (int g = 0; g < b.ngen; ++g) {
-      double2 c = __ldg(b.phase + b.gens[g].phase_off + best[g]);
+      const GenDev& G = b.gens[g];
+      int c0 = q0;
+      if (g > 0) {
+        c0 = (int)(o % (unsigned)G.order);
+        o /= (unsigned)G.order;
+      }
+      double2 c = __ldg(b.phase + G.phase_off + c0);
       double nr = pr * c.x - pi * c.y, ni = pr * c.y + pi * c.x;
       pr = nr; pi = ni;
     }

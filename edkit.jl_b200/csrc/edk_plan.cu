@@ -26,13 +26,12 @@ namespace {
 template <int BK>
 __global__ void __launch_bounds__(256) k_plan_build(BasisDev b, OpDev op, FFParams ff,
                                                     int want_diag,
-                                                    const uint32_t* __restrict__ binom,
                                                     uint4* __restrict__ slot_o,
                                                     double* __restrict__ dg_o,
                                                     int* __restrict__ bad) {
   __shared__ int s_key[kPlanWindow];
   __shared__ uint32_t s_binom[32 * 33];
-  for (int q = threadIdx.x; q < 32 * 33; q += blockDim.x) s_binom[q] = __ldg(binom + q);
+  fill_binom32(s_binom);
   __syncthreads();
   const int t = threadIdx.x;
   const int64_t r0 = (int64_t)blockIdx.x * kPlanWindow, i = r0 + t;
@@ -88,7 +87,7 @@ __global__ void __launch_bounds__(256, plan_min_blocks<BK, VT>())
                  VT* __restrict__ y, int64_t ldx, int64_t ldy, int accumulate, int64_t slot0,
                  int64_t slot1) {
   __shared__ FFTab<BK> sm;
-  ff_tab_fill<BK>(sm, b, op.plan.binom);
+  ff_tab_fill<BK>(sm, b);
   __syncthreads();
   const VT* xk = x + (int64_t)blockIdx.y * ldx;
   VT* yk = y + (int64_t)blockIdx.y * ldy;
@@ -157,18 +156,9 @@ edk_status build_plan_kind(edk_operator* op, const FFParams& ff, int want_diag) 
   EDK_RETURN_IF(op->p_slot.alloc(ns * sizeof(uint4)));
   if (want_diag) EDK_RETURN_IF(op->p_dg.alloc(ns * 8));
   EDK_RETURN_IF(op->p_bad.alloc(sizeof(int)));
-  std::vector<uint32_t> binom(32 * 33, 0);
-  for (int p = 0; p < 32; ++p) {
-    binom[p * 33] = 1;
-    for (int k = 1; k <= p; ++k)
-      binom[p * 33 + k] = binom[(p - 1) * 33 + k - 1] + binom[(p - 1) * 33 + k];
-  }
-  EDK_RETURN_IF(op->p_binom.alloc(binom.size() * 4));
-  EDK_TRY_CUDA(cudaMemcpyAsync(op->p_binom.p, binom.data(), binom.size() * 4,
-                               cudaMemcpyHostToDevice, st));
   EDK_TRY_CUDA(cudaMemsetAsync(op->p_bad.p, 0, sizeof(int), st));
   k_plan_build<BK><<<(unsigned)nwin, kPlanWindow, 0, st>>>(
-      b, op->dev, ff, want_diag, op->p_binom.as<uint32_t>(), op->p_slot.as<uint4>(),
+      b, op->dev, ff, want_diag, op->p_slot.as<uint4>(),
       want_diag ? op->p_dg.as<double>() : nullptr, op->p_bad.as<int>());
   EDK_TRY_CUDA(cudaGetLastError());
   int bad = 0;
@@ -185,7 +175,6 @@ edk_status build_plan_kind(edk_operator* op, const FFParams& ff, int want_diag) 
 void plan_release(edk_operator* op) {
   op->p_slot.release();
   op->p_dg.release();
-  op->p_binom.release();
   op->dev.plan = RowPlanDev{};
 }
 
@@ -227,7 +216,6 @@ edk_status plan_ensure(edk_operator* op) {
   RowPlanDev& pl = op->dev.plan;
   pl.slot = op->p_slot.as<uint4>();
   pl.dg = want_diag ? op->p_dg.as<double>() : nullptr;
-  pl.binom = op->p_binom.as<uint32_t>();
   pl.nslots = ((b.D + kPlanWindow - 1) / kPlanWindow) * kPlanWindow;
   op->plan_state = 1;
   return EDK_OK;

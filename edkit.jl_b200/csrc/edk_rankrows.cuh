@@ -44,7 +44,7 @@ __host__ __device__ inline bool plan_nn(const FFParams& ff) {
 
 // One slot of the plan.  BK is BK_TRANS0_RANK, BK_TRANS_RANK,
 // BK_TRANSPAR_RANK (rank table) or BK_PROJ_RANK (row = rank); `t` holds the
-// block's tables (ff_tab_fill with the plan's binomials).
+// block's tables (ff_tab_fill).
 template <int BK, class VT, int NN = 0>
 __device__ __forceinline__ void plan_row(const BasisDev& b, const OpDev& op, const FFParams& ff,
                                          const FFTab<BK>& t, int64_t slot,

@@ -34,24 +34,21 @@ __device__ __forceinline__ void atv(float2* p, Cx<float> v) {
   atomicAdd(&p->x, v.r); atomicAdd(&p->y, v.i);
 }
 
-__device__ __forceinline__ void fill_binom32(uint32_t* s_binom) {
-  for (int q = threadIdx.x; q < 32 * 33; q += blockDim.x) {
-    int pp = q / 33, kk = q % 33;
-    uint64_t c = 1;
-    if (kk > pp) c = 0;
-    else for (int r = 1; r <= kk; ++r) c = c * (uint64_t)(pp - kk + r) / (uint64_t)r;
-    s_binom[q] = (uint32_t)c;
-  }
-}
-
 // Visit every nonzero of column `s` of H: f_diag(dr, di) once with the summed
 // diagonal, f_hit(hit, vr, vi) for each off-diagonal element found in the basis.
-template <int BK, class S, class FHit>
+// TPR lanes can share the row: lane `sub` then takes the bonds whose position
+// is sub modulo TPR, every TPR-th generic term and its part of the diagonal.
+template <int BK, class S, int TPR = 1, class FHit>
 __device__ __forceinline__ void expand_row(const BasisDev& b, const OpDev& op, S s,
                                            const uint32_t* s_binom, double& dr, double& di,
-                                           FHit&& f_hit) {
+                                           FHit&& f_hit, int sub = 0) {
   const S mask = (S)b.maskL;
   const int L = b.L;
+  S own = ~(S)0;  // bond positions of this lane
+  if constexpr (TPR > 1) {
+    own = 0;
+    for (int p = sub; p < StateBits<S>::bits; p += TPR) own |= (S)1 << p;
+  }
   for (int f = 0; f < op.nfam; ++f) {
     const FamDev* F = op.fam + f;
     const int d = F->d;
@@ -62,33 +59,37 @@ __device__ __forceinline__ void expand_row(const BasisDev& b, const OpDev& op, S
     m[1] = (S)(~X & Y & valid);
     m[2] = (S)(X & ~Y & valid);
     m[3] = (S)(X & Y & valid);
+    S bits = 0;  // bonds with an off-diagonal entry
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-      const double2 dv = F->dval[c];
-      const int cnt = popc_s(m[c]);
-      dr += dv.x * cnt;
-      di += dv.y * cnt;
+      if (TPR == 1 || f % TPR == sub) {
+        const double2 dv = F->dval[c];
+        const int cnt = popc_s(m[c]);
+        dr += dv.x * cnt;
+        di += dv.y * cnt;
+      }
+      if (F->nnz[c] != 0) bits |= m[c];
+    }
+    bits &= own;
+    while (bits) {  // one loop over all local columns: lanes stay together
+      const int p = ffs_s(bits);
+      bits &= bits - 1;
+      const int c = (int)((X >> p) & 1) * 2 + (int)((Y >> p) & 1);
+      int pj = p - d;
+      if (pj < 0) pj += L;
       const int nz = F->nnz[c];
-      if (nz == 0) continue;
-      S bits = m[c];
-      while (bits) {
-        const int p = ffs_s(bits);
-        bits &= bits - 1;
-        int pj = p - d;
-        if (pj < 0) pj += L;
-        for (int q = 0; q < nz; ++q) {
-          const int xr = F->xr[c][q];
-          const S flip = (S)((S)((xr >> 1) & 1) << p) | (S)((S)(xr & 1) << pj);
-          Hit h;
-          if (lookup<BK, S>(b, (S)(s ^ flip), s_binom, h)) {
-            const double2 v = F->val[c][q];
-            f_hit(h, v.x, v.y);
-          }
+      for (int q = 0; q < nz; ++q) {
+        const int xr = F->xr[c][q];
+        const S flip = (S)((S)((xr >> 1) & 1) << p) | (S)((S)(xr & 1) << pj);
+        Hit h;
+        if (lookup<BK, S>(b, (S)(s ^ flip), s_binom, h)) {
+          const double2 v = F->val[c][q];
+          f_hit(h, v.x, v.y);
         }
       }
     }
   }
-  for (int t = 0; t < op.nterm; ++t) {
+  for (int t = sub; t < op.nterm; t += TPR) {
     const TermDev* T = op.term + t;
     const int ns = T->nsites;
     int c = 0;
@@ -108,19 +109,23 @@ __device__ __forceinline__ void expand_row(const BasisDev& b, const OpDev& op, S
 }
 
 // One output row of the general kernels: gather form y[i] (+)= sum conj(H[pos,i]) x[pos],
-// or scatter form y[pos] += H[pos,i] x[i] (atomics).
-template <int BK, class S, class VT, bool GATHER>
+// or scatter form y[pos] += H[pos,i] x[i] (atomics).  TPR lanes (of one warp,
+// lane `sub`) can share a row of the gather form; `valid` is false on lanes
+// past the last row (they take part in the reduction only).
+template <int BK, class S, class VT, bool GATHER, int TPR = 1>
 __device__ __forceinline__ void gen_row(const BasisDev& b, const OpDev& op, int64_t i,
                                         const VT* __restrict__ xk, VT* __restrict__ yk,
-                                        int accumulate, const uint32_t* s_binom) {
+                                        int accumulate, const uint32_t* s_binom, int sub = 0,
+                                        bool valid = true) {
   using A = typename VTraits<VT>::A;
   constexpr bool CX = VTraits<VT>::cx;
+  static_assert(GATHER || TPR == 1, "the scatter form has one lane per row");
   const S s = (BK == BK_TENSOR) ? (S)i : (S)__ldg(b.I + i);
   const A invRi = b.R ? (A)(1.0 / __ldg(b.R + i)) : (A)1;
   double dr = 0.0, di = 0.0;
   if constexpr (GATHER) {
     A ar = 0, ai = 0;
-    expand_row<BK, S>(b, op, s, s_binom, dr, di, [&](const Hit& h, double vr, double vi) {
+    if (valid) expand_row<BK, S, TPR>(b, op, s, s_binom, dr, di, [&](const Hit& h, double vr, double vi) {
       const A pr = (A)h.pre, pi = (A)h.pim, v_r = (A)vr, v_i = (A)vi;
       const A ratio = (A)h.rpos * invRi;
       const A cr = (v_r * pr - v_i * pi) * ratio;
@@ -132,7 +137,17 @@ __device__ __forceinline__ void gen_row(const BasisDev& b, const OpDev& op, int6
       } else {
         ar += cr * xv.r;
       }
-    });
+    }, sub);
+    if constexpr (TPR > 1) {
+#pragma unroll
+      for (int o = 1; o < TPR; o <<= 1) {
+        ar += __shfl_xor_sync(0xffffffffu, ar, o);
+        if constexpr (CX) ai += __shfl_xor_sync(0xffffffffu, ai, o);
+        dr += __shfl_xor_sync(0xffffffffu, dr, o);
+        di += __shfl_xor_sync(0xffffffffu, di, o);
+      }
+      if (sub != 0 || !valid) return;
+    }
     const Cx<A> xi = ldv(xk + i);
     ar += (A)dr * xi.r + (A)di * xi.i;
     if constexpr (CX) ai += (A)dr * xi.i - (A)di * xi.r;
@@ -329,15 +344,12 @@ template <int BK> struct FFTab {
   double2 coef[FFTabSize<BK>::n];
 };
 
-// binom_src: the 32 x 33 table in global memory, or null to compute it
+// (the binomials only where rows follow from ranks: no other kind reads them)
 template <int BK>
-__device__ __forceinline__ void ff_tab_fill(FFTab<BK>& t, const BasisDev& b,
-                                            const uint32_t* binom_src) {
-  if (binom_src) {
-    for (int q = threadIdx.x; q < 32 * 33; q += blockDim.x) t.binom[q] = __ldg(binom_src + q);
-  } else {
+__device__ __forceinline__ void ff_tab_fill(FFTab<BK>& t, const BasisDev& b) {
+  if constexpr (BK == BK_PROJ_RANK || BK == BK_TRANS0_RANK || BK == BK_TRANS_RANK ||
+                BK == BK_TRANSPAR_RANK)
     fill_binom32(t.binom);
-  }
   for (int q = threadIdx.x; q < FFTabSize<BK>::n; q += blockDim.x) {
     const int c = q & 31;
     const double R = (b.packed && c < b.nclass) ? b.Rcls[c] : 1.0;
@@ -608,7 +620,7 @@ __device__ __forceinline__ void ff_tile(const BasisDev& b, const OpDev& op, cons
   __shared__ int s_hist[64];
   __shared__ unsigned short s_order[256];
   __shared__ uint32_t s_state[256];
-  ff_tab_fill<BK>(s_tab, b, RANKED ? b.binom32 : nullptr);
+  ff_tab_fill<BK>(s_tab, b);
   constexpr int RT = 256 / TPS;  // rows per tile
   const int t = threadIdx.x;
   if (t < 64) s_hist[t] = 0;

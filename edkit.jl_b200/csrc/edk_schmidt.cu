@@ -183,14 +183,7 @@ template <bool MATRIX, bool CV>
 __global__ void k_double_map(BasisDev b1, BasisDev b2, double o1, double o2,
                              const void* __restrict__ v, double2* out, uint64_t nfull) {
   __shared__ uint32_t s_binom[32 * 33];
-  for (int q = threadIdx.x; q < 32 * 33; q += blockDim.x) {
-    const int pp = q / 33, kk = q % 33;
-    uint64_t c = 1;
-    if (kk > pp) c = 0;
-    else
-      for (int r = 1; r <= kk; ++r) c = c * (uint64_t)(pp - kk + r) / (uint64_t)r;
-    s_binom[q] = (uint32_t)c;
-  }
+  fill_binom32(s_binom);
   __syncthreads();
   for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < nfull;
        j += (uint64_t)gridDim.x * blockDim.x) {
