@@ -343,6 +343,7 @@ edk_status apply_device(edk_operator* op, int dtype, const void* x, void* y, int
     }
 #undef EDK_FF_TPS
   }
+  if (op->pauli_ok) return apply_pauli(op, dtype, x, y, nvec, ldx, ldy, accumulate, st);
   switch (dtype) {
     case EDK_F64:
       return sc ? launch_apply<double, false>(b, op->dev, x, y, nvec, ldx, ldy, 1, st)
@@ -473,6 +474,68 @@ bool invariant(const std::vector<HostTerm>& terms, const std::vector<int>& perm,
     return true;
   };
   return cmp(a, b) && cmp(b, a);
+}
+
+// Pauli strings of the terms' off-diagonal parts, grouped by flip mask, and of
+// the diagonals of the terms outside the bond families.  False when there are
+// more than kPauliMax: a string costs a row about six instructions and a flip
+// mask one gather, a general term about a hundred (transverse-field Ising,
+// L = 20: 97 per term), so the strings win while they stay few per term.
+constexpr size_t kPauliMax = 512;
+bool pauli_strings(const std::vector<HostTerm>& terms, const std::vector<char>& in_family, int L,
+                   PauliFlips& flips, std::vector<PauliGroup>& group,
+                   std::vector<PauliStr>& str, std::vector<PauliStr>& diag) {
+  std::map<std::pair<uint32_t, uint32_t>, std::pair<double, double>> sum;
+  for (size_t t = 0; t < terms.size(); ++t) {
+    const HostTerm& h = terms[t];
+    const int ns = (int)h.sites.size();
+    if (ns > 4) return false;
+    auto mask = [&](int c) {
+      uint32_t m = 0;
+      for (int k = 0; k < ns; ++k)
+        if ((c >> (ns - 1 - k)) & 1) m |= 1u << (L - h.sites[k]);
+      return m;
+    };
+    for (int x = 0; x < h.dim; ++x) {
+      if (x == 0 && in_family[t]) continue;
+      for (int z = 0; z < h.dim; ++z) {
+        double vr = 0.0, vi = 0.0;
+        for (int c = 0; c < h.dim; ++c) {
+          const double sg = (__builtin_popcount(c & z) & 1) ? -1.0 : 1.0;
+          vr += sg * h.re[(c ^ x) * h.dim + c];
+          vi += sg * h.im[(c ^ x) * h.dim + c];
+        }
+        if (vr == 0.0 && vi == 0.0) continue;
+        auto& v = sum[{mask(x), mask(z)}];
+        v.first += vr / h.dim;
+        v.second += vi / h.dim;
+      }
+    }
+    if (sum.size() > kPauliMax) return false;
+  }
+  std::map<uint32_t, int> per_mask;
+  for (auto it = sum.begin(); it != sum.end();)
+    if (it->second.first == 0.0 && it->second.second == 0.0) it = sum.erase(it);
+    else ++per_mask[(it++)->first.first];
+  flips.n = 0;
+  for (auto& kv : sum) {
+    const uint32_t x = kv.first.first, z = kv.first.second;
+    PauliStr p{};
+    p.v = make_double2(kv.second.first, kv.second.second);
+    p.z = z;
+    if (x == 0) {
+      diag.push_back(p);
+    } else if (z == 0 && per_mask[x] == 1 && p.v.y == 0.0 && flips.n < kPauliFlips) {
+      flips.x[flips.n] = x;
+      flips.v[flips.n++] = p.v.x;
+    } else {
+      if (group.empty() || group.back().x != x)
+        group.push_back(PauliGroup{x, (int)str.size(), (int)str.size(), 0});
+      str.push_back(p);
+      group.back().s1 = (int)str.size();
+    }
+  }
+  return true;
 }
 
 }  // namespace
@@ -687,6 +750,10 @@ extern "C" edk_status edk_operator_create(edk_basis* b, int32_t nterms, const in
       std::memcpy(op->ff_params.data(), &ff, sizeof(FFParams));
     }
   }
+  std::vector<PauliGroup> pgroup;
+  std::vector<PauliStr> pstr, pdiag;
+  op->pauli_ok = op->use_ff && op->gather && !op->ff_ok && b->dev.bk == BK_TENSOR && L <= 31 &&
+                 pauli_strings(terms, in_family, L, op->pauli_flips, pgroup, pstr, pdiag);
   auto upload = [&](DevBuf& buf, const void* src, size_t bytes) -> edk_status {
     if (bytes == 0) return EDK_OK;
     EDK_RETURN_IF(buf.alloc(bytes));
@@ -699,6 +766,13 @@ extern "C" edk_status edk_operator_create(edk_basis* b, int32_t nterms, const in
   EDK_RETURN_IF(upload(op->xmask, xm.data(), xm.size() * sizeof(uint64_t)));
   EDK_RETURN_IF(upload(op->val, vals.data(), vals.size() * sizeof(double2)));
   EDK_RETURN_IF(upload(op->dval, dvals.data(), dvals.size() * sizeof(double2)));
+  if (op->pauli_ok) {
+    EDK_RETURN_IF(upload(op->pa_group, pgroup.data(), pgroup.size() * sizeof(PauliGroup)));
+    EDK_RETURN_IF(upload(op->pa_str, pstr.data(), pstr.size() * sizeof(PauliStr)));
+    EDK_RETURN_IF(upload(op->pa_diag, pdiag.data(), pdiag.size() * sizeof(PauliStr)));
+    op->pauli = PauliDev{(int)pgroup.size(), (int)pdiag.size(), op->pa_group.as<PauliGroup>(),
+                         op->pa_str.as<PauliStr>(), op->pa_diag.as<PauliStr>()};
+  }
   op->dev.nfam = op->nfam;
   op->dev.fam = op->fam.as<FamDev>();
   op->dev.nterm = op->ngeneric;

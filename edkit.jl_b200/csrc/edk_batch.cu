@@ -791,6 +791,7 @@ struct BatchEngine {
   bool plan = false;  // every operator carries a row plan (rank-searched sectors)
   bool plan_nn_all = false;  // ... and is one nearest-neighbour family of equal values
   bool sell = false;
+  const edk_operator* pauli = nullptr;  // a batch of one on the Pauli-string kernel
   int64_t nsblk = 0;
   cudaStream_t st = nullptr;
   std::vector<BOp> hops;
@@ -868,6 +869,7 @@ struct BatchEngine {
       Ds.push_back(o.D);
     }
     totalD = woff;
+    if (nops == 1 && !sell && ops[0]->pauli_ok) pauli = ops[0];
     if (!ops[0]->cstream)
       EDK_TRY_CUDA(cudaStreamCreateWithFlags(&ops[0]->cstream, cudaStreamNonBlocking));
     side = ops[0]->cstream;
@@ -973,6 +975,7 @@ struct BatchEngine {
                                                              stp, dn);
         return EDK_OK;
       }
+      if (pauli) return apply_pauli(pauli, vdt, Vv, wv, 1, totalD, totalD, 0, st, stp, dn);
       if (plan) {
         switch (bk) {
           case BK_PROJ_RANK:

@@ -271,6 +271,22 @@ struct RowPlanDev {
 };
 constexpr uint32_t kPlanRowMask = (1u << 27) - 1u;
 
+// Pauli-string form of an operator on the full space (edk_pauli.cu).
+struct PauliStr { double2 v; uint32_t z, pad; };  // v (-1)^{|s & z|}
+struct PauliGroup { uint32_t x; int s0, s1, pad; };  // strings s0 .. s1-1 flip the bits x
+constexpr int kPauliFlips = 64;
+struct PauliFlips {  // strings without z part, one per flip mask, by ascending mask
+  int n;
+  uint32_t x[kPauliFlips];
+  double v[kPauliFlips];
+};
+struct PauliDev {
+  int ngroup, ndiag;
+  const PauliGroup* group;  // by flip mask, ascending
+  const PauliStr* str;
+  const PauliStr* diag;     // diagonal strings of the terms outside the bond families
+};
+
 struct OpDev {
   SellDev sell;
   RowPlanDev plan;          // row plan of the rank-searched fast path (plan.slot null: none)
@@ -329,6 +345,11 @@ struct edk_operator {
   // first use; plan_state 0 not built, 1 built, -1 not available
   edk::DevBuf p_slot, p_dg, p_bad;
   int plan_state = 0;
+  // Pauli-string form (full space, no flip-flop fast path, few enough strings)
+  edk::DevBuf pa_group, pa_str, pa_diag;
+  edk::PauliDev pauli{};
+  edk::PauliFlips pauli_flips{};
+  bool pauli_ok = false;
   bool use_plan = true;   // tps == 1 on a rank-searched sector runs the plan kernel
   int use_block = -1;     // several right-hand sides through one SpMM: 1 yes, 0 no, -1 auto
                           // (yes unless materialised or on a row plan, whose one-column
@@ -365,6 +386,10 @@ edk_status plan_ensure(edk_operator* op);
 edk_status apply_plan(edk_operator* op, int dtype, const void* x, void* y, int64_t nvec,
                       int64_t ldx, int64_t ldy, int accumulate, cudaStream_t st, int64_t row0,
                       int64_t row1);
+// implemented in edk_pauli.cu
+edk_status apply_pauli(const edk_operator* op, int dtype, const void* x, void* y, int64_t nvec,
+                       int64_t ldx, int64_t ldy, int accumulate, cudaStream_t st,
+                       const int* step = nullptr, const int* done = nullptr);
 // implemented in edk_sell.cu
 edk_status apply_sell_rows(edk_operator* op, int dtype, const void* x, void* y, int64_t row0,
                            int64_t row1, int accumulate, cudaStream_t st);
