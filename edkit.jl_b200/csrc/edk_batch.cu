@@ -690,6 +690,7 @@ __global__ void __launch_bounds__(256) k_bfinish(const BOp* __restrict__ ops, in
         if (!isfinite(nrm)) { done[q] = 4; invb[q] = 0.0; }
         else if (!(nrm > 0.0)) { done[q] = 3; invb[q] = 0.0; }
         else invb[q] = 1.0 / nrm;
+        alpha[(int64_t)q * m] = nrm;  // for the Krylov driver; step 0 overwrites it
       } else {
         const double a = coef1[(int64_t)q * ncap + j].x;
         alpha[(int64_t)q * m + j] = a;
@@ -792,6 +793,10 @@ struct BatchEngine {
   bool plan_nn_all = false;  // ... and is one nearest-neighbour family of equal values
   bool sell = false;
   const edk_operator* pauli = nullptr;  // a batch of one on the Pauli-string kernel
+  // a batch of one whose product has no batched kernel (symmetry groups, more
+  // than 32 sites): launched step by step through apply_device
+  edk_operator* direct = nullptr;
+  int hj = 0;  // the next step of a direct batch
   int64_t nsblk = 0;
   cudaStream_t st = nullptr;
   std::vector<BOp> hops;
@@ -906,8 +911,6 @@ struct BatchEngine {
     EDK_RETURN_IF(step.alloc_async(sizeof(int), st));
     EDK_RETURN_IF(cbuf.alloc_async((size_t)nops * ncap * sizeof(double2), st));
     EDK_RETURN_IF(cnc.alloc_async((size_t)nops * sizeof(int), st));
-    EDK_TRY_CUDA(cudaMemsetAsync(done.p, 0, nops * sizeof(int), st));
-    EDK_TRY_CUDA(cudaMemsetAsync(nsteps.p, 0, nops * sizeof(int), st));
     EDK_TRY_CUDA(cudaMemsetAsync(alpha.p, 0, (size_t)nops * m * sizeof(double), st));
     EDK_TRY_CUDA(cudaMemsetAsync(beta.p, 0, (size_t)nops * m * sizeof(double), st));
     return EDK_OK;
@@ -962,6 +965,9 @@ struct BatchEngine {
   const BOp* d_ops() const { return dops.as<BOp>(); }
 
   edk_status launch_apply() {
+    if (direct)
+      return apply_device(direct, vdt, (const char*)V.p + (size_t)hj * totalD * esz(vdt), wt.p, 1,
+                          totalD, totalD, 0, st);
     const int* t2o = tile2op.as<int>();
     const int* stp = step.as<int>();
     const int* dn = done.as<int>();
@@ -1142,6 +1148,9 @@ struct BatchEngine {
   // V[:, 0] = start / ||start||; start is FP64 (wdt) concatenated on the device
   edk_status setup(const void* start_dev) {
     int minus1 = -1;
+    hj = 0;
+    EDK_TRY_CUDA(cudaMemsetAsync(done.p, 0, nops * sizeof(int), st));
+    EDK_TRY_CUDA(cudaMemsetAsync(nsteps.p, 0, nops * sizeof(int), st));
     EDK_TRY_CUDA(cudaMemcpyAsync(step.p, &minus1, sizeof(int), cudaMemcpyHostToDevice, st));
     launch_split();
     edk_status s = with_vt(vdt, [&](auto vp) -> edk_status {
@@ -1164,7 +1173,7 @@ struct BatchEngine {
   }
 
   edk_status capture() {
-    if (graph_ok) return EDK_OK;
+    if (graph_ok || direct) return EDK_OK;
     cudaError_t e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return EDK_OK;  // replay not available: launch directly
     edk_status s = enqueue_step();
@@ -1184,7 +1193,9 @@ struct BatchEngine {
       EDK_TRY_CUDA(cudaGraphLaunch(gexec, st));
       return EDK_OK;
     }
-    return enqueue_step();
+    EDK_RETURN_IF(enqueue_step());
+    ++hj;
+    return EDK_OK;
   }
 };
 
@@ -1514,6 +1525,53 @@ edk_status batch_lanczos(const std::vector<edk_operator*>& ops, const edk_lanczo
   return EDK_OK;
 }
 
+// ---------------------------------------------------------------------------
+// The Krylov driver's Lanczos basis: a batch of one, advanced in blocks of
+// steps without a host round trip per step.
+// ---------------------------------------------------------------------------
+struct KrylovBasis::Impl {
+  BatchEngine E;
+};
+KrylovBasis::KrylovBasis() = default;
+KrylovBasis::~KrylovBasis() = default;
+
+edk_status KrylovBasis::init(edk_operator* op, int vdt, int m_max, cudaStream_t st) {
+  impl = std::make_unique<Impl>();
+  BatchEngine& E = impl->E;
+  const BasisDev& b = op->b->dev;
+  int bk = b.bk;
+  const bool ff = op->ff_ok && op->use_ff;
+  if (ff && b.search == 2) {
+    if (bk == BK_TRANS0) bk = BK_TRANS0_RANK;
+    else if (bk == BK_TRANS && b.rank_shift == 10) bk = BK_TRANS_RANK;
+    else if (bk == BK_TRANSPAR) bk = BK_TRANSPAR_RANK;
+  }
+  if (!op->sell_ok && !op->pauli_ok && (bk == BK_ABELIAN || b.L > 32)) E.direct = op;
+  return E.init(std::vector<edk_operator*>(1, op), vdt, m_max, bk, ff && !E.direct, st);
+}
+
+const void* KrylovBasis::vectors() const { return impl->E.V.p; }
+
+edk_status KrylovBasis::start(const void* src, double* nrm, int* status) {
+  BatchEngine& E = impl->E;
+  EDK_RETURN_IF(E.setup(src));
+  EDK_RETURN_IF(E.capture());
+  EDK_TRY_CUDA(cudaMemcpyAsync(nrm, E.alpha.p, sizeof(double), cudaMemcpyDeviceToHost, E.st));
+  EDK_TRY_CUDA(cudaMemcpyAsync(status, E.done.p, sizeof(int), cudaMemcpyDeviceToHost, E.st));
+  EDK_TRY_CUDA(cudaStreamSynchronize(E.st));
+  return EDK_OK;
+}
+
+edk_status KrylovBasis::extend(int from, int to, double* alpha, double* beta, int* m) {
+  BatchEngine& E = impl->E;
+  for (int j = from; j < to; ++j) EDK_RETURN_IF(E.run_step());
+  EDK_TRY_CUDA(cudaMemcpyAsync(alpha, E.alpha.p, (size_t)to * sizeof(double), cudaMemcpyDeviceToHost, E.st));
+  EDK_TRY_CUDA(cudaMemcpyAsync(beta, E.beta.p, (size_t)to * sizeof(double), cudaMemcpyDeviceToHost, E.st));
+  EDK_TRY_CUDA(cudaMemcpyAsync(m, E.nsteps.p, sizeof(int), cudaMemcpyDeviceToHost, E.st));
+  EDK_TRY_CUDA(cudaStreamSynchronize(E.st));
+  return EDK_OK;
+}
+
 }  // namespace edk
 
 using namespace edk;
@@ -1535,7 +1593,7 @@ extern "C" edk_status edk_batch_lanczos_e0(int32_t nops, edk_operator* const* op
   cudaStream_t st = v[0]->stream;
   size_t es = v0_dtype == EDK_F64 ? 8 : 16;
   DevBuf v0d;
-  EDK_RETURN_IF(v0d.alloc((size_t)tot * es));
+  EDK_RETURN_IF(v0d.alloc_async((size_t)tot * es, st));
   EDK_TRY_CUDA(cudaMemcpyAsync(v0d.p, v0s, (size_t)tot * es, cudaMemcpyHostToDevice, st));
   std::vector<OpResult> res;
   EDK_RETURN_IF(batch_lanczos(v, *opts, v0d.p, v0_dtype, st, res, diag));

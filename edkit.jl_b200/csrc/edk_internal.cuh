@@ -12,6 +12,7 @@
 #include <stdint.h>
 
 #include <cstdio>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -85,14 +86,17 @@ struct DevBuf {
   template <class T> T* as() const { return reinterpret_cast<T*>(p); }
 };
 
-// keep freed pool memory cached in the process (set once per device)
+// keep freed pool memory cached in the process, up to half of the device's
+// memory; what the pool holds beyond that goes back at the next synchronisation
+// (set once per device)
 inline void keep_pool_memory() {
   static bool done[64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || done[dev]) return;
   cudaMemPool_t pool;
   if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) {
-    uint64_t thr = ~0ull;
+    size_t fr = 0, total = 0;
+    uint64_t thr = cudaMemGetInfo(&fr, &total) == cudaSuccess ? total / 2 : 0;
     cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr);
   }
   done[dev] = true;
@@ -411,6 +415,24 @@ edk_status batch_lanczos(const std::vector<edk_operator*>& ops, const edk_lanczo
                          const void* v0_dev, int v0_dt, cudaStream_t st,
                          std::vector<OpResult>& res, edk_lanczos_diag* diag,
                          void* ritz_out = nullptr);
+// One operator's Lanczos basis on the batched engine, for the Krylov driver.
+// start(): V[:, 0] = src / |src| (src: D values of the FP64 working dtype on
+// the device), *status 3 for a zero and 4 for a non-finite norm; extend(): steps
+// from .. to-1, then alpha / beta [0, to) and the steps taken (fewer than `to`
+// after a breakdown); vectors(): V, D x (m_max + 1) column-major in dtype vdt.
+class KrylovBasis {
+ public:
+  KrylovBasis();
+  ~KrylovBasis();
+  edk_status init(edk_operator* op, int vdt, int m_max, cudaStream_t st);
+  edk_status start(const void* src, double* nrm, int* status);
+  edk_status extend(int from, int to, double* alpha, double* beta, int* m);
+  const void* vectors() const;
+
+ private:
+  struct Impl;
+  std::unique_ptr<Impl> impl;
+};
 // implemented in edk_util.cpp
 int tridiag_eigvals(int m, const double* a, const double* b, double* w);
 // The lowest `nev` distinct eigenvalues of block-tridiagonal Hermitian

@@ -476,11 +476,11 @@ edk_status lanczos_run(Engine& E, int max_steps, int nev, double tol, int check_
 // copy / convert a caller vector to a device buffer of dtype dst_dt
 edk_status stage_vector(const void* src, int src_dt, int ptr_kind, int64_t D, int dst_dt,
                         DevBuf& out, cudaStream_t st) {
-  EDK_RETURN_IF(out.alloc((size_t)D * esize(dst_dt)));
+  EDK_RETURN_IF(out.alloc_async((size_t)D * esize(dst_dt), st));
   DevBuf tmp;
   const void* dsrc = src;
   if (ptr_kind == EDK_HOST) {
-    EDK_RETURN_IF(tmp.alloc((size_t)D * esize(src_dt)));
+    EDK_RETURN_IF(tmp.alloc_async((size_t)D * esize(src_dt), st));
     EDK_TRY_CUDA(cudaMemcpyAsync(tmp.p, src, (size_t)D * esize(src_dt), cudaMemcpyHostToDevice, st));
     dsrc = tmp.p;
   }
@@ -570,8 +570,8 @@ extern "C" edk_status edk_lanczos_ground_state(edk_operator* op, const edk_lancz
   const int64_t D = op->b->D;
   EDK_CHECK_ARG(D >= 1, "edk_lanczos_ground_state: empty basis");
   DevBuf gs, ss;
-  EDK_RETURN_IF(gs.alloc((size_t)D * esize(wdt)));
-  EDK_RETURN_IF(ss.alloc(sizeof(double)));
+  EDK_RETURN_IF(gs.alloc_async((size_t)D * esize(wdt), op->stream));
+  EDK_RETURN_IF(ss.alloc_async(sizeof(double), op->stream));
   EDK_RETURN_IF(lanczos_common(op, opts, v0, v0_dtype, ptr_kind, evals, nullptr, nullptr, diag,
                                gs.p));
   std::lock_guard<std::mutex> lk(op->mu);
@@ -612,7 +612,7 @@ static edk_status lanczos_common(edk_operator* op, const edk_lanczos_opts* opts,
     size_t es = (v0_dtype == EDK_F64 || v0_dtype == EDK_C64) ? 8 : (v0_dtype == EDK_C128 ? 16 : 4);
     const void* src = v0;
     if (ptr_kind == EDK_HOST) {
-      EDK_RETURN_IF(v0d.alloc((size_t)D * es));
+      EDK_RETURN_IF(v0d.alloc_async((size_t)D * es, st));
       EDK_TRY_CUDA(cudaMemcpyAsync(v0d.p, v0, (size_t)D * es, cudaMemcpyHostToDevice, st));
       src = v0d.p;
     }
@@ -711,42 +711,77 @@ static edk_status lanczos_common(edk_operator* op, const edk_lanczos_opts* opts,
 // ---------------------------------------------------------------------------
 namespace edk {
 
+namespace {
+
+constexpr int kTimes = 8;  // states per pass over the Krylov vectors
+struct TimeCols { double2* out[kTimes]; };
+
+// out_t[r] = sum_c V[r, c] coef[c * kTimes + t], t < nt: the states at several
+// times from one read of V.  One read per state (8 of 320 MB at 400,000 rows
+// and 50 vectors: 390 us) is bound by HBM; eight states a read balance it with
+// the FP64 units (35 us of multiply-adds to 49 us of reading).  The sum over c is
+// one chain of FMAs per state, whatever states share the pass.
+template <class VV>
+__global__ void __launch_bounds__(256) k_states(const VV* __restrict__ V, int64_t D, int ncols,
+                                                const double2* __restrict__ coef, int nt,
+                                                TimeCols cols) {
+  constexpr int CH = 64;  // columns of coefficients in shared memory at a time
+  __shared__ double2 sc[CH * kTimes];
+  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool on = r < D;
+  double ar[kTimes], ai[kTimes];
+#pragma unroll
+  for (int t = 0; t < kTimes; ++t) ar[t] = ai[t] = 0.0;
+  for (int c0 = 0; c0 < ncols; c0 += CH) {
+    const int cn = min(CH, ncols - c0);
+    __syncthreads();
+    for (int e = threadIdx.x; e < cn * kTimes; e += blockDim.x) sc[e] = coef[c0 * kTimes + e];
+    __syncthreads();
+    if (!on) continue;
+    const VV* v0 = V + (int64_t)c0 * D + r;
+#pragma unroll 4
+    for (int c = 0; c < cn; ++c) {
+      const double2 v = ld2(v0 + (int64_t)c * D);
+#pragma unroll
+      for (int t = 0; t < kTimes; ++t) {
+        if (t >= nt) break;
+        const double2 k = sc[c * kTimes + t];
+        ar[t] = __fma_rn(-v.y, k.y, __fma_rn(v.x, k.x, ar[t]));
+        ai[t] = __fma_rn(v.y, k.x, __fma_rn(v.x, k.y, ai[t]));
+      }
+    }
+  }
+  if (!on) return;
+#pragma unroll
+  for (int t = 0; t < kTimes; ++t)
+    if (t < nt) cols.out[t][r] = make_double2(ar[t], ai[t]);
+}
+
+}  // namespace
+
 struct KrylovCacheDev {
-  Engine E;
+  KrylovBasis B;
   edk_krylov_opts o;
+  int64_t D = 0;
+  int vdt = EDK_C128;
+  cudaStream_t st = nullptr;
   int m = 0, m_max = 0, m_init = 0;
   double t_anchor = 0.0, t_latest = 0.0, norm_anchor = 0.0;
   std::vector<double> alpha, beta, lam, Q, Qe1, Qem;
   edk_krylov_diag* dg = nullptr;
   DevBuf anchor;  // FP64 complex anchor state
+  DevBuf coef;    // m_max x kTimes combination coefficients
+  DevBuf part;    // |state|^2 partial sums and their total (normalize_output)
+  // states asked for and not yet combined: destination and coefficients
+  std::vector<double2*> due;
+  std::vector<std::vector<std::complex<double>>> due_c;
 
   edk_status build(int m_target) {  // _lanczos_build! :250-306
     m_target = std::min(m_target, m_max);
-    const double seps = std::sqrt(std::numeric_limits<double>::epsilon());
-    for (int j = m; j < m_target; ++j) {
-      EDK_RETURN_IF(apply_device(E.op, E.vdt, E.col(j), E.wt.p, 1, E.D, E.D, 0, E.st));
-      ++E.matvecs;
-      dg->matvecs += 1;
-      EDK_RETURN_IF(E.dots(j + 1, E.wt.p, E.vdt));
-      double2 s_j;
-      EDK_TRY_CUDA(cudaMemcpyAsync(&s_j, E.coef.as<double2>() + j, sizeof(double2),
-                                   cudaMemcpyDeviceToHost, E.st));
-      EDK_RETURN_IF(E.update(j + 1, E.wt.p, E.vdt, E.w.p, false));
-      EDK_RETURN_IF(E.dots(j + 1, E.w.p, E.wdt));
-      EDK_RETURN_IF(E.update(j + 1, E.w.p, E.wdt, E.w.p, true));
-      double n2;
-      EDK_RETURN_IF(E.read_scal(&n2, 1));
-      double aj = s_j.x, bj = std::sqrt(n2);
-      alpha[j] = aj;
-      beta[j] = bj;
-      if (bj <= seps * std::max(1.0, std::fabs(aj))) {
-        m = j + 1;
-        beta[j] = 0.0;
-        return EDK_OK;
-      }
-      m = j + 1;
-      if (j + 1 < E.mcap) EDK_RETURN_IF(E.store_col(j + 1, E.w.p, E.wdt, 1.0 / bj));
-    }
+    if (m_target <= m) return EDK_OK;
+    const int old = m;
+    EDK_RETURN_IF(B.extend(m, m_target, alpha.data(), beta.data(), &m));
+    dg->matvecs += m - old;
     return EDK_OK;
   }
   edk_status reduced() {  // _build_reduced! :311-323
@@ -781,24 +816,64 @@ struct KrylovCacheDev {
     for (int k = 0; k < m; ++k) acc += Qem[k] * std::polar(1.0, -tau * lam[k]) * Qe1[k];
     return std::fabs(bm) * std::abs(acc);
   }
-  edk_status reconstruct(double tau, void* out) {  // :352-362 (out: C128 device)
-    auto c = coeffs(tau);
-    EDK_RETURN_IF(E.combine(m, c, norm_anchor, out, EDK_C128));
-    if (o.normalize_output) {
-      EDK_RETURN_IF(E.update(0, out, EDK_C128, E.w.p, true));
-      double n2;
-      EDK_RETURN_IF(E.read_scal(&n2, 1));
-      double n = std::sqrt(n2);
-      if (n > 0) {
-        edk_status s = with_type(EDK_C128, [&](auto) {
-          k_scale<double2, double2><<<vec_grid(E.D), 256, 0, E.st>>>(
-              (const double2*)out, E.D, 1.0 / n, (double2*)out);
-          return EDK_OK;
-        });
-        EDK_RETURN_IF(s);
+  // combine the states that are due, kTimes in one pass over V
+  edk_status flush() {
+    const auto dst = std::move(due);  // none stays due, also after a failure
+    const auto dst_c = std::move(due_c);
+    due.clear();
+    due_c.clear();
+    for (size_t q0 = 0; q0 < dst.size(); q0 += kTimes) {
+      const int nt = (int)std::min<size_t>(kTimes, dst.size() - q0);
+      size_t nc = 0;
+      TimeCols cols{};
+      for (int t = 0; t < nt; ++t) {
+        nc = std::max(nc, dst_c[q0 + t].size());
+        cols.out[t] = dst[q0 + t];
       }
+      std::vector<double2> h(nc * kTimes, make_double2(0.0, 0.0));
+      for (int t = 0; t < nt; ++t)
+        for (size_t c = 0; c < dst_c[q0 + t].size(); ++c)
+          h[c * kTimes + t] = make_double2(dst_c[q0 + t][c].real(), dst_c[q0 + t][c].imag());
+      EDK_TRY_CUDA(cudaMemcpyAsync(coef.p, h.data(), h.size() * sizeof(double2),
+                                   cudaMemcpyHostToDevice, st));
+      const unsigned grid = (unsigned)((D + 255) / 256);
+      if (vdt == EDK_C64)
+        k_states<float2><<<grid, 256, 0, st>>>((const float2*)B.vectors(), D, (int)nc,
+                                               coef.as<double2>(), nt, cols);
+      else
+        k_states<double2><<<grid, 256, 0, st>>>((const double2*)B.vectors(), D, (int)nc,
+                                                coef.as<double2>(), nt, cols);
+      EDK_TRY_CUDA(cudaGetLastError());
+      if (o.normalize_output)
+        for (int t = 0; t < nt; ++t) EDK_RETURN_IF(normalize(cols.out[t]));
     }
     return EDK_OK;
+  }
+  edk_status normalize(double2* out) {
+    const int g = vec_grid(D);
+    if (!part.p) EDK_RETURN_IF(part.alloc_async((size_t)(g + 1) * sizeof(double), st));
+    double* tot = part.as<double>() + g;
+    k_update<double2, double2, double2><<<g, 256, 0, st>>>(
+        (const double2*)nullptr, D, 0, (const double2*)nullptr, out, out, D, part.as<double>());
+    k_sum<<<1, 256, 0, st>>>(part.as<double>(), g, tot);
+    EDK_TRY_CUDA(cudaGetLastError());
+    double n2 = 0.0;
+    EDK_TRY_CUDA(cudaMemcpyAsync(&n2, tot, sizeof(double), cudaMemcpyDeviceToHost, st));
+    EDK_TRY_CUDA(cudaStreamSynchronize(st));
+    const double n = std::sqrt(n2);
+    if (n > 0) {
+      k_scale<double2, double2><<<g, 256, 0, st>>>(out, D, 1.0 / n, out);
+      EDK_TRY_CUDA(cudaGetLastError());
+    }
+    return EDK_OK;
+  }
+  // the state at anchor time + tau into out (C128 device), at the next flush()
+  // (:352-362)
+  void reconstruct(double tau, void* out) {
+    auto c = coeffs(tau);
+    for (auto& v : c) v *= norm_anchor;
+    due.push_back((double2*)out);
+    due_c.push_back(std::move(c));
   }
   int nsample_eff(double tau_try) const {  // :383-394
     int base_n = o.nsample;
@@ -813,9 +888,29 @@ struct KrylovCacheDev {
     if (!(tau_try > 0)) return 0.0;
     if (std::fabs(beta[m - 1]) <= o.tol) return tau_try;
     int n = nsample_eff(tau_try);
+    // the monitor on the equally spaced samples: the phases of sample k are those
+    // of k - 1 turned by one step, taken afresh every 32 samples
+    std::vector<std::complex<double>> z(m), turn(m);
+    std::vector<double> g(m);
+    const double dx = n > 1 ? tau_try / (double)(n - 1) : 0.0, bm = std::fabs(beta[m - 1]);
+    for (int e = 0; e < m; ++e) {
+      turn[e] = std::polar(1.0, -dx * lam[e]);
+      g[e] = Qem[e] * Qe1[e];
+    }
     for (int k = 0; k < n; ++k) {
       double xk = (n == 1) ? 0.0 : tau_try * (double)k / (double)(n - 1);
-      double eta = monitor(xk);
+      double sr = 0.0, si = 0.0;
+      for (int e = 0; e < m; ++e) {
+        if (k % 32 == 0) {
+          z[e] = std::polar(1.0, -xk * lam[e]);
+        } else {
+          const double zr = z[e].real(), zi = z[e].imag(), tr = turn[e].real(), ti = turn[e].imag();
+          z[e] = {zr * tr - zi * ti, zr * ti + zi * tr};
+        }
+        sr += g[e] * z[e].real();
+        si += g[e] * z[e].imag();
+      }
+      const double eta = bm * std::hypot(sr, si);
       if (!std::isfinite(eta) || eta > o.tol) {
         if (k == 0) return 0.0;
         double lo = tau_try * (double)(k - 1) / (double)(n - 1), hi = xk;
@@ -842,12 +937,12 @@ struct KrylovCacheDev {
     return EDK_OK;
   }
   edk_status restart(double tau_valid) {  // :449-477
-    EDK_RETURN_IF(reconstruct(tau_valid, anchor.p));
+    reconstruct(tau_valid, anchor.p);
+    EDK_RETURN_IF(flush());  // the states due, and the anchor, need the old basis
     t_anchor += tau_valid;
-    EDK_RETURN_IF(E.update(0, anchor.p, EDK_C128, E.w.p, true));
-    double n2;
-    EDK_RETURN_IF(E.read_scal(&n2, 1));
-    double nrm = std::sqrt(n2);
+    double nrm = 0.0;
+    int status = 0;
+    EDK_RETURN_IF(B.start(anchor.p, &nrm, &status));
     if (!(nrm > 0)) {
       set_error("Restart failed: anchor state has zero norm");
       return EDK_ZERO_NORM;
@@ -856,7 +951,6 @@ struct KrylovCacheDev {
     std::fill(alpha.begin(), alpha.end(), 0.0);
     std::fill(beta.begin(), beta.end(), 0.0);
     m = 0;
-    EDK_RETURN_IF(E.store_col(0, anchor.p, EDK_C128, 1.0 / nrm));
     EDK_RETURN_IF(build(m_init));
     EDK_RETURN_IF(reduced());
     dg->basis_builds += 1;
@@ -933,12 +1027,17 @@ static edk_status krylov_start(KrylovCacheDev& K, edk_operator* op, const edk_kr
   K.m_max = (int)std::min<int64_t>(opts->m_max, D);
   K.m_init = std::min(opts->m_init, K.m_max);
   int vdt = opts->precision == EDK_PREC_MIXED ? EDK_C64 : EDK_C128;
-  EDK_RETURN_IF(K.E.init(op, vdt, K.m_max + 1, st));
+  K.D = D;
+  K.vdt = vdt;
+  K.st = st;
+  EDK_RETURN_IF(K.B.init(op, vdt, K.m_max, st));
+  EDK_RETURN_IF(K.coef.alloc_async((size_t)K.m_max * kTimes * sizeof(double2), st));
   K.alpha.assign(K.m_max, 0.0);
   K.beta.assign(K.m_max, 0.0);
   EDK_RETURN_IF(stage_vector(psi0, EDK_C128, ptr_kind, D, EDK_C128, K.anchor, st));
   double nrm = 0.0;
-  EDK_RETURN_IF(K.E.set_start(K.anchor.p, EDK_C128, &nrm));
+  int status = 0;
+  EDK_RETURN_IF(K.B.start(K.anchor.p, &nrm, &status));
   if (!std::isfinite(nrm)) {
     set_error("Initial state has non-finite entries (NaN or Inf)");
     return EDK_INVALID_ARG;
@@ -955,25 +1054,55 @@ static edk_status krylov_start(KrylovCacheDev& K, edk_operator* op, const edk_kr
   return EDK_OK;
 }
 
+// device columns that host results pass through: up to kTimes, at most 1 GiB
+// (one at least); kept when there are enough
+static edk_status stage_columns(DevBuf& psi, int64_t D, int64_t nts, cudaStream_t st) {
+  const size_t col = (size_t)D * 16;
+  const size_t n = std::max<size_t>(1, std::min<size_t>({(size_t)kTimes, (size_t)std::max<int64_t>(nts, 1),
+                                                         ((size_t)1 << 30) / col}));
+  if (psi.bytes >= n * col) return EDK_OK;
+  return psi.alloc_async(n * col, st);
+}
+
 // timeevolve!(cache, t) for each t of a non-decreasing sequence (:586-636):
 // column p of out (device) or of the host array receives the state at ts[p]
 static edk_status krylov_serve(KrylovCacheDev& K, edk_operator* op, const double* ts, int64_t nts,
                                const int64_t* perm, void* out, int32_t ptr_kind, DevBuf& psi) {
   const int64_t D = op->b->D;
   cudaStream_t st = op->stream;
-  for (int64_t q = 0; q < nts; ++q) {
+  // host results pass through the columns of psi, a few at a time
+  const int64_t ncol = ptr_kind == EDK_HOST ? (int64_t)(psi.bytes / ((size_t)D * 16)) : 0;
+  int64_t at = 0;  // columns of psi in use
+  std::vector<int64_t> where;
+  auto drain = [&]() -> edk_status {
+    EDK_RETURN_IF(K.flush());
+    for (int64_t c = 0; c < at; ++c)
+      EDK_TRY_CUDA(cudaMemcpyAsync((double2*)out + (size_t)where[c] * D, psi.as<double2>() + (size_t)c * D,
+                                   (size_t)D * 16, cudaMemcpyDeviceToHost, st));
+    at = 0;
+    where.clear();
+    return EDK_OK;
+  };
+  edk_status rc = EDK_OK;
+  for (int64_t q = 0; q < nts && rc == EDK_OK; ++q) {
     const int64_t p = perm ? perm[q] : q;
     const double tf = ts[p];
     const double tau = tf - K.t_anchor;
-    EDK_RETURN_IF(K.ensure(tau));
-    void* dst = (ptr_kind == EDK_DEVICE) ? (void*)((double2*)out + (size_t)p * D) : psi.p;
-    EDK_RETURN_IF(K.reconstruct(tf - K.t_anchor, dst));
-    if (ptr_kind == EDK_HOST)
-      EDK_TRY_CUDA(cudaMemcpyAsync((double2*)out + (size_t)p * D, psi.p, (size_t)D * 16,
-                                   cudaMemcpyDeviceToHost, st));
+    rc = K.ensure(tau);
+    if (rc != EDK_OK) break;
+    double2* dst = (double2*)out + (size_t)p * D;
+    if (ptr_kind == EDK_HOST) {
+      dst = psi.as<double2>() + (size_t)at++ * D;
+      where.push_back(p);
+    }
+    K.reconstruct(tf - K.t_anchor, dst);
     K.t_latest = tf;
     K.dg->total_times_served += 1;
+    if (ptr_kind == EDK_HOST && at == ncol) rc = drain();
   }
+  const edk_status rc2 = drain();  // also what was served before a failure
+  EDK_RETURN_IF(rc);
+  EDK_RETURN_IF(rc2);
   EDK_TRY_CUDA(cudaStreamSynchronize(st));
   return EDK_OK;
 }
@@ -1014,7 +1143,7 @@ extern "C" edk_status edk_krylov_evolve(edk_operator* op, const edk_krylov_opts*
   std::iota(perm.begin(), perm.end(), 0);
   std::stable_sort(perm.begin(), perm.end(), [&](int64_t a, int64_t b) { return ts[a] < ts[b]; });
   DevBuf psi;
-  if (ptr_kind == EDK_HOST) EDK_RETURN_IF(psi.alloc((size_t)D * 16));
+  if (ptr_kind == EDK_HOST) EDK_RETURN_IF(stage_columns(psi, D, nts, op->stream));
   EDK_RETURN_IF(krylov_serve(K, op, ts, nts, perm.data(), out, ptr_kind, psi));
   dg->seconds = now_s() - t0;
   return EDK_OK;
@@ -1065,7 +1194,7 @@ extern "C" edk_status edk_krylov_cache_evolve(edk_krylov_cache* c, const double*
   edk_operator* op = c->op;
   std::lock_guard<std::mutex> lk(op->mu);
   double t0 = now_s();
-  if (ptr_kind == EDK_HOST && !c->psi.p) EDK_RETURN_IF(c->psi.alloc((size_t)op->b->D * 16));
+  if (ptr_kind == EDK_HOST) EDK_RETURN_IF(stage_columns(c->psi, op->b->D, nts, op->stream));
   c->K.dg = &c->diag;
   edk_status rc = krylov_serve(c->K, op, ts, nts, nullptr, out, ptr_kind, c->psi);
   c->seconds += now_s() - t0;
