@@ -6,7 +6,7 @@
 // only when T has more eigenvalues in a small window around it than T-hat (T
 // without its first block row and column) — the Cullum-Willoughby test
 // generalised to blocks, with exact counts from block Sturm (inertia)
-// sequences.  All operators' T run together: a Lanczos step is seven
+// sequences.  All operators' T run together: a Lanczos step is six
 // launches over every operator, and every Sturm count is one thread block.
 #include <algorithm>
 #include <cmath>
@@ -35,46 +35,52 @@ struct BandDims {
   int64_t nmax;
 };
 
-// w = T v_k for block row jb of operator q (thread a: row a of the block)
+// w = T v_k: a block takes G = blockDim.x / (3 p) block rows of operator q; of the
+// 3 p threads of a block row, thread (t, a) multiplies row a of B_j, A_j or
+// B_{j+1}^H (t = 0, 1, 2) by x_{j-1+t}, and the three sums meet in shared memory.
+// Bound by the latency of the entries a thread walks, so three threads share a
+// row and eight entries are in flight (p is a multiple of 8).
 __global__ void k_band_mv(BandDims d, const double2* __restrict__ A, const double2* __restrict__ B,
                           const int* __restrict__ mq, const double2* __restrict__ V, int k,
                           double2* __restrict__ w, const int* __restrict__ stop) {
-  extern __shared__ double2 sx[];  // x_{jb-1}, x_jb, x_{jb+1}
-  const int q = blockIdx.y, jb = blockIdx.x, p = d.p;
-  if (stop[q] || jb >= mq[q]) return;
-  const int m = mq[q];
-  const double2* x = V + ((size_t)q * d.vcols + k) * d.nmax;
-  const int a = threadIdx.x;
-  for (int t = 0; t < 3; ++t) {
-    const int jj = jb - 1 + t;
-    sx[t * p + a] = (jj >= 0 && jj < m) ? x[(size_t)jj * p + a] : make_double2(0.0, 0.0);
-  }
+  extern __shared__ double2 sx_all[];  // per block row: x_{jb-1}, x_jb, x_{jb+1}, then the sums
+  const int q = blockIdx.y, p = d.p;
+  if (stop[q]) return;
+  const int G = blockDim.x / (3 * p), m = mq[q];
+  const int g = threadIdx.x / (3 * p), e = threadIdx.x - g * 3 * p, t = e / p, a = e - t * p;
+  const int jb = blockIdx.x * G + g, jj = jb - 1 + t;
+  double2* sx = sx_all + 3 * p * g;
+  double2* sum = sx_all + 3 * p * (G + g);
+  const bool in = jb < m && jj >= 0 && jj < m;
+  sx[e] = in ? V[((size_t)q * d.vcols + k) * d.nmax + (size_t)jj * p + a] : make_double2(0.0, 0.0);
   __syncthreads();
-  const size_t pp = (size_t)p * p;
-  const double2* Aj = A + ((size_t)q * d.mmax + jb) * pp;
   double yr = 0.0, yi = 0.0;
-  for (int c = 0; c < p; ++c) {  // A_j x_j
-    const double2 v = Aj[a + (size_t)c * p], xc = sx[p + c];
-    yr += v.x * xc.x - v.y * xc.y;
-    yi += v.x * xc.y + v.y * xc.x;
-  }
-  if (jb >= 1) {  // + B_j x_{j-1}
-    const double2* Bj = B + ((size_t)q * d.mmax + jb) * pp;
-    for (int c = 0; c < p; ++c) {
-      const double2 v = Bj[a + (size_t)c * p], xc = sx[c];
-      yr += v.x * xc.x - v.y * xc.y;
-      yi += v.x * xc.y + v.y * xc.x;
+  if (in) {
+    const size_t pp = (size_t)p * p;
+    const double2* xs = sx + t * p;
+    if (t < 2) {  // B_j x_{j-1}, A_j x_j
+      const double2* M = (t == 0 ? B : A) + ((size_t)q * d.mmax + jb) * pp + a;
+#pragma unroll 8
+      for (int c = 0; c < p; ++c) {
+        const double2 v = M[(size_t)c * p], xc = xs[c];
+        yr += v.x * xc.x - v.y * xc.y;
+        yi += v.x * xc.y + v.y * xc.x;
+      }
+    } else {  // B_{j+1}^H x_{j+1}: conj(B(c, a)) x_c
+      const double2* M = B + ((size_t)q * d.mmax + jb + 1) * pp + (size_t)a * p;
+#pragma unroll 8
+      for (int c = 0; c < p; ++c) {
+        const double2 v = M[c], xc = xs[c];
+        yr += v.x * xc.x + v.y * xc.y;
+        yi += v.x * xc.y - v.y * xc.x;
+      }
     }
   }
-  if (jb + 1 < m) {  // + B_{j+1}^H x_{j+1}: conj(B(c, a)) x_c
-    const double2* Bn = B + ((size_t)q * d.mmax + jb + 1) * pp;
-    for (int c = 0; c < p; ++c) {
-      const double2 v = Bn[c + (size_t)a * p], xc = sx[2 * p + c];
-      yr += v.x * xc.x + v.y * xc.y;
-      yi += v.x * xc.y - v.y * xc.x;
-    }
-  }
-  w[(size_t)q * d.nmax + (size_t)jb * p + a] = make_double2(yr, yi);
+  sum[e] = make_double2(yr, yi);
+  __syncthreads();
+  if (t != 1 || jb >= m) return;
+  const double2 lo = sum[a], up = sum[2 * p + a];
+  w[(size_t)q * d.nmax + (size_t)jb * p + a] = make_double2((yr + lo.x) + up.x, (yi + lo.y) + up.y);
 }
 
 // s[q][c] = V_q[:, c]^H w_q for c <= k: one warp per (column, operator)
@@ -110,41 +116,54 @@ __global__ void __launch_bounds__(256) k_band_dots(BandDims d, const int* __rest
   if (lane == 0) s[(size_t)q * d.vcols + c] = make_double2(r, im);
 }
 
-// w_q -= V_q[:, 0:k+1] s_q (one thread per row)
+// w_q -= V_q[:, 0:k+1] s_q: a block takes 32 rows, its eight warps every eighth
+// column each, and the warps' sums meet in shared memory.  (One thread per row
+// leaves four blocks per operator at order 960 and a serial walk over all
+// columns: 21.6 us a launch over runs of order 160 to 960, 18 operators; this one
+// 12.3 us over the run of order 960, up to 280 columns.)
 __global__ void __launch_bounds__(256) k_band_update(BandDims d, const int* __restrict__ nq,
                                                      const double2* __restrict__ V, int k,
                                                      const double2* __restrict__ s,
                                                      double2* __restrict__ w,
                                                      const int* __restrict__ stop) {
-  extern __shared__ double2 ss[];  // k + 1 coefficients
+  __shared__ double2 sum[8][32];
   const int q = blockIdx.y;
   if (stop[q]) return;
-  for (int c = threadIdx.x; c <= k; c += blockDim.x) ss[c] = s[(size_t)q * d.vcols + c];
-  __syncthreads();
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nq[q]) return;
-  const double2* v = V + (size_t)q * d.vcols * d.nmax + i;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t i = (int64_t)blockIdx.x * 32 + lane;
+  const bool on = i < nq[q];
+  const double2* v = V + (size_t)q * d.vcols * d.nmax + (on ? i : 0);
+  const double2* t = s + (size_t)q * d.vcols;
   double ar = 0.0, ai = 0.0;
-  for (int c = 0; c <= k; ++c) {
-    const double2 x = v[(size_t)c * d.nmax], t = ss[c];
-    ar += x.x * t.x - x.y * t.y;
-    ai += x.x * t.y + x.y * t.x;
+#pragma unroll 4
+  for (int c = warp; c <= k; c += 8) {
+    const double2 x = v[(size_t)c * d.nmax], y = t[c];
+    ar += x.x * y.x - x.y * y.y;
+    ai += x.x * y.y + x.y * y.x;
+  }
+  sum[warp][lane] = make_double2(ar, ai);
+  __syncthreads();
+  if (warp != 0 || !on) return;
+#pragma unroll
+  for (int u = 1; u < 8; ++u) {
+    ar += sum[u][lane].x;
+    ai += sum[u][lane].y;
   }
   double2* wi = w + (size_t)q * d.nmax + i;
   *wi = make_double2(wi->x - ar, wi->y - ai);
 }
 
-// alpha_k (the first sweep's s_k), beta_k = |w|, 1/beta; a negligible beta
-// (the host form's rule b < 1e-12 max(1, |a|)) stops the operator with k + 1
-// steps, recorded in stop[q]
-__global__ void __launch_bounds__(256) k_band_norm(BandDims d, const int* __restrict__ nq, int k,
-                                                   const double2* __restrict__ w,
-                                                   const double2* __restrict__ s1,
-                                                   double* __restrict__ alpha,
-                                                   double* __restrict__ beta,
-                                                   double* __restrict__ invb,
-                                                   int* __restrict__ stop) {
-  __shared__ double sh[8];
+// alpha_k (the first sweep's s_k), beta_k = |w| and v_{k+1} = w / beta (one block
+// per operator); a negligible beta (the host form's rule b < 1e-12 max(1, |a|))
+// stops the operator with k + 1 steps, recorded in stop[q]
+__global__ void __launch_bounds__(1024) k_band_next(BandDims d, const int* __restrict__ nq, int k,
+                                                    const double2* __restrict__ w,
+                                                    const double2* __restrict__ s1,
+                                                    double* __restrict__ alpha,
+                                                    double* __restrict__ beta,
+                                                    double2* __restrict__ V,
+                                                    int* __restrict__ stop) {
+  __shared__ double sh[32];
   const int q = blockIdx.x;
   if (stop[q]) return;
   const int64_t n = nq[q];
@@ -154,33 +173,19 @@ __global__ void __launch_bounds__(256) k_band_norm(BandDims d, const int* __rest
   t = bwsum(t);
   if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = t;
   __syncthreads();
-  if (threadIdx.x != 0) return;
-  double n2 = 0.0;
-  for (int u = 0; u < 8; ++u) n2 += sh[u];
+  const double n2 = bwsum(sh[threadIdx.x & 31]);
   const double a = s1[(size_t)q * d.vcols + k].x, b = sqrt(n2);
-  alpha[(size_t)q * d.vcols + k] = a;
-  beta[(size_t)q * d.vcols + k] = b;
-  if (b < 1e-12 * fmax(1.0, fabs(a))) {
-    stop[q] = k + 1;
-    invb[q] = 0.0;
-  } else {
-    invb[q] = 1.0 / b;
+  const bool end = b < 1e-12 * fmax(1.0, fabs(a));
+  if (threadIdx.x == 0) {
+    alpha[(size_t)q * d.vcols + k] = a;
+    beta[(size_t)q * d.vcols + k] = b;
+    if (end) stop[q] = k + 1;
   }
-}
-
-// v_{k+1} = w / beta
-__global__ void __launch_bounds__(256) k_band_scale(BandDims d, const int* __restrict__ nq,
-                                                    int k, const double2* __restrict__ w,
-                                                    const double* __restrict__ invb,
-                                                    double2* __restrict__ V,
-                                                    const int* __restrict__ stop) {
-  const int q = blockIdx.y;
-  if (stop[q] || k + 1 >= d.vcols) return;
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nq[q]) return;
-  const double sc = invb[q];
-  const double2 x = w[(size_t)q * d.nmax + i];
-  V[((size_t)q * d.vcols + k + 1) * d.nmax + i] = make_double2(x.x * sc, x.y * sc);
+  if (end || k + 1 >= d.vcols) return;
+  const double sc = 1.0 / b;
+  double2* v = V + ((size_t)q * d.vcols + k + 1) * d.nmax;
+  for (int64_t i = threadIdx.x; i < n; i += blockDim.x)
+    v[i] = make_double2(x[i].x * sc, x[i].y * sc);
 }
 
 // One Sturm count: the number of eigenvalues below sigma of the
@@ -334,7 +339,7 @@ edk_status band_lowest_device(int p, int nev, const std::vector<int>& m,
   const size_t pp = (size_t)p * p;
   // T's blocks on the device
   std::vector<double2> hAB((size_t)nops * d.mmax * pp);
-  DevBuf dA, dB, V, w, s1, s2, alpha, beta, invb, stop, nq, mqd;
+  DevBuf dA, dB, V, w, s1, s2, alpha, beta, stop, nq, mqd;
   EDK_RETURN_IF(dA.alloc_async(hAB.size() * sizeof(double2), st));
   EDK_RETURN_IF(dB.alloc_async(hAB.size() * sizeof(double2), st));
   for (int pass = 0; pass < 2; ++pass) {
@@ -356,7 +361,6 @@ edk_status band_lowest_device(int p, int nev, const std::vector<int>& m,
   EDK_RETURN_IF(s2.alloc_async((size_t)nops * d.vcols * sizeof(double2), st));
   EDK_RETURN_IF(alpha.alloc_async((size_t)nops * d.vcols * sizeof(double), st));
   EDK_RETURN_IF(beta.alloc_async((size_t)nops * d.vcols * sizeof(double), st));
-  EDK_RETURN_IF(invb.alloc_async((size_t)nops * sizeof(double), st));
   EDK_RETURN_IF(stop.alloc_async((size_t)nops * sizeof(int), st));
   EDK_RETURN_IF(nq.alloc_async((size_t)nops * sizeof(int), st));
   EDK_RETURN_IF(mqd.alloc_async((size_t)nops * sizeof(int), st));
@@ -394,30 +398,28 @@ edk_status band_lowest_device(int p, int nev, const std::vector<int>& m,
   std::vector<std::vector<double>> prev(nops), cand(nops);
   std::vector<int> finished(nops, 0), hstop(nops, 0);
   // the lowest nk eigenvalues of each Lanczos matrix, on the device
-  // (edk_tridiag.cu): nev + 4 candidates and four more for values that merge
-  int nk = nev + 8;
+  // (edk_tridiag.cu): nev + 4 candidates, more only once values merge
+  int nk = nev + 4;
   DevBuf evd;
   EDK_RETURN_IF(evd.alloc_async((size_t)nops * nk * sizeof(double), st));
   std::vector<double> hev((size_t)nops * nk);
-  const unsigned rows = (unsigned)((d.nmax + 255) / 256);
+  const unsigned rows = (unsigned)((d.nmax + 31) / 32);
+  const int G = std::max(1, 64 / p);  // block rows per block of k_band_mv
   int left = nops;
   for (int k = 0; k < kmax && left > 0; ++k) {
-    k_band_mv<<<dim3(d.mmax, nops), p, 3 * p * sizeof(double2), st>>>(
+    k_band_mv<<<dim3((d.mmax + G - 1) / G, nops), 3 * G * p, 6 * G * p * sizeof(double2), st>>>(
         d, dA.as<double2>(), dB.as<double2>(), mqd.as<int>(), V.as<double2>(), k, w.as<double2>(),
         stop.as<int>());
     for (int pass = 0; pass < 2; ++pass) {
       double2* s = pass == 0 ? s1.as<double2>() : s2.as<double2>();
       k_band_dots<<<dim3((k + 8) / 8, nops), 256, 0, st>>>(d, nq.as<int>(), V.as<double2>(), k,
                                                           w.as<double2>(), s, stop.as<int>());
-      k_band_update<<<dim3(rows, nops), 256, (k + 1) * sizeof(double2), st>>>(
-          d, nq.as<int>(), V.as<double2>(), k, s, w.as<double2>(), stop.as<int>());
+      k_band_update<<<dim3(rows, nops), 256, 0, st>>>(d, nq.as<int>(), V.as<double2>(), k, s,
+                                                      w.as<double2>(), stop.as<int>());
     }
-    k_band_norm<<<nops, 256, 0, st>>>(d, nq.as<int>(), k, w.as<double2>(), s1.as<double2>(),
-                                      alpha.as<double>(), beta.as<double>(), invb.as<double>(),
-                                      stop.as<int>());
-    k_band_scale<<<dim3(rows, nops), 256, 0, st>>>(d, nq.as<int>(), k, w.as<double2>(),
-                                                   invb.as<double>(), V.as<double2>(),
-                                                   stop.as<int>());
+    k_band_next<<<nops, 1024, 0, st>>>(d, nq.as<int>(), k, w.as<double2>(), s1.as<double2>(),
+                                       alpha.as<double>(), beta.as<double>(), V.as<double2>(),
+                                       stop.as<int>());
     EDK_TRY_CUDA(cudaGetLastError());
     bool look = (k + 1) % 10 == 0 || k + 1 == kmax;
     for (int q = 0; q < nops && !look; ++q)

@@ -250,10 +250,6 @@ const char* cublas_msg(cublasStatus_t s) {
     }                                                                               \
   } while (0)
 
-struct BlasHandle {
-  cublasHandle_t h = nullptr;
-  ~BlasHandle() { if (h) cublasDestroy(h); }
-};
 
 // ---------------------------------------------------------------------------
 // eigenvalues of the block-tridiagonal T (host)
@@ -492,7 +488,11 @@ static edk_status block_lanczos(int nops, edk_operator* const* ops,
   cudaStream_t st = ops[0]->stream;
   int64_t Dmax = 0;
   for (int q = 0; q < nops; ++q) Dmax = std::max<int64_t>(Dmax, ops[q]->b->D);
-  const int64_t Kc = std::min<int64_t>(2048, ((Dmax + 31) / 32) * 32);
+  // rows per chunk of the split products: 2,048, fewer when that leaves the GPU
+  // short of chunks (a chunk is one serial sum: 18 sectors of 2,700 rows with 36
+  // chunks of 2,048 rows took 75 us a product, 11.9 us with four chunks per SM)
+  const int64_t Kfit = ((int64_t)nops * Dmax / (4 * 148) + 31) / 32 * 32;
+  const int64_t Kc = std::min<int64_t>({2048, ((Dmax + 31) / 32) * 32, std::max<int64_t>(64, Kfit)});
   const int64_t S = (Dmax + Kc - 1) / Kc;
   const int64_t Dpad = S * Kc;
   const size_t slot = (size_t)nops * Dpad * p;
@@ -519,17 +519,17 @@ static edk_status block_lanczos(int nops, edk_operator* const* ops,
   }
 
   DevBuf d_ops, ring0, ring1, ring2, part, Q1, Q2, G, Rinv, R1, R2, Bm, flags, colx, coly;
-  EDK_RETURN_IF(d_ops.alloc(sizeof(SpmmOp) * nops));
-  EDK_RETURN_IF(ring0.alloc(slot * sizeof(double2)));
-  EDK_RETURN_IF(ring1.alloc(slot * sizeof(double2)));
-  EDK_RETURN_IF(ring2.alloc(slot * sizeof(double2)));
-  EDK_RETURN_IF(part.alloc((size_t)nops * S * pp * sizeof(double2)));
+  EDK_RETURN_IF(d_ops.alloc_async(sizeof(SpmmOp) * nops, st));
+  EDK_RETURN_IF(ring0.alloc_async(slot * sizeof(double2), st));
+  EDK_RETURN_IF(ring1.alloc_async(slot * sizeof(double2), st));
+  EDK_RETURN_IF(ring2.alloc_async(slot * sizeof(double2), st));
+  EDK_RETURN_IF(part.alloc_async((size_t)nops * S * pp * sizeof(double2), st));
   for (DevBuf* bf : {&Q1, &Q2, &G, &Rinv, &R1, &R2, &Bm})
-    EDK_RETURN_IF(bf->alloc((size_t)nops * pp * sizeof(double2)));
-  EDK_RETURN_IF(flags.alloc(nops * sizeof(int)));
+    EDK_RETURN_IF(bf->alloc_async((size_t)nops * pp * sizeof(double2), st));
+  EDK_RETURN_IF(flags.alloc_async(nops * sizeof(int), st));
   if (any_generic) {
-    EDK_RETURN_IF(colx.alloc((size_t)Dmax * p * sizeof(double2)));
-    EDK_RETURN_IF(coly.alloc((size_t)Dmax * p * sizeof(double2)));
+    EDK_RETURN_IF(colx.alloc_async((size_t)Dmax * p * sizeof(double2), st));
+    EDK_RETURN_IF(coly.alloc_async((size_t)Dmax * p * sizeof(double2), st));
   }
   EDK_TRY_CUDA(cudaMemcpyAsync(d_ops.p, hops.data(), sizeof(SpmmOp) * nops,
                                cudaMemcpyHostToDevice, st));
@@ -540,8 +540,13 @@ static edk_status block_lanczos(int nops, edk_operator* const* ops,
   double2* V = ring1.as<double2>();
   double2* W = ring2.as<double2>();
 
-  BlasHandle bh;
-  EDK_TRY_BLAS(cublasCreate(&bh.h));
+  // the first operator keeps its handle (creating one costs milliseconds); its
+  // lock is held here
+  struct { cublasHandle_t h; } bh{static_cast<cublasHandle_t>(ops[0]->blas)};
+  if (!bh.h) {
+    EDK_TRY_BLAS(cublasCreate(&bh.h));
+    ops[0]->blas = bh.h;
+  }
   EDK_TRY_BLAS(cublasSetStream(bh.h, st));
   EDK_TRY_BLAS(cublasSetPointerMode(bh.h, CUBLAS_POINTER_MODE_HOST));
   const cuDoubleComplex one = make_cuDoubleComplex(1.0, 0.0);
@@ -746,8 +751,9 @@ static edk_status block_lanczos(int nops, edk_operator* const* ops,
       if (hflag[q] && broke_at[q] < 0) broke_at[q] = j + 1;
       all_broken = all_broken && broke_at[q] >= 0;
     }
-    const bool check = (o.check_every > 0 && (j + 1) % o.check_every == 0) || j + 1 == m ||
-                       all_broken;
+    // (without a tolerance only the last step's eigenvalues are ever used)
+    const bool check = (o.tol > 0.0 && o.check_every > 0 && (j + 1) % o.check_every == 0) ||
+                       j + 1 == m || all_broken;
     if (check) {
       EDK_RETURN_IF(extract(j + 1));
       if (o.tol > 0.0 && j + 1 < m) {
@@ -780,6 +786,10 @@ static edk_status block_lanczos(int nops, edk_operator* const* ops,
     diag->seconds_eig = t_eig;
   }
   return EDK_OK;
+}
+
+void blas_release(void* handle) {
+  if (handle) cublasDestroy(static_cast<cublasHandle_t>(handle));
 }
 
 }  // namespace edk

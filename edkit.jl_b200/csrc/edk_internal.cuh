@@ -369,6 +369,7 @@ struct edk_operator {
   std::vector<unsigned char> bop_host;   // the record as last uploaded
   cudaStream_t cstream = nullptr;        // copy stream of the pipelined host path
   std::vector<cudaEvent_t> cevents;      // one per row chunk of that path
+  void* blas = nullptr;                  // cuBLAS handle of the block Lanczos, once it ran
   std::mutex mu;
   ~edk_operator();
 };
@@ -433,6 +434,8 @@ class KrylovBasis {
   struct Impl;
   std::unique_ptr<Impl> impl;
 };
+// implemented in edk_block.cu
+void blas_release(void* handle);
 // implemented in edk_util.cpp
 int tridiag_eigvals(int m, const double* a, const double* b, double* w);
 // The lowest `nev` distinct eigenvalues of block-tridiagonal Hermitian
