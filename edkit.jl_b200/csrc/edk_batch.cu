@@ -13,14 +13,16 @@
 // tridiagonal problems and tests convergence (edk_tridiag.cu); the host reads
 // only how many operators are left.  One step per operator q:
 //   wt_q = H_q v_j                       (row-gather matvec)
-//   s = V_q^H wt_q ; alpha_j = Re s_j     (CGS sweep 1, FP64 block partials)
-//   w_q = wt_q - V_q s ; u = V_q^H w_q    (one pass: k_rupdate_dots)
-//   w_q -= V_q u ; beta_j = ||w_q||       (sweep 2 + norm)
-//   lucky breakdown beta <= sqrt(eps) max(1, |alpha|) stops operator q
+//   s = V_q^H v_j, r = V_q^H wt_q          (one read of V for both)
+//   v_j = (v_j - V_q s) / a                (the second sweep of the step before)
+//   w_q = H v_j - V_q V_q^H H v_j          (the first sweep of this step; the same
+//                                          second read of V serves both)
+//   beta_j = ||w_q|| ; lucky breakdown beta <= sqrt(eps) max(1, |alpha|) stops q
 //   v_{j+1} = w_q / beta_j
 // (classical Gram-Schmidt twice, as _lanczos_build! in
 // src/algorithms/TimeEvolution.jl:250-306, with its three-term recurrence
-// folded into the first sweep).
+// folded into the first sweep, and the second sweep delayed by one step; see
+// k_rdots2).
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -37,7 +39,8 @@ namespace edk {
 namespace {
 
 constexpr int kTile = 256;          // rows per matvec / update tile
-constexpr int kSplitBlocks = 4;         // resident reorthogonalisation blocks per SM (register cap)
+// resident reorthogonalisation blocks per SM (128 registers a thread)
+constexpr int kSplitBlocks = 2;
 
 template <class T> struct IsCx;
 template <> struct IsCx<double> { static constexpr bool v = false; };
@@ -329,333 +332,415 @@ __device__ __forceinline__ void for_block_rows(const BOp* __restrict__ ops, RowS
   }
 }
 
-// Rows per thread and pass of the reorthogonalisation kernels: a pass loads
-// U columns (8 real, 4 complex) of R rows in one go, 128 bytes a thread.
+// loads of the Krylov vectors: each is used once per kernel, so it leaves L1 to
+// the vectors every column is combined with
+__device__ __forceinline__ double lv(const double* p) {
+  double v;
+  asm volatile("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ double2 lv(const double2* p) {
+  double2 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float lv(const float* p) {
+  float v;
+  asm volatile("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float2 lv(const float2* p) {
+  float2 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ double2 wide(double v) { return make_double2(v, 0.0); }
+__device__ __forceinline__ double2 wide(double2 v) { return v; }
+__device__ __forceinline__ double2 wide(float v) { return make_double2((double)v, 0.0); }
+__device__ __forceinline__ double2 wide(float2 v) { return make_double2((double)v.x, (double)v.y); }
+
+// ---------------------------------------------------------------------------
+// Gram-Schmidt twice with two reads of V per step.  Each sweep has to know all
+// its dot products before it updates, so two sweeps of one vector read V four
+// times (three with the middle update and dot products fused).  Here the second
+// sweep of v_j waits for the first sweep of the next vector (delayed
+// re-orthogonalisation, as in Bielich, Langou, Thomas, Swirydowicz, Yamazaki and
+// Boman, "Low-synch Gram-Schmidt with delayed reorthogonalization for Krylov
+// solvers", 2022).  With u = v_j after one sweep, normalised, V the final columns
+// before it and wt = H u, one read of V gives s = V^H u and r = V^H wt (and
+// |u|^2, u^H wt from column j).  Then, with a^2 = |u|^2 - |s|^2,
+//   q = (u - V s) / a                                     (v_j, final)
+//   H q = (wt - V T s - beta_{j-1} s_{j-1} q) / a         (H V = V T + beta q e^T)
+//   g = q^H wt / a = (u^H wt - s^H r) / a^2
+//   alpha_j = Re(g - beta_{j-1} s_{j-1} / a)
+//   H q - V V^H H q - q q^H H q = (wt - g u - V (r - g s)) / a
+// so the second read of V updates both vectors.  V^H H q is exact to the
+// rounding of the recurrence times |s|, which one sweep leaves at eps |H| / beta.
+// Mean over the 131 steps of 96 random-field chains of 12 to 20 sites (FP64):
+// 194 + 247 + 173 us for the three passes before, 171 + 177 us for the two here,
+// which is the HBM rate (two blocks of 128 registers per SM; three of 80 spill:
+// 199 + 170; four of 64: slower in every case measured).
+// ---------------------------------------------------------------------------
+
+// part[pofs_q + c nslot_q + slot] = sum over the block's rows of conj(V_q[r, c])
+// V_q[r, j], and the same with wt_q at part + pstride, c <= j.  Bound by HBM: a
+// warp takes four columns over its rows and reduces once at the end, all loads of
+// RU rows of them in flight; the two vectors every warp needs stay in L1.  With
+// few columns the warps split the rows as well (up to eight ways) and meet in
+// shared memory.
 template <class VV>
-constexpr int pass_rows() {
-  return 128 / ((IsCx<VV>::v ? 4 : 8) * (int)sizeof(VV));
-}
-
-// One pass of k_rdots: a += conj(V[rows, cols]) w[rows] for the U columns
-// at Vc[u] and the R rows rb + 256 k (all in range when FULL).
-template <bool FULL, int U, int R, bool CX, class VV, class WV>
-__device__ __forceinline__ void dots_pass(const VV* const (&Vc)[U], const WV* __restrict__ wq,
-                                          int64_t rb, int64_t r1, double (&a)[8]) {
-  double2 wv[R], v[U][R];
-#pragma unroll
-  for (int k = 0; k < R; ++k) {
-    const int64_t r = rb + (int64_t)k * 256;
-    wv[k] = (FULL || r < r1) ? l2(wq + r) : make_double2(0.0, 0.0);
-  }
-#pragma unroll
-  for (int u = 0; u < U; ++u)
-#pragma unroll
-    for (int k = 0; k < R; ++k) {
-      const int64_t r = rb + (int64_t)k * 256;
-      v[u][k] = (FULL || r < r1) ? l2(Vc[u] + r) : make_double2(0.0, 0.0);
-    }
-#pragma unroll
-  for (int u = 0; u < U; ++u)
-#pragma unroll
-    for (int k = 0; k < R; ++k) {
-      if constexpr (CX) {
-        a[2 * u] += v[u][k].x * wv[k].x + v[u][k].y * wv[k].y;
-        a[2 * u + 1] += v[u][k].x * wv[k].y - v[u][k].y * wv[k].x;
-      } else {
-        a[u] += v[u][k].x * wv[k].x;
-      }
-    }
-}
-
-// part[pofs_q + c * nslot_q + slot] = sum over the block's rows r of
-// conj(V_q[r, c]) w_q[r], c <= j.  Columns go eight real (four complex)
-// values at a time through one wsum8 after the thread has summed its rows;
-// the columns of a last, partial group read the segment's last column again
-// (their sums are not kept).  The per-warp sums of 64 columns at a time are
-// added across warps in shared memory.
-template <class VV, class WV>
-__global__ void __launch_bounds__(256, kSplitBlocks) k_rdots(const BOp* __restrict__ ops, RowSplit rs,
-                                               const VV* __restrict__ V,
-                                               const WV* __restrict__ w,
-                                               double2* __restrict__ part,
-                                               const int* __restrict__ step,
-                                               const int* __restrict__ done) {
-  constexpr bool CX = IsCx<VV>::v || IsCx<WV>::v;
-  constexpr int U = CX ? 4 : 8;  // columns per reduction
-  constexpr int SEG = 64;        // columns per shared-memory flush
-  constexpr int R = pass_rows<VV>();
-  __shared__ double s_part[8][SEG][2];
-  const int ncols = *step + 1;
+__global__ void __launch_bounds__(256, kSplitBlocks) k_rdots2(const BOp* __restrict__ ops, RowSplit rs,
+                                                const VV* __restrict__ V,
+                                                const VV* __restrict__ wt,
+                                                double2* __restrict__ part, int64_t pstride,
+                                                const int* __restrict__ step,
+                                                const int* __restrict__ done) {
+  constexpr bool CX = IsCx<VV>::v;
+  constexpr int NC = CX ? 2 : 1;
+  constexpr int RU = sizeof(VV) == 16 ? 2 : 4;
+  __shared__ double2 s_part[256][2];
+  const int ncols = *step + 1, ng = (ncols + 3) / 4;
+  const int nsub = ng <= 8 ? 8 : (ng <= 16 ? 4 : (ng <= 32 ? 2 : 1));
+  const int pad = 256 / nsub;  // columns of a row share in s_part
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for_block_rows(ops, rs, [&](int q, const BOp& o, int64_t r0, int64_t r1, int slot, const SplitOp& sq) {
     if (done[q]) return;
-    const int64_t D = o.D;
+    const int64_t D = o.D, rows = r1 - r0;
     const VV* Vq = V + o.voff;
-    const WV* wq = w + o.woff;
-    for (int s0 = 0; s0 < ncols; s0 += SEG) {
-      const int s1 = min(ncols, s0 + SEG);
-      for (int c = s0; c < s1; c += U) {
-        const VV* Vc[U];
+    const VV* x = Vq + (int64_t)(ncols - 1) * D;
+    const VV* y = wt + o.woff;
+    for (int un = warp; un < ng * nsub; un += 8) {
+      const int cg = un % ng, sub = un / ng;
+      const int64_t a = r0 + rows * sub / nsub, b = r0 + rows * (sub + 1) / nsub;
+      const VV* Vc[4];
 #pragma unroll
-        for (int u = 0; u < U; ++u) Vc[u] = Vq + (int64_t)min(c + u, s1 - 1) * D;
-        double a[8];
+      for (int u = 0; u < 4; ++u) Vc[u] = Vq + (int64_t)min(4 * cg + u, ncols - 1) * D;
+      double fs[4 * NC], fr[4 * NC];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) a[u] = 0.0;
-        int64_t rb = r0 + threadIdx.x;
-        for (; rb + (int64_t)(R - 1) * 256 < r1; rb += 256 * R)
-          dots_pass<true, U, R, CX>(Vc, wq, rb, r1, a);
-        if (rb < r1) dots_pass<false, U, R, CX>(Vc, wq, rb, r1, a);
-        const double t = wsum8(a, lane);
-        if ((lane & 3) == 0) {
-          const int vi = lane >> 2;
-          const int col = CX ? c + (vi >> 1) : c + vi;
-          if (col < s1) s_part[warp][col - s0][CX ? (vi & 1) : 0] = t;
+      for (int u = 0; u < 4 * NC; ++u) fs[u] = fr[u] = 0.0;
+      auto pass = [&](int64_t rb, bool full) {
+        VV v[4][RU], xv[RU], yv[RU];
+#pragma unroll
+        for (int k = 0; k < RU; ++k) {
+          const int64_t r = rb + 32 * k;
+          const bool on = full || r < b;
+#pragma unroll
+          for (int u = 0; u < 4; ++u) v[u][k] = on ? lv(Vc[u] + r) : VV{};
+          xv[k] = on ? x[r] : VV{};
+          yv[k] = on ? y[r] : VV{};
         }
-      }
-      __syncthreads();
-      for (int c = threadIdx.x; c < s1 - s0; c += blockDim.x) {
-        double sr = 0.0, si = 0.0;
 #pragma unroll
-        for (int ww = 0; ww < 8; ++ww) {
-          sr += s_part[ww][c][0];
-          if (CX) si += s_part[ww][c][1];
-        }
-        part[sq.pofs + (int64_t)(s0 + c) * sq.nslot + slot] = make_double2(sr, si);
-      }
-      __syncthreads();
-    }
-  });
-}
-
-// coef[q * ncap + c] = sum of operator q's slots: block (x, q) sums columns
-// 8x .. 8x + 7 of operator q, one warp per column
-__global__ void __launch_bounds__(256) k_breduce(const SplitOp* __restrict__ sp, int ncap,
-                                                 const double2* __restrict__ part,
-                                                 double2* __restrict__ coef,
-                                                 const int* __restrict__ step,
-                                                 const int* __restrict__ done) {
-  const int q = blockIdx.y;
-  const int c = blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (done[q] || c > *step) return;
-  const int lane = threadIdx.x & 31;
-  const SplitOp& o = sp[q];
-  const double2* pc = part + o.pofs + (int64_t)c * o.nslot;
-  // four independent loads in flight a lane (a large operator has hundreds
-  // of slots and only j + 1 columns, so few warps carry the whole reduction)
-  double2 a[4] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0), make_double2(0.0, 0.0),
-                  make_double2(0.0, 0.0)};
-  int k = lane;
-  for (; k + 96 < o.nslot; k += 128) {
+        for (int k = 0; k < RU; ++k) {
+          const double2 xw = wide(xv[k]), yw = wide(yv[k]);
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const double2 v = pc[k + 32 * u];
-      a[u].x += v.x;
-      a[u].y += v.y;
-    }
-  }
-  for (; k < o.nslot; k += 32) {
-    const double2 v = pc[k];
-    a[0].x += v.x;
-    a[0].y += v.y;
-  }
-  double sr = (a[0].x + a[1].x) + (a[2].x + a[3].x);
-  double si = (a[0].y + a[1].y) + (a[2].y + a[3].y);
-  sr = wsum(sr);
-  si = wsum(si);
-  if (lane == 0) coef[(int64_t)q * ncap + c] = make_double2(sr, si);
-}
-
-// acc[k] -= V[rows, cols] coef[cols] for the U columns at Vc[u] (coefficient
-// zero past the last column) and the R rows rb + 256 k (all in range when
-// FULL).
-template <bool FULL, int U, int R, bool CX, class VV>
-__device__ __forceinline__ void update_pass(const VV* const (&Vc)[U], const double2* kc,
-                                            int64_t rb, int64_t r1, double2 (&acc)[R]) {
-  double2 v[U][R];
-#pragma unroll
-  for (int u = 0; u < U; ++u)
-#pragma unroll
-    for (int k = 0; k < R; ++k) {
-      const int64_t r = rb + (int64_t)k * 256;
-      v[u][k] = (FULL || r < r1) ? l2(Vc[u] + r) : make_double2(0.0, 0.0);
-    }
-#pragma unroll
-  for (int u = 0; u < U; ++u) {
-    const double2 cu = kc[u];
-#pragma unroll
-    for (int k = 0; k < R; ++k) {
-      acc[k].x -= v[u][k].x * cu.x;
-      if (CX) {
-        acc[k].x += v[u][k].y * cu.y;
-        acc[k].y -= v[u][k].x * cu.y + v[u][k].y * cu.x;
-      }
-    }
-  }
-}
-
-// wout_q = win_q - V_q[:, 0:ncols] coef_q over the block's rows;
-// normpart[slot0_q + slot] = sum |wout|^2 over them.  ncols = *step + 1 (or 0
-// with zero_cols).  Columns go U at a time (the coefficients are padded with
-// zeros to a multiple of U, the missing columns read the last one again).
-template <class VV, class WI, class WO>
-__global__ void __launch_bounds__(256, kSplitBlocks) k_rupdate(const BOp* __restrict__ ops, RowSplit rs,
-                                                 int ncap, const VV* __restrict__ V,
-                                                 const double2* __restrict__ coef,
-                                                 const WI* __restrict__ win, WO* __restrict__ wout,
-                                                 double* __restrict__ normpart,
-                                                 const int* __restrict__ step,
-                                                 const int* __restrict__ done, int zero_cols) {
-  extern __shared__ double2 s_coef[];  // ncap + 8
-  __shared__ double s_n[8];
-  constexpr bool CX = IsCx<VV>::v || IsCx<WI>::v;
-  constexpr int U = CX ? 4 : 8;
-  constexpr int R = pass_rows<VV>();
-  const int ncols = zero_cols ? 0 : *step + 1;
-  const int npad = (ncols + U - 1) / U * U;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for_block_rows(ops, rs, [&](int q, const BOp& o, int64_t r0, int64_t r1, int slot, const SplitOp& sq) {
-    if (done[q]) return;
-    __syncthreads();  // the previous piece's coefficients and norms are read
-    for (int c = threadIdx.x; c < npad; c += blockDim.x)
-      s_coef[c] = c < ncols ? coef[(int64_t)q * ncap + c] : make_double2(0.0, 0.0);
-    __syncthreads();
-    const int64_t D = o.D;
-    const VV* Vq = V + o.voff;
-    double nrm = 0.0;
-    for (int64_t rb = r0 + threadIdx.x; rb < r1; rb += 256 * R) {
-      const bool full = rb + (int64_t)(R - 1) * 256 < r1;
-      double2 acc[R];
-#pragma unroll
-      for (int k = 0; k < R; ++k) {
-        const int64_t r = rb + (int64_t)k * 256;
-        acc[k] = r < r1 ? l2(win + o.woff + r) : make_double2(0.0, 0.0);
-      }
-      for (int c = 0; c < npad; c += U) {
-        const VV* Vc[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) Vc[u] = Vq + (int64_t)min(c + u, ncols - 1) * D;
-        if (full) update_pass<true, U, R, CX>(Vc, s_coef + c, rb, r1, acc);
-        else update_pass<false, U, R, CX>(Vc, s_coef + c, rb, r1, acc);
-      }
-#pragma unroll
-      for (int k = 0; k < R; ++k) {
-        const int64_t r = rb + (int64_t)k * 256;
-        if (r < r1) {
-          s2(wout + o.woff + r, acc[k]);
-          nrm += acc[k].x * acc[k].x + (CX ? acc[k].y * acc[k].y : 0.0);
-        }
-      }
-    }
-    if (normpart) {
-      nrm = wsum(nrm);
-      if (lane == 0) s_n[warp] = nrm;
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        double t = 0.0;
-        for (int k = 0; k < 8; ++k) t += s_n[k];
-        normpart[sq.slot0 + slot] = t;
-      }
-    }
-  });
-}
-
-// The first sweep's update and the second sweep's dot products in one pass,
-// 256 rows at a time.  Update: one thread per row, wout = win - V coef over
-// all columns; the result (as stored) goes to shared memory.  Dot products:
-// one warp per column (warps take every eighth column, newest first, so the
-// columns the update read last, the most likely to be still in L2, are read
-// again first), each lane over eight of the 256 rows, one warp reduction per
-// column; the sums build up per column in shared memory and go to
-// part[pofs_q + c * nslot_q + slot] at the end of the piece.
-// Shared memory: ncap + 8 coefficients and ncap column sums (double2).
-template <class VV, class WI, class WO>
-__global__ void __launch_bounds__(256, kSplitBlocks) k_rupdate_dots(const BOp* __restrict__ ops, RowSplit rs,
-                                                      int ncap, const VV* __restrict__ V,
-                                                      const double2* __restrict__ coef,
-                                                      const WI* __restrict__ win,
-                                                      WO* __restrict__ wout,
-                                                      double2* __restrict__ part,
-                                                      const int* __restrict__ step,
-                                                      const int* __restrict__ done) {
-  extern __shared__ double2 s_dyn[];
-  double2* s_coef = s_dyn;
-  double2* s_acc = s_dyn + ncap + 8;
-  __shared__ double2 s_w[256];
-  constexpr bool CX = IsCx<VV>::v || IsCx<WI>::v || IsCx<WO>::v;
-  constexpr int U = CX ? 4 : 8;
-  const int ncols = *step + 1;
-  const int npad = (ncols + U - 1) / U * U;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for_block_rows(ops, rs, [&](int q, const BOp& o, int64_t r0, int64_t r1, int slot, const SplitOp& sq) {
-    if (done[q]) return;
-    __syncthreads();  // the previous piece's column sums are written out
-    for (int c = threadIdx.x; c < npad; c += blockDim.x)
-      s_coef[c] = c < ncols ? coef[(int64_t)q * ncap + c] : make_double2(0.0, 0.0);
-    for (int c = threadIdx.x; c < ncols; c += blockDim.x) s_acc[c] = make_double2(0.0, 0.0);
-    __syncthreads();
-    const int64_t D = o.D;
-    const VV* Vq = V + o.voff;
-    for (int64_t rb = r0; rb < r1; rb += 256) {
-      const int64_t r = rb + threadIdx.x;
-      const int nrow = (int)min((int64_t)256, r1 - rb);
-      double2 acc[1] = {make_double2(0.0, 0.0)};
-      if (r < r1) {
-        acc[0] = l2(win + o.woff + r);
-        for (int c = 0; c < npad; c += U) {
-          const VV* Vc[U];
-#pragma unroll
-          for (int u = 0; u < U; ++u) Vc[u] = Vq + (int64_t)min(c + u, ncols - 1) * D;
-          update_pass<true, U, 1, CX>(Vc, s_coef + c, r, r + 1, acc);
-        }
-        WO t;
-        s2(&t, acc[0]);
-        wout[o.woff + r] = t;
-        acc[0] = l2(&t);  // the dot products see the stored value
-      }
-      s_w[threadIdx.x] = acc[0];
-      __syncthreads();
-      // two columns (c and c - 8) per pass: sixteen loads in flight a lane
-      for (int c = ncols - 1 - warp; c >= 0; c -= 16) {
-        const int c2 = c >= 8 ? c - 8 : c;
-        const VV* Va = Vq + (int64_t)c * D + rb;
-        const VV* Vb = Vq + (int64_t)c2 * D + rb;
-        double ar = 0.0, ai = 0.0, br = 0.0, bi = 0.0;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const int i = lane + 32 * k;
-          if (i < nrow) {
-            const double2 va = l2(Va + i), vb = l2(Vb + i), x = s_w[i];
-            ar += va.x * x.x + va.y * x.y;
-            br += vb.x * x.x + vb.y * x.y;
-            if (CX) {
-              ai += va.x * x.y - va.y * x.x;
-              bi += vb.x * x.y - vb.y * x.x;
+          for (int u = 0; u < 4; ++u) {
+            const double2 c = wide(v[u][k]);
+            if constexpr (CX) {
+              fs[2 * u] += c.x * xw.x + c.y * xw.y;
+              fs[2 * u + 1] += c.x * xw.y - c.y * xw.x;
+              fr[2 * u] += c.x * yw.x + c.y * yw.y;
+              fr[2 * u + 1] += c.x * yw.y - c.y * yw.x;
+            } else {
+              fs[u] += c.x * xw.x;
+              fr[u] += c.x * yw.x;
             }
           }
         }
-        ar = wsum(ar);
-        br = wsum(br);
-        if (CX) {
-          ai = wsum(ai);
-          bi = wsum(bi);
+      };
+      int64_t rb = a + lane;
+      for (; rb - lane + 32 * RU <= b; rb += 32 * RU) pass(rb, true);
+      if (rb - lane < b) pass(rb, false);
+      // lane 4 v ends with value v: the sums of a column (and vector) in turn
+      auto put = [&](int col, int vec, int comp, double t) {
+        if (col >= ncols) return;
+        if (nsub > 1) {
+          reinterpret_cast<double*>(&s_part[sub * pad + col][vec])[comp] = t;
+          if (!CX) reinterpret_cast<double*>(&s_part[sub * pad + col][vec])[1] = 0.0;
+        } else {
+          double* d = reinterpret_cast<double*>(part + (vec ? pstride : 0) + sq.pofs +
+                                                (int64_t)col * sq.nslot + slot);
+          d[comp] = t;
+          if (!CX) d[1] = 0.0;
         }
-        if (lane == 0) {
-          s_acc[c].x += ar;
-          s_acc[c].y += ai;
-          if (c2 != c) {
-            s_acc[c2].x += br;
-            s_acc[c2].y += bi;
-          }
+      };
+      const int vi = lane >> 2;
+      if constexpr (CX) {
+        const double ts = wsum8(fs, lane), tr = wsum8(fr, lane);
+        if ((lane & 3) == 0) {
+          put(4 * cg + (vi >> 1), 0, vi & 1, ts);
+          put(4 * cg + (vi >> 1), 1, vi & 1, tr);
         }
+      } else {
+        double f[8];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          f[u] = fs[u];
+          f[u + 4] = fr[u];
+        }
+        const double t = wsum8(f, lane);
+        if ((lane & 3) == 0) put(4 * cg + (vi & 3), vi >> 2, 0, t);
       }
-      __syncthreads();  // s_w is rewritten by the next rows
     }
-    for (int c = threadIdx.x; c < ncols; c += blockDim.x)
-      part[sq.pofs + (int64_t)c * sq.nslot + slot] = s_acc[c];
+    if (nsub > 1) {
+      __syncthreads();
+      for (int e = threadIdx.x; e < 2 * ncols; e += blockDim.x) {
+        const int c = e >> 1, vec = e & 1;
+        double2 t = make_double2(0.0, 0.0);
+        for (int sub = 0; sub < nsub; ++sub) {
+          t.x += s_part[sub * pad + c][vec].x;
+          t.y += s_part[sub * pad + c][vec].y;
+        }
+        part[(vec ? pstride : 0) + sq.pofs + (int64_t)c * sq.nslot + slot] = t;
+      }
+      __syncthreads();  // s_part is free for the next piece
+    }
   });
 }
 
-// per operator: alpha_j, beta_j, breakdown, 1/beta (one block per operator).
+__device__ __forceinline__ double bsum256(double v, double* sh) {  // all threads get the sum
+  v = wsum(v);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+  __syncthreads();
+  double t = 0.0;
+  for (int k = 0; k < 8; ++k) t += sh[k];
+  return t;
+}
+
+// Sums operator q's slots (one warp per column; both vectors), and in the last
+// block of the operator turns them into the update's coefficients:
+// cs = s, ce = r - g s, scal = {1 / a, g}, and alpha_j.
+__global__ void __launch_bounds__(256) k_breduce2(const SplitOp* __restrict__ sp, int ncap, int m,
+                                                  const double2* __restrict__ part, int64_t pstride,
+                                                  double2* __restrict__ cs, double2* __restrict__ ce,
+                                                  double4* __restrict__ scal,
+                                                  double* __restrict__ alpha,
+                                                  const double* __restrict__ beta,
+                                                  unsigned* __restrict__ cnt,
+                                                  const int* __restrict__ step,
+                                                  const int* __restrict__ done) {
+  __shared__ bool s_last;
+  __shared__ double sh[8];
+  const int q = blockIdx.y;
+  if (done[q]) return;
+  const int j = *step, lane = threadIdx.x & 31;
+  const SplitOp& o = sp[q];
+  double2* csq = cs + (int64_t)q * ncap;
+  double2* ceq = ce + (int64_t)q * ncap;
+  for (int c = blockIdx.x * 8 + (threadIdx.x >> 5); c <= j; c += gridDim.x * 8) {
+    const double2* ps = part + o.pofs + (int64_t)c * o.nslot;
+    const double2* pr = ps + pstride;
+    // independent loads in flight a lane (a large operator has hundreds of
+    // slots and few columns, so few warps carry the whole reduction)
+    double2 a[2], b[2];
+    a[0] = a[1] = b[0] = b[1] = make_double2(0.0, 0.0);
+    int k = lane;
+    for (; k + 32 < o.nslot; k += 64) {
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const double2 v = ps[k + 32 * u], w = pr[k + 32 * u];
+        a[u].x += v.x;
+        a[u].y += v.y;
+        b[u].x += w.x;
+        b[u].y += w.y;
+      }
+    }
+    if (k < o.nslot) {
+      const double2 v = ps[k], w = pr[k];
+      a[0].x += v.x;
+      a[0].y += v.y;
+      b[0].x += w.x;
+      b[0].y += w.y;
+    }
+    const double sx = wsum(a[0].x + a[1].x), sy = wsum(a[0].y + a[1].y);
+    const double rx = wsum(b[0].x + b[1].x), ry = wsum(b[0].y + b[1].y);
+    if (lane == 0) {
+      csq[c] = make_double2(sx, sy);
+      ceq[c] = make_double2(rx, ry);
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();  // this block's sums before its count
+    s_last = atomicAdd(cnt + q, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  double ss = 0.0, hx = 0.0, hy = 0.0;  // |s|^2 and s^H r over the final columns
+  for (int c = threadIdx.x; c < j; c += blockDim.x) {
+    const double2 s = __ldcg(csq + c), r = __ldcg(ceq + c);
+    ss += s.x * s.x + s.y * s.y;
+    hx += s.x * r.x + s.y * r.y;
+    hy += s.x * r.y - s.y * r.x;
+  }
+  ss = bsum256(ss, sh);
+  hx = bsum256(hx, sh);
+  hy = bsum256(hy, sh);
+  const double2 uu = __ldcg(csq + j), uw = __ldcg(ceq + j);
+  double a2 = uu.x - ss;
+  if (a2 < 1e-30 * uu.x) a2 = 1e-30 * uu.x;  // (NaN stays)
+  const double inva = 1.0 / sqrt(a2), gx = (uw.x - hx) / a2, gy = (uw.y - hy) / a2;
+  for (int c = threadIdx.x; c < j; c += blockDim.x) {
+    const double2 s = __ldcg(csq + c), r = __ldcg(ceq + c);
+    ceq[c] = make_double2(r.x - (gx * s.x - gy * s.y), r.y - (gx * s.y + gy * s.x));
+  }
+  if (threadIdx.x == 0) {
+    const double last = j > 0 ? beta[(int64_t)q * m + j - 1] * __ldcg(csq + j - 1).x * inva : 0.0;
+    alpha[(int64_t)q * m + j] = gx - last;
+    scal[q] = make_double4(inva, gx, gy, 0.0);
+    cnt[q] = 0;
+  }
+}
+
+// V_q[:, j] = (V_q[:, j] - V_q cs) / a (final) and w_q = (wt_q - g V_q[:, j] - V_q
+// ce) / a over the block's rows, columns below j, newest first: k_rdots2 has read
+// the newest columns last and reads the oldest first in the next step, so each
+// kernel starts with what the other has left in L2.  A thread holds four rows of
+// both vectors and loads 128 bytes a pass; the coefficients go through shared
+// memory 128 columns at a time.  normpart[slot0_q + slot] = sum |w|^2.
+template <class VV, class WD>
+__global__ void __launch_bounds__(256, kSplitBlocks) k_rupdate2(const BOp* __restrict__ ops, RowSplit rs,
+                                                  int ncap, VV* __restrict__ V,
+                                                  const double2* __restrict__ cs,
+                                                  const double2* __restrict__ ce,
+                                                  const double4* __restrict__ scal,
+                                                  const VV* __restrict__ wt, WD* __restrict__ w,
+                                                  double* __restrict__ normpart,
+                                                  const int* __restrict__ step,
+                                                  const int* __restrict__ done) {
+  constexpr bool CX = IsCx<VV>::v;
+  constexpr int R = 4, U = 128 / (R * (int)sizeof(VV)), CH = 128;
+  static_assert(CH % U == 0, "chunks hold whole passes");
+  __shared__ double2 s_k[CH * (CX ? 2 : 1)];  // real: {cs, ce}; complex: cs, ce
+  __shared__ double s_n[8];
+  const int j = *step, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for_block_rows(ops, rs, [&](int q, const BOp& o, int64_t r0, int64_t r1, int slot, const SplitOp& sq) {
+    if (done[q]) return;
+    const int64_t D = o.D;
+    VV* Vq = V + o.voff;
+    VV* uj = Vq + (int64_t)j * D;
+    const double4 k4 = scal[q];
+    double nrm = 0.0;
+    for (int64_t rb0 = r0; rb0 < r1; rb0 += 256 * R) {
+      const int64_t rb = rb0 + threadIdx.x;
+      const bool full = rb0 + 256 * R <= r1;
+      double2 aq[R], au[R];
+#pragma unroll
+      for (int k = 0; k < R; ++k) {
+        const int64_t r = rb + 256 * k;
+        const bool on = full || r < r1;
+        const double2 u = on ? l2(uj + r) : make_double2(0.0, 0.0);
+        const double2 h = on ? l2(wt + o.woff + r) : make_double2(0.0, 0.0);
+        aq[k] = u;
+        au[k].x = h.x - k4.y * u.x;
+        au[k].y = 0.0;
+        if constexpr (CX) {
+          au[k].x += k4.z * u.y;
+          au[k].y = h.y - (k4.y * u.y + k4.z * u.x);
+        }
+      }
+      for (int c1 = j; c1 > 0; c1 = (c1 - 1) / CH * CH) {  // columns [c0, c1) of one chunk
+        const int c0 = (c1 - 1) / CH * CH;
+        const int npad = (c1 - c0 + U - 1) / U * U;
+        __syncthreads();  // the previous chunk's coefficients are read
+        for (int e = threadIdx.x; e < npad; e += blockDim.x) {
+          const int c = c0 + e;
+          const double2 s = c < c1 ? cs[(int64_t)q * ncap + c] : make_double2(0.0, 0.0);
+          const double2 t = c < c1 ? ce[(int64_t)q * ncap + c] : make_double2(0.0, 0.0);
+          if constexpr (CX) {
+            s_k[2 * e] = s;
+            s_k[2 * e + 1] = t;
+          } else {
+            s_k[e] = make_double2(s.x, t.x);
+          }
+        }
+        __syncthreads();
+        for (int e = npad - U; e >= 0; e -= U) {
+          VV v[U][R];
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const VV* Vc = Vq + (int64_t)min(c0 + e + u, c1 - 1) * D + rb;
+#pragma unroll
+            for (int k = 0; k < R; ++k) v[u][k] = full || rb + 256 * k < r1 ? lv(Vc + 256 * k) : VV{};
+          }
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            if constexpr (CX) {
+              const double2 s = s_k[2 * (e + u)], t = s_k[2 * (e + u) + 1];
+#pragma unroll
+              for (int k = 0; k < R; ++k) {
+                const double2 x = wide(v[u][k]);
+                aq[k].x -= x.x * s.x - x.y * s.y;
+                aq[k].y -= x.x * s.y + x.y * s.x;
+                au[k].x -= x.x * t.x - x.y * t.y;
+                au[k].y -= x.x * t.y + x.y * t.x;
+              }
+            } else {
+              const double2 st = s_k[e + u];
+#pragma unroll
+              for (int k = 0; k < R; ++k) {
+                const double x = wide(v[u][k]).x;
+                aq[k].x -= x * st.x;
+                au[k].x -= x * st.y;
+              }
+            }
+          }
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < R; ++k) {
+        const int64_t r = rb + 256 * k;
+        if (full || r < r1) {
+          s2(uj + r, make_double2(aq[k].x * k4.x, aq[k].y * k4.x));
+          const double2 t = make_double2(au[k].x * k4.x, au[k].y * k4.x);
+          s2(w + o.woff + r, t);
+          nrm += t.x * t.x + (CX ? t.y * t.y : 0.0);
+        }
+      }
+    }
+    nrm = wsum(nrm);
+    __syncthreads();
+    if (lane == 0) s_n[warp] = nrm;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double t = 0.0;
+      for (int k = 0; k < 8; ++k) t += s_n[k];
+      normpart[sq.slot0 + slot] = t;
+    }
+  });
+}
+
+// w_q = the start vector, normpart = sum |w|^2 over the block's rows
+template <class WD>
+__global__ void __launch_bounds__(256) k_rstart(const BOp* __restrict__ ops, RowSplit rs,
+                                                const WD* __restrict__ start, WD* __restrict__ w,
+                                                double* __restrict__ normpart,
+                                                const int* __restrict__ done) {
+  __shared__ double s_n[8];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for_block_rows(ops, rs, [&](int q, const BOp& o, int64_t r0, int64_t r1, int slot, const SplitOp& sq) {
+    if (done[q]) return;
+    double nrm = 0.0;
+    for (int64_t r = r0 + threadIdx.x; r < r1; r += 256) {
+      const double2 v = l2(start + o.woff + r);
+      s2(w + o.woff + r, v);
+      nrm += v.x * v.x + v.y * v.y;
+    }
+    nrm = wsum(nrm);
+    __syncthreads();
+    if (lane == 0) s_n[warp] = nrm;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double t = 0.0;
+      for (int k = 0; k < 8; ++k) t += s_n[k];
+      normpart[sq.slot0 + slot] = t;
+    }
+  });
+}
+
+// per operator: beta_j, breakdown, 1/beta (one block per operator; alpha_j is
+// there already).
 // The last block to finish then closes the step: it splits the rows of the
 // operators still running for the next step's reorthogonalisation kernels
 // and advances the step counter (every block has read it by then).
@@ -664,7 +749,6 @@ __global__ void __launch_bounds__(256) k_bfinish(const BOp* __restrict__ ops, in
                                                  int64_t* __restrict__ TG,
                                                  unsigned* __restrict__ nfinished, int ncap, int m,
                                                  const double* __restrict__ normpart,
-                                                 const double2* __restrict__ coef1,
                                                  double* __restrict__ alpha,
                                                  double* __restrict__ beta,
                                                  double* __restrict__ invb,
@@ -692,8 +776,7 @@ __global__ void __launch_bounds__(256) k_bfinish(const BOp* __restrict__ ops, in
         else invb[q] = 1.0 / nrm;
         alpha[(int64_t)q * m] = nrm;  // for the Krylov driver; step 0 overwrites it
       } else {
-        const double a = coef1[(int64_t)q * ncap + j].x;
-        alpha[(int64_t)q * m + j] = a;
+        const double a = alpha[(int64_t)q * m + j];
         beta[(int64_t)q * m + j] = nrm;
         nsteps[q] = j + 1;
         const double seps = 1.4901161193847656e-08;  // sqrt(eps(Float64))
@@ -804,8 +887,7 @@ struct BatchEngine {
   int64_t ntiles = 0, totalD = 0;
   int G = 1;             // blocks of the reorthogonalisation grid
   int nsm = 1;           // SMs of the device
-  bool fused = false;    // first update and second dot products in one kernel
-  DevBuf dops, tile2op, sblk2op, splitops, splitT, nfin, V, w, wt, part, coef1, coef2, normpart, alpha, beta, invb,
+  DevBuf dops, tile2op, sblk2op, splitops, splitT, nfin, V, w, wt, part, cs, ce, scal, cnt, normpart, alpha, beta, invb,
       done, step, nsteps, cbuf, cnc;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t gexec = nullptr;
@@ -895,13 +977,16 @@ struct BatchEngine {
     EDK_RETURN_IF(w.alloc_async((size_t)totalD * esz(wdt), st));
     EDK_RETURN_IF(wt.alloc_async((size_t)totalD * esz(vdt), st));
     // a block meets at most one operator more than it starts in: G + nops slots
-    EDK_RETURN_IF(part.alloc_async((size_t)(G + nops) * ncap * sizeof(double2), st));
+    EDK_RETURN_IF(part.alloc_async(2 * (size_t)(G + nops) * ncap * sizeof(double2), st));
     EDK_RETURN_IF(splitops.alloc_async((size_t)nops * sizeof(SplitOp), st));
     EDK_RETURN_IF(splitT.alloc_async(2 * sizeof(int64_t), st));
     EDK_RETURN_IF(nfin.alloc_async(sizeof(unsigned), st));
     EDK_TRY_CUDA(cudaMemsetAsync(nfin.p, 0, sizeof(unsigned), st));
-    EDK_RETURN_IF(coef1.alloc_async((size_t)nops * ncap * sizeof(double2), st));
-    EDK_RETURN_IF(coef2.alloc_async((size_t)nops * ncap * sizeof(double2), st));
+    EDK_RETURN_IF(cs.alloc_async((size_t)nops * ncap * sizeof(double2), st));
+    EDK_RETURN_IF(ce.alloc_async((size_t)nops * ncap * sizeof(double2), st));
+    EDK_RETURN_IF(scal.alloc_async((size_t)nops * sizeof(double4), st));
+    EDK_RETURN_IF(cnt.alloc_async((size_t)nops * sizeof(unsigned), st));
+    EDK_TRY_CUDA(cudaMemsetAsync(cnt.p, 0, (size_t)nops * sizeof(unsigned), st));
     EDK_RETURN_IF(normpart.alloc_async((size_t)(G + nops) * sizeof(double), st));
     EDK_RETURN_IF(alpha.alloc_async((size_t)nops * m * sizeof(double), st));
     EDK_RETURN_IF(beta.alloc_async((size_t)nops * m * sizeof(double), st));
@@ -916,16 +1001,13 @@ struct BatchEngine {
     return EDK_OK;
   }
 
-  // Opt the reorthogonalisation kernels into the shared memory they need
-  // (outside any capture) and size their grid to what is resident at once.
+  // Size the reorthogonalisation grid to what is resident at once.
   edk_status split_rows() {
-    const size_t us = (size_t)(ncap + 8) * sizeof(double2);
-    if (us > 200 * 1024) {
+    // (a step's coefficients once sat whole in shared memory; the limit stays)
+    if ((size_t)(ncap + 8) * sizeof(double2) > 200 * 1024) {
       set_error("batch Lanczos: too many steps for the shared-memory coefficients (max 12791)");
       return EDK_UNSUPPORTED;
     }
-    const size_t fs = us + (size_t)ncap * sizeof(double2);  // + column sums
-    fused = fs <= 200 * 1024;
     int dev = 0;
     EDK_TRY_CUDA(cudaGetDevice(&dev));
     EDK_TRY_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
@@ -934,24 +1016,12 @@ struct BatchEngine {
       using VV = std::remove_pointer_t<decltype(vp)>;
       return with_vt(wdt, [&](auto wp) -> edk_status {
         using WD = std::remove_pointer_t<decltype(wp)>;
-        const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-        const auto ku1 = k_rupdate<VV, VV, WD>;
-        const auto ku2 = k_rupdate<VV, WD, WD>;
-        const auto kd1 = k_rdots<VV, VV>;
-        const auto kd2 = k_rdots<VV, WD>;
-        const auto kf = k_rupdate_dots<VV, VV, WD>;
-        if (us > 48 * 1024) {
-          EDK_TRY_CUDA(cudaFuncSetAttribute(ku1, attr, (int)us));
-          EDK_TRY_CUDA(cudaFuncSetAttribute(ku2, attr, (int)us));
-        }
-        if (fused && fs > 48 * 1024) EDK_TRY_CUDA(cudaFuncSetAttribute(kf, attr, (int)fs));
-        int n[5] = {0, 0, 0, 0, 0};
-        EDK_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n[0], ku1, 256, us));
-        EDK_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n[1], ku2, 256, us));
-        EDK_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n[2], kd1, 256, 0));
-        EDK_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n[3], kd2, 256, 0));
-        if (fused) EDK_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n[4], kf, 256, fs));
-        per_sm = std::min({n[0], n[1], fused ? n[4] : n[2], n[2], n[3]});
+        int n[2] = {0, 0};
+        const auto kd = k_rdots2<VV>;
+        const auto ku = k_rupdate2<VV, WD>;
+        EDK_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n[0], kd, 256, 0));
+        EDK_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n[1], ku, 256, 0));
+        per_sm = std::min(n[0], n[1]);
         return EDK_OK;
       });
     });
@@ -1071,67 +1141,31 @@ struct BatchEngine {
   void launch_finish(int setup) {
     k_bfinish<<<nops, 256, 0, st>>>(d_ops(), nops, G, splitops.as<SplitOp>(),
                                     splitT.as<int64_t>(), nfin.as<unsigned>(), ncap, m,
-                                    normpart.as<double>(), coef1.as<double2>(),
-                                    alpha.as<double>(), beta.as<double>(), invb.as<double>(),
+                                    normpart.as<double>(), alpha.as<double>(), beta.as<double>(), invb.as<double>(),
                                     nsteps.as<int>(), step.as<int>(), done.as<int>(), setup);
-  }
-
-  template <class XT>
-  edk_status launch_dots(const XT* x) {
-    return with_vt(vdt, [&](auto vp) -> edk_status {
-      using VV = std::remove_pointer_t<decltype(vp)>;
-      k_rdots<VV, XT><<<(unsigned)G, 256, 0, st>>>(d_ops(), rsplit(), V.as<VV>(), x,
-                                                   part.as<double2>(), step.as<int>(),
-                                                   done.as<int>());
-      return EDK_OK;
-    });
-  }
-
-  template <class WI, class WO>
-  edk_status launch_update(const double2* coef, const WI* win, WO* wout, bool norm, int zero) {
-    const size_t smem = (size_t)(ncap + 8) * sizeof(double2);
-    return with_vt(vdt, [&](auto vp) -> edk_status {
-      using VV = std::remove_pointer_t<decltype(vp)>;
-      k_rupdate<VV, WI, WO><<<(unsigned)G, 256, smem, st>>>(
-          d_ops(), rsplit(), ncap, V.as<VV>(), coef, win, wout,
-          norm ? normpart.as<double>() : nullptr, step.as<int>(), done.as<int>(), zero);
-      return EDK_OK;
-    });
-  }
-
-  template <class WI, class WO>
-  edk_status launch_update_dots(const double2* coef, const WI* win, WO* wout) {
-    const size_t smem = (size_t)(2 * ncap + 8) * sizeof(double2);
-    return with_vt(vdt, [&](auto vp) -> edk_status {
-      using VV = std::remove_pointer_t<decltype(vp)>;
-      k_rupdate_dots<VV, WI, WO><<<(unsigned)G, 256, smem, st>>>(
-          d_ops(), rsplit(), ncap, V.as<VV>(), coef, win, wout, part.as<double2>(),
-          step.as<int>(), done.as<int>());
-      return EDK_OK;
-    });
   }
 
   // one Lanczos step for every live operator (graph-capturable)
   edk_status enqueue_step() {
     EDK_RETURN_IF(launch_apply());
+    const int64_t pst = (int64_t)(G + nops) * ncap;
+    // blocks per operator of the sums: two per SM over all operators
+    const int rx = std::max(1, std::min((ncap + 7) / 8, (2 * nsm + nops - 1) / nops));
     edk_status s = with_vt(vdt, [&](auto vp) -> edk_status {
       using VV = std::remove_pointer_t<decltype(vp)>;
       return with_vt(wdt, [&](auto wp) -> edk_status {
         using WD = std::remove_pointer_t<decltype(wp)>;
-        EDK_RETURN_IF(launch_dots<VV>(wt.as<VV>()));
-        k_breduce<<<dim3((ncap + 7) / 8, nops), 256, 0, st>>>(
-            splitops.as<SplitOp>(), ncap, part.as<double2>(), coef1.as<double2>(), step.as<int>(),
+        k_rdots2<VV><<<(unsigned)G, 256, 0, st>>>(d_ops(), rsplit(), V.as<VV>(), wt.as<VV>(),
+                                                  part.as<double2>(), pst, step.as<int>(),
+                                                  done.as<int>());
+        k_breduce2<<<dim3(rx, nops), 256, 0, st>>>(
+            splitops.as<SplitOp>(), ncap, m, part.as<double2>(), pst, cs.as<double2>(),
+            ce.as<double2>(), scal.as<double4>(), alpha.as<double>(), beta.as<double>(),
+            cnt.as<unsigned>(), step.as<int>(), done.as<int>());
+        k_rupdate2<VV, WD><<<(unsigned)G, 256, 0, st>>>(
+            d_ops(), rsplit(), ncap, V.as<VV>(), cs.as<double2>(), ce.as<double2>(),
+            scal.as<double4>(), wt.as<VV>(), w.as<WD>(), normpart.as<double>(), step.as<int>(),
             done.as<int>());
-        if (fused) {
-          EDK_RETURN_IF((launch_update_dots<VV, WD>(coef1.as<double2>(), wt.as<VV>(), w.as<WD>())));
-        } else {
-          EDK_RETURN_IF((launch_update<VV, WD>(coef1.as<double2>(), wt.as<VV>(), w.as<WD>(), false, 0)));
-          EDK_RETURN_IF(launch_dots<WD>(w.as<WD>()));
-        }
-        k_breduce<<<dim3((ncap + 7) / 8, nops), 256, 0, st>>>(
-            splitops.as<SplitOp>(), ncap, part.as<double2>(), coef2.as<double2>(), step.as<int>(),
-            done.as<int>());
-        EDK_RETURN_IF((launch_update<WD, WD>(coef2.as<double2>(), w.as<WD>(), w.as<WD>(), true, 0)));
         launch_finish(0);
         k_bscale<WD, VV><<<(unsigned)ntiles, 256, 0, st>>>(d_ops(), tile2op.as<int>(), ncap,
                                                            w.as<WD>(), V.as<VV>(),
@@ -1157,8 +1191,9 @@ struct BatchEngine {
       using VV = std::remove_pointer_t<decltype(vp)>;
       return with_vt(wdt, [&](auto wp) -> edk_status {
         using WD = std::remove_pointer_t<decltype(wp)>;
-        EDK_RETURN_IF((launch_update<WD, WD>(coef1.as<double2>(), (const WD*)start_dev,
-                                             w.as<WD>(), true, 1)));
+        k_rstart<WD><<<(unsigned)G, 256, 0, st>>>(d_ops(), rsplit(), (const WD*)start_dev,
+                                                  w.as<WD>(), normpart.as<double>(),
+                                                  done.as<int>());
         launch_finish(1);
         k_bscale<WD, VV><<<(unsigned)ntiles, 256, 0, st>>>(d_ops(), tile2op.as<int>(), ncap,
                                                            w.as<WD>(), V.as<VV>(),
