@@ -544,7 +544,7 @@ bool pauli_strings(const std::vector<HostTerm>& terms, const std::vector<char>& 
 using namespace edk;
 
 edk_operator::~edk_operator() {
-  blas_release(blas);
+  handles_unregister(handles);
   for (cudaEvent_t e : cevents) cudaEventDestroy(e);
   if (cstream) cudaStreamDestroy(cstream);
   if (stream) cudaStreamDestroy(stream);

@@ -709,6 +709,7 @@ static edk_status upload_tables(edk_basis* b, const edk_basis_desc& d, cudaStrea
 using namespace edk;
 
 edk_basis::~edk_basis() {
+  edk::handles_unregister(handles);
   if (stream) cudaStreamDestroy(stream);
 }
 

@@ -540,13 +540,9 @@ static edk_status block_lanczos(int nops, edk_operator* const* ops,
   double2* V = ring1.as<double2>();
   double2* W = ring2.as<double2>();
 
-  // the first operator keeps its handle (creating one costs milliseconds); its
-  // lock is held here
-  struct { cublasHandle_t h; } bh{static_cast<cublasHandle_t>(ops[0]->blas)};
-  if (!bh.h) {
-    EDK_TRY_BLAS(cublasCreate(&bh.h));
-    ops[0]->blas = bh.h;
-  }
+  HandleLease lease;
+  EDK_RETURN_IF(lease.take(ops[0]->handles, false, st));
+  struct { cublasHandle_t h; } bh{static_cast<cublasHandle_t>(lease.h.blas)};
   EDK_TRY_BLAS(cublasSetStream(bh.h, st));
   EDK_TRY_BLAS(cublasSetPointerMode(bh.h, CUBLAS_POINTER_MODE_HOST));
   const cuDoubleComplex one = make_cuDoubleComplex(1.0, 0.0);
@@ -786,10 +782,6 @@ static edk_status block_lanczos(int nops, edk_operator* const* ops,
     diag->seconds_eig = t_eig;
   }
   return EDK_OK;
-}
-
-void blas_release(void* handle) {
-  if (handle) cublasDestroy(static_cast<cublasHandle_t>(handle));
 }
 
 }  // namespace edk

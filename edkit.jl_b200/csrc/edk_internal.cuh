@@ -323,6 +323,7 @@ struct edk_basis {
   bool phase_complex = false;
   bool pairnorm = false;  // TranslationFlipBasis norms on the abelian path
   int device = 0;  // CUDA device the tables live on
+  bool handles = false;  // has borrowed library handles (edk_handles.cu)
   cudaStream_t stream = nullptr;
   std::mutex mu;
   ~edk_basis();
@@ -369,7 +370,7 @@ struct edk_operator {
   std::vector<unsigned char> bop_host;   // the record as last uploaded
   cudaStream_t cstream = nullptr;        // copy stream of the pipelined host path
   std::vector<cudaEvent_t> cevents;      // one per row chunk of that path
-  void* blas = nullptr;                  // cuBLAS handle of the block Lanczos, once it ran
+  bool handles = false;                  // has borrowed library handles (edk_handles.cu)
   std::mutex mu;
   ~edk_operator();
 };
@@ -434,8 +435,23 @@ class KrylovBasis {
   struct Impl;
   std::unique_ptr<Impl> impl;
 };
-// implemented in edk_block.cu
-void blas_release(void* handle);
+// implemented in edk_handles.cu: a cuBLAS (and cuSOLVER) handle borrowed for one
+// call on one stream
+struct LibHandles {
+  void *blas = nullptr, *solver = nullptr;
+};
+struct HandleLease {
+  LibHandles h;
+  int device = 0;
+  cudaStream_t stream = nullptr;
+  HandleLease() = default;
+  HandleLease(const HandleLease&) = delete;
+  HandleLease& operator=(const HandleLease&) = delete;
+  ~HandleLease();
+  // `registered`: the borrowing object's flag (edk_basis / edk_operator handles)
+  edk_status take(bool& registered, bool solver, cudaStream_t st);
+};
+void handles_unregister(bool registered);
 // implemented in edk_util.cpp
 int tridiag_eigvals(int m, const double* a, const double* b, double* w);
 // The lowest `nev` distinct eigenvalues of block-tridiagonal Hermitian

@@ -346,34 +346,25 @@ const char* solver_msg(cusolverStatus_t s) {
     }                                                                                \
   } while (0)
 
-struct Handles {
-  cublasHandle_t blas = nullptr;
-  cusolverDnHandle_t solver = nullptr;
-  ~Handles() {
-    if (blas) cublasDestroy(blas);
-    if (solver) cusolverDnDestroy(solver);
-  }
-};
-
 // Squared singular values of the dA x dB column-major device matrix M_d,
 // descending, into s2 (min(dA, dB) values).
-edk_status gram_spectrum(const void* M_d, bool cm, uint64_t dA, uint64_t dB, cudaStream_t st,
+edk_status gram_spectrum(edk_basis* b, const void* M_d, bool cm, uint64_t dA, uint64_t dB,
                          std::vector<double>& s2) {
+  cudaStream_t st = b->stream;
   const uint64_t n64 = std::min(dA, dB), k64 = std::max(dA, dB);
   EDK_CHECK_ARG(n64 <= 32768, "ent_spec: the smaller side of the Schmidt matrix exceeds 32768");
   EDK_CHECK_ARG(k64 < (1ull << 31), "ent_spec: the larger side of the Schmidt matrix exceeds 2^31");
   const int n = (int)n64, k = (int)k64, lda = (int)dA;
   const bool rows = dA <= dB;  // G = M M^H (dA x dA) or M^H M (dB x dB)
-  Handles h;
-  EDK_TRY_CUBLAS(cublasCreate(&h.blas));
-  EDK_TRY_CUBLAS(cublasSetStream(h.blas, st));
-  EDK_TRY_SOLVER(cusolverDnCreate(&h.solver));
-  EDK_TRY_SOLVER(cusolverDnSetStream(h.solver, st));
+  HandleLease lease;
+  EDK_RETURN_IF(lease.take(b->handles, true, st));
+  struct { cublasHandle_t blas; cusolverDnHandle_t solver; } h{
+      static_cast<cublasHandle_t>(lease.h.blas), static_cast<cusolverDnHandle_t>(lease.h.solver)};
   const size_t es = cm ? 16 : 8;
   DevBuf G, W, info, work;
-  EDK_RETURN_IF(G.alloc((size_t)n * n * es));
-  EDK_RETURN_IF(W.alloc((size_t)n * 8));
-  EDK_RETURN_IF(info.alloc(sizeof(int)));
+  EDK_RETURN_IF(G.alloc_async((size_t)n * n * es, st));
+  EDK_RETURN_IF(W.alloc_async((size_t)n * 8, st));
+  EDK_RETURN_IF(info.alloc_async(sizeof(int), st));
   const double one = 1.0, zero = 0.0;
   int lwork = 0;
   if (cm) {
@@ -383,7 +374,7 @@ edk_status gram_spectrum(const void* M_d, bool cm, uint64_t dA, uint64_t dB, cud
     EDK_TRY_SOLVER(cusolverDnZheevd_bufferSize(h.solver, CUSOLVER_EIG_MODE_NOVECTOR,
                                                CUBLAS_FILL_MODE_LOWER, n, G.as<cuDoubleComplex>(),
                                                n, W.as<double>(), &lwork));
-    EDK_RETURN_IF(work.alloc((size_t)std::max(lwork, 1) * 16));
+    EDK_RETURN_IF(work.alloc_async((size_t)std::max(lwork, 1) * 16, st));
     EDK_TRY_SOLVER(cusolverDnZheevd(h.solver, CUSOLVER_EIG_MODE_NOVECTOR, CUBLAS_FILL_MODE_LOWER,
                                     n, G.as<cuDoubleComplex>(), n, W.as<double>(),
                                     work.as<cuDoubleComplex>(), lwork, info.as<int>()));
@@ -394,7 +385,7 @@ edk_status gram_spectrum(const void* M_d, bool cm, uint64_t dA, uint64_t dB, cud
     EDK_TRY_SOLVER(cusolverDnDsyevd_bufferSize(h.solver, CUSOLVER_EIG_MODE_NOVECTOR,
                                                CUBLAS_FILL_MODE_LOWER, n, G.as<double>(), n,
                                                W.as<double>(), &lwork));
-    EDK_RETURN_IF(work.alloc((size_t)std::max(lwork, 1) * 8));
+    EDK_RETURN_IF(work.alloc_async((size_t)std::max(lwork, 1) * 8, st));
     EDK_TRY_SOLVER(cusolverDnDsyevd(h.solver, CUSOLVER_EIG_MODE_NOVECTOR, CUBLAS_FILL_MODE_LOWER,
                                     n, G.as<double>(), n, W.as<double>(), work.as<double>(),
                                     lwork, info.as<int>()));
@@ -458,15 +449,15 @@ edk_status schmidt_for_spectrum(edk_basis* b, int vdt, const void* v, int32_t nA
   DevBuf dv, dM;
   const void* v_d = v;
   if (ptr_kind == EDK_HOST && b->D > 0) {
-    EDK_RETURN_IF(dv.alloc(vb));
+    EDK_RETURN_IF(dv.alloc_async(vb, st));
     EDK_TRY_CUDA(cudaMemcpyAsync(dv.p, v, vb, cudaMemcpyHostToDevice, st));
     v_d = dv.p;
   }
   const size_t mb = (size_t)(dA * dB) * (cm ? 16 : 8);
-  EDK_RETURN_IF(dM.alloc(mb));
+  EDK_RETURN_IF(dM.alloc_async(mb, st));
   EDK_TRY_CUDA(cudaMemsetAsync(dM.p, 0, mb, st));
   EDK_RETURN_IF(schmidt_device(b, vdt, v_d, tab, dA, cm ? EDK_C128 : EDK_F64, dM.p, st));
-  return gram_spectrum(dM.p, cm, dA, dB, st, s2);
+  return gram_spectrum(b, dM.p, cm, dA, dB, s2);
 }
 
 struct BasisPairLock {
@@ -503,6 +494,7 @@ edk_status check_pair(const edk_basis* b1, const edk_basis* b2) {
 }
 
 }  // namespace
+
 }  // namespace edk
 
 using namespace edk;

@@ -133,6 +133,20 @@ def _merge(mats, inds):
     return M, I
 
 
+_TORCH_TYPES: dict = {}
+
+
+def _torch_types():
+    """torch dtype -> (edk dtype, complex torch dtype, its edk dtype), filled on
+    first use (torch is not imported for numpy-only programs)."""
+    if not _TORCH_TYPES:
+        import torch
+        c128, c64 = (torch.complex128, E.C128), (torch.complex64, E.C64)
+        _TORCH_TYPES.update({torch.float64: (E.F64,) + c128, torch.complex128: (E.C128,) + c128,
+                             torch.float32: (E.F32,) + c64, torch.complex64: (E.C64,) + c64})
+    return _TORCH_TYPES
+
+
 def _vec_dtype(a):
     dt = np.dtype(str(a.dtype).replace("torch.", "")) if hasattr(a, "data_ptr") else a.dtype
     return {np.dtype(np.float64): E.F64, np.dtype(np.complex128): E.C128,
@@ -144,7 +158,7 @@ class Operator:
 
     def __init__(self, M, I, B: AbstractBasis):
         self.M, self.I, self.B = M, I, B
-        lib = E.load()
+        self._lib = lib = E.load()
         nsites, sites, nnz, colptr, rowval, nzval = [], [], [], [], [], []
         for m, ind in zip(M, I):
             m = np.asarray(m, dtype=np.complex128)
@@ -259,22 +273,45 @@ class Operator:
                 E.C64: np.complex64}[dt]
         return np.asfortranarray(x.astype(npdt, copy=False))
 
+    def _mul_tensor(self, x):
+        """H x for a torch tensor.  Small products are bound by this function, so
+        it looks the dtype up once and hands plain integers to ctypes (a product
+        of ten sites, 4.8 us on the GPU: 19.7 us a call through the numpy dtype
+        names and pointer objects, 17.8 us here)."""
+        types = _torch_types().get(x.dtype)
+        if types is None:
+            raise TypeError(f"unsupported vector dtype {x.dtype}")
+        dt = types[0]
+        if self.is_complex and dt != types[2]:
+            x, dt = x.to(types[1]), types[2]
+        shape = x.shape
+        D = self.B._D
+        assert shape[0] == D
+        if len(shape) == 1:
+            if x.stride(0) != 1:
+                x = x.contiguous()
+            y = x.new_empty(D)
+            nvec, ldx, ldy = 1, D, D
+        else:  # torch is row-major: a column-major (transposed) view
+            nvec = shape[1]
+            y = x.new_empty((nvec, D)).t()
+            assert x.stride(0) == 1 and y.stride(0) == 1, "need column-major blocks"
+            ldx, ldy = x.stride(1), y.stride(1)
+        st = self._lib.edk_apply(self._h, dt, x.data_ptr(), y.data_ptr(), nvec, ldx, ldy, 0,
+                                 E.DEVICE if x.is_cuda else E.HOST)
+        if st:
+            E.check(st)
+        return y
+
     def __mul__(self, x):
         """opt * v / opt * m — Operator.jl:372-394 (fresh zeroed output)."""
+        if hasattr(x, "data_ptr"):
+            return self._mul_tensor(x)
         if np.isscalar(x):
             return x * self
         x = self._prep(x)
         dt = self._out_dtype(x)
-        if hasattr(x, "data_ptr"):
-            import torch
-            tdt = {E.F64: torch.float64, E.C128: torch.complex128, E.F32: torch.float32,
-                   E.C64: torch.complex64}[dt]
-            if x.dtype != tdt:
-                x = x.to(tdt)
-            y = torch.empty_like(x) if x.ndim == 1 else torch.empty(
-                (x.shape[1], x.shape[0]), dtype=tdt, device=x.device).t()
-        else:
-            y = np.zeros_like(x, order="F")
+        y = np.zeros_like(x, order="F")
         return self._apply(x, y, False, dt)
 
     __matmul__ = __mul__
