@@ -96,6 +96,37 @@ __global__ void __launch_bounds__(256, plan_min_blocks<BK, VT>())
     plan_row<BK, VT, NN>(b, op, ff, sm, s, xk, yk, accumulate);
 }
 
+// Several columns at once (blockIdx.y = group of kPlanCols columns): a target is
+// located once for all of them.  Taken for eight and more real columns: the
+// gathers themselves, one L1 line each whatever the kernel, are most of the time,
+// so a group pays only where it is full and its rows fill the GPU (whole product,
+// FP64: 8 columns of 400,000 rank-searched rows 113 -> 89 us, 16 of 184,756
+// complete-sector rows 72.8 -> 64.5, 13 single-precision of 48,620 33.5 -> 31.9;
+// but 5 of 48,620 27.8 -> 29.9, and complex columns 112 -> 120).
+constexpr int kPlanCols = 4;
+constexpr int64_t kPlanColsMin = 8;
+
+template <int BK, class VT, int NN, int NC>
+__global__ void __launch_bounds__(256, (sizeof(VT) == 4 && NN == 1) ? 5 : 4)
+    k_apply_plan_cols(BasisDev b, OpDev op, FFParams ff, const VT* __restrict__ x,
+                      VT* __restrict__ y, int64_t ldx, int64_t ldy, int accumulate, int nvec,
+                      int64_t slot0, int64_t slot1) {
+  __shared__ FFTab<BK> sm;
+  ff_tab_fill<BK>(sm, b);
+  __syncthreads();
+  const VT* xk[NC];
+  VT* yk[NC];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const int k = (int)blockIdx.y * NC + c;
+    xk[c] = x + (int64_t)(k < nvec ? k : nvec - 1) * ldx;
+    yk[c] = k < nvec ? y + (int64_t)k * ldy : nullptr;
+  }
+  for (int64_t s = slot0 + (int64_t)blockIdx.x * kPlanWindow + threadIdx.x; s < slot1;
+       s += (int64_t)gridDim.x * kPlanWindow)
+    plan_row_cols<BK, VT, NN, NC>(b, op, ff, sm, s, xk, yk, accumulate);
+}
+
 int sm_count() {
   static int n[64] = {};
   int dev = 0;
@@ -116,6 +147,20 @@ edk_status launch_plan_nn(const BasisDev& b, const OpDev& op, const FFParams& ff
       per_sm = 1;
   }
   const int64_t nwin = (slot1 - slot0) / kPlanWindow;
+  if constexpr (!VTraits<VT>::cx) {
+    if (nvec >= kPlanColsMin) {
+      constexpr int NC = kPlanCols;
+      const unsigned gc = (unsigned)std::min<int64_t>(nwin, (int64_t)sm_count() * 4);
+      for (int64_t k0 = 0; k0 < nvec; k0 += (int64_t)NC * 65535) {
+        const int64_t nk = std::min<int64_t>(nvec - k0, (int64_t)NC * 65535);
+        k_apply_plan_cols<BK, VT, NN, NC>
+            <<<dim3(gc, (unsigned)((nk + NC - 1) / NC)), kPlanWindow, 0, st>>>(
+                b, op, ff, X + k0 * ldx, Y + k0 * ldy, ldx, ldy, accumulate, (int)nk, slot0, slot1);
+        EDK_TRY_CUDA(cudaGetLastError());
+      }
+      return EDK_OK;
+    }
+  }
   const unsigned gx = (unsigned)std::min<int64_t>(nwin, (int64_t)sm_count() * per_sm);
   for (int64_t k0 = 0; k0 < nvec; k0 += 65535) {
     const int64_t nk = std::min<int64_t>(nvec - k0, 65535);

@@ -72,4 +72,102 @@ __device__ __forceinline__ void plan_row(const BasisDev& b, const OpDev& op, con
   ff_row_store<VT>(Y, invRi, dr, di, xk, yk, i, accumulate);
 }
 
+// One slot of the plan applied to NC real columns at once (xk[c], yk[c]): every
+// target is located once, then gathered from each column.  Each column's sums
+// run in plan_row's order with its rounding, so a block and its columns one by
+// one agree bit for bit.
+template <int BK, class VT, int NN, int NC>
+__device__ __forceinline__ void plan_row_cols(const BasisDev& b, const OpDev& op,
+                                              const FFParams& ff, const FFTab<BK>& t, int64_t slot,
+                                              const VT* const (&xk)[NC], VT* const (&yk)[NC],
+                                              int accumulate) {
+  using A = typename VTraits<VT>::A;
+  static_assert(!VTraits<VT>::cx, "real columns");
+  constexpr bool RANKED = BK != BK_PROJ_RANK;
+  constexpr bool CT = BK == BK_TRANS_RANK;
+  constexpr uint32_t TM = FFTabSize<BK>::n - 1;
+  const uint4 e = __ldg(op.plan.slot + slot);
+  const uint32_t rw = e.x;
+  if (rw == ~0u) return;
+  const uint32_t st = e.y, rs = e.z, rkw = e.w, mask = (uint32_t)b.maskL;
+  const int64_t i = (int64_t)(rw & kPlanRowMask);
+  const int L = b.L;
+  const A invRi = BK == BK_PROJ_RANK ? (A)1 : (A)(1.0 / t.coef[rw >> 27].x);
+  Cx<A> Y[NC], S[NC];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) Y[c] = Cx<A>{0, 0};
+  auto adj = [&](int a) -> uint32_t {  // sites a, a + 1: rank change C(a, j)
+    const uint32_t d = t.binom[a * 33 + __popc(st & ((1u << a) - 1u))];
+    return ((st >> a) & 1u) ? rs + d : rs - d;
+  };
+  // up to four hits of target ranks k: S += T x in the order of the hits
+  auto take = [&](const uint32_t (&k)[4], const bool (&on_)[4]) {
+    uint32_t v[4];
+    bool on[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] = RANKED ? __ldg(b.rankmap + k[u]) : k[u];
+    Cx<A> x[4][NC];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      on[u] = on_[u] && (!RANKED || v[u] != ~0u);
+      const int64_t pos = RANKED ? (on[u] ? (int64_t)(v[u] >> b.rank_shift) : 0) : (int64_t)v[u];
+#pragma unroll
+      for (int c = 0; c < NC; ++c) x[u][c] = ldv(xk[c] + pos);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (!on[u]) continue;
+      A tr = 1, ti = 0;
+      if constexpr (RANKED) {
+        const double2 q = t.coef[v[u] & TM];
+        tr = (A)q.x;
+        ti = (A)q.y;
+      }
+#pragma unroll
+      for (int c = 0; c < NC; ++c) acc_t<A, false, CT>(S[c], tr, ti, x[u][c]);
+    }
+  };
+  for (int f = 0; f < (NN == 1 ? 1 : ff.nfam); ++f) {
+    const int d = NN == 1 ? 1 : ff.d[f];
+    uint32_t bits = (st ^ rotl_L(st, d, L, mask)) & ff.valid[f];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) S[c] = Cx<A>{0, 0};
+    while (bits) {
+      uint32_t k[4];
+      bool on[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        on[u] = bits != 0;
+        // (a hit past the row's last one repeats the row itself: not accumulated)
+        const int p = on[u] ? __ffs(bits) - 1 : 0;
+        bits &= bits - 1;
+        if (!on[u]) {
+          k[u] = rs;
+        } else if (d == 1 && p != 0) {
+          k[u] = adj(p - 1);
+        } else if (d == 1 && rkw != ~0u) {
+          k[u] = rkw;
+        } else {
+          k[u] = rank_after_swap(st, rs, p, p >= d ? p - d : p - d + L, t.binom);
+        }
+      }
+      take(k, on);
+    }
+    // (real vectors always see equal exchange values, see ff_row_sum)
+#pragma unroll
+    for (int c = 0; c < NC; ++c) fold_w<A, false>(Y[c], ff.v1[f], S[c]);
+  }
+  double dr = 0.0, di = 0.0;
+  if (op.plan.dg) {
+    dr = __ldg(op.plan.dg + slot);
+  } else {
+    for (int f = 0; f < ff.nfam; ++f)
+      ff_diag(ff, f, st, rotl_L(st, ff.d[f], L, mask), ff.valid[f], dr, di);
+    term_diag(op, st, dr, di);
+  }
+#pragma unroll
+  for (int c = 0; c < NC; ++c)
+    if (yk[c]) ff_row_store<VT>(Y[c], invRi, dr, di, xk[c], yk[c], i, accumulate);
+}
+
 }  // namespace edk
