@@ -912,10 +912,11 @@ struct BatchEngine {
     plan = use_ff && (lookup_kind == BK_TRANS0_RANK || lookup_kind == BK_TRANS_RANK ||
                       lookup_kind == BK_TRANSPAR_RANK || lookup_kind == BK_PROJ_RANK);
     plan_nn_all = plan;
+    for (auto* op : ops) plan = plan && plan_applies(op);
+    plan_nn_all = plan;
+    if (plan) EDK_RETURN_IF(plan_ensure(ops, s));
     for (auto* op : ops) {
       if (!plan) break;
-      if (!plan_applies(op)) { plan = false; break; }
-      EDK_RETURN_IF(plan_ensure(op));
       plan = op->plan_state == 1;
       plan_nn_all = plan_nn_all && plan_nn(*reinterpret_cast<const FFParams*>(op->ff_params.data()));
     }

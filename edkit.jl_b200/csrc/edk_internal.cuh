@@ -68,7 +68,7 @@ struct DevBuf {
     bytes = 0;
     pooled = false;
   }
-  edk_status alloc_async(size_t n, cudaStream_t s);
+  edk_status alloc_async(size_t n, cudaStream_t s, cudaMemPool_t from = nullptr);
   edk_status alloc(size_t n) {
     release();
     if (n == 0) return EDK_OK;
@@ -102,11 +102,11 @@ inline void keep_pool_memory() {
   done[dev] = true;
 }
 
-inline edk_status DevBuf::alloc_async(size_t n, cudaStream_t s) {
+inline edk_status DevBuf::alloc_async(size_t n, cudaStream_t s, cudaMemPool_t from) {
   release();
   if (n == 0) return EDK_OK;
   keep_pool_memory();
-  cudaError_t e = cudaMallocAsync(&p, n, s);
+  cudaError_t e = from ? cudaMallocFromPoolAsync(&p, n, from, s) : cudaMallocAsync(&p, n, s);
   if (e != cudaSuccess) {
     cudaGetLastError();  // an allocation failure is not sticky: clear it for later checks
     p = nullptr;
@@ -118,6 +118,31 @@ inline edk_status DevBuf::alloc_async(size_t n, cudaStream_t s) {
   pool_stream = s;
   pooled = true;
   return EDK_OK;
+}
+
+// The pool of what operators keep (row plans): apart from the default pool, whose
+// free space the solvers' large workspaces need in one piece.  It holds at most
+// 512 MB beyond what is in use.  Null (then the default pool serves) on failure.
+inline cudaMemPool_t keep_pool() {
+  static std::mutex mu;
+  static cudaMemPool_t pools[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+  std::lock_guard<std::mutex> lk(mu);
+  if (!pools[dev]) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    if (cudaMemPoolCreate(&pools[dev], &props) != cudaSuccess) {
+      cudaGetLastError();
+      pools[dev] = nullptr;
+      return nullptr;
+    }
+    uint64_t thr = 512ull << 20;
+    cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &thr);
+  }
+  return pools[dev];
 }
 
 // ---------------------------------------------------------------------------
@@ -348,7 +373,7 @@ struct edk_operator {
   int tps = 1;            // threads per state of the fast path (1, 2 or 4; autotuned)
   // row plan of the fast path on rank-searched sectors (edk_plan.cu): built on
   // first use; plan_state 0 not built, 1 built, -1 not available
-  edk::DevBuf p_slot, p_dg, p_bad;
+  std::shared_ptr<edk::DevBuf> p_slab;  // shared by the operators of the batch that built it
   int plan_state = 0;
   // Pauli-string form (full space, no flip-flop fast path, few enough strings)
   edk::DevBuf pa_group, pa_str, pa_diag;
@@ -388,7 +413,7 @@ edk_status apply_rows(edk_operator* op, int dtype, const void* x, void* y, int64
                       int64_t row1, int accumulate, cudaStream_t st);
 // implemented in edk_plan.cu
 bool plan_applies(const edk_operator* op);
-edk_status plan_ensure(edk_operator* op);
+edk_status plan_ensure(const std::vector<edk_operator*>& ops, cudaStream_t st);
 edk_status apply_plan(edk_operator* op, int dtype, const void* x, void* y, int64_t nvec,
                       int64_t ldx, int64_t ldy, int accumulate, cudaStream_t st, int64_t row0,
                       int64_t row1);

