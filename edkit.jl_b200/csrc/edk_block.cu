@@ -541,7 +541,7 @@ static edk_status block_lanczos(int nops, edk_operator* const* ops,
   double2* W = ring2.as<double2>();
 
   HandleLease lease;
-  EDK_RETURN_IF(lease.take(ops[0]->handles, false, st));
+  EDK_RETURN_IF(lease.take(ops[0]->handles, st));
   struct { cublasHandle_t h; } bh{static_cast<cublasHandle_t>(lease.h.blas)};
   EDK_TRY_BLAS(cublasSetStream(bh.h, st));
   EDK_TRY_BLAS(cublasSetPointerMode(bh.h, CUBLAS_POINTER_MODE_HOST));

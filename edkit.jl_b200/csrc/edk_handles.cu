@@ -41,7 +41,7 @@ HandleLease::~HandleLease() {
 }
 
 // The calls of one lease run on `st`; they are finished when it ends.
-edk_status HandleLease::take(bool& registered, bool solver, cudaStream_t st) {
+edk_status HandleLease::take(bool& registered, cudaStream_t st) {
   stream = st;
   EDK_TRY_CUDA(cudaGetDevice(&device));
   {
@@ -64,7 +64,15 @@ edk_status HandleLease::take(bool& registered, bool solver, cudaStream_t st) {
     }
     h.blas = b;
   }
-  if (solver && !h.solver) {
+  if (cublasSetStream(static_cast<cublasHandle_t>(h.blas), st) != CUBLAS_STATUS_SUCCESS) {
+    set_error("cublasSetStream failed");
+    return EDK_CUDA_ERROR;
+  }
+  return EDK_OK;
+}
+
+edk_status HandleLease::add_solver() {
+  if (!h.solver) {
     cusolverDnHandle_t s = nullptr;
     if (cusolverDnCreate(&s) != CUSOLVER_STATUS_SUCCESS) {
       set_error("cusolverDnCreate failed");
@@ -72,10 +80,9 @@ edk_status HandleLease::take(bool& registered, bool solver, cudaStream_t st) {
     }
     h.solver = s;
   }
-  if (cublasSetStream(static_cast<cublasHandle_t>(h.blas), st) != CUBLAS_STATUS_SUCCESS ||
-      (h.solver && cusolverDnSetStream(static_cast<cusolverDnHandle_t>(h.solver), st) !=
-                       CUSOLVER_STATUS_SUCCESS)) {
-    set_error("setting the stream of a cuBLAS or cuSOLVER handle failed");
+  if (cusolverDnSetStream(static_cast<cusolverDnHandle_t>(h.solver), stream) !=
+      CUSOLVER_STATUS_SUCCESS) {
+    set_error("cusolverDnSetStream failed");
     return EDK_CUDA_ERROR;
   }
   return EDK_OK;

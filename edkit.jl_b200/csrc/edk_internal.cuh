@@ -460,8 +460,10 @@ class KrylovBasis {
   struct Impl;
   std::unique_ptr<Impl> impl;
 };
-// implemented in edk_handles.cu: a cuBLAS (and cuSOLVER) handle borrowed for one
-// call on one stream
+// implemented in edk_eig.cu
+edk_status hermitian_eigvals(bool cx, int n, const void* G, double* W, cudaStream_t st);
+// implemented in edk_handles.cu: a cuBLAS handle (and on request a cuSOLVER one)
+// borrowed for one call on one stream
 struct LibHandles {
   void *blas = nullptr, *solver = nullptr;
 };
@@ -474,7 +476,8 @@ struct HandleLease {
   HandleLease& operator=(const HandleLease&) = delete;
   ~HandleLease();
   // `registered`: the borrowing object's flag (edk_basis / edk_operator handles)
-  edk_status take(bool& registered, bool solver, cudaStream_t st);
+  edk_status take(bool& registered, cudaStream_t st);
+  edk_status add_solver();
 };
 void handles_unregister(bool registered);
 // implemented in edk_util.cpp

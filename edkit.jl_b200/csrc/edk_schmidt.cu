@@ -357,38 +357,48 @@ edk_status gram_spectrum(edk_basis* b, const void* M_d, bool cm, uint64_t dA, ui
   const int n = (int)n64, k = (int)k64, lda = (int)dA;
   const bool rows = dA <= dB;  // G = M M^H (dA x dA) or M^H M (dB x dB)
   HandleLease lease;
-  EDK_RETURN_IF(lease.take(b->handles, true, st));
-  struct { cublasHandle_t blas; cusolverDnHandle_t solver; } h{
-      static_cast<cublasHandle_t>(lease.h.blas), static_cast<cusolverDnHandle_t>(lease.h.solver)};
+  EDK_RETURN_IF(lease.take(b->handles, st));
+  const auto blas = static_cast<cublasHandle_t>(lease.h.blas);
   const size_t es = cm ? 16 : 8;
   DevBuf G, W, info, work;
   EDK_RETURN_IF(G.alloc_async((size_t)n * n * es, st));
   EDK_RETURN_IF(W.alloc_async((size_t)n * 8, st));
   EDK_RETURN_IF(info.alloc_async(sizeof(int), st));
+  EDK_TRY_CUDA(cudaMemsetAsync(info.p, 0, sizeof(int), st));
   const double one = 1.0, zero = 0.0;
-  int lwork = 0;
   if (cm) {
-    EDK_TRY_CUBLAS(cublasZherk(h.blas, CUBLAS_FILL_MODE_LOWER, rows ? CUBLAS_OP_N : CUBLAS_OP_C,
-                               n, k, &one, reinterpret_cast<const cuDoubleComplex*>(M_d), lda,
-                               &zero, G.as<cuDoubleComplex>(), n));
-    EDK_TRY_SOLVER(cusolverDnZheevd_bufferSize(h.solver, CUSOLVER_EIG_MODE_NOVECTOR,
-                                               CUBLAS_FILL_MODE_LOWER, n, G.as<cuDoubleComplex>(),
-                                               n, W.as<double>(), &lwork));
-    EDK_RETURN_IF(work.alloc_async((size_t)std::max(lwork, 1) * 16, st));
-    EDK_TRY_SOLVER(cusolverDnZheevd(h.solver, CUSOLVER_EIG_MODE_NOVECTOR, CUBLAS_FILL_MODE_LOWER,
-                                    n, G.as<cuDoubleComplex>(), n, W.as<double>(),
-                                    work.as<cuDoubleComplex>(), lwork, info.as<int>()));
+    EDK_TRY_CUBLAS(cublasZherk(blas, CUBLAS_FILL_MODE_LOWER, rows ? CUBLAS_OP_N : CUBLAS_OP_C, n, k,
+                               &one, reinterpret_cast<const cuDoubleComplex*>(M_d), lda, &zero,
+                               G.as<cuDoubleComplex>(), n));
   } else {
-    EDK_TRY_CUBLAS(cublasDsyrk(h.blas, CUBLAS_FILL_MODE_LOWER, rows ? CUBLAS_OP_N : CUBLAS_OP_T,
-                               n, k, &one, reinterpret_cast<const double*>(M_d), lda, &zero,
+    EDK_TRY_CUBLAS(cublasDsyrk(blas, CUBLAS_FILL_MODE_LOWER, rows ? CUBLAS_OP_N : CUBLAS_OP_T, n, k,
+                               &one, reinterpret_cast<const double*>(M_d), lda, &zero,
                                G.as<double>(), n));
-    EDK_TRY_SOLVER(cusolverDnDsyevd_bufferSize(h.solver, CUSOLVER_EIG_MODE_NOVECTOR,
-                                               CUBLAS_FILL_MODE_LOWER, n, G.as<double>(), n,
-                                               W.as<double>(), &lwork));
-    EDK_RETURN_IF(work.alloc_async((size_t)std::max(lwork, 1) * 8, st));
-    EDK_TRY_SOLVER(cusolverDnDsyevd(h.solver, CUSOLVER_EIG_MODE_NOVECTOR, CUBLAS_FILL_MODE_LOWER,
-                                    n, G.as<double>(), n, W.as<double>(), work.as<double>(),
-                                    lwork, info.as<int>()));
+  }
+  // matrices that fit the SMs' shared memory, then the library for the larger ones
+  const edk_status own = hermitian_eigvals(cm, n, G.p, W.as<double>(), st);
+  if (own != EDK_OK && own != EDK_UNSUPPORTED) return own;
+  if (own == EDK_UNSUPPORTED) {
+    EDK_RETURN_IF(lease.add_solver());
+    const auto solver = static_cast<cusolverDnHandle_t>(lease.h.solver);
+    int lwork = 0;
+    if (cm) {
+      EDK_TRY_SOLVER(cusolverDnZheevd_bufferSize(solver, CUSOLVER_EIG_MODE_NOVECTOR,
+                                                 CUBLAS_FILL_MODE_LOWER, n,
+                                                 G.as<cuDoubleComplex>(), n, W.as<double>(), &lwork));
+      EDK_RETURN_IF(work.alloc_async((size_t)std::max(lwork, 1) * 16, st));
+      EDK_TRY_SOLVER(cusolverDnZheevd(solver, CUSOLVER_EIG_MODE_NOVECTOR, CUBLAS_FILL_MODE_LOWER, n,
+                                      G.as<cuDoubleComplex>(), n, W.as<double>(),
+                                      work.as<cuDoubleComplex>(), lwork, info.as<int>()));
+    } else {
+      EDK_TRY_SOLVER(cusolverDnDsyevd_bufferSize(solver, CUSOLVER_EIG_MODE_NOVECTOR,
+                                                 CUBLAS_FILL_MODE_LOWER, n, G.as<double>(), n,
+                                                 W.as<double>(), &lwork));
+      EDK_RETURN_IF(work.alloc_async((size_t)std::max(lwork, 1) * 8, st));
+      EDK_TRY_SOLVER(cusolverDnDsyevd(solver, CUSOLVER_EIG_MODE_NOVECTOR, CUBLAS_FILL_MODE_LOWER, n,
+                                      G.as<double>(), n, W.as<double>(), work.as<double>(), lwork,
+                                      info.as<int>()));
+    }
   }
   std::vector<double> w(n);
   int hinfo = 0;

@@ -43,8 +43,8 @@ __device__ __forceinline__ void tri_rescale(double& p0, double& p1) {
 }
 
 // Lowest eigenvalues 0 .. nk-1 of T_q (diagonal alpha + q ld, off-diagonal
-// beta + q ld, order nsteps[q], or nfix[q] > 0 ? nfix[q] : nall when nsteps is
-// null), ascending, into ev + q nk; NaN past the order.
+// beta + q ld, order nsteps[q], or nfix[q] if positive, or nall), ascending, into
+// ev + q nk; NaN past the order.  Blocks along y share a matrix's eigenvalues.
 // With CHECK: matrices whose done[q] is set are left alone, the new values
 // are compared with the ones the previous check left in ev (seen[q] says there
 // are some), done[q] becomes 1 when all nk moved by at most tol max(1, |x|),
@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(kTriThreads) k_tri_lowest(
   __shared__ int s_nle[kTriGroups], s_conv, s_open;
   const int q = blockIdx.x, tid = threadIdx.x;
   if (CHECK && done[q]) return;
-  const int n = nsteps ? nsteps[q] : (nfix[q] > 0 ? nfix[q] : nall);
+  const int n = nsteps ? nsteps[q] : (nfix && nfix[q] > 0 ? nfix[q] : nall);
   if (CHECK && n < nk) {
     if (tid == 0) atomicAdd(left, 1);
     return;
@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(kTriThreads) k_tri_lowest(
   }
   const int G = kTriThreads / groups, g = tid / G, t = tid % G;
   const double step = 1.0 / (G + 1);
-  for (int k0 = 0; k0 < nk; k0 += groups) {
+  for (int k0 = blockIdx.y * groups; k0 < nk; k0 += groups * gridDim.y) {
     const int k = k0 + g;
     const bool mine = ok && k < nk && k < n;
     if (t == 0) {
@@ -209,9 +209,10 @@ edk_status tridiag_check_device(int nops, const double* alpha, const double* bet
 edk_status tridiag_lowest_device(int nops, const double* alpha, const double* beta, int64_t ld,
                                  const int* nsteps, const int* nfix, int nall, int nk, double* ev,
                                  cudaStream_t st) {
-  k_tri_lowest<false><<<nops, kTriThreads, 0, st>>>(alpha, beta, ld, nsteps, nfix, nall, nk,
-                                                    tri_groups(nk), ev, 0.0, nullptr, nullptr,
-                                                    nullptr);
+  const int groups = tri_groups(nk);
+  const dim3 grid((unsigned)nops, (unsigned)std::min(65535, (nk + groups - 1) / groups));
+  k_tri_lowest<false><<<grid, kTriThreads, 0, st>>>(alpha, beta, ld, nsteps, nfix, nall, nk, groups,
+                                                    ev, 0.0, nullptr, nullptr, nullptr);
   EDK_TRY_CUDA(cudaGetLastError());
   return EDK_OK;
 }
