@@ -6,7 +6,7 @@
 // only when T has more eigenvalues in a small window around it than T-hat (T
 // without its first block row and column) — the Cullum-Willoughby test
 // generalised to blocks, with exact counts from block Sturm (inertia)
-// sequences.  All operators' T run together: a Lanczos step is six
+// sequences.  All operators' T run together: a Lanczos step is four
 // launches over every operator, and every Sturm count is one thread block.
 #include <algorithm>
 #include <cmath>
@@ -83,11 +83,16 @@ __global__ void k_band_mv(BandDims d, const double2* __restrict__ A, const doubl
   w[(size_t)q * d.nmax + (size_t)jb * p + a] = make_double2((yr + lo.x) + up.x, (yi + lo.y) + up.y);
 }
 
-// s[q][c] = V_q[:, c]^H w_q for c <= k: one warp per (column, operator)
+// The step orthogonalises twice with two passes over V, as the batched Lanczos
+// does (k_rdots2 in edk_batch.cu): V[:, k] arrives after one sweep, its second
+// sweep shares the passes of the next vector's first.
+//
+// s[q][c] = V_q[:, c]^H V_q[:, k] and r[q][c] = V_q[:, c]^H w_q for c <= k: one
+// warp per (column, operator)
 __global__ void __launch_bounds__(256) k_band_dots(BandDims d, const int* __restrict__ nq,
                                                    const double2* __restrict__ V, int k,
                                                    const double2* __restrict__ w,
-                                                   double2* __restrict__ s,
+                                                   double2* __restrict__ s, double2* __restrict__ r,
                                                    const int* __restrict__ stop) {
   const int q = blockIdx.y;
   const int c = blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -95,71 +100,121 @@ __global__ void __launch_bounds__(256) k_band_dots(BandDims d, const int* __rest
   const int lane = threadIdx.x & 31;
   const int64_t n = nq[q];
   const double2* v = V + ((size_t)q * d.vcols + c) * d.nmax;
+  const double2* u = V + ((size_t)q * d.vcols + k) * d.nmax;
   const double2* x = w + (size_t)q * d.nmax;
-  double sr[4] = {0.0, 0.0, 0.0, 0.0}, si[4] = {0.0, 0.0, 0.0, 0.0};
-  int64_t i = lane;
-  for (; i + 96 < n; i += 128) {
+  double f[2][4] = {};  // two rows in flight; s, r (real and imaginary parts)
+#pragma unroll 2
+  for (int64_t i = lane; i < n; i += 64) {
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const double2 a = v[i + 32 * u], b = x[i + 32 * u];
-      sr[u] += a.x * b.x + a.y * b.y;
-      si[u] += a.x * b.y - a.y * b.x;
+    for (int e = 0; e < 2; ++e) {
+      if (i + 32 * e >= n) break;
+      const double2 a = v[i + 32 * e], b = u[i + 32 * e], y = x[i + 32 * e];
+      f[e][0] += a.x * b.x + a.y * b.y;
+      f[e][1] += a.x * b.y - a.y * b.x;
+      f[e][2] += a.x * y.x + a.y * y.y;
+      f[e][3] += a.x * y.y - a.y * y.x;
     }
   }
-  for (; i < n; i += 32) {
-    const double2 a = v[i], b = x[i];
-    sr[0] += a.x * b.x + a.y * b.y;
-    si[0] += a.x * b.y - a.y * b.x;
+  double t[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) t[e] = bwsum(f[0][e] + f[1][e]);
+  if (lane == 0) {
+    s[(size_t)q * d.vcols + c] = make_double2(t[0], t[1]);
+    r[(size_t)q * d.vcols + c] = make_double2(t[2], t[3]);
   }
-  const double r = bwsum((sr[0] + sr[1]) + (sr[2] + sr[3]));
-  const double im = bwsum((si[0] + si[1]) + (si[2] + si[3]));
-  if (lane == 0) s[(size_t)q * d.vcols + c] = make_double2(r, im);
 }
 
-// w_q -= V_q[:, 0:k+1] s_q: a block takes 32 rows, its eight warps every eighth
-// column each, and the warps' sums meet in shared memory.  (One thread per row
-// leaves four blocks per operator at order 960 and a serial walk over all
-// columns: 21.6 us a launch over runs of order 160 to 960, 18 operators; this one
-// 12.3 us over the run of order 960, up to 280 columns.)
+// With a^2 = s_k - sum |s_c|^2 and g = (r_k - s^H r) / a^2 (sums over c < k):
+// V[:, k] = (V[:, k] - V s) / a, final, and w = (w - V r - g (V[:, k] - V s)) / a,
+// alpha_k = Re(g - beta_{k-1} s_{k-1} / a).  A block takes 32 rows, its eight warps
+// every eighth column each, and the warps' sums meet in shared memory; every block
+// adds up a and g for itself.  (One thread per row leaves four blocks per operator
+// at order 960 and a serial walk over all columns.)  18 operators, the run of order
+// 960, up to 280 columns: two sweeps of their own took 2 x (11.8 + 12.3) us a
+// step, this 13.3 + 12.4.
 __global__ void __launch_bounds__(256) k_band_update(BandDims d, const int* __restrict__ nq,
-                                                     const double2* __restrict__ V, int k,
+                                                     double2* __restrict__ V, int k,
                                                      const double2* __restrict__ s,
+                                                     const double2* __restrict__ r,
                                                      double2* __restrict__ w,
+                                                     double* __restrict__ alpha,
+                                                     const double* __restrict__ beta,
                                                      const int* __restrict__ stop) {
-  __shared__ double2 sum[8][32];
+  __shared__ double2 sum[2][8][32];
+  __shared__ double red[8][3];
   const int q = blockIdx.y;
   if (stop[q]) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t i = (int64_t)blockIdx.x * 32 + lane;
   const bool on = i < nq[q];
-  const double2* v = V + (size_t)q * d.vcols * d.nmax + (on ? i : 0);
-  const double2* t = s + (size_t)q * d.vcols;
-  double ar = 0.0, ai = 0.0;
-#pragma unroll 4
-  for (int c = warp; c <= k; c += 8) {
-    const double2 x = v[(size_t)c * d.nmax], y = t[c];
-    ar += x.x * y.x - x.y * y.y;
-    ai += x.x * y.y + x.y * y.x;
+  const double2* sq = s + (size_t)q * d.vcols;
+  const double2* rq = r + (size_t)q * d.vcols;
+  double ss = 0.0, hx = 0.0, hy = 0.0;
+  for (int c = threadIdx.x; c < k; c += 256) {
+    const double2 a = sq[c], b = rq[c];
+    ss += a.x * a.x + a.y * a.y;
+    hx += a.x * b.x + a.y * b.y;
+    hy += a.x * b.y - a.y * b.x;
   }
-  sum[warp][lane] = make_double2(ar, ai);
+  ss = bwsum(ss);
+  hx = bwsum(hx);
+  hy = bwsum(hy);
+  if (lane == 0) {
+    red[warp][0] = ss;
+    red[warp][1] = hx;
+    red[warp][2] = hy;
+  }
+  double2* v = V + (size_t)q * d.vcols * d.nmax + (on ? i : 0);
+  double2 as = make_double2(0.0, 0.0), ar = make_double2(0.0, 0.0);
+#pragma unroll 4
+  for (int c = warp; c < k; c += 8) {
+    const double2 x = v[(size_t)c * d.nmax], y = sq[c], z = rq[c];
+    as.x += x.x * y.x - x.y * y.y;
+    as.y += x.x * y.y + x.y * y.x;
+    ar.x += x.x * z.x - x.y * z.y;
+    ar.y += x.x * z.y + x.y * z.x;
+  }
+  sum[0][warp][lane] = as;
+  sum[1][warp][lane] = ar;
   __syncthreads();
-  if (warp != 0 || !on) return;
+  if (warp != 0) return;
+  ss = hx = hy = 0.0;
+#pragma unroll
+  for (int u = 0; u < 8; ++u) {
+    ss += red[u][0];
+    hx += red[u][1];
+    hy += red[u][2];
+  }
+  const double2 uu = sq[k], uw = rq[k];
+  double a2 = uu.x - ss;
+  if (a2 < 1e-30 * uu.x) a2 = 1e-30 * uu.x;  // (NaN stays)
+  const double inva = 1.0 / sqrt(a2), gx = (uw.x - hx) / a2, gy = (uw.y - hy) / a2;
+  if (blockIdx.x == 0 && lane == 0)
+    alpha[(size_t)q * d.vcols + k] =
+        gx - (k > 0 ? beta[(size_t)q * d.vcols + k - 1] * sq[k - 1].x * inva : 0.0);
+  if (!on) return;
 #pragma unroll
   for (int u = 1; u < 8; ++u) {
-    ar += sum[u][lane].x;
-    ai += sum[u][lane].y;
+    as.x += sum[0][u][lane].x;
+    as.y += sum[0][u][lane].y;
+    ar.x += sum[1][u][lane].x;
+    ar.y += sum[1][u][lane].y;
   }
+  double2* vk = v + (size_t)k * d.nmax;
   double2* wi = w + (size_t)q * d.nmax + i;
-  *wi = make_double2(wi->x - ar, wi->y - ai);
+  const double2 t = *vk, y = *wi;
+  const double2 p = make_double2(t.x - as.x, t.y - as.y);
+  *vk = make_double2(p.x * inva, p.y * inva);
+  *wi = make_double2((y.x - ar.x - (gx * p.x - gy * p.y)) * inva,
+                     (y.y - ar.y - (gx * p.y + gy * p.x)) * inva);
 }
 
-// alpha_k (the first sweep's s_k), beta_k = |w| and v_{k+1} = w / beta (one block
-// per operator); a negligible beta (the host form's rule b < 1e-12 max(1, |a|))
-// stops the operator with k + 1 steps, recorded in stop[q]
+// beta_k = |w| and v_{k+1} = w / beta, after one sweep (one block per operator); a
+// negligible beta (the host form's rule b < 1e-12 max(1, |a|)) stops the operator
+// with k + 1 steps, recorded in stop[q]
 __global__ void __launch_bounds__(1024) k_band_next(BandDims d, const int* __restrict__ nq, int k,
                                                     const double2* __restrict__ w,
-                                                    const double2* __restrict__ s1,
-                                                    double* __restrict__ alpha,
+                                                    const double* __restrict__ alpha,
                                                     double* __restrict__ beta,
                                                     double2* __restrict__ V,
                                                     int* __restrict__ stop) {
@@ -174,10 +229,9 @@ __global__ void __launch_bounds__(1024) k_band_next(BandDims d, const int* __res
   if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = t;
   __syncthreads();
   const double n2 = bwsum(sh[threadIdx.x & 31]);
-  const double a = s1[(size_t)q * d.vcols + k].x, b = sqrt(n2);
+  const double a = alpha[(size_t)q * d.vcols + k], b = sqrt(n2);
   const bool end = b < 1e-12 * fmax(1.0, fabs(a));
   if (threadIdx.x == 0) {
-    alpha[(size_t)q * d.vcols + k] = a;
     beta[(size_t)q * d.vcols + k] = b;
     if (end) stop[q] = k + 1;
   }
@@ -317,12 +371,41 @@ __global__ void __launch_bounds__(256) k_band_sturm(BandDims d, const double2* _
   if (tid == 0) counts[blockIdx.x] = s_neg;
 }
 
+// T's blocks as the kernels read them, from the block Lanczos's per-step products:
+// SA[j][q] is (V_j^H W)^T column-major, so A_j(r, c) = SA[c + r p], made Hermitian;
+// SB[j][q] is B_j already.  diag[q] is the largest |A_j(a, a)| over all j, and over
+// j >= 1 in diag[nops + q] (at least one), as the bits of non-negative doubles.
+__global__ void __launch_bounds__(256) k_band_pack(BandDims d, int nops,
+                                                   const double2* __restrict__ SA,
+                                                   const double2* __restrict__ SB,
+                                                   const int* __restrict__ mq,
+                                                   double2* __restrict__ A, double2* __restrict__ B,
+                                                   unsigned long long* __restrict__ diag) {
+  const int q = blockIdx.y, j = blockIdx.x, p = d.p, pp = p * p;
+  if (j >= mq[q]) return;
+  const double2* a1 = SA + ((size_t)j * nops + q) * pp;
+  const double2* b1 = SB + ((size_t)j * nops + q) * pp;
+  double2* ao = A + ((size_t)q * d.mmax + j) * pp;
+  double2* bo = B + ((size_t)q * d.mmax + j) * pp;
+  for (int e = threadIdx.x; e < pp; e += blockDim.x) {
+    const int r = e % p, c = e / p;
+    const double2 x = a1[c + r * p], y = a1[r + c * p];  // A(r, c), A(c, r)
+    const double2 h = make_double2(0.5 * (x.x + y.x), 0.5 * (x.y - y.y));
+    ao[e] = h;
+    if (j >= 1) bo[e] = b1[e];
+    if (r == c) {
+      const unsigned long long v = (unsigned long long)__double_as_longlong(fmax(1.0, fabs(h.x)));
+      atomicMax(diag + q, v);
+      if (j >= 1) atomicMax(diag + nops + q, v);
+    }
+  }
+}
+
 }  // namespace
 
-edk_status band_lowest_device(int p, int nev, const std::vector<int>& m,
-                              const std::vector<std::vector<const double*>>& A,
-                              const std::vector<std::vector<const double*>>& B,
-                              cudaStream_t st, std::vector<std::vector<double>>& out) {
+edk_status band_lowest_device(int p, int nev, const std::vector<int>& m, const void* SA,
+                              const void* SB, cudaStream_t st,
+                              std::vector<std::vector<double>>& out) {
   const int nops = (int)m.size();
   out.assign(nops, std::vector<double>(nev, NAN));
   if (nops == 0) return EDK_OK;
@@ -337,22 +420,12 @@ edk_status band_lowest_device(int p, int nev, const std::vector<int>& m,
   const int kmax = (int)std::min<int64_t>(d.nmax, kBandSteps);
   d.vcols = kmax + 1;
   const size_t pp = (size_t)p * p;
-  // T's blocks on the device
-  std::vector<double2> hAB((size_t)nops * d.mmax * pp);
-  DevBuf dA, dB, V, w, s1, s2, alpha, beta, stop, nq, mqd;
-  EDK_RETURN_IF(dA.alloc_async(hAB.size() * sizeof(double2), st));
-  EDK_RETURN_IF(dB.alloc_async(hAB.size() * sizeof(double2), st));
-  for (int pass = 0; pass < 2; ++pass) {
-    std::fill(hAB.begin(), hAB.end(), make_double2(0.0, 0.0));
-    for (int q = 0; q < nops; ++q)
-      for (int j = 0; j < m[q]; ++j) {
-        const double* src = pass == 0 ? A[q][j] : (j >= 1 ? B[q][j] : nullptr);
-        if (src) std::memcpy(&hAB[((size_t)q * d.mmax + j) * pp], src, pp * sizeof(double2));
-      }
-    EDK_TRY_CUDA(cudaMemcpyAsync(pass == 0 ? dA.p : dB.p, hAB.data(), hAB.size() * sizeof(double2),
-                                 cudaMemcpyHostToDevice, st));
-    EDK_TRY_CUDA(cudaStreamSynchronize(st));  // hAB is refilled next pass
-  }
+  DevBuf dA, dB, dmax, V, w, s1, s2, alpha, beta, stop, nq, mqd;
+  const size_t ab = (size_t)nops * d.mmax * pp * sizeof(double2);
+  EDK_RETURN_IF(dA.alloc_async(ab, st));
+  EDK_RETURN_IF(dB.alloc_async(ab, st));
+  EDK_RETURN_IF(dmax.alloc_async(2 * (size_t)nops * 8, st));
+  EDK_TRY_CUDA(cudaMemsetAsync(dmax.p, 0, 2 * (size_t)nops * 8, st));
   std::vector<int> hn(nops);
   for (int q = 0; q < nops; ++q) hn[q] = p * m[q];
   EDK_RETURN_IF(V.alloc_async((size_t)nops * d.vcols * d.nmax * sizeof(double2), st));
@@ -366,6 +439,12 @@ edk_status band_lowest_device(int p, int nev, const std::vector<int>& m,
   EDK_RETURN_IF(mqd.alloc_async((size_t)nops * sizeof(int), st));
   EDK_TRY_CUDA(cudaMemcpyAsync(nq.p, hn.data(), nops * sizeof(int), cudaMemcpyHostToDevice, st));
   EDK_TRY_CUDA(cudaMemcpyAsync(mqd.p, m.data(), nops * sizeof(int), cudaMemcpyHostToDevice, st));
+  k_band_pack<<<dim3(d.mmax, nops), 256, 0, st>>>(
+      d, nops, static_cast<const double2*>(SA), static_cast<const double2*>(SB), mqd.as<int>(),
+      dA.as<double2>(), dB.as<double2>(), dmax.as<unsigned long long>());
+  EDK_TRY_CUDA(cudaGetLastError());
+  std::vector<double> hmax(2 * (size_t)nops);
+  EDK_TRY_CUDA(cudaMemcpyAsync(hmax.data(), dmax.p, hmax.size() * 8, cudaMemcpyDeviceToHost, st));
   EDK_TRY_CUDA(cudaMemsetAsync(stop.p, 0, nops * sizeof(int), st));
   EDK_TRY_CUDA(cudaMemsetAsync(V.p, 0, (size_t)nops * d.vcols * d.nmax * sizeof(double2), st));
   // start vectors: the host form's seeded sequence, normalised, in column 0
@@ -410,16 +489,15 @@ edk_status band_lowest_device(int p, int nev, const std::vector<int>& m,
     k_band_mv<<<dim3((d.mmax + G - 1) / G, nops), 3 * G * p, 6 * G * p * sizeof(double2), st>>>(
         d, dA.as<double2>(), dB.as<double2>(), mqd.as<int>(), V.as<double2>(), k, w.as<double2>(),
         stop.as<int>());
-    for (int pass = 0; pass < 2; ++pass) {
-      double2* s = pass == 0 ? s1.as<double2>() : s2.as<double2>();
-      k_band_dots<<<dim3((k + 8) / 8, nops), 256, 0, st>>>(d, nq.as<int>(), V.as<double2>(), k,
-                                                          w.as<double2>(), s, stop.as<int>());
-      k_band_update<<<dim3(rows, nops), 256, 0, st>>>(d, nq.as<int>(), V.as<double2>(), k, s,
-                                                      w.as<double2>(), stop.as<int>());
-    }
-    k_band_next<<<nops, 1024, 0, st>>>(d, nq.as<int>(), k, w.as<double2>(), s1.as<double2>(),
-                                       alpha.as<double>(), beta.as<double>(), V.as<double2>(),
-                                       stop.as<int>());
+    k_band_dots<<<dim3((k + 8) / 8, nops), 256, 0, st>>>(d, nq.as<int>(), V.as<double2>(), k,
+                                                        w.as<double2>(), s1.as<double2>(),
+                                                        s2.as<double2>(), stop.as<int>());
+    k_band_update<<<dim3(rows, nops), 256, 0, st>>>(d, nq.as<int>(), V.as<double2>(), k,
+                                                    s1.as<double2>(), s2.as<double2>(),
+                                                    w.as<double2>(), alpha.as<double>(),
+                                                    beta.as<double>(), stop.as<int>());
+    k_band_next<<<nops, 1024, 0, st>>>(d, nq.as<int>(), k, w.as<double2>(), alpha.as<double>(),
+                                       beta.as<double>(), V.as<double2>(), stop.as<int>());
     EDK_TRY_CUDA(cudaGetLastError());
     bool look = (k + 1) % 10 == 0 || k + 1 == kmax;
     for (int q = 0; q < nops && !look; ++q)
@@ -491,12 +569,8 @@ edk_status band_lowest_device(int p, int nev, const std::vector<int>& m,
   std::vector<BandTask> tasks;
   for (int q = 0; q < nops; ++q) {
     double tiny[2];
-    for (int j0 = 0; j0 < 2; ++j0) {
-      double scale = 1.0;
-      for (int j = j0; j < m[q]; ++j)
-        for (int a = 0; a < p; ++a) scale = std::max(scale, std::fabs(A[q][j][2 * ((size_t)a * p + a)]));
-      tiny[j0] = 1e-300 + 1e-15 * scale;
-    }
+    for (int j0 = 0; j0 < 2; ++j0)
+      tiny[j0] = 1e-300 + 1e-15 * std::max(1.0, hmax[(size_t)j0 * nops + q]);
     const std::vector<double>& c = cand[q];
     for (size_t i = 0; i < c.size();) {
       const double lo = c[i], dl = 1e-10 * std::max(1.0, std::fabs(lo));

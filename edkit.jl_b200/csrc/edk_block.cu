@@ -30,9 +30,7 @@
 #include <algorithm>
 #include <chrono>
 #include <cmath>
-#include <complex>
 #include <cstring>
-#include <thread>
 #include <vector>
 
 #include "edk_spmm.cuh"
@@ -40,8 +38,6 @@
 namespace edk {
 
 namespace {
-
-using cplx = std::complex<double>;
 
 double wall_s() {
   return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch())
@@ -72,22 +68,31 @@ __global__ void k_cols_to_rows(const double2* __restrict__ src, double2* __restr
 // ---------------------------------------------------------------------------
 // small dense kernels
 // ---------------------------------------------------------------------------
-// out[q] = sum over S chunks of part[q * S + s] (p x p each)
-__global__ void k_sum_chunks(const double2* __restrict__ part, double2* __restrict__ out,
-                             int nops, int S, int pp) {
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < (int64_t)nops * pp;
-       e += (int64_t)gridDim.x * blockDim.x) {
-    const int q = (int)(e / pp);
-    const int k = (int)(e - (int64_t)q * pp);
-    double sr = 0.0, si = 0.0;
-    const double2* src = part + (int64_t)q * S * pp + k;
-    for (int s = 0; s < S; ++s) {
-      const double2 v = src[(int64_t)s * pp];
-      sr += v.x;
-      si += v.y;
-    }
-    out[e] = make_double2(sr, si);
+// out[q] = sum over S chunks of part[q * S + s] (p x p each): 32 elements a
+// block, its eight warps every eighth chunk each
+__global__ void __launch_bounds__(256) k_sum_chunks(const double2* __restrict__ part,
+                                                    double2* __restrict__ out, int S, int pp) {
+  __shared__ double2 sh[8][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t e = (int64_t)blockIdx.x * 32 + lane;  // p is a multiple of 8: whole blocks
+  const int64_t q = e / pp;
+  const double2* src = part + q * S * pp + (e - q * pp);
+  double sr = 0.0, si = 0.0;
+#pragma unroll 4
+  for (int s = warp; s < S; s += 8) {
+    const double2 v = src[(int64_t)s * pp];
+    sr += v.x;
+    si += v.y;
   }
+  sh[warp][lane] = make_double2(sr, si);
+  __syncthreads();
+  if (warp != 0) return;
+#pragma unroll
+  for (int u = 1; u < 8; ++u) {
+    sr += sh[u][lane].x;
+    si += sh[u][lane].y;
+  }
+  out[e] = make_double2(sr, si);
 }
 
 // splitmix64 finaliser: a counter-based stream of 64-bit words
@@ -518,15 +523,22 @@ static edk_status block_lanczos(int nops, edk_operator* const* ops,
     }
   }
 
-  DevBuf d_ops, ring0, ring1, ring2, part, Q1, Q2, G, Rinv, R1, R2, Bm, flags, colx, coly;
+  DevBuf d_ops, ring0, ring1, ring2, part, Q2, G, Rinv, R1, R2, SA, SB, flags, SF, colx, coly;
   EDK_RETURN_IF(d_ops.alloc_async(sizeof(SpmmOp) * nops, st));
   EDK_RETURN_IF(ring0.alloc_async(slot * sizeof(double2), st));
   EDK_RETURN_IF(ring1.alloc_async(slot * sizeof(double2), st));
   EDK_RETURN_IF(ring2.alloc_async(slot * sizeof(double2), st));
   EDK_RETURN_IF(part.alloc_async((size_t)nops * S * pp * sizeof(double2), st));
-  for (DevBuf* bf : {&Q1, &Q2, &G, &Rinv, &R1, &R2, &Bm})
+  for (DevBuf* bf : {&Q2, &G, &Rinv, &R1, &R2})
     EDK_RETURN_IF(bf->alloc_async((size_t)nops * pp * sizeof(double2), st));
+  // every step's A_j (transposed) and B_j, and the rank flags after it, stay on the
+  // device for the eigenvalue step
+  const int m = o.max_steps;
+  const size_t npp = (size_t)nops * pp;
+  EDK_RETURN_IF(SA.alloc_async((size_t)m * npp * sizeof(double2), st));
+  EDK_RETURN_IF(SB.alloc_async((size_t)(m + 1) * npp * sizeof(double2), st));
   EDK_RETURN_IF(flags.alloc_async(nops * sizeof(int), st));
+  EDK_RETURN_IF(SF.alloc_async((size_t)m * nops * sizeof(int), st));
   if (any_generic) {
     EDK_RETURN_IF(colx.alloc_async((size_t)Dmax * p * sizeof(double2), st));
     EDK_RETURN_IF(coly.alloc_async((size_t)Dmax * p * sizeof(double2), st));
@@ -558,8 +570,8 @@ static edk_status block_lanczos(int nops, edk_operator* const* ops,
         reinterpret_cast<const cuDoubleComplex*>(Xs), p, Kc * p,
         reinterpret_cast<const cuDoubleComplex*>(Ys), p, Kc * p, &zero, C(part.as<double2>()), p,
         pp, (int)(nops * S)));
-    k_sum_chunks<<<grid_for((int64_t)nops * pp), 256, 0, st>>>(part.as<double2>(), out, nops,
-                                                                (int)S, pp);
+    k_sum_chunks<<<(unsigned)((int64_t)nops * pp / 32), 256, 0, st>>>(
+        part.as<double2>(), out, (int)S, pp);
     EDK_TRY_CUDA(cudaGetLastError());
     return EDK_OK;
   };
@@ -585,8 +597,8 @@ static edk_status block_lanczos(int nops, edk_operator* const* ops,
   EDK_TRY_CUDA(cudaFuncSetAttribute(k_chol, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)chol_smem));
   // Cholesky-QR twice: X (in slot W) = Q B; Q lands back in W, `spare` is
-  // overwritten; B in Bm
-  auto cholqr = [&](double2* Wx, double2* spare) -> edk_status {
+  // overwritten; B to Bm
+  auto cholqr = [&](double2* Wx, double2* spare, double2* Bm) -> edk_status {
     EDK_RETURN_IF(gram(Wx, Wx, G.as<double2>()));
     k_chol<<<nops, 256, chol_smem, st>>>(G.as<double2>(), p, Rinv.as<double2>(),
                                          R1.as<double2>(), nullptr, nullptr, flags.as<int>(), 1);
@@ -594,22 +606,22 @@ static edk_status block_lanczos(int nops, edk_operator* const* ops,
     EDK_RETURN_IF(rmul(Wx, spare));
     EDK_RETURN_IF(gram(spare, spare, G.as<double2>()));
     k_chol<<<nops, 256, chol_smem, st>>>(G.as<double2>(), p, Rinv.as<double2>(),
-                                         R2.as<double2>(), R1.as<double2>(), Bm.as<double2>(),
+                                         R2.as<double2>(), R1.as<double2>(), Bm,
                                          flags.as<int>(), 2);
     EDK_TRY_CUDA(cudaGetLastError());
     EDK_RETURN_IF(rmul(spare, Wx));
     return EDK_OK;
   };
 
+  // The host looks at the rank flags every kLook steps; the steps in between are
+  // enqueued without a round trip (one per step left the GPU idle for 50 us).
+  constexpr int kLook = 8;
   float t_spmm = 0.f, t_orth = 0.f;
-  cudaEvent_t e0, e1, e2;
-  EDK_TRY_CUDA(cudaEventCreate(&e0));
-  EDK_TRY_CUDA(cudaEventCreate(&e1));
-  EDK_TRY_CUDA(cudaEventCreate(&e2));
-  struct EvGuard {
-    cudaEvent_t a, b, c;
-    ~EvGuard() { cudaEventDestroy(a); cudaEventDestroy(b); cudaEventDestroy(c); }
-  } evg{e0, e1, e2};
+  struct Events {
+    cudaEvent_t e[3 * kLook] = {};
+    ~Events() { for (cudaEvent_t x : e) if (x) cudaEventDestroy(x); }
+  } evs;
+  for (cudaEvent_t& x : evs.e) EDK_TRY_CUDA(cudaEventCreate(&x));
 
   auto spmm = [&](const double2* X, double2* Y) -> edk_status {
     EDK_RETURN_IF(launch_spmm<double2>(d_ops.as<SpmmOp>(), nops, bk_ff, smax, Dpad, p, X, Y, 0,
@@ -653,106 +665,79 @@ static edk_status block_lanczos(int nops, edk_operator* const* ops,
                                                                       Dpad, p, o.seed, W);
     EDK_TRY_CUDA(cudaGetLastError());
   }
-  EDK_RETURN_IF(cholqr(W, U));
+  EDK_RETURN_IF(cholqr(W, U, SB.as<double2>()));
   std::swap(V, W);  // V = V_1; U (zero rows not needed: j = 1 skips it)
 
-  // per step host copies: A and B
-  const int m = o.max_steps;
-  std::vector<cplx> hA((size_t)m * nops * pp),
-      hB((size_t)(m + 1) * nops * pp);
-  std::vector<int> hflag(nops, 0), broke_at(nops, -1);
+  std::vector<int> broke_at(nops, -1);
   std::vector<double> cur((size_t)nops * o.nev, NAN), prev((size_t)nops * o.nev, NAN);
   double t_eig = 0.0;
   int steps = 0;
   bool converged = false;
 
-  // eigenvalues of every operator's block tridiagonal T: the blocks are put
-  // together on the host (threads over the operators), the eigenvalue step
-  // itself runs on the device (band_lowest_device)
-  std::vector<std::vector<cplx>> Aall(nops);
+  // eigenvalues of every operator's block tridiagonal T, on the device
   auto extract = [&](int nsteps) -> edk_status {
     const double te = wall_s();
-    const int nth = (int)std::max(1u, std::min<unsigned>(std::thread::hardware_concurrency(), 64));
-    std::vector<std::thread> pool;
     std::vector<int> mqs(nops);
-    std::vector<std::vector<const double*>> Ap(nops), Bp(nops);
-    auto work = [&](int t) {
-      for (int q = t; q < nops; q += nth) {
-        const int mq = broke_at[q] >= 0 ? broke_at[q] : nsteps;
-        mqs[q] = mq;
-        Aall[q].assign((size_t)mq * pp, cplx(0.0, 0.0));
-        Ap[q].assign(mq, nullptr);
-        Bp[q].assign(mq, nullptr);
-        for (int j = 0; j < mq; ++j) {
-          cplx* Aj = Aall[q].data() + (size_t)j * pp;
-          const cplx* a1 = hA.data() + ((size_t)j * nops + q) * pp;
-          // device holds (V^H W)^T column-major = A row-major; make A
-          // column-major and Hermitian
-          for (int r = 0; r < p; ++r)
-            for (int c = 0; c < p; ++c) Aj[r + (size_t)c * p] = a1[c + (size_t)r * p];
-          for (int r = 0; r < p; ++r)
-            for (int c = r; c < p; ++c) {
-              const cplx h = 0.5 * (Aj[r + (size_t)c * p] + std::conj(Aj[c + (size_t)r * p]));
-              Aj[r + (size_t)c * p] = h;
-              Aj[c + (size_t)r * p] = std::conj(h);
-            }
-          Ap[q][j] = reinterpret_cast<const double*>(Aj);
-          if (j >= 1) Bp[q][j] = reinterpret_cast<const double*>(hB.data() + ((size_t)j * nops + q) * pp);
-        }
-      }
-    };
-    for (int t = 0; t < nth; ++t) pool.emplace_back(work, t);
-    for (auto& th : pool) th.join();
+    for (int q = 0; q < nops; ++q) mqs[q] = broke_at[q] >= 0 ? broke_at[q] : nsteps;
     std::vector<std::vector<double>> res;
-    EDK_RETURN_IF(band_lowest_device(p, o.nev, mqs, Ap, Bp, st, res));
+    EDK_RETURN_IF(band_lowest_device(p, o.nev, mqs, SA.p, SB.p, st, res));
     for (int q = 0; q < nops; ++q)
       for (int k = 0; k < o.nev; ++k) cur[(size_t)q * o.nev + k] = res[q][k];
     t_eig += wall_s() - te;
     return EDK_OK;
   };
 
+  int looked = 0;  // steps whose flags and times the host has read
+  std::vector<int> hflag((size_t)kLook * nops);
   for (int j = 0; j < m; ++j) {
-    EDK_TRY_CUDA(cudaEventRecord(e0, st));
+    cudaEvent_t* ev = evs.e + 3 * (j - looked);
+    double2* Q1 = SA.as<double2>() + (size_t)j * npp;
+    EDK_TRY_CUDA(cudaEventRecord(ev[0], st));
     EDK_RETURN_IF(spmm(V, W));
-    EDK_TRY_CUDA(cudaEventRecord(e1, st));
+    EDK_TRY_CUDA(cudaEventRecord(ev[1], st));
     // one classical block Gram-Schmidt pass against V_j and V_{j-1}; the
     // Cholesky-QR below runs twice
-    EDK_RETURN_IF(gram(W, V, Q1.as<double2>()));
+    EDK_RETURN_IF(gram(W, V, Q1));
     if (j > 0) EDK_RETURN_IF(gram(W, U, Q2.as<double2>()));
-    EDK_RETURN_IF(update(Q1.as<double2>(), V, W));
+    EDK_RETURN_IF(update(Q1, V, W));
     if (j > 0) EDK_RETURN_IF(update(Q2.as<double2>(), U, W));
-    EDK_RETURN_IF(cholqr(W, U));  // U (= V_{j-1}) is free now
-    EDK_TRY_CUDA(cudaEventRecord(e2, st));
-    EDK_TRY_CUDA(cudaMemcpyAsync(hA.data() + (size_t)j * nops * pp, Q1.p,
-                                 (size_t)nops * pp * sizeof(double2), cudaMemcpyDeviceToHost, st));
-    EDK_TRY_CUDA(cudaMemcpyAsync(hB.data() + (size_t)(j + 1) * nops * pp, Bm.p,
-                                 (size_t)nops * pp * sizeof(double2), cudaMemcpyDeviceToHost, st));
-    EDK_TRY_CUDA(cudaMemcpyAsync(hflag.data(), flags.p, nops * sizeof(int),
-                                 cudaMemcpyDeviceToHost, st));
-    EDK_TRY_CUDA(cudaStreamSynchronize(st));
-    float a = 0.f, c = 0.f;
-    cudaEventElapsedTime(&a, e0, e1);
-    cudaEventElapsedTime(&c, e1, e2);
-    t_spmm += a;
-    t_orth += c;
+    // U (= V_{j-1}) is free now
+    EDK_RETURN_IF(cholqr(W, U, SB.as<double2>() + (size_t)(j + 1) * npp));
+    EDK_TRY_CUDA(cudaMemcpyAsync(SF.as<int>() + (size_t)j * nops, flags.p, nops * sizeof(int),
+                                 cudaMemcpyDeviceToDevice, st));
+    EDK_TRY_CUDA(cudaEventRecord(ev[2], st));
     // rotate: V_{j-1} <- V_j, V_j <- V_{j+1} (in W), spare <- old U
     double2* oldU = U;
     U = V;
     V = W;
     W = oldU;
-    steps = j + 1;
-    bool all_broken = true;
-    for (int q = 0; q < nops; ++q) {
-      // a flag raised in this step's QR: block j+1 is not part of the space
-      if (hflag[q] && broke_at[q] < 0) broke_at[q] = j + 1;
-      all_broken = all_broken && broke_at[q] >= 0;
-    }
     // (without a tolerance only the last step's eigenvalues are ever used)
-    const bool check = (o.tol > 0.0 && o.check_every > 0 && (j + 1) % o.check_every == 0) ||
-                       j + 1 == m || all_broken;
-    if (check) {
-      EDK_RETURN_IF(extract(j + 1));
-      if (o.tol > 0.0 && j + 1 < m) {
+    bool check = (o.tol > 0.0 && o.check_every > 0 && (j + 1) % o.check_every == 0) || j + 1 == m;
+    if (!check && j + 1 - looked < kLook) continue;
+    EDK_TRY_CUDA(cudaMemcpyAsync(hflag.data(), SF.as<int>() + (size_t)looked * nops,
+                                 (size_t)(j + 1 - looked) * nops * sizeof(int),
+                                 cudaMemcpyDeviceToHost, st));
+    EDK_TRY_CUDA(cudaStreamSynchronize(st));
+    bool all_broken = false;
+    for (int i = looked; i <= j && !all_broken; ++i) {
+      float a = 0.f, c = 0.f;
+      const cudaEvent_t* e = evs.e + 3 * (i - looked);
+      cudaEventElapsedTime(&a, e[0], e[1]);
+      cudaEventElapsedTime(&c, e[1], e[2]);
+      t_spmm += a;
+      t_orth += c;
+      steps = i + 1;
+      all_broken = true;  // (steps enqueued past that point are not counted)
+      for (int q = 0; q < nops; ++q) {
+        // a flag raised in this step's QR: block i + 1 is not part of the space
+        if (hflag[(size_t)(i - looked) * nops + q] && broke_at[q] < 0) broke_at[q] = i + 1;
+        all_broken = all_broken && broke_at[q] >= 0;
+      }
+    }
+    looked = j + 1;
+    if (check || all_broken) {
+      EDK_RETURN_IF(extract(steps));
+      if (o.tol > 0.0 && steps < m) {
         bool conv = true;
         for (int q = 0; q < nops && conv; ++q)
           for (int k = 0; k < o.nev; ++k) {

@@ -482,14 +482,13 @@ struct HandleLease {
 void handles_unregister(bool registered);
 // implemented in edk_util.cpp
 int tridiag_eigvals(int m, const double* a, const double* b, double* w);
-// The lowest `nev` distinct eigenvalues of block-tridiagonal Hermitian
-// matrices (operator q: m[q] blocks of p x p, A[q][j] on the diagonal and
-// B[q][j], j >= 1, below it, column-major interleaved complex on the host),
-// on the device (edk_band.cu); NaN where fewer are found.
-edk_status band_lowest_device(int p, int nev, const std::vector<int>& m,
-                              const std::vector<std::vector<const double*>>& A,
-                              const std::vector<std::vector<const double*>>& B,
-                              cudaStream_t st, std::vector<std::vector<double>>& out);
+// The lowest `nev` distinct eigenvalues of block-tridiagonal Hermitian matrices
+// (edk_band.cu): operator q has m[q] blocks; SA and SB (device) hold step j's
+// p x p products of operator q at (j nops + q) p^2, see k_band_pack; NaN where
+// fewer are found.
+edk_status band_lowest_device(int p, int nev, const std::vector<int>& m, const void* SA,
+                              const void* SB, cudaStream_t st,
+                              std::vector<std::vector<double>>& out);
 int tridiag_eigen(int m, const double* a, const double* b, double* w, double* Q);
 int tridiag_first_row(int m, const double* a, const double* b, double* w, double* z);
 // implemented in edk_tridiag.cu: the lowest nk eigenvalues of nops tridiagonal
