@@ -8,7 +8,10 @@
 // applied to the p vectors with the lanes spread over the vectors.  Blocks are
 // row-major (row i, vector c at i * p + c), so each hit reads one contiguous
 // p-element row of X: coalesced, and reused from L2 across the rows that
-// reach it.  The materialised form reads the sliced-ELL entries instead of
+// reach it.  Up to 16 vectors, half a warp takes a row (LW = 16 lanes): a whole
+// one would leave half of its lanes without a vector and most without a hit (18
+// sectors of 2,700 rows, 16 vectors: 92 us a product with whole warps; the block
+// Lanczos around 60 of them 29.2 -> 27.6 ms).  The materialised form reads the sliced-ELL entries instead of
 // recomputing them.
 #pragma once
 
@@ -30,7 +33,7 @@ struct SpmmOp {
 
 namespace spmm_detail {
 
-template <class VT, int VPL>
+template <class VT, int VPL, int LW>
 __device__ __forceinline__ void acc_row(typename VTraits<VT>::A (&ar)[VPL],
                                         typename VTraits<VT>::A (&ai)[VPL],
                                         const VT* __restrict__ xr, int lane, int p, double cr,
@@ -40,7 +43,7 @@ __device__ __forceinline__ void acc_row(typename VTraits<VT>::A (&ar)[VPL],
   const A r = (A)cr, i = (A)ci;
 #pragma unroll
   for (int v = 0; v < VPL; ++v) {
-    const int c = lane + 32 * v;
+    const int c = lane + LW * v;
     if (c < p) {
       const Cx<A> xv = ldv(xr + c);
       ar[v] += r * xv.r + i * xv.i;  // conj(coefficient) * x
@@ -49,14 +52,14 @@ __device__ __forceinline__ void acc_row(typename VTraits<VT>::A (&ar)[VPL],
   }
 }
 
-template <class VT, int VPL>
+template <class VT, int VPL, int LW>
 __device__ __forceinline__ void store_row(VT* __restrict__ yr, int lane, int p, int accumulate,
                                           typename VTraits<VT>::A (&ar)[VPL],
                                           typename VTraits<VT>::A (&ai)[VPL]) {
   using A = typename VTraits<VT>::A;
 #pragma unroll
   for (int v = 0; v < VPL; ++v) {
-    const int c = lane + 32 * v;
+    const int c = lane + LW * v;
     if (c < p) {
       Cx<A> out{ar[v], ai[v]};
       if (accumulate) {
@@ -72,14 +75,14 @@ __device__ __forceinline__ void store_row(VT* __restrict__ yr, int lane, int p, 
 // Apply the nh hits held one per lane (ok, target row, coefficient) to the
 // lane's columns, four hits at a time: their row gathers are all issued
 // before the multiply-adds, so four rows are in flight per lane.
-template <class VT, int VPL>
+template <class VT, int VPL, int LW>
 __device__ __forceinline__ void apply_hits(typename VTraits<VT>::A (&ar)[VPL],
                                            typename VTraits<VT>::A (&ai)[VPL],
                                            const VT* __restrict__ xb, int lane, int p, int nh,
                                            int ok, int64_t pos, double cr, double ci) {
   using A = typename VTraits<VT>::A;
   constexpr bool CX = VTraits<VT>::cx;
-  const unsigned full = 0xffffffffu;
+  const unsigned full = LW == 32 ? 0xffffffffu : 0xffffu << (threadIdx.x & 16);  // the row's lanes
   int hh = 0;
   for (; hh + 4 <= nh; hh += 4) {
     int okq[4];
@@ -87,17 +90,17 @@ __device__ __forceinline__ void apply_hits(typename VTraits<VT>::A (&ar)[VPL],
     double crq[4], ciq[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      okq[u] = __shfl_sync(full, ok, hh + u);
-      pq[u] = __shfl_sync(full, pos, hh + u);
-      crq[u] = __shfl_sync(full, cr, hh + u);
-      ciq[u] = __shfl_sync(full, ci, hh + u);
+      okq[u] = __shfl_sync(full, ok, hh + u, LW);
+      pq[u] = __shfl_sync(full, pos, hh + u, LW);
+      crq[u] = __shfl_sync(full, cr, hh + u, LW);
+      ciq[u] = __shfl_sync(full, ci, hh + u, LW);
     }
     Cx<A> xv[4][VPL];
 #pragma unroll
     for (int u = 0; u < 4; ++u)
 #pragma unroll
       for (int v = 0; v < VPL; ++v) {
-        const int c = lane + 32 * v;
+        const int c = lane + LW * v;
         xv[u][v] = (okq[u] && c < p) ? ldv(xb + pq[u] * p + c) : Cx<A>{0, 0};
       }
 #pragma unroll
@@ -111,16 +114,16 @@ __device__ __forceinline__ void apply_hits(typename VTraits<VT>::A (&ar)[VPL],
     }
   }
   for (; hh < nh; ++hh) {
-    if (!__shfl_sync(full, ok, hh)) continue;
-    const int64_t ph = __shfl_sync(full, pos, hh);
-    const double crh = __shfl_sync(full, cr, hh), cih = __shfl_sync(full, ci, hh);
-    acc_row<VT, VPL>(ar, ai, xb + ph * p, lane, p, crh, cih);
+    if (!__shfl_sync(full, ok, hh, LW)) continue;
+    const int64_t ph = __shfl_sync(full, pos, hh, LW);
+    const double crh = __shfl_sync(full, cr, hh, LW), cih = __shfl_sync(full, ci, hh, LW);
+    acc_row<VT, VPL, LW>(ar, ai, xb + ph * p, lane, p, crh, cih);
   }
 }
 
 }  // namespace spmm_detail
 
-template <int BK, class VT, int VPL>
+template <int BK, class VT, int VPL, int LW>
 __global__ void __launch_bounds__(256) k_spmm_ff(const SpmmOp* __restrict__ ops, int nops,
                                                  int64_t Dpad, int p,
                                                  const VT* __restrict__ X, VT* __restrict__ Y,
@@ -131,14 +134,14 @@ __global__ void __launch_bounds__(256) k_spmm_ff(const SpmmOp* __restrict__ ops,
     fill_binom32(s_binom);
     __syncthreads();
   }
-  const int lane = threadIdx.x & 31;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  const int lane = threadIdx.x & (LW - 1);
+  const int64_t nw = (int64_t)gridDim.x * (blockDim.x / LW);
   const int64_t total = (int64_t)nops * Dpad;
-  for (int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < total; g += nw) {
+  for (int64_t g = (int64_t)blockIdx.x * (blockDim.x / LW) + threadIdx.x / LW; g < total; g += nw) {
     const int q = (int)(g / Dpad);
     const int64_t i = g - (int64_t)q * Dpad;
     const SpmmOp& o = ops[q];
-    if (o.kind != 0 || i >= o.D) continue;  // warp-uniform
+    if (o.kind != 0 || i >= o.D) continue;  // the row's lanes agree
     const BasisDev& b = o.b;
     const FFParams& ff = o.ff;
     const uint32_t mask = (uint32_t)b.maskL;
@@ -173,8 +176,8 @@ __global__ void __launch_bounds__(256) k_spmm_ff(const SpmmOp* __restrict__ ops,
     A ar[VPL], ai[VPL];
 #pragma unroll
     for (int v = 0; v < VPL; ++v) ar[v] = ai[v] = 0;
-    spmm_detail::acc_row<VT, VPL>(ar, ai, xb + i * p, lane, p, dr, di);  // conj(diag) x_i
-    for (int base = 0; base < nhit; base += 32) {
+    spmm_detail::acc_row<VT, VPL, LW>(ar, ai, xb + i * p, lane, p, dr, di);  // conj(diag) x_i
+    for (int base = 0; base < nhit; base += LW) {
       const int l = base + lane;
       int ok = 0;
       int64_t pos = 0;
@@ -202,10 +205,10 @@ __global__ void __launch_bounds__(256) k_spmm_ff(const SpmmOp* __restrict__ ops,
           ok = 1;
         }
       }
-      const int nh = min(32, nhit - base);
-      spmm_detail::apply_hits<VT, VPL>(ar, ai, xb, lane, p, nh, ok, pos, cr, ci);
+      const int nh = min(LW, nhit - base);
+      spmm_detail::apply_hits<VT, VPL, LW>(ar, ai, xb, lane, p, nh, ok, pos, cr, ci);
     }
-    spmm_detail::store_row<VT, VPL>(Y + (int64_t)q * Dpad * p + i * p, lane, p, accumulate, ar,
+    spmm_detail::store_row<VT, VPL, LW>(Y + (int64_t)q * Dpad * p + i * p, lane, p, accumulate, ar,
                                     ai);
   }
 }
@@ -238,7 +241,7 @@ __global__ void __launch_bounds__(256) k_spmm_sell(const SpmmOp* __restrict__ op
     A ar[VPL], ai[VPL];
 #pragma unroll
     for (int v = 0; v < VPL; ++v) ar[v] = ai[v] = 0;
-    spmm_detail::acc_row<VT, VPL>(ar, ai, xb + row * p, lane, p, d.x, d.y);
+    spmm_detail::acc_row<VT, VPL, 32>(ar, ai, xb + row * p, lane, p, d.x, d.y);
     for (int kb = 0; kb < w; kb += 32) {
       const int k = kb + lane;
       int col = 0;
@@ -265,9 +268,9 @@ __global__ void __launch_bounds__(256) k_spmm_sell(const SpmmOp* __restrict__ op
       }
       const int nh = min(32, w - kb);
       // padding entries carry a zero coefficient: applying them adds nothing
-      spmm_detail::apply_hits<VT, VPL>(ar, ai, xb, lane, p, nh, 1, (int64_t)col, cr, ci);
+      spmm_detail::apply_hits<VT, VPL, 32>(ar, ai, xb, lane, p, nh, 1, (int64_t)col, cr, ci);
     }
-    spmm_detail::store_row<VT, VPL>(Y + (int64_t)q * Dpad * p + row * p, lane, p, accumulate,
+    spmm_detail::store_row<VT, VPL, 32>(Y + (int64_t)q * Dpad * p + row * p, lane, p, accumulate,
                                     ar, ai);
   }
 }
@@ -281,11 +284,15 @@ edk_status launch_spmm(const SpmmOp* d_ops, int nops, int bk_ff, int64_t smax, i
   const bool two = p > 32;
   if (bk_ff >= 0) {
     const int64_t nw = (int64_t)nops * Dpad;
-    const int grid = (int)std::min<int64_t>((nw + 7) / 8, 148 * 64);
-#define EDK_SPMM_FF(BK)                                                                          \
-  case BK:                                                                                       \
-    if (two) k_spmm_ff<BK, VT, 2><<<grid, 256, 0, st>>>(d_ops, nops, Dpad, p, X, Y, accumulate); \
-    else k_spmm_ff<BK, VT, 1><<<grid, 256, 0, st>>>(d_ops, nops, Dpad, p, X, Y, accumulate);    \
+    const int rpb = p <= 16 ? 16 : 8;  // rows per block
+    const int grid = (int)std::min<int64_t>((nw + rpb - 1) / rpb, 148 * 64);
+#define EDK_SPMM_FF(BK)                                                                              \
+  case BK:                                                                                           \
+    if (two) k_spmm_ff<BK, VT, 2, 32><<<grid, 256, 0, st>>>(d_ops, nops, Dpad, p, X, Y, accumulate); \
+    else if (p > 16)                                                                                 \
+      k_spmm_ff<BK, VT, 1, 32><<<grid, 256, 0, st>>>(d_ops, nops, Dpad, p, X, Y, accumulate);        \
+    else                                                                                             \
+      k_spmm_ff<BK, VT, 1, 16><<<grid, 256, 0, st>>>(d_ops, nops, Dpad, p, X, Y, accumulate);        \
     break;
     switch (bk_ff) {
       EDK_SPMM_FF(BK_TENSOR)
