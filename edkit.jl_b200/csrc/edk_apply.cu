@@ -70,14 +70,16 @@ bool lanes_fit(int64_t rows, int lanes) { return rows * lanes <= (int64_t)2 * 14
 // Resident blocks per SM asked of the compiler: the rank-search kernels are
 // latency bound and fit 32 registers (8 blocks of 256 threads fill every warp
 // slot) for real and single-precision complex vectors, or single precision
-// when the sector has a phase or a parity; the others keep the compiler's
-// choice.
+// when the sector has a phase or a parity; double complex on the hashed kinds
+// with a phase or a parity fits 48 (5 blocks instead of 4 at 56: 25 sites, 697
+// blocks, 64 -> 58 us, and no second wave); the others keep the compiler's choice.
 template <int BK, class VT>
 constexpr int ff_min_blocks() {
   constexpr bool single = std::is_same<VT, float>::value || std::is_same<VT, float2>::value;
-  return (BK == BK_TRANS0_RANK && !std::is_same<VT, double2>::value) ||
-                 ((BK == BK_TRANS_RANK || BK == BK_TRANSPAR_RANK) && single)
-             ? 8 : 1;
+  if ((BK == BK_TRANS0_RANK && !std::is_same<VT, double2>::value) ||
+      ((BK == BK_TRANS_RANK || BK == BK_TRANSPAR_RANK) && single))
+    return 8;
+  return (BK == BK_TRANS || BK == BK_TRANSPAR) && std::is_same<VT, double2>::value ? 5 : 1;
 }
 
 template <int BK, class VT, int TPS>

@@ -358,12 +358,12 @@ __global__ void k_rank_map(BasisDev b, int K, uint64_t n, uint32_t* out) {
     uint32_t key, extra = 0;  // extra: M (BK_TRANS) or the sign bit (BK_TRANSPAR)
     if (b.bk == BK_TRANS) {
       int M = 0;
-      key = canon_arg32(s, b.L, b.A, b.len, mask, M);
+      key = canon_arg32(s, b.L, b.A, b.len, mask, M, b.A == 1);
       extra = (uint32_t)M;
     } else if (b.bk == BK_TRANSPAR) {  // the coefficient rule of lookup<BK_TRANSPAR>
       uint32_t Iam, Ibm;
       int Rr, M;
-      canon_par32(s, b.L, b.A, b.len, mask, Iam, Rr, Ibm, M);
+      canon_par32(s, b.L, b.A, b.len, mask, Iam, Rr, Ibm, M, b.A == 1);
       double n;
       if (Ibm < Iam) { key = Ibm; n = (double)b.P * __ldg(b.phase + M).x; }
       else { key = Iam; n = __ldg(b.phase + Rr).x; }
@@ -889,6 +889,7 @@ extern "C" edk_status edk_basis_create(const edk_basis_desc* desc, edk_basis** o
     } else if (b->kind == EDK_TRANSLATIONAL) {
       dv.bk = (b->Kmom == 0) ? BK_TRANS0 : BK_TRANS;
       const char* e = std::getenv("EDK_CANON_RUNS");
+      dv.runs_arg = (b->A == 1 && b->L <= 32 && b->D >= 150000) ? 1 : 0;
       dv.runs_canon = (dv.bk == BK_TRANS0 && b->A == 1 && b->L <= 32 && e && e[0] == '1') ? 1 : 0;
     } else if (b->kind == EDK_TRANSPARITY) {
       dv.bk = BK_TRANSPAR;

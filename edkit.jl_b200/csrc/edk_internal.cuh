@@ -223,6 +223,12 @@ struct BasisDev {
   int P;                 // parity sign (TranslationParityBasis)
   int phase_real;        // 1 when every phase is real
   int runs_canon;        // 1: canonicalise from zero-run tops (unit cell 1, phase-free)
+  // 1: compare rotations at the zero-run tops where the shift counts too (unit cell
+  // 1, at least 150,000 rows).  Fewer, but serial, candidates: where rows fill the
+  // GPU the kernel is bound by issue and gains (c128 products: 28 sites 311 -> 279
+  // us, 27 163 -> 148, 25 59.4 -> 57.7), below by latency and loses (22 sites 45.7
+  // -> 48, 20 sites 34.5 -> 37.5).
+  int runs_arg;
   // abelian generators
   int ngen;
   const GenDev* gens;

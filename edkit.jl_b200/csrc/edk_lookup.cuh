@@ -285,9 +285,10 @@ __device__ __forceinline__ uint32_t runs_arg32(uint32_t s, int L, uint32_t mask,
   return m;
 }
 // first minimum and its translation count M
+// (with `runs`, see BasisDev::runs_arg, at the zero-run tops only)
 __device__ __forceinline__ uint32_t canon_arg32(uint32_t s, int L, int A, int len, uint32_t mask,
-                                                int& M) {
-  if (A == 1) return runs_arg32<false>(s, L, mask, M);
+                                                int& M, bool runs) {
+  if (runs) return runs_arg32<false>(s, L, mask, M);
   if (L <= 27) {
     // the spare low bits carry q, so min() keeps the smallest q on ties
     const Dbl32 d = dbl32_top(s, L);
@@ -319,9 +320,9 @@ __device__ __forceinline__ uint32_t canon_arg32(uint32_t s, int L, int A, int le
 // translations and reflected translations (TranslationParityBasis):
 // rev(rotr(s, i)) = rotl(rev(s), i) = rotr(rev(s), L - i).
 __device__ __forceinline__ void canon_par32(uint32_t s, int L, int A, int len, uint32_t mask,
-                                            uint32_t& Iam, int& Rr, uint32_t& Ibm, int& M) {
+                                            uint32_t& Iam, int& Rr, uint32_t& Ibm, int& M, bool runs) {
   const uint32_t rs = __brev(s) >> (32 - L);
-  if (A == 1) {
+  if (runs) {
     Iam = runs_arg32<false>(s, L, mask, Rr);
     Ibm = runs_arg32<true>(rs, L, mask, M);
     return;
@@ -455,7 +456,7 @@ __device__ __forceinline__ bool lookup(const BasisDev& b, S s, const uint32_t* b
     S Im = s;
     int M = 0;
     if constexpr (sizeof(S) == 4) {
-      Im = canon_arg32(s, b.L, b.A, b.len, mask, M);
+      Im = canon_arg32(s, b.L, b.A, b.len, mask, M, b.runs_arg != 0);
     } else {
       S I0 = s, t = s;
       for (int i = 1; i < b.len; ++i) {
@@ -476,7 +477,7 @@ __device__ __forceinline__ bool lookup(const BasisDev& b, S s, const uint32_t* b
     int Rr = 0, M = 0;
     if constexpr (sizeof(S) == 4) {
       uint32_t a_, b_;
-      canon_par32(s, b.L, b.A, b.len, mask, a_, Rr, b_, M);
+      canon_par32(s, b.L, b.A, b.len, mask, a_, Rr, b_, M, b.runs_arg != 0);
       Iam = a_; Ibm = b_;
     } else {
       S Ia0 = s, t = s;

@@ -196,14 +196,14 @@ __device__ __forceinline__ void canon_ctx(const BasisDev& b, uint32_t s, HitCtx&
     c.key = b.runs_canon ? canon_runs32(s, b.L, mask) : canon_min32(s, b.L, b.A, b.len, mask);
   } else if constexpr (BK == BK_TRANS) {
     int M;
-    c.key = canon_arg32(s, b.L, b.A, b.len, mask, M);
+    c.key = canon_arg32(s, b.L, b.A, b.len, mask, M, b.runs_arg != 0);
     const double2 ph = __ldg(b.phase + M);
     c.pre = ph.x;
     c.pim = ph.y;
   } else if constexpr (BK == BK_TRANSPAR) {
     uint32_t Iam, Ibm;
     int Rr, M;
-    canon_par32(s, b.L, b.A, b.len, mask, Iam, Rr, Ibm, M);
+    canon_par32(s, b.L, b.A, b.len, mask, Iam, Rr, Ibm, M, b.runs_arg != 0);
     if (Ibm < Iam) { c.key = Ibm; c.pre = (double)b.P * __ldg(b.phase + M).x; }
     else { c.key = Iam; c.pre = __ldg(b.phase + Rr).x; }
   } else {

@@ -42,12 +42,12 @@ __device__ __forceinline__ bool sell_target(const BasisDev& b, uint32_t s, const
       key = canon_min32(s, b.L, b.A, b.len, mask);
     } else if constexpr (BK == BK_TRANS) {
       int M;
-      key = canon_arg32(s, b.L, b.A, b.len, mask, M);
+      key = canon_arg32(s, b.L, b.A, b.len, mask, M, b.runs_arg != 0);
       ph = M;
     } else if constexpr (BK == BK_TRANSPAR) {
       uint32_t Iam, Ibm;
       int Rr, M;
-      canon_par32(s, b.L, b.A, b.len, mask, Iam, Rr, Ibm, M);
+      canon_par32(s, b.L, b.A, b.len, mask, Iam, Rr, Ibm, M, b.runs_arg != 0);
       double n;
       if (Ibm < Iam) { key = Ibm; n = (double)b.P * __ldg(b.phase + M).x; }
       else { key = Iam; n = __ldg(b.phase + Rr).x; }
