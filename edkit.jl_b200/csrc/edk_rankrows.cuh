@@ -147,6 +147,8 @@ __device__ __forceinline__ void plan_row_cols(const BasisDev& b, const OpDev& op
           k[u] = adj(p - 1);
         } else if (d == 1 && rkw != ~0u) {
           k[u] = rkw;
+        } else if (d == 2 && p >= 2) {
+          k[u] = rank_after_swap2(st, rs, p - 2, t.binom);
         } else {
           k[u] = rank_after_swap(st, rs, p, p >= d ? p - d : p - d + L, t.binom);
         }

@@ -256,3 +256,24 @@ def test_rank_search_translation_parity_bit_exact(ek, O, L, N, k, p):
                                     tol=1e-13, check_every=5)
         for q in range(2):
             assert abs(ev[q][0] - refs[q]) <= 1e-10 * abs(refs[q]), q
+
+
+@pytest.mark.parametrize("L,N", [(5, 1), (5, 4), (6, 3), (14, 7), (26, 3), (31, 2), (32, 30)])
+def test_next_nearest_swaps_bit_exact_with_hash(ek, L, N):
+    """Two bond families on row plans (k = 0, one thread per row): swaps two sites
+    apart at both ends of the ring, one to four and more hits per row, few and
+    many particles, up to 32 sites.  The same columns in the same order of
+    addition as the hash search, so bit for bit."""
+    rng = np.random.default_rng(100 * L + N)
+    b = ek.TranslationalBasis(L=L, k=0, N=N)
+    H = j1j2(ek, L, b, h=0.3)
+    H.configure_("fast", 1)
+    for dt in (np.float64, np.float32, np.complex128):
+        x = rng.standard_normal(b.size(1)).astype(dt)
+        if np.iscomplexobj(x):
+            x = x + 1j * rng.standard_normal(b.size(1))
+        b.set_search("hash")
+        want = H * x
+        b.set_search("rank")
+        assert np.array_equal(H * x, want), dt
+    b.set_search("hash")
