@@ -593,8 +593,9 @@ edk_status band_lowest_device(int p, int nev, const std::vector<int>& m, const v
     EDK_TRY_CUDA(cudaMemcpyAsync(dt.p, tasks.data(), tasks.size() * sizeof(BandTask),
                                  cudaMemcpyHostToDevice, st));
     const size_t smem = 3 * pp * sizeof(double2) + p * sizeof(double);
+    // the largest block's size (p = 64), the same from every calling thread
     EDK_TRY_CUDA(cudaFuncSetAttribute(k_band_sturm, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
+                                      (int)(3 * 64 * 64 * sizeof(double2) + 64 * sizeof(double))));
     k_band_sturm<<<(unsigned)tasks.size(), 256, smem, st>>>(d, dA.as<double2>(), dB.as<double2>(),
                                                              mqd.as<int>(), dt.as<BandTask>(),
                                                              dc.as<int>());

@@ -594,8 +594,9 @@ static edk_status block_lanczos(int nops, edk_operator* const* ops,
     return EDK_OK;
   };
   const size_t chol_smem = 3 * (size_t)pp * sizeof(double2);
+  // the largest block's size (p = 64), the same from every calling thread
   EDK_TRY_CUDA(cudaFuncSetAttribute(k_chol, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)chol_smem));
+                                    (int)(3 * 64 * 64 * sizeof(double2))));
   // Cholesky-QR twice: X (in slot W) = Q B; Q lands back in W, `spare` is
   // overwritten; B to Bm
   auto cholqr = [&](double2* Wx, double2* spare, double2* Bm) -> edk_status {

@@ -242,8 +242,10 @@ edk_status eig_run(int n, const void* G, double* W, cudaStream_t st) {
   int nb = std::max(1, std::min(nsm, (n + 7) / 8));
   const size_t smem = eig_smem<T>(n, nb);
   if (smem + 1024 > (size_t)optin) return EDK_UNSUPPORTED;
+  // the device's limit rather than this call's size: threads with different
+  // sizes would take the attribute from one another between here and the launch
   EDK_TRY_CUDA(cudaFuncSetAttribute(k_tridiagonalise<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)smem));
+                                    optin - 1024));
   DevBuf buf;
   const size_t vb = 2 * (size_t)n * sizeof(T);
   EDK_RETURN_IF(buf.alloc_async(2 * vb + 2 * (size_t)n * 8 + 16, st));

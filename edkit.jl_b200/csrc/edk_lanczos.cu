@@ -314,7 +314,9 @@ struct Engine {
         using XV = std::remove_pointer_t<decltype(xp)>;
         auto kern = k_dots<VV, XV>;
         if (smem > 48 * 1024)
-          cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+          // one value up to 1,024 columns, so that concurrent threads agree on it
+          cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)std::max<size_t>(smem, 128 * 1024));
         kern<<<nblk, kDotThreads, smem, st>>>((const VV*)V.p, D, ncols, (const XV*)x, D,
                                                part.as<double2>());
         return EDK_OK;
