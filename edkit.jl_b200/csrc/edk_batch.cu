@@ -1430,8 +1430,7 @@ edk_status batch_lanczos(const std::vector<edk_operator*>& ops, const edk_lanczo
   // the FP64 refinement (1e-5), several levels a better one (1e-7) — and, for
   // a few operators, it checks every 5 steps so that it stops early
   double tol1 = mixed ? std::max(o.tol, o.nev > 1 ? 1e-7 : 1e-5) : o.tol;
-  // (a check solves every operator's tridiagonal problem on the host, so
-  // large batches keep the caller's interval)
+  // (larger batches keep the caller's interval)
   const int check1 = (mixed && nops <= 8)
                          ? std::max(1, std::min(o.check_every > 0 ? o.check_every : 5, 5))
                          : o.check_every;

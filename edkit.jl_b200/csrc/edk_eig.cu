@@ -1,7 +1,7 @@
-// edk_eig.cu — eigenvalues of a dense Hermitian matrix of up to some 1,500 rows
-// (the Gram matrices of ent_spec / ent_S, src/Schmidt.jl:84-165): Householder
-// tridiagonalisation in the shared memory of all SMs, then the multi-section
-// Sturm kernel (edk_tridiag.cu) for all eigenvalues at once.
+// edk_eig.cu — eigenvalues of a dense Hermitian matrix that fits the shared memory
+// of all SMs, 1,808 rows real, 1,205 complex (the Gram matrices of ent_spec /
+// ent_S, src/Schmidt.jl:84-165): Householder tridiagonalisation there, then the
+// multi-section Sturm kernel (edk_tridiag.cu) for all eigenvalues at once.
 //
 // A tridiagonalisation is n dependent steps of one matrix-vector product and one
 // rank-two update, so it is bound by what a step cannot overlap: a product needs

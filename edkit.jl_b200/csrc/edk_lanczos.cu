@@ -1,10 +1,13 @@
-// edk_lanczos.cu — Lanczos ground state and adaptive Krylov exp(-iHt) on the
-// device.
+// edk_lanczos.cu — the adaptive Krylov controller exp(-iHt), on the batched
+// engine's steps (edk_batch.cu, KrylovBasis), and a single-operator Lanczos
+// engine for what that one does not take: lanczos_e0 without
+// reorthogonalisation, on symmetry-group bases and on chains of more than 32
+// sites.
 //
-// The Krylov basis V (D x (m+1), column-major) lives in HBM in the storage
-// precision (f64/c128, or f32/c64 for the mixed path); the working vector w,
-// every inner product and the Gram-Schmidt coefficients are FP64.  One
-// Lanczos step is
+// In the single-operator engine the Krylov basis V (D x (m+1), column-major)
+// lives in HBM in the storage precision (f64/c128, or f32/c64 for the mixed
+// path); the working vector w, every inner product and the Gram-Schmidt
+// coefficients are FP64.  One step is
 //   wt = H v_j                        (row-gather matvec)
 //   s  = V^H wt ; alpha_j = Re s_j     (pass 1 over V, FP64 block partials)
 //   w  = wt - V s                      (pass 2)

@@ -18,8 +18,8 @@
 // Orbits of different representatives are disjoint, so every entry is owned
 // by one thread and updated without atomics, in the reference's summation
 // order.  Singular values come from the Gram matrix (cuBLAS SYRK / HERK on
-// the smaller side) and a dense symmetric eigensolver (cuSOLVER SYEVD /
-// HEEVD), the GEMM-shaped route; eigenvalues of the Gram matrix below
+// the smaller side) and a dense Hermitian eigensolver (edk_eig.cu, or cuSOLVER
+// SYEVD / HEEVD where the matrix does not fit its shared memory); eigenvalues of the Gram matrix below
 // n * eps * lambda_max (its rounding floor) are reported as zero.
 //
 // DoubleBasis: one thread per full-space state looks the state up in the

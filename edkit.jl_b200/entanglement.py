@@ -6,7 +6,7 @@ src/LinearMap.jl (``DoubleBasis``, ``symmetrizer``) with the reference's names,
 keyword arguments and error messages.  The work runs in libedk
 (edk_schmidt.cu): the Schmidt matrix and the DoubleBasis map are CUDA kernels,
 the singular values come from a Gram matrix (cuBLAS) and a dense Hermitian
-eigensolver (cuSOLVER).  Vectors may be numpy arrays (host) or CUDA torch
+eigensolver (edk_eig.cu; cuSOLVER above 1,024 rows).  Vectors may be numpy arrays (host) or CUDA torch
 tensors (device); results of ``schmidt`` and ``DoubleBasis`` come back on the
 side the input came from.
 """

@@ -236,8 +236,10 @@ edk_status edk_block_lanczos(int32_t nops, edk_operator* const* ops,
 /* Kernel choice of the matrix-free application.  EDK_KERNEL_FAST: the
  * bond-family kernel (operators whose off-diagonal part is flip-flop bonds),
  * with `tps` threads (1, 2, 4) sharing each state; EDK_KERNEL_GENERIC: the
- * row kernel that handles every operator.  block = 1 applies four or more
- * right-hand sides as one SpMM on the bond-family and materialised paths
+ * row kernel that handles every operator (on TensorBasis with L <= 31 operators
+ * other than flip-flop bonds run as Pauli strings instead, with either choice;
+ * EDK_DISABLE_FAST=1 in the environment at their creation keeps the row kernel).
+ * block = 1 applies four or more right-hand sides as one SpMM on the bond-family and materialised paths
  * (each nonzero located once for all columns, as colmn! does,
  * Operator.jl:417-465); block = 0 runs them one column at a time; block = -1
  * (the default) uses the SpMM matrix-free, and the columns on a materialised
@@ -293,8 +295,7 @@ typedef enum {
 } edk_precision;
 
 typedef struct {
-  int32_t max_steps;     /* Lanczos steps (m); at most 12,791 on the batched
-                            engine (its step coefficients sit in shared memory) */
+  int32_t max_steps;     /* Lanczos steps (m); at most 12,791 on the batched engine */
   int32_t nev;           /* number of lowest eigenvalues wanted */
   double tol;            /* relative stop tolerance on the Ritz values; 0 = run max_steps */
   int32_t check_every;   /* steps between convergence checks */
@@ -317,7 +318,7 @@ typedef struct {
   double seconds_stage1; /* first Lanczos stage (FP64, or FP32 storage when mixed) */
   double seconds_refine; /* FP64 refinement stages (mixed precision) */
   int32_t refine_rounds; /* FP64 refinement restarts taken */
-  int32_t checks;        /* host convergence checks */
+  int32_t checks;        /* convergence checks */
 } edk_lanczos_diag;
 
 /* v0: starting vector (dtype v0_dtype, host or device); evals: nev values.
@@ -432,8 +433,9 @@ edk_status edk_schmidt(const edk_basis* b, int32_t vdtype, const void* v, int32_
 /* ent_spec(v, Aind, b) — Schmidt.jl:84: singular values of the Schmidt matrix,
  * descending, into s (host, min(2^nA, 2^(L-nA)) values, count in *ns; s may
  * be NULL to query the count).  Computed as square roots of the eigenvalues
- * of the Gram matrix of the smaller side (cuBLAS SYRK/HERK + cuSOLVER
- * SYEVD/HEEVD); squared values below n * eps * max are returned as 0.
+ * of the Gram matrix of the smaller side (cuBLAS SYRK/HERK, then the library's
+ * tridiagonalisation in shared memory up to 1,024 rows and cuSOLVER
+ * SYEVD/HEEVD above); squared values below n * eps * max are returned as 0.
  * min side <= 32768.  ptr_kind applies to v. */
 edk_status edk_ent_spec(const edk_basis* b, int32_t vdtype, const void* v, int32_t nA,
                         const int32_t* Ainds, double* s, int64_t* ns, int32_t ptr_kind);
