@@ -21,7 +21,7 @@
 // zero.  Read as column-major p x Dpad matrices (ld = p) these are what the
 // strided-batched cuBLAS ZGEMMs consume: the K = D reductions are split in
 // chunks of Kc rows (one batch entry each) and the partial p x p products
-// summed by a kernel.  H V is this file's own SpMM: one warp per row, the
+// summed by a kernel.  H V is this file's own SpMM: one warp per row (half a warp for up to 16 vectors), the
 // row's off-diagonal hits found by different lanes, then every hit applied to
 // the p vectors with the lanes spread over the vectors (coalesced p x 16-byte
 // row gathers).

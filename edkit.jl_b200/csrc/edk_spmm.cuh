@@ -3,7 +3,7 @@
 //
 // EDKit's colmn! (src/Operator.jl:417-465) finds each nonzero's target index
 // once and then loops over the RHS columns.  The GPU form keeps that order of
-// work: one warp per row, the row's off-diagonal hits located by different
+// work: one warp per row (half a warp for up to 16 vectors), the row's off-diagonal hits located by different
 // lanes (canonicalisation and lookup done once per hit), then every hit
 // applied to the p vectors with the lanes spread over the vectors.  Blocks are
 // row-major (row i, vector c at i * p + c), so each hit reads one contiguous
