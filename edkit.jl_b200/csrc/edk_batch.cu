@@ -376,6 +376,10 @@ __device__ __forceinline__ double2 wide(float2 v) { return make_double2((double)
 //   H q - V V^H H q - q q^H H q = (wt - g u - V (r - g s)) / a
 // so the second read of V updates both vectors.  V^H H q is exact to the
 // rounding of the recurrence times |s|, which one sweep leaves at eps |H| / beta.
+// In a space that V already spans (a sector with fewer levels than steps) u is the
+// rounding of the first sweep, s takes in all of it and a is close to zero: beta a,
+// the length the second sweep leaves, then ends the run (k_breduce2) by the rule
+// that a vector orthogonalised twice in its own step would meet there.
 // Mean over the 131 steps of 96 random-field chains of 12 to 20 sites (FP64):
 // 194 + 247 + 173 us for the three passes before, 171 + 177 us for the two here,
 // which is the HBM rate (two blocks of 128 registers per SM; three of 80 spill:
@@ -507,18 +511,27 @@ __device__ __forceinline__ double bsum256(double v, double* sh) {  // all thread
   return t;
 }
 
+constexpr double kBreakdown = 1.4901161193847656e-08;  // sqrt(eps(Float64))
+// Part of |u|^2 outside the span of V below which column u is taken as inside it:
+// dividing by a would raise u's rounding (6e-8 in FP32 storage) by more than 100.
+// In storage of either width a vector whose beta is above the breakdown rule's
+// limit leaves 1 - O(eps |H| / beta)^2.
+constexpr double kInSpan = 1e-4;
+
 // Sums operator q's slots (one warp per column; both vectors), and in the last
 // block of the operator turns them into the update's coefficients:
-// cs = s, ce = r - g s, scal = {1 / a, g}, and alpha_j.
+// cs = s, ce = r - g s, scal = {1 / a, g}, and alpha_j; or stops the operator with
+// j steps and beta_{j-1} = 0 when the second sweep leaves nothing of column j.
+// `closing`: only that test, for the column past the last step.
 __global__ void __launch_bounds__(256) k_breduce2(const SplitOp* __restrict__ sp, int ncap, int m,
                                                   const double2* __restrict__ part, int64_t pstride,
                                                   double2* __restrict__ cs, double2* __restrict__ ce,
                                                   double4* __restrict__ scal,
                                                   double* __restrict__ alpha,
-                                                  const double* __restrict__ beta,
+                                                  double* __restrict__ beta,
                                                   unsigned* __restrict__ cnt,
-                                                  const int* __restrict__ step,
-                                                  const int* __restrict__ done) {
+                                                  const int* __restrict__ step, int* done,
+                                                  int closing) {
   __shared__ bool s_last;
   __shared__ double sh[8];
   const int q = blockIdx.y;
@@ -578,8 +591,24 @@ __global__ void __launch_bounds__(256) k_breduce2(const SplitOp* __restrict__ sp
   hx = bsum256(hx, sh);
   hy = bsum256(hy, sh);
   const double2 uu = __ldcg(csq + j), uw = __ldcg(ceq + j);
-  double a2 = uu.x - ss;
-  if (a2 < 1e-30 * uu.x) a2 = 1e-30 * uu.x;  // (NaN stays)
+  const double a2 = uu.x - ss;
+  if (j > 0) {  // (NaN runs on)
+    double* bj = beta + (int64_t)q * m + j - 1;
+    const double left = *bj * sqrt(a2 < 0.0 ? 0.0 : a2), a = alpha[(int64_t)q * m + j - 1];
+    if (a2 <= kInSpan * uu.x || left <= kBreakdown * fmax(1.0, fabs(a))) {
+      __syncthreads();  // beta_{j-1} is read
+      if (threadIdx.x == 0) {
+        *bj = 0.0;
+        done[q] = 2;  // (every block of the operator has read the flag: all have counted)
+        cnt[q] = 0;
+      }
+      return;
+    }
+  }
+  if (closing) {
+    if (threadIdx.x == 0) cnt[q] = 0;
+    return;
+  }
   const double inva = 1.0 / sqrt(a2), gx = (uw.x - hx) / a2, gy = (uw.y - hy) / a2;
   for (int c = threadIdx.x; c < j; c += blockDim.x) {
     const double2 s = __ldcg(csq + c), r = __ldcg(ceq + c);
@@ -779,8 +808,7 @@ __global__ void __launch_bounds__(256) k_bfinish(const BOp* __restrict__ ops, in
         const double a = alpha[(int64_t)q * m + j];
         beta[(int64_t)q * m + j] = nrm;
         nsteps[q] = j + 1;
-        const double seps = 1.4901161193847656e-08;  // sqrt(eps(Float64))
-        if (nrm <= seps * fmax(1.0, fabs(a))) {
+        if (nrm <= kBreakdown * fmax(1.0, fabs(a))) {
           beta[(int64_t)q * m + j] = 0.0;
           done[q] = 2;
           invb[q] = 0.0;
@@ -1146,23 +1174,55 @@ struct BatchEngine {
                                     nsteps.as<int>(), step.as<int>(), done.as<int>(), setup);
   }
 
-  // one Lanczos step for every live operator (graph-capturable)
-  edk_status enqueue_step() {
-    EDK_RETURN_IF(launch_apply());
+  // the dot products of column *step and their sums; see k_breduce2 for `closing`
+  void launch_dots(int closing) {
     const int64_t pst = (int64_t)(G + nops) * ncap;
     // blocks per operator of the sums: two per SM over all operators
     const int rx = std::max(1, std::min((ncap + 7) / 8, (2 * nsm + nops - 1) / nops));
+    with_vt(vdt, [&](auto vp) -> edk_status {
+      using VV = std::remove_pointer_t<decltype(vp)>;
+      k_rdots2<VV><<<(unsigned)G, 256, 0, st>>>(d_ops(), rsplit(), V.as<VV>(), wt.as<VV>(),
+                                                part.as<double2>(), pst, step.as<int>(),
+                                                done.as<int>());
+      k_breduce2<<<dim3(rx, nops), 256, 0, st>>>(
+          splitops.as<SplitOp>(), ncap, m, part.as<double2>(), pst, cs.as<double2>(),
+          ce.as<double2>(), scal.as<double4>(), alpha.as<double>(), beta.as<double>(),
+          cnt.as<unsigned>(), step.as<int>(), done.as<int>(), closing);
+      return EDK_OK;
+    });
+  }
+
+  // After a run's last step: true when some running operator's last vector is
+  // so short beside its T that its second sweep, which comes with the next step,
+  // could take all of it.  (Above 1e-3 one sweep leaves |s| below 1e-3 even in FP32
+  // storage.)
+  bool may_close(const double* a, const double* b, const int* dn, const int* ns) const {
+    for (int q = 0; q < nops; ++q) {
+      if (dn[q] != 0 || ns[q] < 1) continue;
+      const double *aq = a + (size_t)q * m, *bq = b + (size_t)q * m;
+      double big = 0.0;
+      for (int k = 0; k < ns[q]; ++k) big = std::max({big, std::fabs(aq[k]), std::fabs(bq[k])});
+      if (bq[ns[q] - 1] <= 1e-3 * big) return true;
+    }
+    return false;
+  }
+
+  // Test the vector past the last step: beta of that step becomes 0 and the
+  // operator stops (status 2) when the space is closed.
+  edk_status close() {
+    launch_dots(1);
+    EDK_TRY_CUDA(cudaGetLastError());
+    return EDK_OK;
+  }
+
+  // one Lanczos step for every live operator (graph-capturable)
+  edk_status enqueue_step() {
+    EDK_RETURN_IF(launch_apply());
+    launch_dots(0);
     edk_status s = with_vt(vdt, [&](auto vp) -> edk_status {
       using VV = std::remove_pointer_t<decltype(vp)>;
       return with_vt(wdt, [&](auto wp) -> edk_status {
         using WD = std::remove_pointer_t<decltype(wp)>;
-        k_rdots2<VV><<<(unsigned)G, 256, 0, st>>>(d_ops(), rsplit(), V.as<VV>(), wt.as<VV>(),
-                                                  part.as<double2>(), pst, step.as<int>(),
-                                                  done.as<int>());
-        k_breduce2<<<dim3(rx, nops), 256, 0, st>>>(
-            splitops.as<SplitOp>(), ncap, m, part.as<double2>(), pst, cs.as<double2>(),
-            ce.as<double2>(), scal.as<double4>(), alpha.as<double>(), beta.as<double>(),
-            cnt.as<unsigned>(), step.as<int>(), done.as<int>());
         k_rupdate2<VV, WD><<<(unsigned)G, 256, 0, st>>>(
             d_ops(), rsplit(), ncap, V.as<VV>(), cs.as<double2>(), ce.as<double2>(),
             scal.as<double4>(), wt.as<VV>(), w.as<WD>(), normpart.as<double>(), step.as<int>(),
@@ -1283,6 +1343,12 @@ edk_status run_batch(BatchEngine& E, int max_steps, int nev, double tol, int che
   EDK_TRY_CUDA(cudaMemcpyAsync(hb.data(), E.beta.p, hb.size() * 8, cudaMemcpyDeviceToHost, E.st));
   EDK_TRY_CUDA(cudaMemcpyAsync(he.data(), ev.p, he.size() * 8, cudaMemcpyDeviceToHost, E.st));
   EDK_TRY_CUDA(cudaStreamSynchronize(E.st));
+  if (E.may_close(ha.data(), hb.data(), hdone.data(), hsteps.data())) {
+    EDK_RETURN_IF(E.close());
+    EDK_TRY_CUDA(cudaMemcpyAsync(hdone.data(), E.done.p, nops * sizeof(int), cudaMemcpyDeviceToHost, E.st));
+    EDK_TRY_CUDA(cudaMemcpyAsync(hb.data(), E.beta.p, hb.size() * 8, cudaMemcpyDeviceToHost, E.st));
+    EDK_TRY_CUDA(cudaStreamSynchronize(E.st));
+  }
   for (int q = 0; q < nops; ++q) {
     OpResult& r = res[q];
     r.status = hdone[q];
@@ -1478,6 +1544,12 @@ edk_status batch_lanczos(const std::vector<edk_operator*>& ops, const edk_lanczo
       std::vector<int> keep;  // positions in `active` of the operators to restart
       for (size_t i = 0; i < active.size(); ++i) {
         const int q = active[i];
+        bool finite = r2[i].status < 3;  // (3, 4: the refinement's start vector is none)
+        for (double x : r2[i].ev) finite = finite && std::isfinite(x);
+        if (!finite) {
+          set_error("batch Lanczos: the FP64 refinement of a mixed-precision run is not finite");
+          return EDK_NOT_CONVERGED;
+        }
         bool still = r2[i].ev.size() == res[q].ev.size();
         for (size_t k = 0; k < r2[i].ev.size() && still; ++k) {
           const double a = r2[i].ev[k], b = res[q].ev[k];
@@ -1602,8 +1674,16 @@ edk_status KrylovBasis::extend(int from, int to, double* alpha, double* beta, in
   for (int j = from; j < to; ++j) EDK_RETURN_IF(E.run_step());
   EDK_TRY_CUDA(cudaMemcpyAsync(alpha, E.alpha.p, (size_t)to * sizeof(double), cudaMemcpyDeviceToHost, E.st));
   EDK_TRY_CUDA(cudaMemcpyAsync(beta, E.beta.p, (size_t)to * sizeof(double), cudaMemcpyDeviceToHost, E.st));
+  int done = 0;
   EDK_TRY_CUDA(cudaMemcpyAsync(m, E.nsteps.p, sizeof(int), cudaMemcpyDeviceToHost, E.st));
+  EDK_TRY_CUDA(cudaMemcpyAsync(&done, E.done.p, sizeof(int), cudaMemcpyDeviceToHost, E.st));
   EDK_TRY_CUDA(cudaStreamSynchronize(E.st));
+  if (E.may_close(alpha, beta, &done, m)) {  // the controller stops at beta = 0
+    EDK_RETURN_IF(E.close());
+    EDK_TRY_CUDA(cudaMemcpyAsync(beta + *m - 1, E.beta.as<double>() + *m - 1, sizeof(double),
+                                 cudaMemcpyDeviceToHost, E.st));
+    EDK_TRY_CUDA(cudaStreamSynchronize(E.st));
+  }
   return EDK_OK;
 }
 

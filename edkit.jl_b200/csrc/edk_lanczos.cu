@@ -938,6 +938,8 @@ struct KrylovCacheDev {
       dg->basis_extensions += 1;
       dg->max_dim_used = std::max(dg->max_dim_used, m);
       ok = true;
+    } else if (beta[m - 1] == 0.0) {
+      ok = true;  // the space turned out closed at m vectors: valid for every time
     }
     return EDK_OK;
   }
