@@ -907,7 +907,7 @@ struct BatchEngine {
   // a batch of one whose product has no batched kernel (symmetry groups, more
   // than 32 sites): launched step by step through apply_device
   edk_operator* direct = nullptr;
-  int hj = 0;  // the next step of a direct batch
+  int hj = 0;  // the next step, where steps are launched one by one
   int64_t nsblk = 0;
   cudaStream_t st = nullptr;
   std::vector<BOp> hops;
@@ -929,32 +929,33 @@ struct BatchEngine {
     if (graph) cudaGraphDestroy(graph);
   }
 
-  edk_status init(const std::vector<edk_operator*>& ops, int vdtype, int m_, int lookup_kind,
-                  bool use_ff, cudaStream_t s) {
-    nops = (int)ops.size();
-    if (nops > 65535) {
-      set_error("batch Lanczos: at most 65535 operators per batch");
-      return EDK_UNSUPPORTED;
-    }
+  // The operators as they are now: their device records, tile maps and the
+  // kernel of the product.  Called again (with the stream idle) when one of them
+  // has been materialised, cleared or configured since.
+  edk_status load(const std::vector<edk_operator*>& ops, int lookup_kind, bool use_ff) {
+    if (gexec) cudaGraphExecDestroy(gexec);
+    if (graph) cudaGraphDestroy(graph);
+    gexec = nullptr;
+    graph = nullptr;
+    graph_ok = false;
+    hops.clear();
+    Ds.clear();
+    ntiles = nsblk = 0;
+    pauli = nullptr;
     // row plans (built here, outside any capture) when the sectors are ranked
     plan = use_ff && (lookup_kind == BK_TRANS0_RANK || lookup_kind == BK_TRANS_RANK ||
                       lookup_kind == BK_TRANSPAR_RANK || lookup_kind == BK_PROJ_RANK);
     plan_nn_all = plan;
     for (auto* op : ops) plan = plan && plan_applies(op);
     plan_nn_all = plan;
-    if (plan) EDK_RETURN_IF(plan_ensure(ops, s));
+    if (plan) EDK_RETURN_IF(plan_ensure(ops, st));
     for (auto* op : ops) {
       if (!plan) break;
       plan = op->plan_state == 1;
       plan_nn_all = plan_nn_all && plan_nn(*reinterpret_cast<const FFParams*>(op->ff_params.data()));
     }
-    vdt = vdtype;
-    wdt = (vdt == EDK_C128 || vdt == EDK_C64) ? EDK_C128 : EDK_F64;
-    m = m_;
-    ncap = m + 1;
     bk = lookup_kind;
     ff = use_ff;
-    st = s;
     std::vector<int> t2o, s2o;
     int64_t voff = 0, woff = 0;
     sell = true;
@@ -986,11 +987,6 @@ struct BatchEngine {
     }
     totalD = woff;
     if (nops == 1 && !sell && ops[0]->pauli_ok) pauli = ops[0];
-    if (!ops[0]->cstream)
-      EDK_TRY_CUDA(cudaStreamCreateWithFlags(&ops[0]->cstream, cudaStreamNonBlocking));
-    side = ops[0]->cstream;
-    EDK_TRY_CUDA(cudaEventCreateWithFlags(&checked, cudaEventDisableTiming));
-    EDK_RETURN_IF(split_rows());
     EDK_RETURN_IF(dops.alloc_async(hops.size() * sizeof(BOp), st));
     EDK_TRY_CUDA(cudaMemcpyAsync(dops.p, hops.data(), hops.size() * sizeof(BOp),
                                  cudaMemcpyHostToDevice, st));
@@ -1002,7 +998,28 @@ struct BatchEngine {
         EDK_TRY_CUDA(cudaMemcpyAsync(sblk2op.p, s2o.data(), s2o.size() * 4,
                                      cudaMemcpyHostToDevice, st));
     }
-    EDK_RETURN_IF(V.alloc_async((size_t)voff * esz(vdt), st));
+    return EDK_OK;
+  }
+
+  edk_status init(const std::vector<edk_operator*>& ops, int vdtype, int m_, int lookup_kind,
+                  bool use_ff, cudaStream_t s) {
+    nops = (int)ops.size();
+    if (nops > 65535) {
+      set_error("batch Lanczos: at most 65535 operators per batch");
+      return EDK_UNSUPPORTED;
+    }
+    vdt = vdtype;
+    wdt = (vdt == EDK_C128 || vdt == EDK_C64) ? EDK_C128 : EDK_F64;
+    m = m_;
+    ncap = m + 1;
+    st = s;
+    EDK_RETURN_IF(load(ops, lookup_kind, use_ff));
+    if (!ops[0]->cstream)
+      EDK_TRY_CUDA(cudaStreamCreateWithFlags(&ops[0]->cstream, cudaStreamNonBlocking));
+    side = ops[0]->cstream;
+    EDK_TRY_CUDA(cudaEventCreateWithFlags(&checked, cudaEventDisableTiming));
+    EDK_RETURN_IF(split_rows());
+    EDK_RETURN_IF(V.alloc_async((size_t)totalD * ncap * esz(vdt), st));
     EDK_RETURN_IF(w.alloc_async((size_t)totalD * esz(wdt), st));
     EDK_RETURN_IF(wt.alloc_async((size_t)totalD * esz(vdt), st));
     // a block meets at most one operator more than it starts in: G + nops slots
@@ -1638,29 +1655,66 @@ edk_status batch_lanczos(const std::vector<edk_operator*>& ops, const edk_lanczo
 // ---------------------------------------------------------------------------
 struct KrylovBasis::Impl {
   BatchEngine E;
+  edk_operator* op = nullptr;
+  // the operator as the engine's record and graph have it
+  struct Form {
+    uint64_t tables;
+    bool ff;
+    int tps, search;
+    bool operator==(const Form& o) const {
+      return tables == o.tables && ff == o.ff && tps == o.tps && search == o.search;
+    }
+  } form{};
+  bool loaded = false;
+
+  Form now() const { return Form{op->sell_tables, op->use_ff, op->tps, op->b->dev.search}; }
+  // the lookup kind and kernel family of the product, as apply_device takes them
+  int kind(bool& ff) {
+    const BasisDev& b = op->b->dev;
+    int bk = b.bk;
+    ff = op->ff_ok && op->use_ff;
+    if (ff && b.search == 2) {
+      if (bk == BK_TRANS0) bk = BK_TRANS0_RANK;
+      else if (bk == BK_TRANS && b.rank_shift == 10) bk = BK_TRANS_RANK;
+      else if (bk == BK_TRANSPAR) bk = BK_TRANSPAR_RANK;
+    }
+    E.direct = !op->sell_ok && !op->pauli_ok && (bk == BK_ABELIAN || b.L > 32) ? op : nullptr;
+    ff = ff && !E.direct;
+    return bk;
+  }
+  // A cache outlives calls that materialise, clear or configure its operator: the
+  // matrix that the record and the graph point to may be gone by then.
+  edk_status refresh() {
+    if (loaded && form == now()) return EDK_OK;
+    loaded = false;  // also after a failure below: the next call tries again
+    EDK_TRY_CUDA(cudaStreamSynchronize(E.st));
+    bool ff = false;
+    const int bk = kind(ff);
+    EDK_RETURN_IF(E.load(std::vector<edk_operator*>(1, op), bk, ff));
+    form = now();
+    loaded = true;
+    return E.capture();
+  }
 };
 KrylovBasis::KrylovBasis() = default;
 KrylovBasis::~KrylovBasis() = default;
 
 edk_status KrylovBasis::init(edk_operator* op, int vdt, int m_max, cudaStream_t st) {
   impl = std::make_unique<Impl>();
-  BatchEngine& E = impl->E;
-  const BasisDev& b = op->b->dev;
-  int bk = b.bk;
-  const bool ff = op->ff_ok && op->use_ff;
-  if (ff && b.search == 2) {
-    if (bk == BK_TRANS0) bk = BK_TRANS0_RANK;
-    else if (bk == BK_TRANS && b.rank_shift == 10) bk = BK_TRANS_RANK;
-    else if (bk == BK_TRANSPAR) bk = BK_TRANSPAR_RANK;
-  }
-  if (!op->sell_ok && !op->pauli_ok && (bk == BK_ABELIAN || b.L > 32)) E.direct = op;
-  return E.init(std::vector<edk_operator*>(1, op), vdt, m_max, bk, ff && !E.direct, st);
+  impl->op = op;
+  bool ff = false;
+  const int bk = impl->kind(ff);
+  EDK_RETURN_IF(impl->E.init(std::vector<edk_operator*>(1, op), vdt, m_max, bk, ff, st));
+  impl->form = impl->now();
+  impl->loaded = true;
+  return EDK_OK;
 }
 
 const void* KrylovBasis::vectors() const { return impl->E.V.p; }
 
 edk_status KrylovBasis::start(const void* src, double* nrm, int* status) {
   BatchEngine& E = impl->E;
+  EDK_RETURN_IF(impl->refresh());
   EDK_RETURN_IF(E.setup(src));
   EDK_RETURN_IF(E.capture());
   EDK_TRY_CUDA(cudaMemcpyAsync(nrm, E.alpha.p, sizeof(double), cudaMemcpyDeviceToHost, E.st));
@@ -1671,6 +1725,8 @@ edk_status KrylovBasis::start(const void* src, double* nrm, int* status) {
 
 edk_status KrylovBasis::extend(int from, int to, double* alpha, double* beta, int* m) {
   BatchEngine& E = impl->E;
+  EDK_RETURN_IF(impl->refresh());
+  E.hj = from;
   for (int j = from; j < to; ++j) EDK_RETURN_IF(E.run_step());
   EDK_TRY_CUDA(cudaMemcpyAsync(alpha, E.alpha.p, (size_t)to * sizeof(double), cudaMemcpyDeviceToHost, E.st));
   EDK_TRY_CUDA(cudaMemcpyAsync(beta, E.beta.p, (size_t)to * sizeof(double), cudaMemcpyDeviceToHost, E.st));

@@ -369,6 +369,7 @@ struct edk_operator {
   int64_t sell_wincap = 0;  // entries of the largest 256-row window
   bool sell_tma_ok = false;  // the staged (bulk-copy) product applies (stages fit in shared memory)
   bool sell_tma = false;     // ... and is used (set by the autotuner)
+  uint64_t sell_tables = 0;  // raised when the tables below dev.sell come or go
   bool sell_ok = false;
   int64_t sell_entries = 0;
   edk::OpDev dev{};

@@ -874,6 +874,7 @@ extern "C" edk_status edk_operator_materialize(edk_operator* op, int32_t enable,
   EDK_CHECK_ARG(op != nullptr, "edk_operator_materialize: NULL operator");
   std::lock_guard<std::mutex> lk(op->mu);
   if (!enable) {
+    ++op->sell_tables;
     op->sell_ok = false;
     op->dev.sell = SellDev{};
     op->s_rowid.release(); op->s_off.release(); op->s_width.release(); op->s_col.release();
@@ -883,7 +884,10 @@ extern "C" edk_status edk_operator_materialize(edk_operator* op, int32_t enable,
     if (entries) *entries = 0;
     return EDK_OK;
   }
-  if (!op->sell_ok) EDK_RETURN_IF(materialize(op));
+  if (!op->sell_ok) {
+    ++op->sell_tables;
+    EDK_RETURN_IF(materialize(op));
+  }
   if (entries) *entries = op->sell_entries;
   return EDK_OK;
 }
