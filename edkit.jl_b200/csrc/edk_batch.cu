@@ -1761,6 +1761,7 @@ extern "C" edk_status edk_batch_lanczos_e0(int32_t nops, edk_operator* const* op
     EDK_CHECK_ARG(op != nullptr, "edk_batch_lanczos_e0: NULL operator");
     tot += op->b->D;
   }
+  const OperatorLocks locks(v);
   cudaStream_t st = v[0]->stream;
   size_t es = v0_dtype == EDK_F64 ? 8 : 16;
   DevBuf v0d;

@@ -820,12 +820,7 @@ extern "C" edk_status edk_block_lanczos(int32_t nops, edk_operator* const* ops,
     EDK_CHECK_ARG((int64_t)o.block * o.max_steps < ops[q]->b->D,
                   "edk_block_lanczos: block * max_steps must stay below every dimension");
   }
-  std::vector<std::unique_lock<std::mutex>> locks;
-  for (int q = 0; q < nops; ++q) {
-    bool seen = false;
-    for (int r = 0; r < q; ++r) seen = seen || ops[r] == ops[q];
-    if (!seen) locks.emplace_back(ops[q]->mu);
-  }
+  const OperatorLocks locks(std::vector<edk_operator*>(ops, ops + nops));
   EDK_TRY_CUDA(cudaSetDevice(dev));
   return block_lanczos(nops, ops, o, x0, evals, diag);
 }

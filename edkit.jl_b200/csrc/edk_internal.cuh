@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <memory>
 #include <mutex>
@@ -405,6 +406,17 @@ struct edk_operator {
   bool handles = false;                  // has borrowed library handles (edk_handles.cu)
   std::mutex mu;
   ~edk_operator();
+};
+
+// Locks every operator of a batch, each once, in the order of their addresses
+// (two batches that share operators cannot wait for each other).
+struct OperatorLocks {
+  std::vector<std::unique_lock<std::mutex>> held;
+  explicit OperatorLocks(std::vector<edk_operator*> ops) {
+    std::sort(ops.begin(), ops.end());
+    ops.erase(std::unique(ops.begin(), ops.end()), ops.end());
+    for (edk_operator* op : ops) held.emplace_back(op->mu);
+  }
 };
 
 namespace edk {

@@ -526,7 +526,8 @@ static edk_status ritz_vector(Engine& E, const RunResult& R, void* out) {
 using namespace edk;
 
 // gs_out (optional, device, D elements of the FP64 working dtype): the lowest
-// Ritz vector, normalised
+// Ritz vector, normalised.  The caller holds op->mu: whatever goes to the operator's
+// stream, allocations included, must stay out of another thread's capture of it.
 static edk_status lanczos_common(edk_operator* op, const edk_lanczos_opts* opts, const void* v0,
                                  int32_t v0_dtype, int32_t ptr_kind, double* evals,
                                  double* alpha, double* beta, edk_lanczos_diag* diag,
@@ -536,6 +537,8 @@ extern "C" edk_status edk_lanczos_e0(edk_operator* op, const edk_lanczos_opts* o
                                      const void* v0, int32_t v0_dtype, int32_t ptr_kind,
                                      double* evals, double* alpha, double* beta,
                                      edk_lanczos_diag* diag) {
+  EDK_CHECK_ARG(op && opts && v0 && evals, "edk_lanczos_e0: NULL argument");
+  std::lock_guard<std::mutex> lk(op->mu);
   return lanczos_common(op, opts, v0, v0_dtype, ptr_kind, evals, alpha, beta, diag, nullptr);
 }
 
@@ -574,12 +577,12 @@ extern "C" edk_status edk_lanczos_ground_state(edk_operator* op, const edk_lancz
   }
   const int64_t D = op->b->D;
   EDK_CHECK_ARG(D >= 1, "edk_lanczos_ground_state: empty basis");
+  std::lock_guard<std::mutex> lk(op->mu);  // before the buffers, which go back under it
   DevBuf gs, ss;
   EDK_RETURN_IF(gs.alloc_async((size_t)D * esize(wdt), op->stream));
   EDK_RETURN_IF(ss.alloc_async(sizeof(double), op->stream));
   EDK_RETURN_IF(lanczos_common(op, opts, v0, v0_dtype, ptr_kind, evals, nullptr, nullptr, diag,
                                gs.p));
-  std::lock_guard<std::mutex> lk(op->mu);
   cudaStream_t st = op->stream;
   const int64_t nd = D * (cx ? 2 : 1);  // real doubles
   EDK_TRY_CUDA(cudaMemsetAsync(ss.p, 0, sizeof(double), st));
@@ -598,7 +601,6 @@ static edk_status lanczos_common(edk_operator* op, const edk_lanczos_opts* opts,
                                  int32_t v0_dtype, int32_t ptr_kind, double* evals,
                                  double* alpha, double* beta, edk_lanczos_diag* diag,
                                  void* gs_out) {
-  EDK_CHECK_ARG(op && opts && v0 && evals, "edk_lanczos_e0: NULL argument");
   EDK_CHECK_ARG(opts->max_steps >= 1, "edk_lanczos_e0: max_steps < 1");
   EDK_CHECK_ARG(opts->nev >= 1, "edk_lanczos_e0: nev < 1");
   EDK_CHECK_ARG(v0_dtype >= EDK_F64 && v0_dtype <= EDK_C64, "edk_lanczos_e0: bad v0 dtype");
@@ -606,7 +608,6 @@ static edk_status lanczos_common(edk_operator* op, const edk_lanczos_opts* opts,
     set_error("edk_lanczos_e0: the operator is not Hermitian in this basis");
     return EDK_NOT_HERMITIAN;
   }
-  std::lock_guard<std::mutex> lk(op->mu);
   double t0 = now_s();
   cudaStream_t st = op->stream;
   const int64_t D = op->b->D;
