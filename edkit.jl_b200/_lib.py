@@ -189,6 +189,16 @@ def check(status):
         raise EDKError(status, msg or f"libedk status {status}")
 
 
+def settled(new, old):
+    """`new`, a CUDA tensor that torch may have just made from `old` (a conversion
+    or a copy on its current stream), ready for libedk, which works on streams of
+    its own."""
+    if new is not old and new.is_cuda:
+        import torch
+        torch.cuda.current_stream(new.device).synchronize()
+    return new
+
+
 def ptr(a):
     """Raw address of a numpy array or torch tensor."""
     if hasattr(a, "data_ptr"):

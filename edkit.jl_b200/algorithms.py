@@ -162,7 +162,7 @@ class KrylovEvolutionCache:
         self._dev = hasattr(psi0, "data_ptr") and getattr(psi0, "is_cuda", False)
         if self._dev:
             import torch
-            psi0 = psi0.to(torch.complex128).contiguous()
+            psi0 = E.settled(psi0.to(torch.complex128).contiguous(), psi0)
             self._device = psi0.device
         else:
             psi0 = np.ascontiguousarray(psi0, dtype=np.complex128)
@@ -236,7 +236,7 @@ def timeevolve(H: Operator, psi0, t, *, return_diagnostics=False, tol=1e-10, m_i
     on_device = hasattr(psi0, "data_ptr") and getattr(psi0, "is_cuda", False)
     if on_device:
         import torch
-        psi0 = psi0.to(torch.complex128).contiguous()
+        psi0 = E.settled(psi0.to(torch.complex128).contiguous(), psi0)
     else:
         psi0 = np.ascontiguousarray(psi0, dtype=np.complex128)
     if psi0.shape[0] != D:

@@ -26,7 +26,7 @@ def _vec(v):
         import torch
         if v.dtype not in (torch.float64, torch.complex128):
             raise TypeError("vectors must be float64 or complex128")
-        v = v.contiguous()
+        v = E.settled(v.contiguous(), v)
         kind = E.DEVICE if v.is_cuda else E.HOST
         return (E.ptr(v), E.C128 if v.is_complex() else E.F64, kind, v, True,
                 v.device)

@@ -273,23 +273,29 @@ class Operator:
                 E.C64: np.complex64}[dt]
         return np.asfortranarray(x.astype(npdt, copy=False))
 
+    def _tensor_in(self, x):
+        """(x, edk dtype) as libedk reads a torch tensor: complex where the operator
+        is, a vector without gaps."""
+        types = _torch_types().get(x.dtype)
+        if types is None:
+            raise TypeError(f"unsupported vector dtype {x.dtype}")
+        dt, given = types[0], x
+        if self.is_complex and dt != types[2]:
+            x, dt = x.to(types[1]), types[2]
+        if x.dim() == 1 and x.stride(0) != 1:
+            x = x.contiguous()
+        return (x if x is given else E.settled(x, given)), dt
+
     def _mul_tensor(self, x):
         """H x for a torch tensor.  Small products are bound by this function, so
         it looks the dtype up once and hands plain integers to ctypes (a product
         of ten sites, 4.8 us on the GPU: 19.7 us a call through the numpy dtype
         names and pointer objects, 17.8 us here)."""
-        types = _torch_types().get(x.dtype)
-        if types is None:
-            raise TypeError(f"unsupported vector dtype {x.dtype}")
-        dt = types[0]
-        if self.is_complex and dt != types[2]:
-            x, dt = x.to(types[1]), types[2]
+        x, dt = self._tensor_in(x)
         shape = x.shape
         D = self.B._D
         assert shape[0] == D
         if len(shape) == 1:
-            if x.stride(0) != 1:
-                x = x.contiguous()
             y = x.new_empty(D)
             nvec, ldx, ldy = 1, D, D
         else:  # torch is row-major: a column-major (transposed) view
@@ -407,13 +413,24 @@ def trans_inv_operator(mat, ind, B):
 
 def mul_(target, opt: Operator, v):
     """mul!(target, opt, v): accumulates into target (Operator.jl:309-328)."""
-    v = opt._prep(v)
-    dt = opt._out_dtype(v)
+    if hasattr(v, "data_ptr"):
+        v, dt = opt._tensor_in(v)
+    else:
+        v = opt._prep(v)
+        dt = opt._out_dtype(v)
     if not hasattr(target, "data_ptr"):
         if not (target.flags.f_contiguous or target.ndim == 1):
             raise ValueError("target must be column-major")
-        if _vec_dtype(target) != dt:
-            raise TypeError("target dtype does not match the product dtype")
+    if _vec_dtype(target) != dt:
+        raise TypeError("target dtype does not match the product dtype")
+    if target.ndim == 1:  # a vector with gaps gets its sum through one without
+        if hasattr(target, "data_ptr"):
+            if target.stride(0) != 1:
+                whole = E.settled(target.contiguous(), target)
+                return target.copy_(opt._apply(v, whole, True, dt))
+        elif not target.flags.c_contiguous:
+            target[...] = opt._apply(v, np.ascontiguousarray(target), True, dt)
+            return target
     return opt._apply(v, target, True, dt)
 
 
