@@ -478,26 +478,129 @@ bool invariant(const std::vector<HostTerm>& terms, const std::vector<int>& perm,
   return cmp(a, b) && cmp(b, a);
 }
 
+uint32_t site_mask(const HostTerm& h, int L, int c) {
+  const int ns = (int)h.sites.size();
+  uint32_t m = 0;
+  for (int k = 0; k < ns; ++k)
+    if ((c >> (ns - 1 - k)) & 1) m |= 1u << (L - h.sites[k]);
+  return m;
+}
+
+// True when the strings of every flip mask give the matrix elements back: to a few
+// roundings of the entries they are made of, in both widths and in the kernel's order
+// of summation, and exactly zero where no term has an entry (the kernel reads the
+// vector at nonzeros only, as the row kernel does, so an infinity or NaN stays in
+// the rows that have an element with it).  (1.7, 0.3) as 1.0 +- 0.7 passes;
+// 1e10 and 1e-10 in one matrix, or three couplings that cancel only up to
+// rounding, do not.
+using PauliSum = std::map<std::pair<uint32_t, uint32_t>, std::pair<double, double>>;
+bool strings_give_entries(const std::vector<HostTerm>& terms, const std::vector<char>& in_family,
+                          int L, const PauliSum& sum) {
+  constexpr int kBits = 10;  // patterns are enumerated over at most 2^10
+  struct Part { const HostTerm* t; int x; };
+  std::map<uint32_t, std::vector<Part>> parts;
+  for (size_t q = 0; q < terms.size(); ++q) {
+    const HostTerm& h = terms[q];
+    for (int x = 0; x < h.dim; ++x) {
+      bool any = false;
+      for (int c = 0; c < h.dim && !any; ++c) {
+        const double re = h.re[(c ^ x) * h.dim + c], im = h.im[(c ^ x) * h.dim + c];
+        any = !(re == 0.0 && im == 0.0);
+      }
+      if (any && !(x == 0 && in_family[q])) parts[site_mask(h, L, x)].push_back({&h, x});
+    }
+  }
+  auto near = [](double got, double want, double scale, double eps) {
+    return scale == 0.0 ? got == 0.0 : std::fabs(got - want) <= 8.0 * eps * scale;
+  };
+  auto walsh = [](const HostTerm& h, int x, int z, double& vr, double& vi) {
+    vr = vi = 0.0;
+    for (int c = 0; c < h.dim; ++c) {
+      const double sg = (__builtin_popcount(c & z) & 1) ? -1.0 : 1.0;
+      vr += sg * h.re[(c ^ x) * h.dim + c];
+      vi += sg * h.im[(c ^ x) * h.dim + c];
+    }
+    vr /= h.dim;
+    vi /= h.dim;
+  };
+  for (const auto& kv : parts) {
+    uint32_t sites = 0;
+    for (const Part& p : kv.second) sites |= site_mask(*p.t, L, p.t->dim - 1);
+    if (kv.first == 0 || __builtin_popcount(sites) > kBits) {
+      // term by term: the diagonal (every row multiplies it, so a rounding beside a
+      // zero entry spreads nothing), and flips that reach many sites, where each term
+      // has to be one string (an entry in every column, so no pattern is empty)
+      for (const Part& p : kv.second) {
+        const HostTerm& h = *p.t;
+        std::vector<double> vr(h.dim), vi(h.dim);
+        int strings = 0;
+        for (int z = 0; z < h.dim; ++z) {
+          walsh(h, p.x, z, vr[z], vi[z]);
+          strings += vr[z] != 0.0 || vi[z] != 0.0;
+        }
+        if (kv.first != 0 && strings != 1) return false;
+        for (int c = 0; c < h.dim; ++c) {
+          double re = 0.0, im = 0.0;
+          for (int z = 0; z < h.dim; ++z) {
+            const double sg = (__builtin_popcount(c & z) & 1) ? -1.0 : 1.0;
+            re += sg * vr[z];
+            im += sg * vi[z];
+          }
+          const double er = h.re[(c ^ p.x) * h.dim + c], ei = h.im[(c ^ p.x) * h.dim + c];
+          const double s = std::fabs(er) + std::fabs(ei);
+          if (!near(re, er, s, 2.220446049250313e-16) || !near(im, ei, s, 2.220446049250313e-16))
+            return false;
+        }
+      }
+      continue;
+    }
+    const auto first = sum.lower_bound({kv.first, 0u}), last = sum.upper_bound({kv.first, ~0u});
+    uint32_t pat = 0;  // the patterns of the sites, in ascending order
+    do {
+      double re = 0.0, im = 0.0, s = 0.0, dr = 0.0, di = 0.0;
+      float fr = 0.f, fi = 0.f;
+      for (const Part& p : kv.second) {
+        const HostTerm& h = *p.t;
+        int c = 0;
+        for (int v : h.sites) c = 2 * c + (int)((pat >> (L - v)) & 1u);
+        const double er = h.re[(c ^ p.x) * h.dim + c], ei = h.im[(c ^ p.x) * h.dim + c];
+        re += er;
+        im += ei;
+        s += std::fabs(er) + std::fabs(ei);
+      }
+      for (auto it = first; it != last; ++it) {
+        const bool neg = __builtin_popcount(pat & it->first.second) & 1;
+        const double vr = it->second.first, vi = it->second.second;
+        dr += neg ? -vr : vr;
+        di += neg ? -vi : vi;
+        fr += neg ? -(float)vr : (float)vr;
+        fi += neg ? -(float)vi : (float)vi;
+      }
+      const double e64 = 2.220446049250313e-16, e32 = 1.1920928955078125e-07;
+      if (!near(dr, re, s, e64) || !near(di, im, s, e64) || !near(fr, re, s, e32) ||
+          !near(fi, im, s, e32))
+        return false;
+      pat = (pat - sites) & sites;
+    } while (pat != 0);
+  }
+  return true;
+}
+
 // Pauli strings of the terms' off-diagonal parts, grouped by flip mask, and of
 // the diagonals of the terms outside the bond families.  False when there are
-// more than kPauliMax: a string costs a row about six instructions and a flip
+// more than kPauliMax, or they do not give the matrix elements back: a string costs a row about six instructions and a flip
 // mask one gather, a general term about a hundred (transverse-field Ising,
 // L = 20: 97 per term), so the strings win while they stay few per term.
 constexpr size_t kPauliMax = 512;
 bool pauli_strings(const std::vector<HostTerm>& terms, const std::vector<char>& in_family, int L,
                    PauliFlips& flips, std::vector<PauliGroup>& group,
                    std::vector<PauliStr>& str, std::vector<PauliStr>& diag) {
-  std::map<std::pair<uint32_t, uint32_t>, std::pair<double, double>> sum;
+  PauliSum sum;
   for (size_t t = 0; t < terms.size(); ++t) {
     const HostTerm& h = terms[t];
     const int ns = (int)h.sites.size();
     if (ns > 4) return false;
-    auto mask = [&](int c) {
-      uint32_t m = 0;
-      for (int k = 0; k < ns; ++k)
-        if ((c >> (ns - 1 - k)) & 1) m |= 1u << (L - h.sites[k]);
-      return m;
-    };
+    auto mask = [&](int c) { return site_mask(h, L, c); };
     for (int x = 0; x < h.dim; ++x) {
       if (x == 0 && in_family[t]) continue;
       for (int z = 0; z < h.dim; ++z) {
@@ -515,6 +618,7 @@ bool pauli_strings(const std::vector<HostTerm>& terms, const std::vector<char>& 
     }
     if (sum.size() > kPauliMax) return false;
   }
+  if (!strings_give_entries(terms, in_family, L, sum)) return false;
   std::map<uint32_t, int> per_mask;
   for (auto it = sum.begin(); it != sum.end();)
     if (it->second.first == 0.0 && it->second.second == 0.0) it = sum.erase(it);

@@ -114,6 +114,8 @@ __global__ void __launch_bounds__(kPauliThreads, 4) k_apply_pauli(
     for (int r = 0; r < RPT; ++r) {
       const uint32_t l = t + r * kPauliThreads;
       if (!FULL && l >= rows) continue;
+      // no element, no read: an infinity or NaN there is not this row's
+      if (cr[r] == 0 && (!CX || ci[r] == 0)) continue;
       const Cx<A> xv = xm < R ? ldout(sx + (l ^ xm)) : ldv(xk + ((base + l) ^ xm));
       acc[r].r = fma_(cr[r], xv.r, acc[r].r);
       if constexpr (CX) {
