@@ -345,7 +345,7 @@ edk_status apply_device(edk_operator* op, int dtype, const void* x, void* y, int
     }
 #undef EDK_FF_TPS
   }
-  if (op->pauli_ok) return apply_pauli(op, dtype, x, y, nvec, ldx, ldy, accumulate, st);
+  if (op->pauli_ok && op->use_ff) return apply_pauli(op, dtype, x, y, nvec, ldx, ldy, accumulate, st);
   switch (dtype) {
     case EDK_F64:
       return sc ? launch_apply<double, false>(b, op->dev, x, y, nvec, ldx, ldy, 1, st)

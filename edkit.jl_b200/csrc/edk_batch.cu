@@ -986,7 +986,7 @@ struct BatchEngine {
       Ds.push_back(o.D);
     }
     totalD = woff;
-    if (nops == 1 && !sell && ops[0]->pauli_ok) pauli = ops[0];
+    if (nops == 1 && !sell && ops[0]->pauli_ok && ops[0]->use_ff) pauli = ops[0];
     EDK_RETURN_IF(dops.alloc_async(hops.size() * sizeof(BOp), st));
     EDK_TRY_CUDA(cudaMemcpyAsync(dops.p, hops.data(), hops.size() * sizeof(BOp),
                                  cudaMemcpyHostToDevice, st));
@@ -1678,7 +1678,7 @@ struct KrylovBasis::Impl {
       else if (bk == BK_TRANS && b.rank_shift == 10) bk = BK_TRANS_RANK;
       else if (bk == BK_TRANSPAR) bk = BK_TRANSPAR_RANK;
     }
-    E.direct = !op->sell_ok && !op->pauli_ok && (bk == BK_ABELIAN || b.L > 32) ? op : nullptr;
+    E.direct = !op->sell_ok && (bk == BK_ABELIAN || b.L > 32) ? op : nullptr;
     ff = ff && !E.direct;
     return bk;
   }

@@ -377,13 +377,14 @@ struct edk_operator {
   bool gather = true;
   bool is_complex = false;
   bool ff_ok = false;     // flip-flop bond-family fast path applies
-  bool use_ff = true;     // callers may switch the fast path off (A/B checks)
+  bool use_ff = true;     // callers may switch the fast path (either one) off
   int tps = 1;            // threads per state of the fast path (1, 2 or 4; autotuned)
   // row plan of the fast path on rank-searched sectors (edk_plan.cu): built on
   // first use; plan_state 0 not built, 1 built, -1 not available
   std::shared_ptr<edk::DevBuf> p_slab;  // shared by the operators of the batch that built it
   int plan_state = 0;
-  // Pauli-string form (full space, no flip-flop fast path, few enough strings)
+  // Pauli-string form (full space, no flip-flop fast path, few enough strings): the
+  // fast kernel of such an operator, taken while use_ff
   edk::DevBuf pa_group, pa_str, pa_diag;
   edk::PauliDev pauli{};
   edk::PauliFlips pauli_flips{};

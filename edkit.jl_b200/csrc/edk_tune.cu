@@ -1,7 +1,8 @@
 // edk_tune.cu — autotuner of the operator application.
 //
 // The best way to apply H depends on the basis and the operator: the
-// flip-flop fast kernel or the generic row kernel, how many threads share one
+// flip-flop fast kernel (Pauli strings where those apply) or the generic row
+// kernel, how many threads share one
 // state (row) in the fast kernel, which index search finds a target
 // representative (hash table or binary search over the sorted array), and
 // whether materialising the matrix once (the device counterpart of EDKit's
@@ -85,7 +86,7 @@ extern "C" edk_status edk_operator_configure(edk_operator* op, int32_t kernel, i
     op->use_block = block < 0 ? -1 : (block != 0);
     return EDK_OK;
   }
-  if (kernel == EDK_KERNEL_FAST && !(op->ff_ok && op->gather)) {
+  if (kernel == EDK_KERNEL_FAST && !((op->ff_ok && op->gather) || op->pauli_ok)) {
     set_error("edk_operator_configure: the fast kernel does not apply to this operator");
     return EDK_UNSUPPORTED;
   }
@@ -108,7 +109,7 @@ extern "C" edk_status edk_operator_autotune(edk_operator* op, int32_t dtype, int
   const int64_t D = b->D;
   edk_tune_result out{};
   if (D == 0) {
-    out.kernel = op->use_ff && op->ff_ok ? EDK_KERNEL_FAST : EDK_KERNEL_GENERIC;
+    out.kernel = op->use_ff && (op->ff_ok || op->pauli_ok) ? EDK_KERNEL_FAST : EDK_KERNEL_GENERIC;
     out.tps = op->tps;
     edk_basis_get_search(b, &out.search);
     if (res) *res = out;
@@ -145,6 +146,7 @@ extern "C" edk_status edk_operator_autotune(edk_operator* op, int32_t dtype, int
   for (int s : searches) {
     if (fast)
       for (int t : {1, 2, 4}) cands.push_back({EDK_KERNEL_FAST, s, t, 0});
+    if (op->pauli_ok) cands.push_back({EDK_KERNEL_FAST, s, 1, 0});
     if (s == EDK_SEARCH_RANK) continue;  // only the bond-family row kernel reads the rank table
     if (fast && multi && op->b->dev.L <= 32) cands.push_back({EDK_KERNEL_FAST, s, 1, 1});
     cands.push_back({EDK_KERNEL_GENERIC, s, 1, 0});

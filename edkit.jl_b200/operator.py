@@ -340,7 +340,7 @@ class Operator:
 
     def configure_(self, kernel="fast", tps=1, block=None):
         """Pick the matrix-free kernel by hand: "fast" (bond families, `tps`
-        threads per state) or "generic"; `block` True/False forces four or
+        threads per state; Pauli strings on the full space) or "generic"; `block` True/False forces four or
         more right-hand sides through one SpMM or one column at a time (None:
         automatic).  Every choice gives the same product."""
         E.check(E.load().edk_operator_configure(self._h, self._KERNELS[kernel], int(tps),

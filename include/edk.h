@@ -235,10 +235,12 @@ edk_status edk_block_lanczos(int32_t nops, edk_operator* const* ops,
 
 /* Kernel choice of the matrix-free application.  EDK_KERNEL_FAST: the
  * bond-family kernel (operators whose off-diagonal part is flip-flop bonds),
- * with `tps` threads (1, 2, 4) sharing each state; EDK_KERNEL_GENERIC: the
- * row kernel that handles every operator (on TensorBasis with L <= 31 operators
- * other than flip-flop bonds run as Pauli strings instead, with either choice;
- * EDK_DISABLE_FAST=1 in the environment at their creation keeps the row kernel).
+ * with `tps` threads (1, 2, 4) sharing each state, or the Pauli-string kernel
+ * (operators other than flip-flop bonds on TensorBasis with L <= 31, where few
+ * strings hold them; tps ignored); EDK_KERNEL_GENERIC: the row kernel that handles
+ * every operator.  The fast kernel is taken where it applies until the other is
+ * chosen (EDK_DISABLE_FAST=1 in the environment at an operator's creation chooses
+ * the row kernel from the start).
  * block = 1 applies four or more right-hand sides as one SpMM on the bond-family and materialised paths
  * (each nonzero located once for all columns, as colmn! does,
  * Operator.jl:417-465); block = 0 runs them one column at a time; block = -1
