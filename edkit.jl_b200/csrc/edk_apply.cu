@@ -490,13 +490,15 @@ uint32_t site_mask(const HostTerm& h, int L, int c) {
 // roundings of the entries they are made of, in both widths and in the kernel's order
 // of summation, and exactly zero where no term has an entry (the kernel reads the
 // vector at nonzeros only, as the row kernel does, so an infinity or NaN stays in
-// the rows that have an element with it).  (1.7, 0.3) as 1.0 +- 0.7 passes;
-// 1e10 and 1e-10 in one matrix, or three couplings that cancel only up to
+// the rows that have an element with it).  An entry of at least a hundredth of the
+// largest one beside it may carry that one's rounding.  (1.7, 0.3) as 1.0 +- 0.7
+// passes; 1e10 and 1e-10 in one matrix, or three couplings that cancel only up to
 // rounding, do not.
 using PauliSum = std::map<std::pair<uint32_t, uint32_t>, std::pair<double, double>>;
 bool strings_give_entries(const std::vector<HostTerm>& terms, const std::vector<char>& in_family,
                           int L, const PauliSum& sum) {
   constexpr int kBits = 10;  // patterns are enumerated over at most 2^10
+  constexpr double e64 = 2.220446049250313e-16, e32 = 1.1920928955078125e-07;
   struct Part { const HostTerm* t; int x; };
   std::map<uint32_t, std::vector<Part>> parts;
   for (size_t q = 0; q < terms.size(); ++q) {
@@ -510,8 +512,11 @@ bool strings_give_entries(const std::vector<HostTerm>& terms, const std::vector<
       if (any && !(x == 0 && in_family[q])) parts[site_mask(h, L, x)].push_back({&h, x});
     }
   }
-  auto near = [](double got, double want, double scale, double eps) {
-    return scale == 0.0 ? got == 0.0 : std::fabs(got - want) <= 8.0 * eps * scale;
+  // scale: the entries at this pattern, big: the largest over all patterns
+  auto near = [](double got, double want, double scale, double big, double eps) {
+    if (scale == 0.0) return got == 0.0;
+    if (scale >= 0.01 * big) scale = std::max(scale, 0.25 * big);
+    return std::fabs(got - want) <= 8.0 * eps * scale;
   };
   auto walsh = [](const HostTerm& h, int x, int z, double& vr, double& vi) {
     vr = vi = 0.0;
@@ -539,6 +544,10 @@ bool strings_give_entries(const std::vector<HostTerm>& terms, const std::vector<
           strings += vr[z] != 0.0 || vi[z] != 0.0;
         }
         if (kv.first != 0 && strings != 1) return false;
+        double big = 0.0;
+        for (int c = 0; c < h.dim; ++c)
+          big = std::max(big, std::fabs(h.re[(c ^ p.x) * h.dim + c]) +
+                                  std::fabs(h.im[(c ^ p.x) * h.dim + c]));
         for (int c = 0; c < h.dim; ++c) {
           double re = 0.0, im = 0.0;
           for (int z = 0; z < h.dim; ++z) {
@@ -547,18 +556,18 @@ bool strings_give_entries(const std::vector<HostTerm>& terms, const std::vector<
             im += sg * vi[z];
           }
           const double er = h.re[(c ^ p.x) * h.dim + c], ei = h.im[(c ^ p.x) * h.dim + c];
-          const double s = std::fabs(er) + std::fabs(ei);
-          if (!near(re, er, s, 2.220446049250313e-16) || !near(im, ei, s, 2.220446049250313e-16))
-            return false;
+          // (a zero on the diagonal may carry a rounding, and so may what is near it)
+          const double s = kv.first == 0 ? big : std::fabs(er) + std::fabs(ei);
+          if (kv.first == 0 && er != 0.0 && std::fabs(er) < 1e-3 * big) return false;
+          if (!near(re, er, s, big, e64) || !near(im, ei, s, big, e64)) return false;
         }
       }
       continue;
     }
     const auto first = sum.lower_bound({kv.first, 0u}), last = sum.upper_bound({kv.first, ~0u});
-    uint32_t pat = 0;  // the patterns of the sites, in ascending order
-    do {
-      double re = 0.0, im = 0.0, s = 0.0, dr = 0.0, di = 0.0;
-      float fr = 0.f, fi = 0.f;
+    auto entries = [&](uint32_t pat, double& re, double& im) {  // the terms' sum; its size
+      double s = 0.0;
+      re = im = 0.0;
       for (const Part& p : kv.second) {
         const HostTerm& h = *p.t;
         int c = 0;
@@ -568,6 +577,18 @@ bool strings_give_entries(const std::vector<HostTerm>& terms, const std::vector<
         im += ei;
         s += std::fabs(er) + std::fabs(ei);
       }
+      return s;
+    };
+    double re, im, big = 0.0;
+    uint32_t pat = 0;  // the patterns of the sites, in ascending order
+    do {
+      big = std::max(big, entries(pat, re, im));
+      pat = (pat - sites) & sites;
+    } while (pat != 0);
+    do {
+      const double s = entries(pat, re, im);
+      double dr = 0.0, di = 0.0;
+      float fr = 0.f, fi = 0.f;
       for (auto it = first; it != last; ++it) {
         const bool neg = __builtin_popcount(pat & it->first.second) & 1;
         const double vr = it->second.first, vi = it->second.second;
@@ -576,9 +597,8 @@ bool strings_give_entries(const std::vector<HostTerm>& terms, const std::vector<
         fr += neg ? -(float)vr : (float)vr;
         fi += neg ? -(float)vi : (float)vi;
       }
-      const double e64 = 2.220446049250313e-16, e32 = 1.1920928955078125e-07;
-      if (!near(dr, re, s, e64) || !near(di, im, s, e64) || !near(fr, re, s, e32) ||
-          !near(fi, im, s, e32))
+      if (!near(dr, re, s, big, e64) || !near(di, im, s, big, e64) || !near(fr, re, s, big, e32) ||
+          !near(fi, im, s, big, e32))
         return false;
       pat = (pat - sites) & sites;
     } while (pat != 0);
@@ -586,11 +606,38 @@ bool strings_give_entries(const std::vector<HostTerm>& terms, const std::vector<
   return true;
 }
 
-// Pauli strings of the terms' off-diagonal parts, grouped by flip mask, and of
-// the diagonals of the terms outside the bond families.  False when there are
-// more than kPauliMax, or they do not give the matrix elements back: a string costs a row about six instructions and a flip
-// mask one gather, a general term about a hundred (transverse-field Ising,
-// L = 20: 97 per term), so the strings win while they stay few per term.
+// True when the strings cost a row less than the terms.  Both kernels are bound by
+// instructions, so the rule counts them; units of 0.1 us for 2^20 rows, fitted to
+// measured products (FP64, 20 sites, 19.5 us of launch and host taken off):
+//   strings: 0.4 a plain flip, 0.55 a string, 0.6 a flip mask of several strings;
+//   terms: 2.4 a term and 0.9 an off-diagonal entry of its columns (their mean);
+//   bond families: 3.8 an off-diagonal entry; diagonals are popcounts in both.
+// Small spaces, whose rows eight lanes share, run the terms in about a third of that
+// (16 sites, 15 projected flips of two sites: 30 / 25 us; 16 fields: 21 / 26).
+// Measured at 20 sites, strings / terms in us a product: 20 x fields 30 / 87, 20
+// fields of x and z 41 / 89, 19 projected flips of two sites 58 / 65, 18 of three 68 /
+// 72, 17 of four 94 / 67; dense two-site terms 30 / 23 (one) and 128 / 114 (19),
+// three-site 53 / 26 and 196 / 86 (eight), four-site 131 / 34 and 219 / 48 (two).
+bool strings_win(const std::vector<HostTerm>& terms, const std::vector<char>& in_family, int L,
+                 const PauliFlips& flips, size_t groups, size_t strings) {
+  double rows = 0.0;
+  for (size_t t = 0; t < terms.size(); ++t) {
+    const HostTerm& h = terms[t];
+    int off = 0;
+    for (int r = 0; r < h.dim; ++r)
+      for (int c = 0; c < h.dim; ++c)
+        off += r != c && !(h.re[r * h.dim + c] == 0.0 && h.im[r * h.dim + c] == 0.0);
+    const double entries = (double)off / h.dim;
+    rows += in_family[t] ? 38.0 * entries : 24.0 + 9.0 * entries;
+  }
+  if (lanes_fit((int64_t)1 << L, many_lanes<BK_TENSOR>())) rows *= 0.35;
+  return 4.0 * flips.n + 5.5 * strings + 6.0 * groups <= rows;
+}
+
+// Pauli strings of the terms' off-diagonal parts, grouped by flip mask, and of the
+// diagonals of the terms outside the bond families.  False when there are more than
+// kPauliMax (tables and host time), they do not give the matrix elements back, or the
+// terms cost less.
 constexpr size_t kPauliMax = 512;
 bool pauli_strings(const std::vector<HostTerm>& terms, const std::vector<char>& in_family, int L,
                    PauliFlips& flips, std::vector<PauliGroup>& group,
@@ -641,7 +688,7 @@ bool pauli_strings(const std::vector<HostTerm>& terms, const std::vector<char>& 
       group.back().s1 = (int)str.size();
     }
   }
-  return true;
+  return strings_win(terms, in_family, L, flips, group.size(), str.size() + diag.size());
 }
 
 }  // namespace
