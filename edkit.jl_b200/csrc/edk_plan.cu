@@ -125,14 +125,21 @@ __global__ void __launch_bounds__(256, plan_min_blocks<BK, VT>())
 }
 
 // Several columns at once (blockIdx.y = group of kPlanCols columns): a target is
-// located once for all of them.  Taken for eight and more real columns: the
-// gathers themselves, one L1 line each whatever the kernel, are most of the time,
-// so a group pays only where it is full and its rows fill the GPU (whole product,
-// FP64: 8 columns of 400,000 rank-searched rows 113 -> 89 us, 16 of 184,756
-// complete-sector rows 72.8 -> 64.5, 13 single-precision of 48,620 33.5 -> 31.9;
-// but 5 of 48,620 27.8 -> 29.9, and complex columns 112 -> 120).
+// located once for all of them.  Taken for eight and more real columns (5 of 48,620
+// rows 27.8 -> 29.9 us a product, complex columns 112 -> 120) whose groups and windows
+// make two blocks per SM, one where rows have more than nearest neighbours: fewer, and the single-column kernel's larger number of
+// blocks counts for more than its repeated searches.  FP64, one by one / grouped:
+// 16 columns of 924 rows 24.9 / 26.9, of 12,870 28.4 / 29.3, of 48,620 35.8 / 38.9,
+// of 184,756 74 / 65, of 400,024 rank-searched 196 / 143; 31 of 12,870 rows with two
+// families 40.8 / 36.2; single precision, 13 of 48,620 34.0 / 32.8, of 12,870 with two
+// families 27.3 / 25.5.
+// A last group of two or three columns repeats its last one (11 of 400,024 rows: 111
+// us, 124 with the three one by one); a single column goes alone where the windows
+// fill the GPU by themselves (9 of 400,024 rows 107 -> 100 us, of 705,432 135 -> 122;
+// but of 112,720 48.6 -> 50.8: the second launch).
 constexpr int kPlanCols = 4;
 constexpr int64_t kPlanColsMin = 8;
+constexpr int kPlanColsBlocks = 4;  // resident blocks per SM of the grouped kernel
 
 template <int BK, class VT, int NN, int NC>
 __global__ void __launch_bounds__(256, (sizeof(VT) == 4 && NN == 1) ? 5 : 4)
@@ -176,17 +183,23 @@ edk_status launch_plan_nn(const BasisDev& b, const OpDev& op, const FFParams& ff
   }
   const int64_t nwin = (slot1 - slot0) / kPlanWindow;
   if constexpr (!VTraits<VT>::cx) {
-    if (nvec >= kPlanColsMin) {
-      constexpr int NC = kPlanCols;
-      const unsigned gc = (unsigned)std::min<int64_t>(nwin, (int64_t)sm_count() * 4);
-      for (int64_t k0 = 0; k0 < nvec; k0 += (int64_t)NC * 65535) {
-        const int64_t nk = std::min<int64_t>(nvec - k0, (int64_t)NC * 65535);
+    constexpr int NC = kPlanCols;
+    const int64_t nsm = sm_count();
+    if (nvec >= kPlanColsMin && nwin * ((nvec + NC - 1) / NC) >= (NN == 1 ? 2 : 1) * nsm) {
+      const unsigned gc = (unsigned)std::min<int64_t>(nwin, nsm * kPlanColsBlocks);
+      const bool alone = nvec % NC == 1 && nwin >= nsm * kPlanColsBlocks;
+      const int64_t grouped = alone ? nvec - 1 : nvec;
+      for (int64_t k0 = 0; k0 < grouped; k0 += (int64_t)NC * 65535) {
+        const int64_t nk = std::min<int64_t>(grouped - k0, (int64_t)NC * 65535);
         k_apply_plan_cols<BK, VT, NN, NC>
             <<<dim3(gc, (unsigned)((nk + NC - 1) / NC)), kPlanWindow, 0, st>>>(
                 b, op, ff, X + k0 * ldx, Y + k0 * ldy, ldx, ldy, accumulate, (int)nk, slot0, slot1);
         EDK_TRY_CUDA(cudaGetLastError());
       }
-      return EDK_OK;
+      if (!alone) return EDK_OK;
+      X += grouped * ldx;
+      Y += grouped * ldy;
+      nvec = 1;
     }
   }
   const unsigned gx = (unsigned)std::min<int64_t>(nwin, (int64_t)sm_count() * per_sm);
