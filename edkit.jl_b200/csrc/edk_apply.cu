@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(256) k_apply(BasisDev b, OpDev op, const VT* _
 // Lanes per row of the general gather kernel.  A row is a serial chain of
 // lookups, so a small sector with one lane per row leaves most of the GPU
 // idle: lanes share a row while the rows times the lanes still fit two rounds
-// of the resident threads (148 x 2,048).  Symmetry groups, whose lookup is the
+// of the resident threads (2,048 per SM).  Symmetry groups, whose lookup is the
 // longest, take sixteen or four lanes, the others eight.
 // (k, p, z) group sector of L = 22, some 8,360 rows, real vector: 621 us with
 // one lane per row and every group element stepped through the generators, 45
@@ -65,7 +65,9 @@ __global__ void __launch_bounds__(256) k_apply(BasisDev b, OpDev op, const VT* _
 // lanes and rotations compared at the zero-run tops (runs_arg32).
 template <int BK> constexpr int many_lanes() { return BK == BK_ABELIAN ? 16 : 8; }
 template <int BK> constexpr int few_lanes() { return BK == BK_ABELIAN ? 4 : 1; }
-bool lanes_fit(int64_t rows, int lanes) { return rows * lanes <= (int64_t)2 * 148 * 2048; }
+bool lanes_fit(const BasisDev& b, int64_t rows, int lanes) {
+  return rows * lanes <= (int64_t)2 * b.sms * 2048;
+}
 
 // Resident blocks per SM asked of the compiler: the rank-search kernels are
 // latency bound and fit 32 registers (8 blocks of 256 threads fill every warp
@@ -161,8 +163,8 @@ edk_status launch_apply(const BasisDev& b, const OpDev& op, const void* x, void*
       <<<dim3(apply_grid(b.D * (GATHER ? (T) : 1)), (unsigned)nk), 256, 0, st>>>(              \
           b, op, Xk, Yk, ldx, ldy, accumulate);
 #define EDK_APPLY_S(BK, S)                                                                     \
-  if (GATHER && lanes_fit(rows, many_lanes<BK>())) { EDK_APPLY_T(BK, S, many_lanes<BK>()) }    \
-  else if (GATHER && lanes_fit(rows, few_lanes<BK>())) { EDK_APPLY_T(BK, S, few_lanes<BK>()) } \
+  if (GATHER && lanes_fit(b, rows, many_lanes<BK>())) { EDK_APPLY_T(BK, S, many_lanes<BK>()) }    \
+  else if (GATHER && lanes_fit(b, rows, few_lanes<BK>())) { EDK_APPLY_T(BK, S, few_lanes<BK>()) } \
   else { EDK_APPLY_T(BK, S, 1) }
 #define EDK_APPLY(BK)                       \
   case BK:                                  \
@@ -618,8 +620,8 @@ bool strings_give_entries(const std::vector<HostTerm>& terms, const std::vector<
 // fields of x and z 41 / 89, 19 projected flips of two sites 58 / 65, 18 of three 68 /
 // 72, 17 of four 94 / 67; dense two-site terms 30 / 23 (one) and 128 / 114 (19),
 // three-site 53 / 26 and 196 / 86 (eight), four-site 131 / 34 and 219 / 48 (two).
-bool strings_win(const std::vector<HostTerm>& terms, const std::vector<char>& in_family, int L,
-                 const PauliFlips& flips, size_t groups, size_t strings) {
+bool strings_win(const std::vector<HostTerm>& terms, const std::vector<char>& in_family,
+                 const BasisDev& b, const PauliFlips& flips, size_t groups, size_t strings) {
   double rows = 0.0;
   for (size_t t = 0; t < terms.size(); ++t) {
     const HostTerm& h = terms[t];
@@ -630,7 +632,7 @@ bool strings_win(const std::vector<HostTerm>& terms, const std::vector<char>& in
     const double entries = (double)off / h.dim;
     rows += in_family[t] ? 38.0 * entries : 24.0 + 9.0 * entries;
   }
-  if (lanes_fit((int64_t)1 << L, many_lanes<BK_TENSOR>())) rows *= 0.35;
+  if (lanes_fit(b, b.D, many_lanes<BK_TENSOR>())) rows *= 0.35;
   return 4.0 * flips.n + 5.5 * strings + 6.0 * groups <= rows;
 }
 
@@ -639,9 +641,10 @@ bool strings_win(const std::vector<HostTerm>& terms, const std::vector<char>& in
 // kPauliMax (tables and host time), they do not give the matrix elements back, or the
 // terms cost less.
 constexpr size_t kPauliMax = 512;
-bool pauli_strings(const std::vector<HostTerm>& terms, const std::vector<char>& in_family, int L,
-                   PauliFlips& flips, std::vector<PauliGroup>& group,
+bool pauli_strings(const std::vector<HostTerm>& terms, const std::vector<char>& in_family,
+                   const BasisDev& b, PauliFlips& flips, std::vector<PauliGroup>& group,
                    std::vector<PauliStr>& str, std::vector<PauliStr>& diag) {
+  const int L = b.L;
   PauliSum sum;
   for (size_t t = 0; t < terms.size(); ++t) {
     const HostTerm& h = terms[t];
@@ -688,7 +691,7 @@ bool pauli_strings(const std::vector<HostTerm>& terms, const std::vector<char>& 
       group.back().s1 = (int)str.size();
     }
   }
-  return strings_win(terms, in_family, L, flips, group.size(), str.size() + diag.size());
+  return strings_win(terms, in_family, b, flips, group.size(), str.size() + diag.size());
 }
 
 }  // namespace
@@ -911,7 +914,7 @@ extern "C" edk_status edk_operator_create(edk_basis* b, int32_t nterms, const in
   std::vector<PauliGroup> pgroup;
   std::vector<PauliStr> pstr, pdiag;
   op->pauli_ok = op->use_ff && op->gather && !op->ff_ok && b->dev.bk == BK_TENSOR && L <= 31 &&
-                 pauli_strings(terms, in_family, L, op->pauli_flips, pgroup, pstr, pdiag);
+                 pauli_strings(terms, in_family, b->dev, op->pauli_flips, pgroup, pstr, pdiag);
   auto upload = [&](DevBuf& buf, const void* src, size_t bytes) -> edk_status {
     if (bytes == 0) return EDK_OK;
     EDK_RETURN_IF(buf.alloc(bytes));

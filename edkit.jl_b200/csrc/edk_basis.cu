@@ -733,6 +733,7 @@ extern "C" edk_status edk_basis_create(const edk_basis_desc* desc, edk_basis** o
   b->desc.gen_inv = nullptr;
   b->desc.allow = nullptr;
   EDK_TRY_CUDA(cudaGetDevice(&b->device));
+  EDK_TRY_CUDA(cudaDeviceGetAttribute(&b->dev.sms, cudaDevAttrMultiProcessorCount, b->device));
   EDK_TRY_CUDA(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
   cudaStream_t st = b->stream;
   BasisDev& dv = b->dev;

@@ -496,7 +496,7 @@ static edk_status block_lanczos(int nops, edk_operator* const* ops,
   // rows per chunk of the split products: 2,048, fewer when that leaves the GPU
   // short of chunks (a chunk is one serial sum: 18 sectors of 2,700 rows with 36
   // chunks of 2,048 rows took 75 us a product, 11.9 us with four chunks per SM)
-  const int64_t Kfit = ((int64_t)nops * Dmax / (4 * 148) + 31) / 32 * 32;
+  const int64_t Kfit = ((int64_t)nops * Dmax / (4 * ops[0]->b->dev.sms) + 31) / 32 * 32;
   const int64_t Kc = std::min<int64_t>({2048, ((Dmax + 31) / 32) * 32, std::max<int64_t>(64, Kfit)});
   const int64_t S = (Dmax + Kc - 1) / Kc;
   const int64_t Dpad = S * Kc;

@@ -230,6 +230,7 @@ struct BasisDev {
   // us, 27 163 -> 148, 25 59.4 -> 57.7), below by latency and loses (22 sites 45.7
   // -> 48, 20 sites 34.5 -> 37.5).
   int runs_arg;
+  int sms;               // SMs of the device (host side: rules that fill the GPU)
   // abelian generators
   int ngen;
   const GenDev* gens;

@@ -149,11 +149,11 @@ edk_status launch_pauli(const edk_operator* op, const void* x, void* y, int64_t 
   const BasisDev& b = op->b->dev;
   const VT* X = static_cast<const VT*>(x);
   VT* Y = static_cast<VT*>(y);
-  // eight rows a thread once that leaves two blocks for every SM (148 x 4,096
+  // eight rows a thread once that leaves two blocks for every SM (4,096
   // rows), two below: small spaces need the blocks more than the wide tile
   // (four for double complex, whose eight rows do not fit the registers)
   constexpr int W = sizeof(VT) == 16 ? 4 : 8;
-  const bool wide = b.D >= (int64_t)148 * 4096;
+  const bool wide = b.D >= (int64_t)b.sms * 4096;
   const int64_t R = kPauliThreads * (wide ? W : 2);
   int nlow = 0;  // flips in ascending order
   while (nlow < op->pauli_flips.n && op->pauli_flips.x[nlow] < R) ++nlow;
