@@ -890,7 +890,7 @@ extern "C" edk_status edk_basis_create(const edk_basis_desc* desc, edk_basis** o
     } else if (b->kind == EDK_TRANSLATIONAL) {
       dv.bk = (b->Kmom == 0) ? BK_TRANS0 : BK_TRANS;
       const char* e = std::getenv("EDK_CANON_RUNS");
-      dv.runs_arg = (b->A == 1 && b->L <= 32 && b->D >= 150000) ? 1 : 0;
+      dv.runs_arg = (b->A == 1 && b->L <= 32 && b->D >= (int64_t)512 * dv.sms) ? 1 : 0;
       dv.runs_canon = (dv.bk == BK_TRANS0 && b->A == 1 && b->L <= 32 && e && e[0] == '1') ? 1 : 0;
     } else if (b->kind == EDK_TRANSPARITY) {
       dv.bk = BK_TRANSPAR;

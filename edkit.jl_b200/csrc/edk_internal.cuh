@@ -225,10 +225,13 @@ struct BasisDev {
   int phase_real;        // 1 when every phase is real
   int runs_canon;        // 1: canonicalise from zero-run tops (unit cell 1, phase-free)
   // 1: compare rotations at the zero-run tops where the shift counts too (unit cell
-  // 1, at least 150,000 rows).  Fewer, but serial, candidates: where rows fill the
-  // GPU the kernel is bound by issue and gains (c128 products: 28 sites 311 -> 279
-  // us, 27 163 -> 148, 25 59.4 -> 57.7), below by latency and loses (22 sites 45.7
-  // -> 48, 20 sites 34.5 -> 37.5).
+  // 1, at least 512 rows, two blocks, per SM).  Fewer, but serial, candidates: where
+  // rows fill the GPU the kernel is bound by issue and gains, below by latency and
+  // loses.  Products with nearest neighbours, every rotation -> zero-run tops, us
+  // (double / double complex): 2,704 rows 33.9 -> 34.8 / 33.7 -> 35.7; 32,066 45.0 ->
+  // 47.8 / 46.7 -> 48.1; 58,786 - / 48.9 -> 50.7; 81,752 43.7 -> 43.5 / 45.5 -> 45.5;
+  // 111,038 53.3 -> 49.3 / 52.7 -> 50.1; 204,248 68.4 -> 65.2 / 71.3 -> 66.7; 476,913
+  // 132 -> 114 / 136 -> 118; single precision and next-nearest neighbours alike.
   int runs_arg;
   int sms;               // SMs of the device (host side: rules that fill the GPU)
   // abelian generators
