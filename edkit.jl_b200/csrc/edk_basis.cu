@@ -363,7 +363,8 @@ __global__ void k_rank_map(BasisDev b, int K, uint64_t n, uint32_t* out) {
     } else if (b.bk == BK_TRANSPAR) {  // the coefficient rule of lookup<BK_TRANSPAR>
       uint32_t Iam, Ibm;
       int Rr, M;
-      canon_par32(s, b.L, b.A, b.len, mask, Iam, Rr, Ibm, M, b.A == 1);
+      if (b.A == 1) canon_par32<true>(s, b.L, b.A, b.len, mask, Iam, Rr, Ibm, M);
+      else canon_par32<false>(s, b.L, b.A, b.len, mask, Iam, Rr, Ibm, M);
       double n;
       if (Ibm < Iam) { key = Ibm; n = (double)b.P * __ldg(b.phase + M).x; }
       else { key = Iam; n = __ldg(b.phase + Rr).x; }

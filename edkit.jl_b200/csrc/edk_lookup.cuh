@@ -319,10 +319,13 @@ __device__ __forceinline__ uint32_t canon_arg32(uint32_t s, int L, int A, int le
 }
 // translations and reflected translations (TranslationParityBasis):
 // rev(rotr(s, i)) = rotl(rev(s), i) = rotr(rev(s), L - i).
+// RUNS: at the zero-run tops only (unit cell 1): the rank table's build, one lookup per
+// state of the charge sector.  The lookups of products compare every rotation.
+template <bool RUNS>
 __device__ __forceinline__ void canon_par32(uint32_t s, int L, int A, int len, uint32_t mask,
-                                            uint32_t& Iam, int& Rr, uint32_t& Ibm, int& M, bool runs) {
+                                            uint32_t& Iam, int& Rr, uint32_t& Ibm, int& M) {
   const uint32_t rs = __brev(s) >> (32 - L);
-  if (runs) {
+  if constexpr (RUNS) {
     Iam = runs_arg32<false>(s, L, mask, Rr);
     Ibm = runs_arg32<true>(rs, L, mask, M);
     return;
@@ -477,7 +480,7 @@ __device__ __forceinline__ bool lookup(const BasisDev& b, S s, const uint32_t* b
     int Rr = 0, M = 0;
     if constexpr (sizeof(S) == 4) {
       uint32_t a_, b_;
-      canon_par32(s, b.L, b.A, b.len, mask, a_, Rr, b_, M, b.runs_arg != 0);
+      canon_par32<false>(s, b.L, b.A, b.len, mask, a_, Rr, b_, M);
       Iam = a_; Ibm = b_;
     } else {
       S Ia0 = s, t = s;

@@ -205,7 +205,7 @@ __device__ __forceinline__ void canon_ctx(const BasisDev& b, uint32_t s, HitCtx&
   } else if constexpr (BK == BK_TRANSPAR) {
     uint32_t Iam, Ibm;
     int Rr, M;
-    canon_par32(s, b.L, b.A, b.len, mask, Iam, Rr, Ibm, M, b.runs_arg != 0);
+    canon_par32<false>(s, b.L, b.A, b.len, mask, Iam, Rr, Ibm, M);
     if (Ibm < Iam) { c.key = Ibm; c.pre = (double)b.P * __ldg(b.phase + M).x; }
     else { c.key = Iam; c.pre = __ldg(b.phase + Rr).x; }
   } else {

@@ -47,7 +47,7 @@ __device__ __forceinline__ bool sell_target(const BasisDev& b, uint32_t s, const
     } else if constexpr (BK == BK_TRANSPAR) {
       uint32_t Iam, Ibm;
       int Rr, M;
-      canon_par32(s, b.L, b.A, b.len, mask, Iam, Rr, Ibm, M, b.runs_arg != 0);
+      canon_par32<false>(s, b.L, b.A, b.len, mask, Iam, Rr, Ibm, M);
       double n;
       if (Ibm < Iam) { key = Ibm; n = (double)b.P * __ldg(b.phase + M).x; }
       else { key = Iam; n = __ldg(b.phase + Rr).x; }
