@@ -375,7 +375,8 @@ edk_status gram_spectrum(edk_basis* b, const void* M_d, bool cm, uint64_t dA, ui
                                &one, reinterpret_cast<const double*>(M_d), lda, &zero,
                                G.as<double>(), n));
   }
-  // matrices that fit the SMs' shared memory, then the library for the larger ones
+  // matrices that fit the SMs' shared memory; the library for the larger ones, and where
+  // the blocks of one launch could not meet (G is as it was)
   const edk_status own = hermitian_eigvals(cm, n, G.p, W.as<double>(), st);
   if (own != EDK_OK && own != EDK_UNSUPPORTED) return own;
   if (own == EDK_UNSUPPORTED) {
