@@ -182,13 +182,16 @@ __global__ void __launch_bounds__(kEigThreads, 1) k_tridiagonalise(
     const double ar = re(alpha), ai = im(alpha);
     double beta, inv_r = 0.0, inv_i = 0.0;
     T taun;
-    if (s > 0.0) {
+    // (a column below 1e-140 of the matrix, whose squares leave the range of doubles, is
+    // dropped: its reflector would not be unitary in what bits are left, and it meets
+    // entries of size one)
+    if (s > 0.0 && ar * ar + ai * ai + s > 1e-280) {
       beta = -copysign(sqrt(ar * ar + ai * ai + s), ar);
       mk(taun, (beta - ar) / beta, -ai / beta);
       const double q = (ar - beta) * (ar - beta) + ai * ai;
       inv_r = (ar - beta) / q;
       inv_i = -ai / q;
-    } else {  // nothing to eliminate (a phase of beta does not move eigenvalues)
+    } else {  // nothing to eliminate, or nothing that counts (a phase of beta does not move eigenvalues)
       beta = sqrt(ar * ar + ai * ai);
       mk(taun, 0.0, 0.0);
     }
