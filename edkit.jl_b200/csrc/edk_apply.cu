@@ -701,9 +701,6 @@ using namespace edk;
 
 edk_operator::~edk_operator() {
   handles_unregister(handles);
-  // the plan goes back to its pool: products that other streams still run on it
-  // (edk_apply_async) have to end first, as cudaFree makes them
-  if (p_slab) cudaDeviceSynchronize();
   p_slab.reset();
   for (cudaEvent_t e : cevents) cudaEventDestroy(e);
   if (cstream) cudaStreamDestroy(cstream);

@@ -295,6 +295,25 @@ struct SellDev {
   const float2* vt32;      // the same table rounded to FP32
 };
 
+// Device memory of the row plans of a batch of operators.  The last of them to go gives
+// it back, on the device it lives on, whichever is current then, and after every
+// product that still runs there (edk_apply_async, on any stream): one synchronisation
+// for the batch.
+struct PlanSlab {
+  DevBuf buf;
+  int device = 0;
+  ~PlanSlab() {
+    if (!buf.p) return;
+    int prev = device;
+    cudaGetDevice(&prev);
+    if (prev != device) cudaSetDevice(device);
+    cudaDeviceSynchronize();
+    buf.pool_stream = nullptr;  // the stream it came from may be gone by now
+    buf.release();
+    if (prev != device) cudaSetDevice(prev);
+  }
+};
+
 constexpr int kPlanWindow = 256;  // rows per window of a row plan (and per thread block)
 // Device view of a row plan: slot k of window w describes row
 // rw[k] & kPlanRowMask of that window (rows sorted by their number of hits).
@@ -385,7 +404,7 @@ struct edk_operator {
   int tps = 1;            // threads per state of the fast path (1, 2 or 4; autotuned)
   // row plan of the fast path on rank-searched sectors (edk_plan.cu): built on
   // first use; plan_state 0 not built, 1 built, -1 not available
-  std::shared_ptr<edk::DevBuf> p_slab;  // shared by the operators of the batch that built it
+  std::shared_ptr<edk::PlanSlab> p_slab;  // shared by the operators of the batch that built it
   int plan_state = 0;
   // Pauli-string form (full space, no flip-flop fast path, few enough strings): the
   // fast kernel of such an operator, taken while use_ff

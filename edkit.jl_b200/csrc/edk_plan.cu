@@ -272,12 +272,10 @@ edk_status plan_ensure(const std::vector<edk_operator*>& ops, cudaStream_t st) {
   if (need.empty()) return EDK_OK;
   const size_t flags = total;
   total += need.size() * sizeof(int);
-  auto slab = std::make_shared<DevBuf>();
-  EDK_RETURN_IF(slab->alloc_async(total, st, keep_pool()));
-  // freed on the legacy stream, after the last operator has synchronised the
-  // device: the stream it came from may be gone by then
-  slab->pool_stream = nullptr;
-  char* base = slab->as<char>();
+  auto slab = std::make_shared<PlanSlab>();
+  slab->device = need[0]->b->device;
+  EDK_RETURN_IF(slab->buf.alloc_async(total, st, keep_pool()));
+  char* base = slab->buf.as<char>();
   int* bad = reinterpret_cast<int*>(base + flags);
   EDK_TRY_CUDA(cudaMemsetAsync(bad, 0, need.size() * sizeof(int), st));
   for (size_t i = 0; i < need.size(); ++i) {
