@@ -14,6 +14,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <memory>
+#include <set>
 #include <type_traits>
 
 #include "edk_rankrows.cuh"
@@ -251,38 +252,48 @@ bool plan_applies(const edk_operator* op) {
          (b.bk == BK_PROJ_RANK || b.packed) && op->plan_state >= 0;
 }
 
+// A batch's plans share allocations of up to this size (a larger plan has its own), so
+// what one operator that stays holds of the others' memory is bounded.
+constexpr size_t kPlanSlab = (size_t)64 << 20;
+
 // Build the plans of the operators that need one and have none yet (plan_state: 0
 // not built yet, 1 built, -1 not available for this operator).  Allocates and
-// synchronises: call it outside any stream capture.  All plans of a call share
-// one allocation and one synchronisation: the first solve of a new batch pays
+// synchronises: call it outside any stream capture.  The plans of a call share
+// allocations and one synchronisation: the first solve of a new batch pays
 // for them (96 chains of 12 to 20 sites: 21 ms one by one, 1.9 ms together).
 edk_status plan_ensure(const std::vector<edk_operator*>& ops, cudaStream_t st) {
   auto pad = [](size_t n) { return (n + 255) / 256 * 256; };
+  struct Place { size_t slab, at; };
   std::vector<edk_operator*> need;
-  std::vector<size_t> at;
-  size_t total = 0;
+  std::set<edk_operator*> seen;
+  std::vector<Place> place;
+  std::vector<size_t> size;  // of each slab
   for (edk_operator* op : ops) {
-    if (op->plan_state != 0 || plan_kind(op->b->dev) < 0) continue;
-    if (std::find(need.begin(), need.end(), op) != need.end()) continue;
+    if (op->plan_state != 0 || plan_kind(op->b->dev) < 0 || !seen.insert(op).second) continue;
     const size_t ns = (size_t)((op->b->D + kPlanWindow - 1) / kPlanWindow) * kPlanWindow;
+    const size_t n = pad(ns * sizeof(uint4)) + (op->ngeneric > 0 ? pad(ns * 8) : 0);
+    if (size.empty() || size.back() + n > kPlanSlab) size.push_back(0);
     need.push_back(op);
-    at.push_back(total);
-    total += pad(ns * sizeof(uint4)) + (op->ngeneric > 0 ? pad(ns * 8) : 0);
+    place.push_back({size.size() - 1, size.back()});
+    size.back() += n;
   }
   if (need.empty()) return EDK_OK;
-  const size_t flags = total;
-  total += need.size() * sizeof(int);
-  auto slab = std::make_shared<PlanSlab>();
-  slab->device = need[0]->b->device;
-  EDK_RETURN_IF(slab->buf.alloc_async(total, st, keep_pool()));
-  char* base = slab->buf.as<char>();
-  int* bad = reinterpret_cast<int*>(base + flags);
+  std::vector<std::shared_ptr<PlanSlab>> slabs;
+  for (size_t n : size) {
+    slabs.push_back(std::make_shared<PlanSlab>());
+    slabs.back()->device = need[0]->b->device;
+    EDK_RETURN_IF(slabs.back()->buf.alloc_async(std::max<size_t>(n, 1), st, keep_pool()));
+  }
+  auto where = [&](size_t i) { return slabs[place[i].slab]->buf.as<char>() + place[i].at; };
+  DevBuf flags;
+  EDK_RETURN_IF(flags.alloc_async(need.size() * sizeof(int), st));
+  int* bad = flags.as<int>();
   EDK_TRY_CUDA(cudaMemsetAsync(bad, 0, need.size() * sizeof(int), st));
   for (size_t i = 0; i < need.size(); ++i) {
     edk_operator* op = need[i];
     const int64_t ns = (op->b->D + kPlanWindow - 1) / kPlanWindow * kPlanWindow;
-    uint4* slot = reinterpret_cast<uint4*>(base + at[i]);
-    double* dg = op->ngeneric > 0 ? reinterpret_cast<double*>(base + at[i] + pad(ns * sizeof(uint4)))
+    uint4* slot = reinterpret_cast<uint4*>(where(i));
+    double* dg = op->ngeneric > 0 ? reinterpret_cast<double*>(where(i) + pad(ns * sizeof(uint4)))
                                   : nullptr;
     switch (plan_kind(op->b->dev)) {
       case BK_PROJ_RANK: launch_plan_build<BK_PROJ_RANK>(op, slot, dg, bad + i, st); break;
@@ -307,11 +318,11 @@ edk_status plan_ensure(const std::vector<edk_operator*>& ops, cudaStream_t st) {
     }
     const int64_t ns = (op->b->D + kPlanWindow - 1) / kPlanWindow * kPlanWindow;
     RowPlanDev& pl = op->dev.plan;
-    pl.slot = reinterpret_cast<uint4*>(base + at[i]);
-    pl.dg = op->ngeneric > 0 ? reinterpret_cast<double*>(base + at[i] + pad(ns * sizeof(uint4)))
+    pl.slot = reinterpret_cast<uint4*>(where(i));
+    pl.dg = op->ngeneric > 0 ? reinterpret_cast<double*>(where(i) + pad(ns * sizeof(uint4)))
                              : nullptr;
     pl.nslots = ns;
-    op->p_slab = slab;
+    op->p_slab = slabs[place[i].slab];
     op->plan_state = 1;
   }
   return EDK_OK;

@@ -52,3 +52,23 @@ def test_last_operator_goes_while_its_product_runs(ek):
         op * x  # plans where the first one was
     torch.cuda.synchronize()
     assert torch.equal(y, ref)
+
+
+def test_memory_of_a_batch_comes_back_with_its_operators(ek):
+    """Six plans of some 166 MB built together: five operators go, their memory comes
+    back (what the pool keeps for the next plans is 512 MB at most)."""
+    import torch
+    L = 26
+    B = ek.ProjectedBasis(L=L, N=L // 2)
+    bond = ek.spin((1.0, "xx"), (1.0, "yy"), (0.8, "zz"))
+    ops = [ek.operator([(1 + 0.1 * q) * bond] * (L - 1), [[i, i + 1] for i in range(1, L)], B)
+           for q in range(6)]
+    ev, _ = ek.batch_lanczos_e0(ops, m=2)
+    plan = 16 * B.size(1)
+    before = torch.cuda.mem_get_info()[0]
+    del ops[1:]
+    torch.cuda.synchronize()
+    back = torch.cuda.mem_get_info()[0] - before
+    assert back >= 5 * plan - (512 << 20) - (64 << 20)
+    # (alone the rows split differently over the blocks: other orders of summation)
+    assert abs(ek.batch_lanczos_e0(ops, m=2)[0][0, 0] - ev[0, 0]) < 1e-12
