@@ -28,11 +28,13 @@ __device__ __forceinline__ double bwsum(double v) {
 }
 
 // Shapes shared by the kernels: T_q has mq[q] blocks (at most mmax), rows
-// n_q = p * mq[q] (at most nmax); A and B hold mmax blocks per operator
-// (B_0 unused); V holds `vcols` columns of nmax rows per operator.
+// n_q = p * mq[q] (at most nmax); A and B hold block j of operator q at
+// (j nops + q) p^2 (B_0 unused), as the block Lanczos wrote its steps; V holds
+// `vcols` columns of nmax rows per operator.
 struct BandDims {
-  int p, mmax, vcols;
+  int p, nops, mmax, vcols;
   int64_t nmax;
+  __device__ size_t block(int q, int j) const { return ((size_t)j * nops + q) * p * p; }
 };
 
 // w = T v_k: a block takes G = blockDim.x / (3 p) block rows of operator q; of the
@@ -56,10 +58,9 @@ __global__ void k_band_mv(BandDims d, const double2* __restrict__ A, const doubl
   __syncthreads();
   double yr = 0.0, yi = 0.0;
   if (in) {
-    const size_t pp = (size_t)p * p;
     const double2* xs = sx + t * p;
     if (t < 2) {  // B_j x_{j-1}, A_j x_j
-      const double2* M = (t == 0 ? B : A) + ((size_t)q * d.mmax + jb) * pp + a;
+      const double2* M = (t == 0 ? B : A) + d.block(q, jb) + a;
 #pragma unroll 8
       for (int c = 0; c < p; ++c) {
         const double2 v = M[(size_t)c * p], xc = xs[c];
@@ -67,7 +68,7 @@ __global__ void k_band_mv(BandDims d, const double2* __restrict__ A, const doubl
         yi += v.x * xc.y + v.y * xc.x;
       }
     } else {  // B_{j+1}^H x_{j+1}: conj(B(c, a)) x_c
-      const double2* M = B + ((size_t)q * d.mmax + jb + 1) * pp + (size_t)a * p;
+      const double2* M = B + d.block(q, jb + 1) + (size_t)a * p;
 #pragma unroll 8
       for (int c = 0; c < p; ++c) {
         const double2 v = M[c], xc = xs[c];
@@ -273,12 +274,12 @@ __global__ void __launch_bounds__(256) k_band_sturm(BandDims d, const double2* _
   if (tid == 0) s_neg = 0;
   bool have_x = false;
   for (int j = tk.j0; j < m; ++j) {
-    const double2* Aj = A + ((size_t)q * d.mmax + j) * pp;
+    const double2* Aj = A + d.block(q, j);
     for (int e = tid; e < pp; e += nt) {
       double2 v = Aj[e];
       if (e % (p + 1) == 0) v.x -= tk.sigma;  // the diagonal entries a (p + 1)
       M[e] = v;
-      if (have_x) L[e] = B[((size_t)q * d.mmax + j) * pp + e];  // B_j, staged
+      if (have_x) L[e] = B[d.block(q, j) + e];  // B_j, staged
     }
     __syncthreads();
     if (have_x) {  // M -= B_j X
@@ -324,7 +325,7 @@ __global__ void __launch_bounds__(256) k_band_sturm(BandDims d, const double2* _
     if (j + 1 < m) {
       // X = M^{-1} B_{j+1}^H: column c (four lanes of one warp each, p a
       // multiple of 8 so a warp's columns are all inside or all outside)
-      const double2* Bn = B + ((size_t)q * d.mmax + j + 1) * pp;
+      const double2* Bn = B + d.block(q, j + 1);
       const int c = tid >> 2, part = tid & 3;
       if (c < p) {
         double2* x = X + (size_t)c * p;
@@ -371,40 +372,37 @@ __global__ void __launch_bounds__(256) k_band_sturm(BandDims d, const double2* _
   if (tid == 0) counts[blockIdx.x] = s_neg;
 }
 
-// T's blocks as the kernels read them, from the block Lanczos's per-step products:
-// SA[j][q] is (V_j^H W)^T column-major, so A_j(r, c) = SA[c + r p], made Hermitian;
-// SB[j][q] is B_j already.  diag[q] is the largest |A_j(a, a)| over all j, and over
-// j >= 1 in diag[nops + q] (at least one), as the bits of non-negative doubles.
-__global__ void __launch_bounds__(256) k_band_pack(BandDims d, int nops,
-                                                   const double2* __restrict__ SA,
-                                                   const double2* __restrict__ SB,
+// The diagonal blocks of the steps since the last call, from[q] .. mq[q] - 1, as the
+// kernels read them, in place: A[j][q] arrives as (V_j^H W)^T column-major, so A_j(r, c) =
+// A[c + r p], and is made Hermitian.  diag[q] rises to the largest |A_j(a, a)| over all j,
+// diag[nops + q] over j >= 1 (at least one), as the bits of non-negative doubles.
+__global__ void __launch_bounds__(256) k_band_pack(BandDims d, double2* __restrict__ A,
+                                                   const int* __restrict__ from,
                                                    const int* __restrict__ mq,
-                                                   double2* __restrict__ A, double2* __restrict__ B,
                                                    unsigned long long* __restrict__ diag) {
-  const int q = blockIdx.y, j = blockIdx.x, p = d.p, pp = p * p;
+  const int q = blockIdx.y, j = from[q] + blockIdx.x, p = d.p;
   if (j >= mq[q]) return;
-  const double2* a1 = SA + ((size_t)j * nops + q) * pp;
-  const double2* b1 = SB + ((size_t)j * nops + q) * pp;
-  double2* ao = A + ((size_t)q * d.mmax + j) * pp;
-  double2* bo = B + ((size_t)q * d.mmax + j) * pp;
-  for (int e = threadIdx.x; e < pp; e += blockDim.x) {
+  double2* a = A + d.block(q, j);
+  for (int e = threadIdx.x; e < p * p; e += blockDim.x) {
     const int r = e % p, c = e / p;
-    const double2 x = a1[c + r * p], y = a1[r + c * p];  // A(r, c), A(c, r)
+    if (r > c) continue;
+    const double2 x = a[c + r * p], y = a[r + c * p];  // A(r, c), A(c, r)
     const double2 h = make_double2(0.5 * (x.x + y.x), 0.5 * (x.y - y.y));
-    ao[e] = h;
-    if (j >= 1) bo[e] = b1[e];
-    if (r == c) {
+    a[r + c * p] = h;
+    if (r != c) {
+      a[c + r * p] = make_double2(h.x, -h.y);
+    } else {
       const unsigned long long v = (unsigned long long)__double_as_longlong(fmax(1.0, fabs(h.x)));
       atomicMax(diag + q, v);
-      if (j >= 1) atomicMax(diag + nops + q, v);
+      if (j >= 1) atomicMax(diag + d.nops + q, v);
     }
   }
 }
 
 }  // namespace
 
-edk_status band_lowest_device(int p, int nev, const std::vector<int>& m, const void* SA,
-                              const void* SB, cudaStream_t st,
+edk_status band_lowest_device(int p, int nev, const std::vector<int>& m, void* SA, const void* SB,
+                              BandState& state, cudaStream_t st,
                               std::vector<std::vector<double>>& out) {
   const int nops = (int)m.size();
   out.assign(nops, std::vector<double>(nev, NAN));
@@ -415,17 +413,20 @@ edk_status band_lowest_device(int p, int nev, const std::vector<int>& m, const v
   }
   BandDims d;
   d.p = p;
+  d.nops = nops;
   d.mmax = std::max(1, *std::max_element(m.begin(), m.end()));
   d.nmax = (int64_t)p * d.mmax;
   const int kmax = (int)std::min<int64_t>(d.nmax, kBandSteps);
   d.vcols = kmax + 1;
   const size_t pp = (size_t)p * p;
-  DevBuf dA, dB, dmax, V, w, s1, s2, alpha, beta, stop, nq, mqd;
-  const size_t ab = (size_t)nops * d.mmax * pp * sizeof(double2);
-  EDK_RETURN_IF(dA.alloc_async(ab, st));
-  EDK_RETURN_IF(dB.alloc_async(ab, st));
-  EDK_RETURN_IF(dmax.alloc_async(2 * (size_t)nops * 8, st));
-  EDK_TRY_CUDA(cudaMemsetAsync(dmax.p, 0, 2 * (size_t)nops * 8, st));
+  DevBuf V, w, s1, s2, alpha, beta, stop, nq, mqd, from;
+  double2* dA = static_cast<double2*>(SA);
+  const double2* dB = static_cast<const double2*>(SB);
+  if (state.packed.empty()) {
+    state.packed.assign(nops, 0);
+    EDK_RETURN_IF(state.diag.alloc_async(2 * (size_t)nops * 8, st));
+    EDK_TRY_CUDA(cudaMemsetAsync(state.diag.p, 0, 2 * (size_t)nops * 8, st));
+  }
   std::vector<int> hn(nops);
   for (int q = 0; q < nops; ++q) hn[q] = p * m[q];
   EDK_RETURN_IF(V.alloc_async((size_t)nops * d.vcols * d.nmax * sizeof(double2), st));
@@ -439,12 +440,18 @@ edk_status band_lowest_device(int p, int nev, const std::vector<int>& m, const v
   EDK_RETURN_IF(mqd.alloc_async((size_t)nops * sizeof(int), st));
   EDK_TRY_CUDA(cudaMemcpyAsync(nq.p, hn.data(), nops * sizeof(int), cudaMemcpyHostToDevice, st));
   EDK_TRY_CUDA(cudaMemcpyAsync(mqd.p, m.data(), nops * sizeof(int), cudaMemcpyHostToDevice, st));
-  k_band_pack<<<dim3(d.mmax, nops), 256, 0, st>>>(
-      d, nops, static_cast<const double2*>(SA), static_cast<const double2*>(SB), mqd.as<int>(),
-      dA.as<double2>(), dB.as<double2>(), dmax.as<unsigned long long>());
-  EDK_TRY_CUDA(cudaGetLastError());
+  EDK_RETURN_IF(from.alloc_async((size_t)nops * sizeof(int), st));
+  EDK_TRY_CUDA(cudaMemcpyAsync(from.p, state.packed.data(), nops * sizeof(int),
+                               cudaMemcpyHostToDevice, st));
+  int fresh = 0;
+  for (int q = 0; q < nops; ++q) fresh = std::max(fresh, m[q] - state.packed[q]);
+  if (fresh > 0) {
+    k_band_pack<<<dim3(fresh, nops), 256, 0, st>>>(d, dA, from.as<int>(), mqd.as<int>(),
+                                                   state.diag.as<unsigned long long>());
+    EDK_TRY_CUDA(cudaGetLastError());
+  }
   std::vector<double> hmax(2 * (size_t)nops);
-  EDK_TRY_CUDA(cudaMemcpyAsync(hmax.data(), dmax.p, hmax.size() * 8, cudaMemcpyDeviceToHost, st));
+  EDK_TRY_CUDA(cudaMemcpyAsync(hmax.data(), state.diag.p, hmax.size() * 8, cudaMemcpyDeviceToHost, st));
   EDK_TRY_CUDA(cudaMemsetAsync(stop.p, 0, nops * sizeof(int), st));
   EDK_TRY_CUDA(cudaMemsetAsync(V.p, 0, (size_t)nops * d.vcols * d.nmax * sizeof(double2), st));
   // start vectors: the host form's seeded sequence, normalised, in column 0
@@ -472,6 +479,7 @@ edk_status band_lowest_device(int p, int nev, const std::vector<int>& m, const v
     }
     EDK_TRY_CUDA(cudaStreamSynchronize(st));
   }
+  state.packed = m;
   // Lanczos on every T in lockstep; the host looks every 10 steps (and at
   // each operator's own last step), as the host form does
   std::vector<std::vector<double>> prev(nops), cand(nops);
@@ -487,7 +495,7 @@ edk_status band_lowest_device(int p, int nev, const std::vector<int>& m, const v
   int left = nops;
   for (int k = 0; k < kmax && left > 0; ++k) {
     k_band_mv<<<dim3((d.mmax + G - 1) / G, nops), 3 * G * p, 6 * G * p * sizeof(double2), st>>>(
-        d, dA.as<double2>(), dB.as<double2>(), mqd.as<int>(), V.as<double2>(), k, w.as<double2>(),
+        d, dA, dB, mqd.as<int>(), V.as<double2>(), k, w.as<double2>(),
         stop.as<int>());
     k_band_dots<<<dim3((k + 8) / 8, nops), 256, 0, st>>>(d, nq.as<int>(), V.as<double2>(), k,
                                                         w.as<double2>(), s1.as<double2>(),
@@ -596,7 +604,7 @@ edk_status band_lowest_device(int p, int nev, const std::vector<int>& m, const v
     // the largest block's size (p = 64), the same from every calling thread
     EDK_TRY_CUDA(cudaFuncSetAttribute(k_band_sturm, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)(3 * 64 * 64 * sizeof(double2) + 64 * sizeof(double))));
-    k_band_sturm<<<(unsigned)tasks.size(), 256, smem, st>>>(d, dA.as<double2>(), dB.as<double2>(),
+    k_band_sturm<<<(unsigned)tasks.size(), 256, smem, st>>>(d, dA, dB,
                                                              mqd.as<int>(), dt.as<BandTask>(),
                                                              dc.as<int>());
     EDK_TRY_CUDA(cudaGetLastError());

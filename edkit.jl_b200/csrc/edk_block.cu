@@ -676,12 +676,13 @@ static edk_status block_lanczos(int nops, edk_operator* const* ops,
   bool converged = false;
 
   // eigenvalues of every operator's block tridiagonal T, on the device
+  BandState bands;
   auto extract = [&](int nsteps) -> edk_status {
     const double te = wall_s();
     std::vector<int> mqs(nops);
     for (int q = 0; q < nops; ++q) mqs[q] = broke_at[q] >= 0 ? broke_at[q] : nsteps;
     std::vector<std::vector<double>> res;
-    EDK_RETURN_IF(band_lowest_device(p, o.nev, mqs, SA.p, SB.p, st, res));
+    EDK_RETURN_IF(band_lowest_device(p, o.nev, mqs, SA.p, SB.p, bands, st, res));
     for (int q = 0; q < nops; ++q)
       for (int k = 0; k < o.nev; ++k) cur[(size_t)q * o.nev + k] = res[q][k];
     t_eig += wall_s() - te;

@@ -527,10 +527,15 @@ void handles_unregister(bool registered);
 int tridiag_eigvals(int m, const double* a, const double* b, double* w);
 // The lowest `nev` distinct eigenvalues of block-tridiagonal Hermitian matrices
 // (edk_band.cu): operator q has m[q] blocks; SA and SB (device) hold step j's
-// p x p products of operator q at (j nops + q) p^2, see k_band_pack; NaN where
+// p x p products of operator q at (j nops + q) p^2.  SA's steps are brought into their
+// final form in place (k_band_pack); `state`, one per run, keeps how far.  NaN where
 // fewer are found.
-edk_status band_lowest_device(int p, int nev, const std::vector<int>& m, const void* SA,
-                              const void* SB, cudaStream_t st,
+struct BandState {
+  std::vector<int> packed;  // steps of each operator in their final form
+  DevBuf diag;              // largest diagonal entries so far
+};
+edk_status band_lowest_device(int p, int nev, const std::vector<int>& m, void* SA, const void* SB,
+                              BandState& state, cudaStream_t st,
                               std::vector<std::vector<double>>& out);
 int tridiag_eigen(int m, const double* a, const double* b, double* w, double* Q);
 int tridiag_first_row(int m, const double* a, const double* b, double* w, double* z);

@@ -202,7 +202,10 @@ edk_status edk_operator_materialize(edk_operator* op, int32_t enable, int64_t* e
  * Hermitian in the row-gather form and block * max_steps below its dimension.
  * tol > 0 stops when every operator's nev values move less than
  * tol * max(1, |E0|) between checks (every check_every steps); tol = 0 runs
- * max_steps.  No reference counterpart (EDKit runs one vector). */
+ * max_steps.  Device memory, in bytes, with D the largest dimension: 3 x 16 nops D
+ * block for the vectors, 32 nops max_steps block^2 for T, held for the whole run, and
+ * 16 nops n min(n, 1201) with n = block * steps for an eigenvalue step.  What does not
+ * fit ends in EDK_OOM.  No reference counterpart (EDKit runs one vector). */
 typedef struct {
   int32_t block;        /* vectors per operator: multiple of 8, 8..64 */
   int32_t max_steps;    /* block steps */
