@@ -39,6 +39,10 @@ namespace edk {
 namespace {
 
 constexpr int kTile = 256;          // rows per matvec / update tile
+// Steps of a run, as edk.h has it.  No kernel needs a limit; a longer run would spend
+// its time in T's eigenvalues (a chain of as many dependent multiply-adds a count).
+// Krylov bases, which look at no eigenvalues here, may have more vectors.
+constexpr int kMaxSteps = 12791;
 // resident reorthogonalisation blocks per SM (128 registers a thread)
 constexpr int kSplitBlocks = 2;
 
@@ -1049,11 +1053,6 @@ struct BatchEngine {
 
   // Size the reorthogonalisation grid to what is resident at once.
   edk_status split_rows() {
-    // (a step's coefficients once sat whole in shared memory; the limit stays)
-    if ((size_t)(ncap + 8) * sizeof(double2) > 200 * 1024) {
-      set_error("batch Lanczos: too many steps for the shared-memory coefficients (max 12791)");
-      return EDK_UNSUPPORTED;
-    }
     int dev = 0;
     EDK_TRY_CUDA(cudaGetDevice(&dev));
     EDK_TRY_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
@@ -1485,6 +1484,10 @@ edk_status batch_lanczos(const std::vector<edk_operator*>& ops, const edk_lanczo
     bk = bk == BK_TRANS0 ? BK_TRANS0_RANK : (bk == BK_TRANS ? BK_TRANS_RANK : BK_TRANSPAR_RANK);
   if (bk == BK_ABELIAN && !all_mat) {
     set_error("batch Lanczos: symmetry-group (abelian) bases run one at a time unless materialised");
+    return EDK_UNSUPPORTED;
+  }
+  if (o.max_steps > kMaxSteps) {
+    set_error("batch Lanczos: at most " + std::to_string(kMaxSteps) + " steps");
     return EDK_UNSUPPORTED;
   }
   (void)Dmin;  // operators smaller than max_steps stop by the breakdown rule
