@@ -542,6 +542,9 @@ __global__ void __launch_bounds__(256) k_breduce2(const SplitOp* __restrict__ sp
   if (done[q]) return;
   const int j = *step, lane = threadIdx.x & 31;
   const SplitOp& o = sp[q];
+  // of the step before, for the last block (read here, behind the sums' loads)
+  const double aprev = j > 0 ? alpha[(int64_t)q * m + j - 1] : 0.0;
+  const double bprev = j > 0 ? beta[(int64_t)q * m + j - 1] : 0.0;
   double2* csq = cs + (int64_t)q * ncap;
   double2* ceq = ce + (int64_t)q * ncap;
   for (int c = blockIdx.x * 8 + (threadIdx.x >> 5); c <= j; c += gridDim.x * 8) {
@@ -597,12 +600,10 @@ __global__ void __launch_bounds__(256) k_breduce2(const SplitOp* __restrict__ sp
   const double2 uu = __ldcg(csq + j), uw = __ldcg(ceq + j);
   const double a2 = uu.x - ss;
   if (j > 0) {  // (NaN runs on)
-    double* bj = beta + (int64_t)q * m + j - 1;
-    const double left = *bj * sqrt(a2 < 0.0 ? 0.0 : a2), a = alpha[(int64_t)q * m + j - 1];
-    if (a2 <= kInSpan * uu.x || left <= kBreakdown * fmax(1.0, fabs(a))) {
-      __syncthreads();  // beta_{j-1} is read
+    const double left = bprev * sqrt(a2 < 0.0 ? 0.0 : a2);
+    if (a2 <= kInSpan * uu.x || left <= kBreakdown * fmax(1.0, fabs(aprev))) {
       if (threadIdx.x == 0) {
-        *bj = 0.0;
+        beta[(int64_t)q * m + j - 1] = 0.0;
         done[q] = 2;  // (every block of the operator has read the flag: all have counted)
         cnt[q] = 0;
       }
@@ -619,7 +620,7 @@ __global__ void __launch_bounds__(256) k_breduce2(const SplitOp* __restrict__ sp
     ceq[c] = make_double2(r.x - (gx * s.x - gy * s.y), r.y - (gx * s.y + gy * s.x));
   }
   if (threadIdx.x == 0) {
-    const double last = j > 0 ? beta[(int64_t)q * m + j - 1] * __ldcg(csq + j - 1).x * inva : 0.0;
+    const double last = j > 0 ? bprev * __ldcg(csq + j - 1).x * inva : 0.0;
     alpha[(int64_t)q * m + j] = gx - last;
     scal[q] = make_double4(inva, gx, gy, 0.0);
     cnt[q] = 0;

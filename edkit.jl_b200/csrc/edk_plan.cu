@@ -278,16 +278,16 @@ edk_status plan_ensure(const std::vector<edk_operator*>& ops, cudaStream_t st) {
     size.back() += n;
   }
   if (need.empty()) return EDK_OK;
+  const size_t flags = size[0];  // the build's flags, at the end of the first
+  size[0] += need.size() * sizeof(int);
   std::vector<std::shared_ptr<PlanSlab>> slabs;
   for (size_t n : size) {
     slabs.push_back(std::make_shared<PlanSlab>());
     slabs.back()->device = need[0]->b->device;
-    EDK_RETURN_IF(slabs.back()->buf.alloc_async(std::max<size_t>(n, 1), st, keep_pool()));
+    EDK_RETURN_IF(slabs.back()->buf.alloc_async(n, st, keep_pool()));
   }
   auto where = [&](size_t i) { return slabs[place[i].slab]->buf.as<char>() + place[i].at; };
-  DevBuf flags;
-  EDK_RETURN_IF(flags.alloc_async(need.size() * sizeof(int), st));
-  int* bad = flags.as<int>();
+  int* bad = reinterpret_cast<int*>(slabs[0]->buf.as<char>() + flags);
   EDK_TRY_CUDA(cudaMemsetAsync(bad, 0, need.size() * sizeof(int), st));
   for (size_t i = 0; i < need.size(); ++i) {
     edk_operator* op = need[i];
