@@ -629,8 +629,10 @@ static edk_status lanczos_common(edk_operator* op, const edk_lanczos_opts* opts,
     EDK_RETURN_IF(batch_lanczos(one, o, src, v0_dtype, st, res, diag, gs_out));
     const OpResult& r = res[0];
     for (int q = 0; q < opts->nev; ++q) evals[q] = q < (int)r.ev.size() ? r.ev[q] : NAN;
-    if (alpha) for (int q = 0; q < r.steps; ++q) alpha[q] = r.a[q];
-    if (beta) for (int q = 0; q < r.steps; ++q) beta[q] = r.b[q];
+    // (a mixed run's FP64 refinement may take more steps than max_steps)
+    const int nc = std::min(r.steps, opts->max_steps);
+    if (alpha) std::copy_n(r.a.begin(), nc, alpha);
+    if (beta) std::copy_n(r.b.begin(), nc, beta);
     return EDK_OK;
   }
   bool cx = op->is_complex || opts->complex_vectors || is_cx(v0_dtype);
@@ -693,8 +695,9 @@ static edk_status lanczos_common(edk_operator* op, const edk_lanczos_opts* opts,
   }
   if (!mixed && gs_out) EDK_RETURN_IF(ritz_vector(E, R, gs_out));
   for (int q = 0; q < opts->nev; ++q) evals[q] = q < (int)ev.size() ? ev[q] : NAN;
-  if (alpha) for (int q = 0; q < R.steps; ++q) alpha[q] = R.a[q];
-  if (beta) for (int q = 0; q < R.steps; ++q) beta[q] = R.b[q];
+  const int nc = std::min(R.steps, opts->max_steps);
+  if (alpha) std::copy_n(R.a.begin(), nc, alpha);
+  if (beta) std::copy_n(R.b.begin(), nc, beta);
   if (diag) {
     diag->steps = R.steps;
     diag->steps_low = mixed ? steps_low : R.steps;

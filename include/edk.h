@@ -328,7 +328,8 @@ typedef struct {
 
 /* v0: starting vector (dtype v0_dtype, host or device); evals: nev values.
  * alpha/beta (optional, may be NULL): the last stage's recurrence
- * coefficients, max_steps entries each. */
+ * coefficients, max_steps entries each (the first ones, where the FP64 refinement of a
+ * mixed run took more steps). */
 edk_status edk_lanczos_e0(edk_operator* op, const edk_lanczos_opts* opts, const void* v0,
                           int32_t v0_dtype, int32_t ptr_kind, double* evals, double* alpha,
                           double* beta, edk_lanczos_diag* diag);
