@@ -78,7 +78,7 @@ def test_mul_into_a_target(ek, late, kind):
     assert out is td
     assert np.allclose(td.cpu().numpy(), ref, rtol=0, atol=1e-13 * np.abs(ref).max())
     with pytest.raises(TypeError, match="target dtype"):
-        ek.mul_(td.to(torch.float32), H, xd)
+        ek.mul_(torch.zeros(D, dtype=torch.float32, device="cuda"), H, xd)
 
 
 def test_mul_into_a_numpy_target_with_gaps(ek):
