@@ -920,8 +920,9 @@ struct BatchEngine {
   int64_t ntiles = 0, totalD = 0;
   int G = 1;             // blocks of the reorthogonalisation grid
   int nsm = 1;           // SMs of the device
-  DevBuf dops, tile2op, sblk2op, splitops, splitT, nfin, V, w, wt, part, cs, ce, scal, cnt, normpart, alpha, beta, invb,
-      done, step, nsteps, cbuf, cnc;
+  DevBuf maps, work;  // what the parts below lie in
+  DevBuf dops, tile2op, sblk2op, splitops, splitT, nfin, V, w, wt, part, cs, ce, scal, cnt,
+      normpart, alpha, beta, invb, done, step, nsteps, cbuf, cnc;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t gexec = nullptr;
   bool graph_ok = false;
@@ -992,17 +993,16 @@ struct BatchEngine {
     }
     totalD = woff;
     if (nops == 1 && !sell && ops[0]->pauli_ok && ops[0]->use_ff) pauli = ops[0];
-    EDK_RETURN_IF(dops.alloc_async(hops.size() * sizeof(BOp), st));
+    DevParts parts;
+    parts.add(dops, hops.size() * sizeof(BOp));
+    parts.add(tile2op, t2o.size() * 4);
+    if (sell) parts.add(sblk2op, std::max<size_t>(s2o.size(), 1) * 4);
+    EDK_RETURN_IF(parts.alloc(maps, st));
     EDK_TRY_CUDA(cudaMemcpyAsync(dops.p, hops.data(), hops.size() * sizeof(BOp),
                                  cudaMemcpyHostToDevice, st));
-    EDK_RETURN_IF(tile2op.alloc_async(t2o.size() * 4, st));
     EDK_TRY_CUDA(cudaMemcpyAsync(tile2op.p, t2o.data(), t2o.size() * 4, cudaMemcpyHostToDevice, st));
-    if (sell) {
-      EDK_RETURN_IF(sblk2op.alloc_async(std::max<size_t>(s2o.size(), 1) * 4, st));
-      if (!s2o.empty())
-        EDK_TRY_CUDA(cudaMemcpyAsync(sblk2op.p, s2o.data(), s2o.size() * 4,
-                                     cudaMemcpyHostToDevice, st));
-    }
+    if (sell && !s2o.empty())
+      EDK_TRY_CUDA(cudaMemcpyAsync(sblk2op.p, s2o.data(), s2o.size() * 4, cudaMemcpyHostToDevice, st));
     return EDK_OK;
   }
 
@@ -1024,29 +1024,31 @@ struct BatchEngine {
     side = ops[0]->cstream;
     EDK_TRY_CUDA(cudaEventCreateWithFlags(&checked, cudaEventDisableTiming));
     EDK_RETURN_IF(split_rows());
-    EDK_RETURN_IF(V.alloc_async((size_t)totalD * ncap * esz(vdt), st));
-    EDK_RETURN_IF(w.alloc_async((size_t)totalD * esz(wdt), st));
-    EDK_RETURN_IF(wt.alloc_async((size_t)totalD * esz(vdt), st));
+    DevParts parts;
+    parts.add(V, (size_t)totalD * ncap * esz(vdt));
+    parts.add(w, (size_t)totalD * esz(wdt));
+    parts.add(wt, (size_t)totalD * esz(vdt));
     // a block meets at most one operator more than it starts in: G + nops slots
-    EDK_RETURN_IF(part.alloc_async(2 * (size_t)(G + nops) * ncap * sizeof(double2), st));
-    EDK_RETURN_IF(splitops.alloc_async((size_t)nops * sizeof(SplitOp), st));
-    EDK_RETURN_IF(splitT.alloc_async(2 * sizeof(int64_t), st));
-    EDK_RETURN_IF(nfin.alloc_async(sizeof(unsigned), st));
+    parts.add(part, 2 * (size_t)(G + nops) * ncap * sizeof(double2));
+    parts.add(splitops, (size_t)nops * sizeof(SplitOp));
+    parts.add(splitT, 2 * sizeof(int64_t));
+    parts.add(nfin, sizeof(unsigned));
+    parts.add(cs, (size_t)nops * ncap * sizeof(double2));
+    parts.add(ce, (size_t)nops * ncap * sizeof(double2));
+    parts.add(scal, (size_t)nops * sizeof(double4));
+    parts.add(cnt, (size_t)nops * sizeof(unsigned));
+    parts.add(normpart, (size_t)(G + nops) * sizeof(double));
+    parts.add(alpha, (size_t)nops * m * sizeof(double));
+    parts.add(beta, (size_t)nops * m * sizeof(double));
+    parts.add(invb, (size_t)nops * sizeof(double));
+    parts.add(done, (size_t)nops * sizeof(int));
+    parts.add(nsteps, (size_t)nops * sizeof(int));
+    parts.add(step, sizeof(int));
+    parts.add(cbuf, (size_t)nops * ncap * sizeof(double2));
+    parts.add(cnc, (size_t)nops * sizeof(int));
+    EDK_RETURN_IF(parts.alloc(work, st));
     EDK_TRY_CUDA(cudaMemsetAsync(nfin.p, 0, sizeof(unsigned), st));
-    EDK_RETURN_IF(cs.alloc_async((size_t)nops * ncap * sizeof(double2), st));
-    EDK_RETURN_IF(ce.alloc_async((size_t)nops * ncap * sizeof(double2), st));
-    EDK_RETURN_IF(scal.alloc_async((size_t)nops * sizeof(double4), st));
-    EDK_RETURN_IF(cnt.alloc_async((size_t)nops * sizeof(unsigned), st));
     EDK_TRY_CUDA(cudaMemsetAsync(cnt.p, 0, (size_t)nops * sizeof(unsigned), st));
-    EDK_RETURN_IF(normpart.alloc_async((size_t)(G + nops) * sizeof(double), st));
-    EDK_RETURN_IF(alpha.alloc_async((size_t)nops * m * sizeof(double), st));
-    EDK_RETURN_IF(beta.alloc_async((size_t)nops * m * sizeof(double), st));
-    EDK_RETURN_IF(invb.alloc_async((size_t)nops * sizeof(double), st));
-    EDK_RETURN_IF(done.alloc_async((size_t)nops * sizeof(int), st));
-    EDK_RETURN_IF(nsteps.alloc_async((size_t)nops * sizeof(int), st));
-    EDK_RETURN_IF(step.alloc_async(sizeof(int), st));
-    EDK_RETURN_IF(cbuf.alloc_async((size_t)nops * ncap * sizeof(double2), st));
-    EDK_RETURN_IF(cnc.alloc_async((size_t)nops * sizeof(int), st));
     EDK_TRY_CUDA(cudaMemsetAsync(alpha.p, 0, (size_t)nops * m * sizeof(double), st));
     EDK_TRY_CUDA(cudaMemsetAsync(beta.p, 0, (size_t)nops * m * sizeof(double), st));
     return EDK_OK;
@@ -1322,10 +1324,12 @@ edk_status run_batch(BatchEngine& E, int max_steps, int nev, double tol, int che
   const int nops = E.nops;
   res.assign(nops, OpResult{});
   EDK_RETURN_IF(E.capture());
-  DevBuf ev, seen, left;
-  EDK_RETURN_IF(ev.alloc_async((size_t)nops * nev * sizeof(double), E.st));
-  EDK_RETURN_IF(seen.alloc_async((size_t)nops * sizeof(int), E.st));
-  EDK_RETURN_IF(left.alloc_async(sizeof(int), E.st));
+  DevBuf whole, ev, seen, left;
+  DevParts parts;
+  parts.add(ev, (size_t)nops * nev * sizeof(double));
+  parts.add(seen, (size_t)nops * sizeof(int));
+  parts.add(left, sizeof(int));
+  EDK_RETURN_IF(parts.alloc(whole, E.st));
   EDK_TRY_CUDA(cudaMemsetAsync(seen.p, 0, (size_t)nops * sizeof(int), E.st));
   const int every = check_every > 0 ? check_every : 10;
   bool pending = false;
