@@ -542,9 +542,6 @@ __global__ void __launch_bounds__(256) k_breduce2(const SplitOp* __restrict__ sp
   if (done[q]) return;
   const int j = *step, lane = threadIdx.x & 31;
   const SplitOp& o = sp[q];
-  // of the step before, for the last block (read here, behind the sums' loads)
-  const double aprev = j > 0 ? alpha[(int64_t)q * m + j - 1] : 0.0;
-  const double bprev = j > 0 ? beta[(int64_t)q * m + j - 1] : 0.0;
   double2* csq = cs + (int64_t)q * ncap;
   double2* ceq = ce + (int64_t)q * ncap;
   for (int c = blockIdx.x * 8 + (threadIdx.x >> 5); c <= j; c += gridDim.x * 8) {
@@ -587,6 +584,9 @@ __global__ void __launch_bounds__(256) k_breduce2(const SplitOp* __restrict__ sp
   __syncthreads();
   if (!s_last) return;
   __threadfence();
+  // of the step before (read here, beside the loads of the sums)
+  const double aprev = j > 0 ? alpha[(int64_t)q * m + j - 1] : 0.0;
+  const double bprev = j > 0 ? beta[(int64_t)q * m + j - 1] : 0.0;
   double ss = 0.0, hx = 0.0, hy = 0.0;  // |s|^2 and s^H r over the final columns
   for (int c = threadIdx.x; c < j; c += blockDim.x) {
     const double2 s = __ldcg(csq + c), r = __ldcg(ceq + c);
@@ -598,10 +598,9 @@ __global__ void __launch_bounds__(256) k_breduce2(const SplitOp* __restrict__ sp
   hx = bsum256(hx, sh);
   hy = bsum256(hy, sh);
   const double2 uu = __ldcg(csq + j), uw = __ldcg(ceq + j);
-  const double a2 = uu.x - ss;
+  const double a2 = uu.x - ss, root = sqrt(a2 < 0.0 ? 0.0 : a2);  // (NaN stays)
   if (j > 0) {  // (NaN runs on)
-    const double left = bprev * sqrt(a2 < 0.0 ? 0.0 : a2);
-    if (a2 <= kInSpan * uu.x || left <= kBreakdown * fmax(1.0, fabs(aprev))) {
+    if (a2 <= kInSpan * uu.x || bprev * root <= kBreakdown * fmax(1.0, fabs(aprev))) {
       if (threadIdx.x == 0) {
         beta[(int64_t)q * m + j - 1] = 0.0;
         done[q] = 2;  // (every block of the operator has read the flag: all have counted)
@@ -614,7 +613,7 @@ __global__ void __launch_bounds__(256) k_breduce2(const SplitOp* __restrict__ sp
     if (threadIdx.x == 0) cnt[q] = 0;
     return;
   }
-  const double inva = 1.0 / sqrt(a2), gx = (uw.x - hx) / a2, gy = (uw.y - hy) / a2;
+  const double inva = 1.0 / root, gx = (uw.x - hx) / a2, gy = (uw.y - hy) / a2;
   for (int c = threadIdx.x; c < j; c += blockDim.x) {
     const double2 s = __ldcg(csq + c), r = __ldcg(ceq + c);
     ceq[c] = make_double2(r.x - (gx * s.x - gy * s.y), r.y - (gx * s.y + gy * s.x));
@@ -1738,11 +1737,11 @@ edk_status KrylovBasis::extend(int from, int to, double* alpha, double* beta, in
   for (int j = from; j < to; ++j) EDK_RETURN_IF(E.run_step());
   EDK_TRY_CUDA(cudaMemcpyAsync(alpha, E.alpha.p, (size_t)to * sizeof(double), cudaMemcpyDeviceToHost, E.st));
   EDK_TRY_CUDA(cudaMemcpyAsync(beta, E.beta.p, (size_t)to * sizeof(double), cudaMemcpyDeviceToHost, E.st));
-  int done = 0;
   EDK_TRY_CUDA(cudaMemcpyAsync(m, E.nsteps.p, sizeof(int), cudaMemcpyDeviceToHost, E.st));
-  EDK_TRY_CUDA(cudaMemcpyAsync(&done, E.done.p, sizeof(int), cudaMemcpyDeviceToHost, E.st));
   EDK_TRY_CUDA(cudaStreamSynchronize(E.st));
-  if (E.may_close(alpha, beta, &done, m)) {  // the controller stops at beta = 0
+  const int running = 0;  // all `to` steps, and no breakdown in the last
+  if (*m == to && beta[to - 1] != 0.0 && E.may_close(alpha, beta, &running, m)) {
+    // (the controller stops at beta = 0)
     EDK_RETURN_IF(E.close());
     EDK_TRY_CUDA(cudaMemcpyAsync(beta + *m - 1, E.beta.as<double>() + *m - 1, sizeof(double),
                                  cudaMemcpyDeviceToHost, E.st));
