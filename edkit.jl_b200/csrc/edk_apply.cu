@@ -23,6 +23,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <set>
 #include <memory>
 #include <type_traits>
 
@@ -495,10 +496,10 @@ uint32_t site_mask(const HostTerm& h, int L, int c) {
 // the rows that have an element with it).  An entry of at least a hundredth of the
 // largest one beside it may carry that one's rounding.  (1.7, 0.3) as 1.0 +- 0.7
 // passes; 1e10 and 1e-10 in one matrix, or three couplings that cancel only up to
-// rounding, do not.
+// rounding, do not.  `empty`: the flip masks that have no entry for some pattern.
 using PauliSum = std::map<std::pair<uint32_t, uint32_t>, std::pair<double, double>>;
 bool strings_give_entries(const std::vector<HostTerm>& terms, const std::vector<char>& in_family,
-                          int L, const PauliSum& sum) {
+                          int L, const PauliSum& sum, std::set<uint32_t>& empty) {
   constexpr int kBits = 10;  // patterns are enumerated over at most 2^10
   constexpr double e64 = 2.220446049250313e-16, e32 = 1.1920928955078125e-07;
   struct Part { const HostTerm* t; int x; };
@@ -584,7 +585,9 @@ bool strings_give_entries(const std::vector<HostTerm>& terms, const std::vector<
     double re, im, big = 0.0;
     uint32_t pat = 0;  // the patterns of the sites, in ascending order
     do {
-      big = std::max(big, entries(pat, re, im));
+      const double s = entries(pat, re, im);
+      big = std::max(big, s);
+      if (s == 0.0) empty.insert(kv.first);
       pat = (pat - sites) & sites;
     } while (pat != 0);
     do {
@@ -609,20 +612,23 @@ bool strings_give_entries(const std::vector<HostTerm>& terms, const std::vector<
 }
 
 // True when the strings cost a row less than the terms.  Both kernels are bound by
-// instructions, so the rule counts them; units of 0.1 us for 2^20 rows, fitted to
-// measured products (FP64, 20 sites, 19.5 us of launch and host taken off):
+// instructions, so the rule counts them, in units of 0.1 us fitted to measured products.
+// Large spaces, for 2^20 rows (FP64, 20 sites, launch and host taken off):
 //   strings: 0.4 a plain flip, 0.55 a string, 0.6 a flip mask of several strings;
-//   terms: 2.4 a term and 0.9 an off-diagonal entry of its columns (their mean);
+//   terms: 2.8 a term and 0.9 an off-diagonal entry of its columns (their mean);
 //   bond families: 3.8 an off-diagonal entry; diagonals are popcounts in both.
-// Small spaces, whose rows eight lanes share, run the terms in about a third of that
-// (16 sites, 15 projected flips of two sites: 30 / 25 us; 16 fields: 21 / 26).
-// Measured at 20 sites, strings / terms in us a product: 20 x fields 30 / 87, 20
-// fields of x and z 41 / 89, 19 projected flips of two sites 58 / 65, 18 of three 68 /
-// 72, 17 of four 94 / 67; dense two-site terms 30 / 23 (one) and 128 / 114 (19),
-// three-site 53 / 26 and 196 / 86 (eight), four-site 131 / 34 and 219 / 48 (two).
+// Strings / terms in us a product there: 20 x fields 26 / 87, of x and z 37 / 89; 19
+// projected flips of two sites 52 / 65, eight 35 / 35, 18 of three 64 / 72, eight 40 / 41,
+// 17 of four 90 / 67; dense two-site terms 28 / 23 (one) and 124 / 114 (19), three-site 50
+// / 28 and 190 / 86 (eight), four-site 128 / 34 and 217 / 49 (two).
+// Small spaces, whose rows eight lanes share (16 sites): terms 3 once, 0.2 a term or
+// entry; strings 0.05 a plain flip, 0.16 a string, 0.4 a flip mask of several.  16
+// fields 21 / 26, complex 31 / 29; 15 projected flips of two sites 30 / 25, 14 of three
+// 28 / 26; dense two-site terms 23 / 24 (one) and 41 / 32 (15), four-site 42 / 29 (one).
 bool strings_win(const std::vector<HostTerm>& terms, const std::vector<char>& in_family,
                  const BasisDev& b, const PauliFlips& flips, size_t groups, size_t strings) {
-  double rows = 0.0;
+  const bool small = lanes_fit(b, b.D, many_lanes<BK_TENSOR>());
+  double rows = small ? 30.0 : 0.0;
   for (size_t t = 0; t < terms.size(); ++t) {
     const HostTerm& h = terms[t];
     int off = 0;
@@ -630,10 +636,11 @@ bool strings_win(const std::vector<HostTerm>& terms, const std::vector<char>& in
       for (int c = 0; c < h.dim; ++c)
         off += r != c && !(h.re[r * h.dim + c] == 0.0 && h.im[r * h.dim + c] == 0.0);
     const double entries = (double)off / h.dim;
-    rows += in_family[t] ? 38.0 * entries : 24.0 + 9.0 * entries;
+    if (small) rows += (in_family[t] ? 0.0 : 2.0) + 2.0 * entries;
+    else rows += in_family[t] ? 38.0 * entries : 28.0 + 9.0 * entries;
   }
-  if (lanes_fit(b, b.D, many_lanes<BK_TENSOR>())) rows *= 0.35;
-  return 4.0 * flips.n + 5.5 * strings + 6.0 * groups <= rows;
+  return (small ? 0.5 * flips.n + 1.6 * strings + 4.0 * groups
+                : 4.0 * flips.n + 5.5 * strings + 6.0 * groups) <= rows;
 }
 
 // Pauli strings of the terms' off-diagonal parts, grouped by flip mask, and of the
@@ -668,7 +675,8 @@ bool pauli_strings(const std::vector<HostTerm>& terms, const std::vector<char>& 
     }
     if (sum.size() > kPauliMax) return false;
   }
-  if (!strings_give_entries(terms, in_family, L, sum)) return false;
+  std::set<uint32_t> empty;
+  if (!strings_give_entries(terms, in_family, L, sum, empty)) return false;
   std::map<uint32_t, int> per_mask;
   for (auto it = sum.begin(); it != sum.end();)
     if (it->second.first == 0.0 && it->second.second == 0.0) it = sum.erase(it);
@@ -686,7 +694,7 @@ bool pauli_strings(const std::vector<HostTerm>& terms, const std::vector<char>& 
       flips.v[flips.n++] = p.v.x;
     } else {
       if (group.empty() || group.back().x != x)
-        group.push_back(PauliGroup{x, (int)str.size(), (int)str.size(), 0});
+        group.push_back(PauliGroup{x, (int)str.size(), (int)str.size(), (int)empty.count(x)});
       str.push_back(p);
       group.back().s1 = (int)str.size();
     }

@@ -356,7 +356,8 @@ constexpr uint32_t kPlanRowMask = (1u << 27) - 1u;
 
 // Pauli-string form of an operator on the full space (edk_pauli.cu).
 struct PauliStr { double2 v; uint32_t z, pad; };  // v (-1)^{|s & z|}
-struct PauliGroup { uint32_t x; int s0, s1, pad; };  // strings s0 .. s1-1 flip the bits x
+// strings s0 .. s1-1 flip the bits x; empty: some rows have no element with that flip
+struct PauliGroup { uint32_t x; int s0, s1, empty; };
 constexpr int kPauliFlips = 64;
 struct PauliFlips {  // strings without z part, one per flip mask, by ascending mask
   int n;

@@ -97,6 +97,7 @@ __global__ void __launch_bounds__(kPauliThreads, 4) k_apply_pauli(
   for (int g = 0; g < pd.ngroup; ++g) {
     const uint32_t xm = __ldg(&pd.group[g].x);
     const int s0 = __ldg(&pd.group[g].s0), s1 = __ldg(&pd.group[g].s1);
+    const bool empty = __ldg(&pd.group[g].empty) != 0;
     A cr[RPT], ci[RPT];
 #pragma unroll
     for (int r = 0; r < RPT; ++r) cr[r] = ci[r] = 0;
@@ -110,18 +111,23 @@ __global__ void __launch_bounds__(kPauliThreads, 4) k_apply_pauli(
         if constexpr (CX) ci[r] += neg ? -vi : vi;
       }
     }
-#pragma unroll
-    for (int r = 0; r < RPT; ++r) {
+    auto take = [&](int r) {
       const uint32_t l = t + r * kPauliThreads;
-      if (!FULL && l >= rows) continue;
-      // no element, no read: an infinity or NaN there is not this row's
-      if (cr[r] == 0 && (!CX || ci[r] == 0)) continue;
       const Cx<A> xv = xm < R ? ldout(sx + (l ^ xm)) : ldv(xk + ((base + l) ^ xm));
       acc[r].r = fma_(cr[r], xv.r, acc[r].r);
       if constexpr (CX) {
         acc[r].r = fma_(ci[r], xv.i, acc[r].r);
         acc[r].i = fma_(-ci[r], xv.r, fma_(cr[r], xv.i, acc[r].i));
       }
+    };
+    if (empty) {  // no element, no read: an infinity or NaN there is not this row's
+#pragma unroll
+      for (int r = 0; r < RPT; ++r)
+        if ((FULL || t + r * kPauliThreads < rows) && !(cr[r] == 0 && (!CX || ci[r] == 0))) take(r);
+    } else {  // (a test per row would keep its gathers from being in flight together)
+#pragma unroll
+      for (int r = 0; r < RPT; ++r)
+        if (FULL || t + r * kPauliThreads < rows) take(r);
     }
   }
 #pragma unroll

@@ -1,7 +1,6 @@
 """Where the strings stop: dense terms of three and four sites hold 36 to 256 strings
-against 8 or 16 entries a column, and run on the row kernel; real fields (one string
-each) keep the strings, complex ones (two, on one flip) only in spaces too large for
-eight lanes a row.  Both sides of the rule against the oracle."""
+against 8 or 16 entries a column, and run on the row kernel; fields keep the strings.
+Both sides of the rule against the oracle."""
 import numpy as np
 import pytest
 
@@ -38,7 +37,7 @@ def test_dense_terms_run_on_the_row_kernel(ek, O, make, k, n, strings, cx):
     mats, inds = make(k, n, cx)
     H = ek.operator(mats, inds, ek.TensorBasis(L=L))
     ref = O.operator(mats, inds, O.tensor(L))
-    if strings and not cx:
+    if strings:
         H.configure_("fast")
     else:
         with pytest.raises(ek.EDKError, match="fast kernel does not apply"):
