@@ -291,8 +291,13 @@ class Operator:
         it looks the dtype up once and hands plain integers to ctypes (a product
         of ten sites, 4.8 us on the GPU: 19.7 us a call through the numpy dtype
         names and pointer objects, 17.8 us here)."""
-        x, dt = self._tensor_in(x)
+        types = _torch_types().get(x.dtype)
         shape = x.shape
+        if types is None or (self.is_complex and types[0] != types[2]) or (
+                len(shape) == 1 and x.stride(0) != 1):
+            x, dt = self._tensor_in(x)
+        else:  # as it is (the usual case, without another call)
+            dt = types[0]
         D = self.B._D
         assert shape[0] == D
         if len(shape) == 1:
